@@ -439,6 +439,26 @@ def test_linear_float32(kernels, m, n, k):
     assert torch.equal(alone[0], out[m // 2])
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 2048, 6144), (1, 50, 24), (9, 640, 68), (17, 12288, 40), (33, 2048, 100), (65, 4096, 36), (130, 129, 20),
+                                   (257, 12288, 20), (1030, 8200, 12), (131, 2052, 33), (200, 4100, 7)])
+def test_linear_float32_every_tile(kernels, m, n, k):
+    """Sizes that the choice of tiles gives to every tile, with remainders in all three sizes and inner sizes that are no multiple of
+    four.  A sum of k products in float32 is off by at most k 2^-24 of the sum of their magnitudes; and a row's bits do not
+    depend on how many rows there are."""
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda")
+    w = torch.randn(n, k, generator=g, device="cuda")
+    out = torch.full((m, n), float("nan"), device="cuda")
+    kernels.linear(x, w, out)
+    want = x.double() @ w.double().T
+    bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-30
+    assert torch.all((out.double() - want).abs() <= bound)
+    for row in {0, m // 2, m - 1}:
+        alone = torch.empty((1, n), device="cuda")
+        kernels.linear(x[row:row + 1].contiguous(), w, alone)
+        assert torch.equal(alone[0], out[row])
+
+
 @pytest.mark.parametrize("out_dtype", DTYPES)
 @pytest.mark.parametrize("m,n,k", [(1, 331, 72), (37, 384, 96), (130, 264, 1032)])
 def test_linear_bfloat16(kernels, out_dtype, m, n, k):
