@@ -1,0 +1,843 @@
+// Recurrences with one decay per token and head, S_t = g_t S_(t-1) + w_t v_t k_t^T, y_t = S_t q_t, for portions of many tokens: what
+// ms_matrix_scan (memory, delta and constant-decay forms) and ms_selective_scan do token after token, as matrix products over chunks
+// of 64 tokens.  Walked, a portion is a chain of as many steps as it has tokens, whose every step waits for shared memory and for a
+// butterfly of shuffles; in chunks nearly all of it is products whose operands a thread uses several times.
+//
+// With D(t, s) = g_(s+1) .. g_t (products of the factors themselves, not differences of their logarithms: a difference of two large
+// sums would cost the digits that the products keep) and G_t = g_0 .. g_t within a chunk that starts from S_0,
+//
+//   y_t = G_t S_0 q_t + sum_(s <= t) D(t, s) w_s (q_t . k_s) v_s,      S_end = G_end S_0 + sum_s D(end, s) w_s v_s k_s^T.
+//
+//   memory, constant decay, selective:
+//     local_kernel   every chunk's sum D(end, s) w_s v_s k_s^T and its G_end
+//     join_kernel    S <- G_end S + sum over a portion's chunks: what each starts from, and the request's new state
+//     read_kernel    y
+//   delta (u_t = beta_t (v_t - S k_t) takes the place of w_t v_t, and depends on S):
+//     solve_kernel   within a chunk, u = U - W S_0 with (I + A) [U | W] = [beta v | beta G k], A(t, s) = beta_t D(t, s) k_t . k_s below
+//                    the diagonal: forward substitution, a thread per column
+//     carry_kernel   the chunks in order, sixteen columns of S a block: u, S_end; S_0 of every chunk
+//     read_kernel    y, with u for v
+//
+// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 124 us; selective,
+// 64 heads of 128 x 64, 2,048 tokens 496 -> 237 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 315 us.
+//
+// All arithmetic is float32 on float32 copies of the projections.  A token's result uses nothing of the tokens behind it (what is
+// masked is not multiplied: a zero would turn an infinity behind it into a NaN before it).
+#include "common.cuh"
+#include "mma_common.cuh"
+
+namespace ms {
+namespace chunk_scan {
+
+constexpr int kC = 64, kThreads = 256, kTile = 64;       // tokens of a chunk; value columns of a block
+constexpr int kLd = kTile + 4;
+enum Form : int { kMemory = 0, kDelta = 1, kDecay = 2, kSelective = 3 };
+
+struct Rows { const void* at; int ld, col; };            // a head's rows: column col + head * size
+
+struct Problem {
+  Rows q, k, v;
+  int heads, kv_heads, dim, vdim, columns;               // columns of a head's state: vdim, and one more in the memory form
+  int input_act, wide;                                   // SiLU on q, k, v; rows on 16-byte boundaries in whole 16-byte pieces
+  float q_scale;
+  const float* gates;                                    // memory [N, H, 3], delta [N, H, 2], decay [H]
+  const void* step;                                      // selective: step sizes' logits, type, rows, first column
+  int step_dtype, step_ld, step_col;
+  const float *step_bias, *a_log, *skip;
+  float* states;
+  long long state_stride;
+  int state_offset;
+  const int *state_slots, *query_start;
+  int most;                                              // chunks of the longest portion: blockIdx.z = request * most + chunk
+  float *chunk_states, *chunk_decays;                    // [places][heads][columns][dim], [places][heads]
+  float *y, *bottom;
+};
+
+struct Where { int request, first, len, left; size_t place; };      // a block's chunk: its first token, its tokens, those from it on
+__device__ __forceinline__ Where where_of(const Problem& p) {
+  Where w;
+  w.request = blockIdx.z / p.most;
+  const int c = blockIdx.z % p.most, first = p.query_start[w.request];
+  w.left = p.query_start[w.request + 1] - first - c * kC;
+  w.len = min(w.left, kC);
+  w.first = first + c * kC;
+  // (places of different requests do not meet: a portion of n tokens has at most one chunk more than it holds borders of 64
+  // tokens counted from the step's first token)
+  w.place = (size_t)(first / kC + w.request + c);
+  return w;
+}
+
+__device__ __forceinline__ float silu_of(float v) { return v * (1.f / (1.f + expf(-v))); }
+
+// (g_t, w_t) of a token (delta: w is beta).
+template <int FORM>
+__device__ __forceinline__ float2 gate_of(const Problem& p, int token, int head) {
+  const size_t at = (size_t)token * p.heads + head;
+  if (FORM == kMemory) return make_float2(p.gates[at * 3], p.gates[at * 3 + 1]);
+  if (FORM == kDelta) return make_float2(p.gates[at * 2], p.gates[at * 2 + 1]);
+  if (FORM == kDecay) return make_float2(p.gates[head], 1.f);
+  const float raw = load_as_float(p.step, p.step_dtype, (size_t)token * p.step_ld + p.step_col + head) + p.step_bias[head];
+  const float step = raw > 20.f ? raw : log1pf(expf(raw));           // softplus; above 20 the two agree in float32
+  return make_float2(expf(-expf(p.a_log[head]) * step), step);
+}
+
+// 64 rows of WIDTH numbers into shared memory as float32, zeros beyond `len` rows and `width` numbers.
+template <typename T, int WIDTH>
+__device__ __forceinline__ void load_rows(float* to, int to_ld, const T* from, size_t ld, int len, int width, int wide, int act) {
+  constexpr int E = 16 / sizeof(T), PER_ROW = WIDTH / E, TIMES = kC * PER_ROW / kThreads;
+  if (wide) {
+    uint4 raw[TIMES];
+#pragma unroll
+    for (int i = 0; i < TIMES; ++i) {
+      const int piece = threadIdx.x + i * kThreads, t = piece / PER_ROW, c = piece % PER_ROW * E;
+      raw[i] = t < len && c < width ? *reinterpret_cast<const uint4*>(from + (size_t)t * ld + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < TIMES; ++i) {
+      const int piece = threadIdx.x + i * kThreads, t = piece / PER_ROW, c = piece % PER_ROW * E;
+      const T* v = reinterpret_cast<const T*>(&raw[i]);
+#pragma unroll
+      for (int e = 0; e < E; e += 4) {
+        float4 four = make_float4(to_float(v[e]), to_float(v[e + 1]), to_float(v[e + 2]), to_float(v[e + 3]));
+        if (act) four = make_float4(silu_of(four.x), silu_of(four.y), silu_of(four.z), silu_of(four.w));
+        *reinterpret_cast<float4*>(to + t * to_ld + c + e) = four;
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < kC * WIDTH; i += kThreads) {
+      const int t = i / WIDTH, c = i % WIDTH;
+      float v = t < len && c < width ? to_float(from[(size_t)t * ld + c]) : 0.f;
+      if (act) v = silu_of(v);
+      to[t * to_ld + c] = v;
+    }
+  }
+}
+
+// Sixteen rows of a warp's scores at a time would leave half of them masked: a warp takes the eight rows of one band, and the
+// bands are dealt so that the two warps of a scheduler (w and w + 4) have nine of them together.
+__device__ __forceinline__ int band_of(int warp) { return warp < 4 ? warp : 11 - warp; }
+
+// a_t . b_s for rows t = 8 band + ty + 2 i and s = 16 j + tx up to the band's last row (tx 0..15, ty 0..1), pairs of entries apart.
+template <int NP>
+__device__ __forceinline__ void dot_band(const float* a, const float* b, int band, int tx, int ty, unsigned long long (&acc)[4][4]) {
+  const int last = band / 2;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll 4
+  for (int n = 0; n < NP; n += 4) {
+    ulonglong2 x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(a + (8 * band + ty + 2 * i) * (NP + 4) + n);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j > last) continue;
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(b + (16 * j + tx) * (NP + 4) + n);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i][j] = fma2(x[i].y, w.y, fma2(x[i].x, w.x, acc[i][j]));
+    }
+  }
+}
+__device__ __forceinline__ float both(unsigned long long two) {
+  float a, b;
+  unpack2(two, a, b);
+  return a + b;
+}
+
+// G_t, the product of a chunk's decays up to token t, into every g[t] (64 threads).  Products of decays are formed in double precision and
+// rounded once: their errors would be the same for a whole row of scores, where the walk's fall on each number of S alone (float32
+// products left the delta form's state 1.6 times as far from the definition as the walk's).
+__device__ __forceinline__ void prefix_products(const double* keep, float* g, int t) {
+  double p = 1.0;
+#pragma unroll 8
+  for (int r = 0; r < kC; ++r)
+    if (r <= t) p *= keep[r];
+  g[t] = (float)p;
+}
+
+// ------------------------------------------------------------------------------------------------- a chunk's own matrix
+// grid (value tiles, heads, chunks).  Bound by its multiply-adds, 64 x 64 x dim a block: a thread has four value columns and dim / 16
+// key entries, a token costs it one read of values and dim / 64 of keys for dim / 8 packed multiply-adds.
+template <typename T, int FORM, int NP>
+__global__ void __launch_bounds__(kThreads)
+local_kernel(const Problem p) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const Where w = where_of(p);
+  if (w.len <= 0) return;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float* ks = chunk_smem;                     // [64][NP + 4]
+  float* vs = ks + kC * (NP + 4);             // [64][kLd]
+  double* keep = reinterpret_cast<double*>(vs + kC * kLd);
+  float* weight = reinterpret_cast<float*>(keep + kC);
+  const int tid = threadIdx.x, head = blockIdx.y, kv_head = head / (p.heads / p.kv_heads), first_column = blockIdx.x * kTile;
+  const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
+  const T* v = reinterpret_cast<const T*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim + first_column;
+  float2 gate = make_float2(1.f, 0.f);
+  if (tid < w.len) gate = gate_of<FORM>(p, w.first + tid, head);
+  load_rows<T, NP>(ks, NP + 4, k, p.k.ld, w.len, p.dim, p.wide, p.input_act);
+  load_rows<T, kTile>(vs, kLd, v, p.v.ld, w.len, p.vdim - first_column, p.wide, p.input_act);
+  if (tid < kC) keep[tid] = gate.x;
+  __syncthreads();
+  if (tid < kC) {
+    double after = 1.0;                        // the decays behind the token
+#pragma unroll 8
+    for (int r = kC - 1; r > 0; --r)
+      if (r > tid) after *= keep[r];
+    weight[tid] = tid < w.len ? gate.y * (float)after : 0.f;
+    if (tid == 0 && blockIdx.x == 0) p.chunk_decays[w.place * p.heads + head] = (float)(after * keep[0]);
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  unsigned long long acc[4][NP / 32];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NP / 32; ++j) acc[i][j] = 0ull;
+#pragma unroll 4
+  for (int s = 0; s < w.len; ++s) {
+    const float4 four = *reinterpret_cast<const float4*>(vs + s * kLd + 4 * ty);
+    const float scale = weight[s];
+    unsigned long long value[4] = {pack2(scale * four.x, scale * four.x), pack2(scale * four.y, scale * four.y),
+                                   pack2(scale * four.z, scale * four.z), pack2(scale * four.w, scale * four.w)};
+#pragma unroll
+    for (int g = 0; g < NP / 64; ++g) {
+      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(ks + s * (NP + 4) + 64 * g + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i][2 * g] = fma2(value[i], key.x, acc[i][2 * g]);
+        acc[i][2 * g + 1] = fma2(value[i], key.y, acc[i][2 * g + 1]);
+      }
+    }
+  }
+  float* out = p.chunk_states + (w.place * p.heads + head) * (size_t)p.columns * p.dim;
+  const bool four_wide = p.dim % 4 == 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int column = first_column + 4 * ty + i;
+    if (column >= p.vdim) continue;
+#pragma unroll
+    for (int g = 0; g < NP / 64; ++g) {
+      const int n = 64 * g + 4 * tx;
+      float* at = out + (size_t)column * p.dim + n;
+      float e[4];
+      unpack2(acc[i][2 * g], e[0], e[1]);
+      unpack2(acc[i][2 * g + 1], e[2], e[3]);
+      if (four_wide) {
+        if (n < p.dim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (n + u < p.dim) at[u] = e[u];
+      }
+    }
+  }
+  if (FORM == kMemory && blockIdx.x == 0 && tid < p.dim) {       // the column n: its "value" is 1
+    float sum = 0.f;
+    for (int s = 0; s < w.len; ++s) sum += weight[s] * ks[s * (NP + 4) + tid];
+    out[(size_t)p.vdim * p.dim + tid] = sum;
+  }
+}
+
+// --------------------------------------------------------------------------------------------------- chunks joined
+// grid (pieces of the heads' states, requests), PER numbers a thread: bound by memory (each chunk's matrix read and written once), four
+// chunks' matrices requested at a time.
+template <int PER> struct alignas(4 * PER) Piece { float v[PER]; };
+
+template <int PER>
+__global__ void __launch_bounds__(256)
+join_kernel(const Problem p) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const int request = blockIdx.y, first = p.query_start[request];
+  const int count = (p.query_start[request + 1] - first + kC - 1) / kC;
+  const size_t all = (size_t)p.heads * p.columns * p.dim, at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * PER;
+  if (count <= 0 || at >= all) return;
+  const int head = (int)(at / ((size_t)p.columns * p.dim));
+  const size_t place = (size_t)(first / kC + request);
+  float* kept = p.states + (long long)p.state_slots[request] * p.state_stride + p.state_offset + at;
+  Piece<PER> s;
+#pragma unroll
+  for (int e = 0; e < PER; ++e) s.v[e] = kept[e];
+  for (int c0 = 0; c0 < count; c0 += 4) {
+    Piece<PER> wrote[4];
+    float decay[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (c0 + u >= count) continue;
+      wrote[u] = *reinterpret_cast<const Piece<PER>*>(p.chunk_states + (place + c0 + u) * all + at);
+      decay[u] = p.chunk_decays[(place + c0 + u) * p.heads + head];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (c0 + u >= count) break;
+      *reinterpret_cast<Piece<PER>*>(p.chunk_states + (place + c0 + u) * all + at) = s;
+#pragma unroll
+      for (int e = 0; e < PER; ++e) s.v[e] = decay[u] * s.v[e] + wrote[u].v[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < PER; ++e) kept[e] = s.v[e];
+}
+
+// ------------------------------------------------------------------------------------------------------- the rows of y
+// grid (value tiles, heads, chunks).  Bound by its multiply-adds: q k^T below the diagonal, scores times values, q S_0.  A warp owns
+// eight tokens from the scores to the results, so that between the two only the warp waits; S_0 arrives in the keys' place.
+template <typename T, typename V, int FORM, int NP>
+__global__ void __launch_bounds__(kThreads, 2)
+read_kernel(const Problem p) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const Where w = where_of(p);
+  if (w.len <= 0) return;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float* qs = chunk_smem;                     // [64][NP + 4]
+  float* ks = qs + kC * (NP + 4);             // [64][NP + 4], then S_0: value column c in row (c % 4) * 16 + c / 4
+  float* vs = ks + kC * (NP + 4);             // [64][kLd]
+  float* scores = vs + kC * kLd;              // [64][kLd]
+  double* keep = reinterpret_cast<double*>(scores + kC * kLd);
+  float* weight = reinterpret_cast<float*>(keep + kC);
+  float* decayed = weight + kC;               // G_t
+  float* n0 = decayed + kC;                   // [NP] (memory form)
+  const int tid = threadIdx.x, head = blockIdx.y, kv_head = head / (p.heads / p.kv_heads), first_column = blockIdx.x * kTile;
+  const T* q = reinterpret_cast<const T*>(p.q.at) + (size_t)w.first * p.q.ld + p.q.col + kv_head * p.dim;
+  const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
+  const V* v = reinterpret_cast<const V*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim + first_column;
+  const float* start = p.chunk_states + (w.place * p.heads + head) * (size_t)p.columns * p.dim;
+  const bool four_wide = p.dim % 4 == 0;
+  float2 gate = make_float2(1.f, 0.f);
+  if (tid < w.len) gate = gate_of<FORM>(p, w.first + tid, head);
+  load_rows<T, NP>(qs, NP + 4, q, p.q.ld, w.len, p.dim, p.wide, p.input_act);
+  load_rows<T, NP>(ks, NP + 4, k, p.k.ld, w.len, p.dim, p.wide, p.input_act);
+  load_rows<V, kTile>(vs, kLd, v, p.v.ld, w.len, p.vdim - first_column, p.wide, p.input_act);
+  if (tid < kC) {
+    keep[tid] = gate.x;
+    weight[tid] = FORM == kDelta ? 1.f : gate.y;
+  }
+  if (FORM == kMemory && tid < NP) n0[tid] = tid < p.dim ? start[(size_t)p.vdim * p.dim + tid] : 0.f;
+  __syncthreads();
+  {
+    // scores[t][s] = D(t, s) w_s: a thread has column s and sixteen rows
+    const int s = tid & (kC - 1), t0 = (tid >> 6) * 16;
+    double product = 1.0;
+#pragma unroll 8
+    for (int r = 0; r < t0; ++r)
+      if (r > s) product *= keep[r];
+    const float mine = weight[s];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (t0 + r > s) product *= keep[t0 + r];
+      scores[(t0 + r) * kLd + s] = (float)product * mine;
+    }
+    if (tid < kC) prefix_products(keep, decayed, tid);
+  }
+  __syncthreads();
+  const int warp = tid >> 5, lane = tid & 31, band = band_of(warp), tx = lane & 15, ty = lane >> 4;
+  const bool busy = 8 * band < w.len;
+  if (busy) {
+    unsigned long long acc[4][4];
+    dot_band<NP>(qs, ks, band, tx, ty, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j > band / 2) continue;
+        float* at = scores + (8 * band + ty + 2 * i) * kLd + 16 * j + tx;
+        *at *= p.q_scale * both(acc[i][j]);                            // (s > t is never read)
+      }
+  }
+  __syncthreads();                            // the keys have been read
+  if (four_wide) {
+    for (int i = tid; i < kTile * (NP / 4); i += kThreads) {
+      const int c = i / (NP / 4), n = i % (NP / 4) * 4;
+      const bool real = first_column + c < p.vdim && n < p.dim;
+      cp_async_16(ks + ((c & 3) * 16 + (c >> 2)) * (NP + 4) + n, start + (real ? (size_t)(first_column + c) * p.dim + n : 0), real);
+    }
+  } else {
+    for (int i = tid; i < kTile * NP; i += kThreads) {
+      const int c = i / NP, n = i % NP;
+      ks[((c & 3) * 16 + (c >> 2)) * (NP + 4) + n] = first_column + c < p.vdim && n < p.dim ? start[(size_t)(first_column + c) * p.dim + n] : 0.f;
+    }
+  }
+  cp_async_commit();
+  unsigned long long out[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) out[i][0] = out[i][1] = 0ull;
+  const float* my_scores = scores + (8 * band + ty) * kLd;
+  if (busy) {
+    for (int s = 0; s < 8 * band; s += 4) {
+      float4 row[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) row[i] = *reinterpret_cast<const float4*>(my_scores + 2 * i * kLd + s);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(vs + (s + u) * kLd + 4 * tx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float f = u == 0 ? row[i].x : u == 1 ? row[i].y : u == 2 ? row[i].z : row[i].w;
+          out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
+          out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {               // the band's own tokens: each row up to itself
+      const int s = 8 * band + u;
+      const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(vs + s * kLd + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (u <= ty + 2 * i) {
+          const float f = my_scores[2 * i * kLd + s];
+          out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
+          out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+        }
+    }
+    if (FORM == kMemory && blockIdx.x == 0) {
+      for (int r = 0; r < 8; ++r) {
+        const int t = 8 * band + r;
+        if (t >= w.len) break;
+        float sum = 0.f, read = 0.f;
+#pragma unroll
+        for (int s = lane; s < kC; s += 32)
+          if (s <= t) sum += scores[t * kLd + s];
+#pragma unroll
+        for (int n = lane; n < NP; n += 32) read += qs[t * (NP + 4) + n] * n0[n];
+        const float total = warp_sum(sum + decayed[t] * p.q_scale * read);
+        const size_t at = (size_t)(w.first + t) * p.heads + head;
+        if (lane == 0) p.bottom[at] = fmaxf(fabsf(total), p.gates[at * 3 + 2]) + 1e-6f;
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  if (!busy) return;
+  unsigned long long acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll 4
+  for (int n = 0; n < NP; n += 4) {
+    ulonglong2 x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(qs + (8 * band + ty + 2 * i) * (NP + 4) + n);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const ulonglong2 s0 = *reinterpret_cast<const ulonglong2*>(ks + (16 * j + tx) * (NP + 4) + n);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i][j] = fma2(x[i].y, s0.y, fma2(x[i].x, s0.x, acc[i][j]));
+    }
+  }
+  const float skip = FORM == kSelective ? p.skip[head] : 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = 8 * band + ty + 2 * i;
+    if (t >= w.len) continue;
+    const float factor = p.q_scale * decayed[t];
+    float e[4];
+    unpack2(out[i][0], e[0], e[1]);
+    unpack2(out[i][1], e[2], e[3]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      e[j] += factor * both(acc[i][j]);
+      if (FORM == kSelective) e[j] += skip * vs[t * kLd + 4 * tx + j];
+    }
+    float* at = p.y + ((size_t)(w.first + t) * p.heads + head) * p.vdim + first_column + 4 * tx;
+    if (p.vdim % 4 == 0) {
+      if (first_column + 4 * tx < p.vdim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (first_column + 4 * tx + j < p.vdim) at[j] = e[j];
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------- delta: within the chunks
+// grid (256 columns of [W | U], heads, chunks).  Forward substitution by sixteen rows: what the rows before them contribute, a read of
+// the column's own earlier result and four broadcast reads of A for sixteen multiply-adds, then the sixteen among themselves.
+struct Solved { float *w, *u, *ke; };         // [N][heads][dim], [N][heads][vdim], [N][heads][dim]: W, U, D(end, t) k_t
+
+template <typename T, int NP>
+__global__ void __launch_bounds__(kThreads, 2)
+solve_kernel(const Problem p, const Solved out) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const Where w = where_of(p);
+  if (w.len <= 0) return;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float* ks = chunk_smem;                     // [64][NP + 4]
+  float* a = ks + kC * (NP + 4);              // [s][t], rows of kLd
+  float* x = a + kC * kLd;                    // [48][256]
+  double* keep = reinterpret_cast<double*>(x + 48 * kThreads);
+  float* beta = reinterpret_cast<float*>(keep + kC);
+  float* decayed = beta + kC;
+  float* after = decayed + kC;                // D(end, t)
+  const int tid = threadIdx.x, head = blockIdx.y, kv_head = head / (p.heads / p.kv_heads);
+  const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
+  const T* v = reinterpret_cast<const T*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim;
+  float2 gate = make_float2(1.f, 0.f);
+  if (tid < w.len) gate = gate_of<kDelta>(p, w.first + tid, head);
+  load_rows<T, NP>(ks, NP + 4, k, p.k.ld, w.len, p.dim, p.wide, 0);
+  if (tid < kC) {
+    keep[tid] = gate.x;
+    beta[tid] = gate.y;
+  }
+  __syncthreads();
+  {
+    // a[s][t] = beta_t D(t, s): a thread has row t and sixteen s, the latest first
+    const int t = tid & (kC - 1), s0 = (tid >> 6) * 16;
+    double product = 1.0;
+#pragma unroll 8
+    for (int r = kC - 1; r > s0 + 15; --r)
+      if (r <= t) product *= keep[r];
+    const float mine = beta[t];
+#pragma unroll
+    for (int r = 15; r >= 0; --r) {
+      a[(s0 + r) * kLd + t] = mine * (float)product;
+      if (s0 + r <= t) product *= keep[s0 + r];
+    }
+    if (tid < kC) {
+      prefix_products(keep, decayed, tid);
+      double behind = 1.0;
+#pragma unroll 8
+      for (int r = kC - 1; r > 0; --r)
+        if (r > tid) behind *= keep[r];
+      after[tid] = (float)behind;
+      if (tid == 0 && blockIdx.x == 0) p.chunk_decays[w.place * p.heads + head] = (float)(behind * keep[0]);
+    }
+  }
+  __syncthreads();
+  {
+    const int lane = tid & 31, band = band_of(tid >> 5), tx = lane & 15, ty = lane >> 4;
+    if (8 * band < w.len) {
+      unsigned long long acc[4][4];
+      dot_band<NP>(ks, ks, band, tx, ty, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j <= band / 2) a[(16 * j + tx) * kLd + 8 * band + ty + 2 * i] *= both(acc[i][j]);
+    }
+  }
+  __syncthreads();
+  const int column = blockIdx.x * kThreads + tid;
+  const bool of_w = column < p.dim, real = column < p.dim + p.vdim;
+  if (!real) return;
+  for (int b = 0; b < 4; ++b) {
+    const int t0 = 16 * b;
+    if (t0 >= w.len) break;
+    unsigned long long sum[8];                // rows t0 + 2 r, t0 + 2 r + 1
+    {
+      float right[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int t = t0 + r;
+        if (of_w) {
+          const float key = ks[t * (NP + 4) + column];
+          right[r] = beta[t] * decayed[t] * key;
+          if (t < w.len) out.ke[((size_t)(w.first + t) * p.heads + head) * p.dim + column] = after[t] * key;
+        } else {
+          const float value = t < w.len ? to_float(v[(size_t)t * p.v.ld + column - p.dim]) : 0.f;
+          right[r] = beta[t] * value;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) sum[r] = pack2(right[2 * r], right[2 * r + 1]);
+    }
+#pragma unroll 4
+    for (int s = 0; s < t0; ++s) {
+      const float before = -x[s * kThreads + tid];
+      const unsigned long long two = pack2(before, before);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const ulonglong2 four = *reinterpret_cast<const ulonglong2*>(a + s * kLd + t0 + 4 * r);
+        sum[2 * r] = fma2(four.x, two, sum[2 * r]);
+        sum[2 * r + 1] = fma2(four.y, two, sum[2 * r + 1]);
+      }
+    }
+    float row[16];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) unpack2(sum[r], row[2 * r], row[2 * r + 1]);
+#pragma unroll
+    for (int s = 0; s < 15; ++s)
+#pragma unroll
+      for (int r = s + 1; r < 16; ++r) row[r] = fmaf(-a[(t0 + s) * kLd + t0 + r], row[s], row[r]);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      if (b < 3) x[(t0 + r) * kThreads + tid] = row[r];
+      if (t0 + r < w.len) {
+        const size_t token = (size_t)(w.first + t0 + r) * p.heads + head;
+        if (of_w) out.w[token * p.dim + column] = row[r];
+        else out.u[token * p.vdim + column - p.dim] = row[r];
+      }
+    }
+  }
+}
+
+// --------------------------------------------------------------------------------------- delta: from chunk to chunk
+// grid (16 value columns, heads, requests): the only part that is a chain, of chunks instead of tokens.  A thread has NP / 64 value
+// columns and four key entries of S in registers; shared memory holds two chunks of W, D(end, t) k_t and U (the next one on its way).
+constexpr int kCarry = 16;
+
+template <int NP>
+__global__ void __launch_bounds__(kThreads)
+carry_kernel(const Problem p, const Solved in) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  constexpr int LD = NP + 4, MINE = NP / 64, QUADS = NP / 4;
+  extern __shared__ __align__(16) float chunk_smem[];
+  float* ws = chunk_smem;                     // [2][64][LD]
+  float* es = ws + 2 * kC * LD;               // [2][64][LD]
+  float* us = es + 2 * kC * LD;               // [2][64][16]
+  float* s_at = us + 2 * kC * kCarry;         // [16][LD]
+  float* u_now = s_at + kCarry * LD;          // [64][16]
+  const int tid = threadIdx.x, head = blockIdx.y, request = blockIdx.z, first_column = blockIdx.x * kCarry;
+  const int first = p.query_start[request], q_len = p.query_start[request + 1] - first, count = (q_len + kC - 1) / kC;
+  if (count <= 0) return;
+  const size_t place = (size_t)(first / kC + request);
+  const int columns_here = min(kCarry, p.vdim - first_column);
+  const bool four_wide = p.dim % 4 == 0, four_values = p.vdim % 4 == 0;
+  auto fetch = [&](int c, int stage) {
+    const int len = min(kC, q_len - c * kC);
+    const size_t token = (size_t)(first + c * kC) * p.heads + head;
+    float* to_w = ws + stage * kC * LD;
+    float* to_e = es + stage * kC * LD;
+    float* to_u = us + stage * kC * kCarry;
+    if (four_wide) {
+      for (int i = tid; i < kC * (NP / 4); i += kThreads) {
+        const int t = i / (NP / 4), n = i % (NP / 4) * 4;
+        const bool real = t < len && n < p.dim;
+        const size_t at = real ? (token + (size_t)t * p.heads) * p.dim + n : 0;
+        cp_async_16(to_w + t * LD + n, in.w + at, real);
+        cp_async_16(to_e + t * LD + n, in.ke + at, real);
+      }
+    } else {
+      for (int i = tid; i < kC * NP; i += kThreads) {
+        const int t = i / NP, n = i % NP;
+        const bool real = t < len && n < p.dim;
+        const size_t at = (token + (size_t)t * p.heads) * p.dim + n;
+        to_w[t * LD + n] = real ? in.w[at] : 0.f;
+        to_e[t * LD + n] = real ? in.ke[at] : 0.f;
+      }
+    }
+    if (four_values) {
+      const int t = tid >> 2, c4 = (tid & 3) * 4;
+      const bool real = t < len && c4 < columns_here;
+      cp_async_16(to_u + t * kCarry + c4, in.u + (real ? (token + (size_t)t * p.heads) * p.vdim + first_column + c4 : 0), real);
+    } else {
+      for (int i = tid; i < kC * kCarry; i += kThreads) {
+        const int t = i / kCarry, c16 = i % kCarry;
+        to_u[i] = t < len && c16 < columns_here ? in.u[(token + (size_t)t * p.heads) * p.vdim + first_column + c16] : 0.f;
+      }
+    }
+    cp_async_commit();
+  };
+  const int n = (tid % QUADS) * 4, column = (tid / QUADS) * MINE;      // this thread's part of S
+  float* kept = p.states + (long long)p.state_slots[request] * p.state_stride + p.state_offset + ((size_t)head * p.vdim + first_column) * p.dim;
+  float s[MINE][4];
+#pragma unroll
+  for (int m = 0; m < MINE; ++m)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[m][e] = column + m < columns_here && n + e < p.dim ? kept[(size_t)(column + m) * p.dim + n + e] : 0.f;
+  auto store = [&](float* to) {
+#pragma unroll
+    for (int m = 0; m < MINE; ++m) {
+      if (column + m >= columns_here) continue;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n + e < p.dim) to[(size_t)(column + m) * p.dim + n + e] = s[m][e];
+    }
+  };
+  fetch(0, 0);
+  for (int c = 0; c < count; ++c) {
+    const int stage = c & 1, len = min(kC, q_len - c * kC);
+    const float decay = p.chunk_decays[(place + c) * p.heads + head];
+#pragma unroll
+    for (int m = 0; m < MINE; ++m) *reinterpret_cast<float4*>(s_at + (column + m) * LD + n) = make_float4(s[m][0], s[m][1], s[m][2], s[m][3]);
+    cp_async_wait<0>();
+    __syncthreads();                          // this chunk is there, S is there, the chunk before has been read
+    if (c + 1 < count) fetch(c + 1, stage ^ 1);
+    store(p.chunk_states + ((place + c) * p.heads + head) * (size_t)p.vdim * p.dim + (size_t)first_column * p.dim);
+    {
+      // u = U - W S_0: tokens tt, tt + 32 and columns tp, tp + 8
+      const int tp = tid & 7, tt = tid >> 3;
+      const float* w0 = ws + stage * kC * LD + tt * LD;
+      unsigned long long acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll 8
+      for (int i = 0; i < NP; i += 4) {
+        const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(w0 + i), wb = *reinterpret_cast<const ulonglong2*>(w0 + 32 * LD + i);
+        const ulonglong2 sa = *reinterpret_cast<const ulonglong2*>(s_at + tp * LD + i);
+        const ulonglong2 sb = *reinterpret_cast<const ulonglong2*>(s_at + (tp + 8) * LD + i);
+        acc[0][0] = fma2(wa.y, sa.y, fma2(wa.x, sa.x, acc[0][0]));
+        acc[0][1] = fma2(wa.y, sb.y, fma2(wa.x, sb.x, acc[0][1]));
+        acc[1][0] = fma2(wb.y, sa.y, fma2(wb.x, sa.x, acc[1][0]));
+        acc[1][1] = fma2(wb.y, sb.y, fma2(wb.x, sb.x, acc[1][1]));
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int t = tt + 32 * i, c16 = tp + 8 * j;
+          const float u = us[stage * kC * kCarry + t * kCarry + c16] - both(acc[i][j]);
+          u_now[t * kCarry + c16] = u;
+          if (t < len && c16 < columns_here) in.u[((size_t)(first + c * kC + t) * p.heads + head) * p.vdim + first_column + c16] = u;
+        }
+    }
+    __syncthreads();
+    unsigned long long sum[MINE][2];
+#pragma unroll
+    for (int m = 0; m < MINE; ++m) sum[m][0] = pack2(decay * s[m][0], decay * s[m][1]), sum[m][1] = pack2(decay * s[m][2], decay * s[m][3]);
+    const float* e_row = es + stage * kC * LD + n;
+#pragma unroll 8
+    for (int t = 0; t < len; ++t) {
+      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(e_row + t * LD);
+#pragma unroll
+      for (int m = 0; m < MINE; ++m) {
+        const float u = u_now[t * kCarry + column + m];
+        sum[m][0] = fma2(pack2(u, u), key.x, sum[m][0]);
+        sum[m][1] = fma2(pack2(u, u), key.y, sum[m][1]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < MINE; ++m) {
+      unpack2(sum[m][0], s[m][0], s[m][1]);
+      unpack2(sum[m][1], s[m][2], s[m][3]);
+    }
+  }
+  store(kept);
+}
+
+// ------------------------------------------------------------------------------------------------------------ launches
+constexpr size_t local_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 3 * kC); }
+constexpr size_t read_bytes(int np) { return sizeof(float) * (size_t)(2 * kC * (np + 4) + 2 * kC * kLd + 4 * kC + np); }
+constexpr size_t solve_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 48 * kThreads + 5 * kC); }
+constexpr size_t carry_bytes(int np) { return sizeof(float) * (size_t)(4 * kC * (np + 4) + 3 * kC * kCarry + kCarry * (np + 4)); }
+
+template <typename Kernel>
+static bool allow(Kernel kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
+template <typename T, int FORM, int NP>
+static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
+  const int tiles = (p.vdim + kTile - 1) / kTile;
+  const dim3 grid(tiles, p.heads, n_requests * p.most);
+  if constexpr (FORM == kDelta) {
+    auto solve = solve_kernel<T, NP>;
+    auto carry = carry_kernel<NP>;
+    auto read = read_kernel<T, float, kDelta, NP>;
+    if (!allow(solve, solve_bytes(NP)) || !allow(carry, carry_bytes(NP)) || !allow(read, read_bytes(NP)))
+      MS_FAIL("chunk_scan: shared memory refused");
+    ms::launch(solve, dim3((p.dim + p.vdim + kThreads - 1) / kThreads, p.heads, n_requests * p.most), kThreads, solve_bytes(NP), stream, p,
+               solved);
+    MS_CHECK_LAUNCH("chunk_scan: within the chunks");
+    ms::launch(carry, dim3((p.vdim + kCarry - 1) / kCarry, p.heads, n_requests), kThreads, carry_bytes(NP), stream, p, solved);
+    MS_CHECK_LAUNCH("chunk_scan: from chunk to chunk");
+    Problem reading = p;
+    reading.v = Rows{solved.u, p.heads * p.vdim, 0};
+    if (p.vdim % 4) reading.wide = 0;
+    ms::launch(read, grid, kThreads, read_bytes(NP), stream, reading);
+  } else {
+    auto local = local_kernel<T, FORM, NP>;
+    auto read = read_kernel<T, T, FORM, NP>;
+    if (!allow(local, local_bytes(NP)) || !allow(read, read_bytes(NP))) MS_FAIL("chunk_scan: shared memory refused");
+    ms::launch(local, grid, kThreads, local_bytes(NP), stream, p);
+    MS_CHECK_LAUNCH("chunk_scan: chunks alone");
+    const bool four = p.dim % 4 == 0;
+    const size_t threads = (size_t)p.heads * p.columns * p.dim / (four ? 4 : 1);
+    ms::launch(four ? join_kernel<4> : join_kernel<1>, dim3((unsigned)((threads + 255) / 256), n_requests), 256, 0, stream, p);
+    MS_CHECK_LAUNCH("chunk_scan: chunks joined");
+    ms::launch(read, grid, kThreads, read_bytes(NP), stream, p);
+  }
+  MS_CHECK_LAUNCH("chunk_scan: rows");
+  return 0;
+}
+
+template <typename T, int FORM>
+static int scan_keys(const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
+  return p.dim <= 64 ? scan<T, FORM, 64>(p, n_requests, solved, stream) : scan<T, FORM, 128>(p, n_requests, solved, stream);
+}
+
+template <typename T>
+static int scan_form(int form, const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
+  if (form == kMemory) return scan_keys<T, kMemory>(p, n_requests, solved, stream);
+  if (form == kDelta) return scan_keys<T, kDelta>(p, n_requests, solved, stream);
+  return scan_keys<T, kDecay>(p, n_requests, solved, stream);
+}
+
+}  // namespace chunk_scan
+}  // namespace ms
+
+using namespace ms;
+using namespace ms::chunk_scan;
+
+// The tokens of a chunk (64) if the step's portions should be scanned in chunks, 0 if the walk, token after token, is the better
+// one or the only one: few tokens (a walk takes about 0.3 us a token, the launches of a scan 20 to 40 us before they have much to
+// do), keys of more than 128 entries, or more chunks than a launch's grid holds.
+MS_EXPORT int ms_chunk_scan_chunk(int n_requests, int max_query_len, int heads, int dim) {
+  if (n_requests <= 0 || heads <= 0 || heads > 65535 || dim <= 0 || dim > 128 || max_query_len < 96) return 0;
+  if ((long long)n_requests * ((max_query_len + kC - 1) / kC) > 65535) return 0;
+  return kC;
+}
+
+// Arguments as ms_matrix_scan's forms 0 (memory), 1 (delta) and 2 (constant decay).  chunk_states float32 [places, heads, columns, dim] and
+// chunk_decays float32 [places, heads], places = n_tokens / 64 + n_requests; delta: w, ke float32 [n_tokens, heads, dim], u float32
+// [n_tokens, heads, vdim].  chunk_states and u on 16-byte boundaries.
+MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const void* k, int k_ld, int k_col, const void* v, int v_ld,
+                            int v_col, int dtype, float q_scale, const float* gates, float* states, long long state_stride,
+                            int state_offset, const int* state_slots, const int* query_start, int n_requests, int max_query_len,
+                            int heads, int kv_heads, int dim, int vdim, float* y, float* bottom, int input_act, float* chunk_states,
+                            float* chunk_decays, float* w, float* u, float* ke, cudaStream_t stream) {
+  if (n_requests == 0 || max_query_len <= 0 || heads == 0) return 0;
+  MS_REQUIRE(form >= kMemory && form <= kDecay, "chunk_scan: form %d", form);
+  MS_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && dim >= 1 && dim <= 128 && vdim >= 1, "chunk_scan: %d/%d heads of %d/%d", heads,
+             kv_heads, dim, vdim);
+  MS_REQUIRE(form != kDelta || !input_act, "chunk_scan: the delta form takes its inputs as they are");
+  MS_REQUIRE(form != kMemory || bottom != nullptr, "chunk_scan: the memory form writes the tokens' divisors");
+  MS_REQUIRE(chunk_states && chunk_decays && (form != kDelta || (w && u && ke)), "chunk_scan: scratch is missing");
+  const int most = (max_query_len + kC - 1) / kC;
+  MS_REQUIRE(heads <= 65535 && (long long)n_requests * most <= 65535, "chunk_scan: %d heads, %d requests of %d chunks exceed the launch limits",
+             heads, n_requests, most);
+  const int per = dtype == MS_F32 ? 4 : 8;
+  auto aligned = [](const void* at) { return reinterpret_cast<size_t>(at) % 16 == 0; };
+  const int wide = aligned(q) && aligned(k) && aligned(v) && q_ld % per == 0 && k_ld % per == 0 && v_ld % per == 0 && q_col % per == 0 &&
+                   k_col % per == 0 && v_col % per == 0 && dim % per == 0 && vdim % per == 0;
+  Problem p = {};
+  p.q = Rows{q, q_ld, q_col}, p.k = Rows{k, k_ld, k_col}, p.v = Rows{v, v_ld, v_col};
+  p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim, p.columns = form == kMemory ? vdim + 1 : vdim;
+  p.input_act = input_act, p.wide = wide, p.q_scale = q_scale, p.gates = gates;
+  p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
+  p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
+  const Solved solved{w, u, ke};
+  if (dtype == MS_F32) return scan_form<float>(form, p, n_requests, solved, stream);
+  if (dtype == MS_BF16) return scan_form<__nv_bfloat16>(form, p, n_requests, solved, stream);
+  MS_FAIL("unknown element type code %d", dtype);
+}
+
+// Arguments as ms_selective_scan; scratch as above with columns = p (a head's channels) and dim = n_state.
+MS_EXPORT int ms_selective_chunk_scan(const float* conv, int conv_ld, const void* proj, int dtype, int ld, int dt_col, const float* dt_bias,
+                                      const float* a_log, const float* d, float* states, long long state_stride, int state_offset,
+                                      const int* state_slots, const int* query_start, int n_requests, int max_query_len, int heads,
+                                      int channels, int n_state, int groups, float* y, float* chunk_states, float* chunk_decays,
+                                      cudaStream_t stream) {
+  if (n_requests == 0 || max_query_len <= 0) return 0;
+  MS_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "selective_chunk_scan: %d heads in %d groups", heads, groups);
+  MS_REQUIRE(n_state >= 1 && n_state <= 128 && channels >= 1, "selective_chunk_scan: a state of %d numbers for %d channels", n_state, channels);
+  MS_REQUIRE(dtype == MS_F32 || dtype == MS_BF16, "unknown element type code %d", dtype);
+  MS_REQUIRE(chunk_states && chunk_decays, "selective_chunk_scan: scratch is missing");
+  const int most = (max_query_len + kC - 1) / kC;
+  MS_REQUIRE(heads <= 65535 && (long long)n_requests * most <= 65535,
+             "selective_chunk_scan: %d heads, %d requests of %d chunks exceed the launch limits", heads, n_requests, most);
+  const int inner = heads * channels;
+  Problem p = {};
+  p.v = Rows{conv, conv_ld, 0}, p.k = Rows{conv, conv_ld, inner}, p.q = Rows{conv, conv_ld, inner + groups * n_state};
+  p.heads = heads, p.kv_heads = groups, p.dim = n_state, p.vdim = channels, p.columns = channels;
+  p.wide = conv_ld % 4 == 0 && inner % 4 == 0 && n_state % 4 == 0 && channels % 4 == 0 && reinterpret_cast<size_t>(conv) % 16 == 0;
+  p.q_scale = 1.f;
+  p.step = proj, p.step_dtype = dtype, p.step_ld = ld, p.step_col = dt_col, p.step_bias = dt_bias, p.a_log = a_log, p.skip = d;
+  p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
+  p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
+  return scan_keys<float, kSelective>(p, n_requests, Solved{}, stream);
+}

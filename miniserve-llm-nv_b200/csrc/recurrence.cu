@@ -19,7 +19,8 @@
 // Everything here is float32 arithmetic on float32 state; only the projections that the kernels read and the last kernels'
 // outputs are in the model's compute type.  A request's tokens are walked in order and every sum has a fixed order, so a
 // position's result depends on the tokens before it alone, not on how they were cut into steps, on what else is in the
-// batch or on which state slot the request holds.
+// batch or on which state slot the request holds.  (Steps with portions of 96 tokens and more are scanned in chunks, chunk_scan.cu and
+// channel_scan.cu: there the cutting changes the order of sums, and with it a result's last bits.)
 #include "common.cuh"
 
 namespace ms {

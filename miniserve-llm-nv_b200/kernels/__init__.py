@@ -911,6 +911,19 @@ def _state_rows(states: torch.Tensor, offset: int, length: int) -> int:
 
 
 CONV_ACTIVATIONS = {"none": 0, "silu": 1}
+MAX_CHUNK_SCRATCH = 1 << 30   # bytes of chunk states beyond which a scan walks its tokens
+
+
+def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device) -> Optional[tuple]:
+    """(chunk states, chunk decays) for the scans in chunks, or None where the step's tokens are walked one after the other."""
+    chunk = library().ms_chunk_scan_chunk(_i(n_requests), _i(longest), _i(heads), _i(dim))
+    if not chunk:
+        return None
+    places = n // chunk + n_requests
+    if 4 * places * heads * columns * dim > MAX_CHUNK_SCRATCH:
+        return None
+    return (torch.empty((places, heads, columns, dim), dtype=torch.float32, device=device),
+            torch.empty((places, heads), dtype=torch.float32, device=device))
 
 
 def causal_conv_silu(proj: torch.Tensor, col: int, weight: torch.Tensor, bias: torch.Tensor, states: torch.Tensor,
@@ -955,13 +968,14 @@ def causal_conv(proj: torch.Tensor, col: int, weight: torch.Tensor, bias: Option
 def selective_scan(conv: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, a_log: torch.Tensor,
                    d: torch.Tensor, states: torch.Tensor, state_offset: int, state_slots: torch.Tensor,
                    query_start: torch.Tensor, heads: int, head_dim: int, state: int, groups: int, y: torch.Tensor,
-                   max_query_len: Optional[int] = None) -> None:
+                   max_query_len: Optional[int] = None, chunked: bool = True) -> None:
     """The selective recurrence over each request's tokens, from and into the request's state.  ``conv`` float32
     ``[N, heads * head_dim + 2 * groups * state]`` = ``[x | B | C]``; the step size of head h is ``softplus(proj[t,
     dt_col + h] + dt_bias[h])``; per head (group ``h // (heads / groups)``) ``S = exp(-exp(a_log) dt) S + dt B x^T`` and
     ``y = S^T C + d x``.  ``states[slot, state_offset:]`` holds float32 ``[heads, head_dim, state]``.  ``y`` float32
     ``[N, heads * head_dim]``.  ``max_query_len``: an upper bound of the tokens a request brings (None: the batch's size); the
-    kernel sizes its chunks by it, so a step of single tokens should say 1."""
+    kernel sizes its chunks by it, so a step of single tokens should say 1.  Portions of many tokens are scanned as matrix products over
+    chunks (``csrc/chunk_scan.cu``); ``chunked=False`` walks them token after token."""
     n, ld = proj.shape
     inner = heads * head_dim
     _want(proj, "proj")
@@ -975,9 +989,17 @@ def selective_scan(conv: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias:
     if dt_col < 0 or dt_col + heads > ld or heads % groups or state > MAX_SCAN_STATE:
         raise KernelError(f"selective_scan: {heads} heads in {groups} groups, state {state}, dt from column {dt_col} of rows of {ld}")
     stride = _state_rows(states, state_offset, inner * state)
+    longest = n if max_query_len is None else max_query_len
+    scratch = _chunk_scratch(n, n_requests, longest, heads, state, head_dim, y.device) if chunked else None
+    if scratch is not None:
+        _check(library().ms_selective_chunk_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
+                                                 _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
+                                                 _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(longest), _i(heads),
+                                                 _i(head_dim), _i(state), _i(groups), _ptr(y), _ptr(scratch[0]), _ptr(scratch[1]), _stream()))
+        return
     _check(library().ms_selective_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
                                        _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
-                                       _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n if max_query_len is None else max_query_len),
+                                       _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(longest),
                                        _i(heads), _i(head_dim), _i(state), _i(groups), _ptr(y), _stream()))
 
 
@@ -1079,7 +1101,8 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
 
     ``"channel_decay"`` of few long portions runs in chunks that need not wait for one another (a walk from zero per chunk, a join
     of the chunks' matrices, a walk from the joined ones): ``chunk`` None lets the library choose, 0 forbids it, a number is
-    the chunk's tokens."""
+    the chunk's tokens.  ``"memory"``, ``"delta"`` and ``"decay"`` of portions of many tokens run as matrix products over chunks of 64
+    tokens (``csrc/chunk_scan.cu``) unless ``chunk`` is 0."""
     code = MATRIX_SCAN_MODES[mode]
     n = y.shape[0]
     for name, tensor in (("q", q), ("k", k), ("v", v)):
@@ -1123,6 +1146,20 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
                                          _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(max_query_len),
                                          _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _i(chunk), _ptr(chunk_states),
                                          _ptr(chunk_decays), _stream()))
+        return
+    scratch = None
+    if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
+        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device)
+    if scratch is not None:
+        solved = [None] * 3
+        if code == 1:
+            solved = [torch.empty((n, heads, size), dtype=torch.float32, device=y.device) for size in (dim, vdim, dim)]
+        _check(library().ms_chunk_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
+                                       _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
+                                       _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(max_query_len),
+                                       _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _ptr(bottom),
+                                       _i(CONV_ACTIVATIONS[input_activation]), _ptr(scratch[0]), _ptr(scratch[1]), _ptr(solved[0]),
+                                       _ptr(solved[1]), _ptr(solved[2]), _stream()))
         return
     _check(library().ms_matrix_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                     _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
