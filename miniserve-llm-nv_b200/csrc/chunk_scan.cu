@@ -18,8 +18,8 @@
 //     carry_kernel   the chunks in order, sixteen columns of S a block: u, S_end; S_0 of every chunk
 //     read_kernel    y, with u for v
 //
-// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 124 us; selective,
-// 64 heads of 128 x 64, 2,048 tokens 496 -> 237 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 315 us.
+// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 120 us; selective,
+// 64 heads of 128 x 64, 2,048 tokens 496 -> 231 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 243 us.
 //
 // All arithmetic is float32 on float32 copies of the projections.  A token's result uses nothing of the tokens behind it (what is
 // masked is not multiplied: a zero would turn an infinity behind it into a NaN before it).
@@ -113,31 +113,43 @@ __device__ __forceinline__ void load_rows(float* to, int to_ld, const T* from, s
   }
 }
 
-// Sixteen rows of a warp's scores at a time would leave half of them masked: a warp takes the eight rows of one band, and the
-// bands are dealt so that the two warps of a scheduler (w and w + 4) have nine of them together.
-__device__ __forceinline__ int band_of(int warp) { return warp < 4 ? warp : 11 - warp; }
-
-// a_t . b_s for rows t = 8 band + ty + 2 i and s = 16 j + tx up to the band's last row (tx 0..15, ty 0..1), pairs of entries apart.
+// a_t . b_s for a warp's tile of 16 rows and 32 columns: rows row0 + ty + 4 i, columns column0 + tx + 8 j for the first `blocks` of four
+// (ty 0..3, tx 0..7; pairs of entries apart).  Eight reads of shared memory, each of at most eight different rows (one pass of its
+// banks), for 32 packed multiply-adds: tiles of 8 x 64 take half as many passes again and were bound by them (72 % busy).
 template <int NP>
-__device__ __forceinline__ void dot_band(const float* a, const float* b, int band, int tx, int ty, unsigned long long (&acc)[4][4]) {
-  const int last = band / 2;
+__device__ __forceinline__ void dot_tile(const float* a, const float* b, int row0, int column0, int blocks, int tx, int ty,
+                                         unsigned long long (&acc)[4][4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  const float* a_at = a + (row0 + ty) * (NP + 4);
+  const float* b_at = b + (column0 + tx) * (NP + 4);
 #pragma unroll 4
   for (int n = 0; n < NP; n += 4) {
     ulonglong2 x[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(a + (8 * band + ty + 2 * i) * (NP + 4) + n);
+    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(a_at + 4 * i * (NP + 4) + n);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (j > last) continue;
-      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(b + (16 * j + tx) * (NP + 4) + n);
+      if (j >= blocks) continue;
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(b_at + 8 * j * (NP + 4) + n);
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[i][j] = fma2(x[i].y, w.y, fma2(x[i].x, w.x, acc[i][j]));
     }
   }
+}
+
+// The warps' tiles of a chunk's scores: (16 rows, 32 columns) where any column is at or below the diagonal, six of eight, dealt so
+// that the two warps of a scheduler (w and w + 4) have few blocks of eight columns together.  blocks: those that a tile needs.
+struct Tile { int row0, column0, blocks; };
+__device__ __forceinline__ Tile score_tile(int warp) {
+  if (warp < 2) return Tile{48, 32 * warp, 4};
+  if (warp == 2) return Tile{32, 0, 4};
+  if (warp == 3) return Tile{16, 0, 4};
+  if (warp == 4) return Tile{32, 32, 2};
+  if (warp == 5) return Tile{0, 0, 2};
+  return Tile{kC, 0, 0};
 }
 __device__ __forceinline__ float both(unsigned long long two) {
   float a, b;
@@ -157,8 +169,8 @@ __device__ __forceinline__ void prefix_products(const double* keep, float* g, in
 }
 
 // ------------------------------------------------------------------------------------------------- a chunk's own matrix
-// grid (value tiles, heads, chunks).  Bound by its multiply-adds, 64 x 64 x dim a block: a thread has four value columns and dim / 16
-// key entries, a token costs it one read of values and dim / 64 of keys for dim / 8 packed multiply-adds.
+// grid (value tiles, heads, chunks).  Bound by its multiply-adds, 64 x 64 x dim a block: a thread has four or eight value columns and
+// four key entries, a token costs it a read of keys and one or two of values for eight or sixteen packed multiply-adds.
 template <typename T, int FORM, int NP>
 __global__ void __launch_bounds__(kThreads)
 local_kernel(const Problem p) {
@@ -189,41 +201,48 @@ local_kernel(const Problem p) {
     if (tid == 0 && blockIdx.x == 0) p.chunk_decays[w.place * p.heads + head] = (float)(after * keep[0]);
   }
   __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  unsigned long long acc[4][NP / 32];
+  for (int i = tid; i < kC * (kTile / 4); i += kThreads) {       // the values times their weights
+    const int t = i / (kTile / 4);
+    float4* at = reinterpret_cast<float4*>(vs + t * kLd + i % (kTile / 4) * 4);
+    const float f = weight[t];
+    *at = make_float4(f * at->x, f * at->y, f * at->z, f * at->w);
+  }
+  __syncthreads();
+  constexpr int GROUPS = NP / 64;               // of four value columns a thread has
+  const int warp = tid >> 5, lane = tid & 31, tx = lane & 7, ty = lane >> 3;
+  const int value0 = NP == 128 ? 32 * (warp & 1) + 4 * ty : 16 * (warp >> 1) + 4 * ty;
+  const int n = 32 * (NP == 128 ? warp >> 1 : warp & 1) + 4 * tx;
+  unsigned long long acc[GROUPS][4][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int g = 0; g < GROUPS; ++g)
 #pragma unroll
-    for (int j = 0; j < NP / 32; ++j) acc[i][j] = 0ull;
+    for (int i = 0; i < 4; ++i) acc[g][i][0] = acc[g][i][1] = 0ull;
 #pragma unroll 4
   for (int s = 0; s < w.len; ++s) {
-    const float4 four = *reinterpret_cast<const float4*>(vs + s * kLd + 4 * ty);
-    const float scale = weight[s];
-    unsigned long long value[4] = {pack2(scale * four.x, scale * four.x), pack2(scale * four.y, scale * four.y),
-                                   pack2(scale * four.z, scale * four.z), pack2(scale * four.w, scale * four.w)};
+    const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(ks + s * (NP + 4) + n);
 #pragma unroll
-    for (int g = 0; g < NP / 64; ++g) {
-      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(ks + s * (NP + 4) + 64 * g + 4 * tx);
+    for (int g = 0; g < GROUPS; ++g) {
+      const float4 four = *reinterpret_cast<const float4*>(vs + s * kLd + value0 + 16 * g);
+      const unsigned long long value[4] = {pack2(four.x, four.x), pack2(four.y, four.y), pack2(four.z, four.z), pack2(four.w, four.w)};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        acc[i][2 * g] = fma2(value[i], key.x, acc[i][2 * g]);
-        acc[i][2 * g + 1] = fma2(value[i], key.y, acc[i][2 * g + 1]);
+        acc[g][i][0] = fma2(value[i], key.x, acc[g][i][0]);
+        acc[g][i][1] = fma2(value[i], key.y, acc[g][i][1]);
       }
     }
   }
   float* out = p.chunk_states + (w.place * p.heads + head) * (size_t)p.columns * p.dim;
   const bool four_wide = p.dim % 4 == 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int column = first_column + 4 * ty + i;
-    if (column >= p.vdim) continue;
+  for (int g = 0; g < GROUPS; ++g)
 #pragma unroll
-    for (int g = 0; g < NP / 64; ++g) {
-      const int n = 64 * g + 4 * tx;
+    for (int i = 0; i < 4; ++i) {
+      const int column = first_column + value0 + 16 * g + i;
+      if (column >= p.vdim) continue;
       float* at = out + (size_t)column * p.dim + n;
       float e[4];
-      unpack2(acc[i][2 * g], e[0], e[1]);
-      unpack2(acc[i][2 * g + 1], e[2], e[3]);
+      unpack2(acc[g][i][0], e[0], e[1]);
+      unpack2(acc[g][i][1], e[2], e[3]);
       if (four_wide) {
         if (n < p.dim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
       } else {
@@ -232,7 +251,6 @@ local_kernel(const Problem p) {
           if (n + u < p.dim) at[u] = e[u];
       }
     }
-  }
   if (FORM == kMemory && blockIdx.x == 0 && tid < p.dim) {       // the column n: its "value" is 1
     float sum = 0.f;
     for (int s = 0; s < w.len; ++s) sum += weight[s] * ks[s * (NP + 4) + tid];
@@ -282,8 +300,11 @@ join_kernel(const Problem p) {
 }
 
 // ------------------------------------------------------------------------------------------------------- the rows of y
-// grid (value tiles, heads, chunks).  Bound by its multiply-adds: q k^T below the diagonal, scores times values, q S_0.  A warp owns
-// eight tokens from the scores to the results, so that between the two only the warp waits; S_0 arrives in the keys' place.
+// grid (value tiles, heads, chunks).  Bound by its multiply-adds: q k^T below the diagonal, scores times values, q S_0, which arrives
+// in the keys' place while the values are summed.
+// (neighbouring threads have every fourth column of S_0: those lie in neighbouring rows)
+__device__ __forceinline__ int place_of_column(int c) { return (c & 32) + (c & 3) * 8 + ((c >> 2) & 7); }
+
 template <typename T, typename V, int FORM, int NP>
 __global__ void __launch_bounds__(kThreads, 2)
 read_kernel(const Problem p) {
@@ -293,7 +314,7 @@ read_kernel(const Problem p) {
   if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* qs = chunk_smem;                     // [64][NP + 4]
-  float* ks = qs + kC * (NP + 4);             // [64][NP + 4], then S_0: value column c in row (c % 4) * 16 + c / 4
+  float* ks = qs + kC * (NP + 4);             // [64][NP + 4], then S_0, value column c in row place_of_column(c)
   float* vs = ks + kC * (NP + 4);             // [64][kLd]
   float* scores = vs + kC * kLd;              // [64][kLd]
   double* keep = reinterpret_cast<double*>(scores + kC * kLd);
@@ -333,46 +354,50 @@ read_kernel(const Problem p) {
     if (tid < kC) prefix_products(keep, decayed, tid);
   }
   __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31, band = band_of(warp), tx = lane & 15, ty = lane >> 4;
-  const bool busy = 8 * band < w.len;
-  if (busy) {
+  const int warp = tid >> 5, lane = tid & 31, tx = lane & 7, ty = lane >> 3;
+  const Tile tile = score_tile(warp);
+  if (tile.row0 < w.len) {
     unsigned long long acc[4][4];
-    dot_band<NP>(qs, ks, band, tx, ty, acc);
+    dot_tile<NP>(qs, ks, tile.row0, tile.column0, tile.blocks, tx, ty, acc);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (j > band / 2) continue;
-        float* at = scores + (8 * band + ty + 2 * i) * kLd + 16 * j + tx;
+        if (j >= tile.blocks) continue;
+        float* at = scores + (tile.row0 + ty + 4 * i) * kLd + tile.column0 + tx + 8 * j;
         *at *= p.q_scale * both(acc[i][j]);                            // (s > t is never read)
       }
   }
-  __syncthreads();                            // the keys have been read
+  __syncthreads();                            // the scores are there, the keys have been read
   if (four_wide) {
     for (int i = tid; i < kTile * (NP / 4); i += kThreads) {
       const int c = i / (NP / 4), n = i % (NP / 4) * 4;
       const bool real = first_column + c < p.vdim && n < p.dim;
-      cp_async_16(ks + ((c & 3) * 16 + (c >> 2)) * (NP + 4) + n, start + (real ? (size_t)(first_column + c) * p.dim + n : 0), real);
+      cp_async_16(ks + place_of_column(c) * (NP + 4) + n, start + (real ? (size_t)(first_column + c) * p.dim + n : 0), real);
     }
   } else {
     for (int i = tid; i < kTile * NP; i += kThreads) {
       const int c = i / NP, n = i % NP;
-      ks[((c & 3) * 16 + (c >> 2)) * (NP + 4) + n] = first_column + c < p.vdim && n < p.dim ? start[(size_t)(first_column + c) * p.dim + n] : 0.f;
+      ks[place_of_column(c) * (NP + 4) + n] = first_column + c < p.vdim && n < p.dim ? start[(size_t)(first_column + c) * p.dim + n] : 0.f;
     }
   }
   cp_async_commit();
+  // results: 16 tokens and 32 value columns a warp, four neighbouring columns a thread; the two warps of a scheduler have 80 tokens' scores
+  const int half = warp >> 2, row0 = 16 * (half ? 3 - (warp & 3) : warp & 3);
+  const bool busy = row0 < w.len;
   unsigned long long out[4][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i) out[i][0] = out[i][1] = 0ull;
-  const float* my_scores = scores + (8 * band + ty) * kLd;
+  const float* my_scores = scores + (row0 + ty) * kLd;
+  const float* my_values = vs + 32 * half + 4 * tx;
   if (busy) {
-    for (int s = 0; s < 8 * band; s += 4) {
+    for (int s = 0; s < row0; s += 4) {
       float4 row[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) row[i] = *reinterpret_cast<const float4*>(my_scores + 2 * i * kLd + s);
+      for (int i = 0; i < 4; ++i) row[i] = *reinterpret_cast<const float4*>(my_scores + 4 * i * kLd + s);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(vs + (s + u) * kLd + 4 * tx);
+        const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (s + u) * kLd);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float f = u == 0 ? row[i].x : u == 1 ? row[i].y : u == 2 ? row[i].z : row[i].w;
@@ -382,57 +407,39 @@ read_kernel(const Problem p) {
       }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {               // the band's own tokens: each row up to itself
-      const int s = 8 * band + u;
-      const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(vs + s * kLd + 4 * tx);
+    for (int u = 0; u < 16; ++u) {              // the tile's own tokens: each row up to itself
+      const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (row0 + u) * kLd);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (u <= ty + 2 * i) {
-          const float f = my_scores[2 * i * kLd + s];
+        if (u <= ty + 4 * i) {
+          const float f = my_scores[4 * i * kLd + row0 + u];
           out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
           out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
         }
     }
-    if (FORM == kMemory && blockIdx.x == 0) {
-      for (int r = 0; r < 8; ++r) {
-        const int t = 8 * band + r;
-        if (t >= w.len) break;
-        float sum = 0.f, read = 0.f;
+  }
+  if (FORM == kMemory && blockIdx.x == 0) {
+    for (int t = 8 * warp; t < min(8 * warp + 8, w.len); ++t) {
+      float sum = 0.f, read = 0.f;
 #pragma unroll
-        for (int s = lane; s < kC; s += 32)
-          if (s <= t) sum += scores[t * kLd + s];
+      for (int s = lane; s < kC; s += 32)
+        if (s <= t) sum += scores[t * kLd + s];
 #pragma unroll
-        for (int n = lane; n < NP; n += 32) read += qs[t * (NP + 4) + n] * n0[n];
-        const float total = warp_sum(sum + decayed[t] * p.q_scale * read);
-        const size_t at = (size_t)(w.first + t) * p.heads + head;
-        if (lane == 0) p.bottom[at] = fmaxf(fabsf(total), p.gates[at * 3 + 2]) + 1e-6f;
-      }
+      for (int n = lane; n < NP; n += 32) read += qs[t * (NP + 4) + n] * n0[n];
+      const float total = warp_sum(sum + decayed[t] * p.q_scale * read);
+      const size_t at = (size_t)(w.first + t) * p.heads + head;
+      if (lane == 0) p.bottom[at] = fmaxf(fabsf(total), p.gates[at * 3 + 2]) + 1e-6f;
     }
   }
   cp_async_wait<0>();
   __syncthreads();
   if (!busy) return;
   unsigned long long acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-#pragma unroll 4
-  for (int n = 0; n < NP; n += 4) {
-    ulonglong2 x[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(qs + (8 * band + ty + 2 * i) * (NP + 4) + n);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const ulonglong2 s0 = *reinterpret_cast<const ulonglong2*>(ks + (16 * j + tx) * (NP + 4) + n);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i][j] = fma2(x[i].y, s0.y, fma2(x[i].x, s0.x, acc[i][j]));
-    }
-  }
+  dot_tile<NP>(qs, ks, row0, 32 * half, 4, tx, ty, acc);
   const float skip = FORM == kSelective ? p.skip[head] : 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int t = 8 * band + ty + 2 * i;
+    const int t = row0 + ty + 4 * i;
     if (t >= w.len) continue;
     const float factor = p.q_scale * decayed[t];
     float e[4];
@@ -441,15 +448,16 @@ read_kernel(const Problem p) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       e[j] += factor * both(acc[i][j]);
-      if (FORM == kSelective) e[j] += skip * vs[t * kLd + 4 * tx + j];
+      if (FORM == kSelective) e[j] += skip * my_values[t * kLd + j];
     }
-    float* at = p.y + ((size_t)(w.first + t) * p.heads + head) * p.vdim + first_column + 4 * tx;
+    const int column = first_column + 32 * half + 4 * tx;
+    float* at = p.y + ((size_t)(w.first + t) * p.heads + head) * p.vdim + column;
     if (p.vdim % 4 == 0) {
-      if (first_column + 4 * tx < p.vdim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
+      if (column < p.vdim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (first_column + 4 * tx + j < p.vdim) at[j] = e[j];
+        if (column + j < p.vdim) at[j] = e[j];
     }
   }
 }
@@ -472,8 +480,8 @@ solve_kernel(const Problem p, const Solved out) {
   float* x = a + kC * kLd;                    // [48][256]
   double* keep = reinterpret_cast<double*>(x + 48 * kThreads);
   float* beta = reinterpret_cast<float*>(keep + kC);
-  float* decayed = beta + kC;
-  float* after = decayed + kC;                // D(end, t)
+  float* factor = beta + kC;                  // beta_t G_t
+  float* after = factor + kC;                 // D(end, t)
   const int tid = threadIdx.x, head = blockIdx.y, kv_head = head / (p.heads / p.kv_heads);
   const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
   const T* v = reinterpret_cast<const T*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim;
@@ -499,8 +507,11 @@ solve_kernel(const Problem p, const Solved out) {
       if (s0 + r <= t) product *= keep[s0 + r];
     }
     if (tid < kC) {
-      prefix_products(keep, decayed, tid);
-      double behind = 1.0;
+      double upto = 1.0, behind = 1.0;
+#pragma unroll 8
+      for (int r = 0; r < kC; ++r)
+        if (r <= tid) upto *= keep[r];
+      factor[tid] = beta[tid] * (float)upto;
 #pragma unroll 8
       for (int r = kC - 1; r > 0; --r)
         if (r > tid) behind *= keep[r];
@@ -510,38 +521,60 @@ solve_kernel(const Problem p, const Solved out) {
   }
   __syncthreads();
   {
-    const int lane = tid & 31, band = band_of(tid >> 5), tx = lane & 15, ty = lane >> 4;
-    if (8 * band < w.len) {
+    const int lane = tid & 31, tx = lane & 7, ty = lane >> 3;
+    const Tile tile = score_tile(tid >> 5);
+    if (tile.row0 < w.len) {
       unsigned long long acc[4][4];
-      dot_band<NP>(ks, ks, band, tx, ty, acc);
+      dot_tile<NP>(ks, ks, tile.row0, tile.column0, tile.blocks, tx, ty, acc);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (j <= band / 2) a[(16 * j + tx) * kLd + 8 * band + ty + 2 * i] *= both(acc[i][j]);
+          if (j < tile.blocks) a[(tile.column0 + tx + 8 * j) * kLd + tile.row0 + ty + 4 * i] *= both(acc[i][j]);
+    }
+    if (blockIdx.x == 0) {                    // the keys as the chunk's end sees them
+      float* ke = out.ke + ((size_t)w.first * p.heads + head) * p.dim;
+      if (p.dim % 4 == 0) {
+        for (int i = tid; i < w.len * (NP / 4); i += kThreads) {
+          const int t = i / (NP / 4), n = i % (NP / 4) * 4;
+          if (n >= p.dim) continue;
+          const float4 key = *reinterpret_cast<const float4*>(ks + t * (NP + 4) + n);
+          const float f = after[t];
+          *reinterpret_cast<float4*>(ke + (size_t)t * p.heads * p.dim + n) = make_float4(f * key.x, f * key.y, f * key.z, f * key.w);
+        }
+      } else {
+        for (int i = tid; i < w.len * NP; i += kThreads) {
+          const int t = i / NP, n = i % NP;
+          if (n < p.dim) ke[(size_t)t * p.heads * p.dim + n] = after[t] * ks[t * (NP + 4) + n];
+        }
+      }
     }
   }
   __syncthreads();
   const int column = blockIdx.x * kThreads + tid;
   const bool of_w = column < p.dim, real = column < p.dim + p.vdim;
   if (!real) return;
-  for (int b = 0; b < 4; ++b) {
-    const int t0 = 16 * b;
-    if (t0 >= w.len) break;
+  float* result = of_w ? out.w + ((size_t)w.first * p.heads + head) * p.dim + column
+                       : out.u + ((size_t)w.first * p.heads + head) * p.vdim + column - p.dim;
+  const int result_ld = p.heads * (of_w ? p.dim : p.vdim);
+  const T* value = v + (of_w ? 0 : column - p.dim);
+  for (int t0 = 0; t0 < w.len; t0 += 16) {
+    const int here = min(16, w.len - t0);
     unsigned long long sum[8];                // rows t0 + 2 r, t0 + 2 r + 1
     {
       float right[16];
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
-        const int t = t0 + r;
         if (of_w) {
-          const float key = ks[t * (NP + 4) + column];
-          right[r] = beta[t] * decayed[t] * key;
-          if (t < w.len) out.ke[((size_t)(w.first + t) * p.heads + head) * p.dim + column] = after[t] * key;
+          right[r] = factor[t0 + r] * ks[(t0 + r) * (NP + 4) + column];
         } else {
-          const float value = t < w.len ? to_float(v[(size_t)t * p.v.ld + column - p.dim]) : 0.f;
-          right[r] = beta[t] * value;
+          right[r] = r < here ? to_float(*value) : 0.f;
+          if (r < here) value += p.v.ld;
         }
+      }
+      if (!of_w) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) right[r] *= beta[t0 + r];
       }
 #pragma unroll
       for (int r = 0; r < 8; ++r) sum[r] = pack2(right[2 * r], right[2 * r + 1]);
@@ -563,36 +596,44 @@ solve_kernel(const Problem p, const Solved out) {
 #pragma unroll
     for (int s = 0; s < 15; ++s)
 #pragma unroll
-      for (int r = s + 1; r < 16; ++r) row[r] = fmaf(-a[(t0 + s) * kLd + t0 + r], row[s], row[r]);
+      for (int q = (s + 1) / 4; q < 4; ++q) {
+        const float4 four = *reinterpret_cast<const float4*>(a + (t0 + s) * kLd + t0 + 4 * q);
+        if (4 * q > s) row[4 * q] = fmaf(-four.x, row[s], row[4 * q]);
+        if (4 * q + 1 > s) row[4 * q + 1] = fmaf(-four.y, row[s], row[4 * q + 1]);
+        if (4 * q + 2 > s) row[4 * q + 2] = fmaf(-four.z, row[s], row[4 * q + 2]);
+        if (4 * q + 3 > s) row[4 * q + 3] = fmaf(-four.w, row[s], row[4 * q + 3]);
+      }
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      if (b < 3) x[(t0 + r) * kThreads + tid] = row[r];
-      if (t0 + r < w.len) {
-        const size_t token = (size_t)(w.first + t0 + r) * p.heads + head;
-        if (of_w) out.w[token * p.dim + column] = row[r];
-        else out.u[token * p.vdim + column - p.dim] = row[r];
+      if (t0 < 48) x[(t0 + r) * kThreads + tid] = row[r];
+      if (r < here) {
+        *result = row[r];
+        result += result_ld;
       }
     }
   }
 }
 
 // --------------------------------------------------------------------------------------- delta: from chunk to chunk
-// grid (16 value columns, heads, requests): the only part that is a chain, of chunks instead of tokens.  A thread has NP / 64 value
-// columns and four key entries of S in registers; shared memory holds two chunks of W, D(end, t) k_t and U (the next one on its way).
-constexpr int kCarry = 16;
+// grid (16 value columns, heads, requests): the only part that is a chain, of chunks instead of tokens.  S is in registers, and in shared
+// memory for W S_0; beside it lie two chunks of W, D(end, t) k_t and U (the next one on its way).  Both products are cut along the
+// sum (key entries by four, tokens by two or four) so that a thread has sixteen results of either, not two or four: the reads of
+// shared memory bound them otherwise (a chunk took 4.5 us).
+constexpr int kCarry = 16, kPartLd = 20;
 
 template <int NP>
 __global__ void __launch_bounds__(kThreads)
 carry_kernel(const Problem p, const Solved in) {
   grid_dependency_wait();
   grid_dependency_launch();
-  constexpr int LD = NP + 4, MINE = NP / 64, QUADS = NP / 4;
+  constexpr int LD = NP + 4, NWARPS = NP / 32, TOKENS = 8 / NWARPS;
   extern __shared__ __align__(16) float chunk_smem[];
   float* ws = chunk_smem;                     // [2][64][LD]
   float* es = ws + 2 * kC * LD;               // [2][64][LD]
   float* us = es + 2 * kC * LD;               // [2][64][16]
   float* s_at = us + 2 * kC * kCarry;         // [16][LD]
   float* u_now = s_at + kCarry * LD;          // [64][16]
+  float* parts = u_now + kC * kCarry;         // [4][64][kPartLd]: quarters of W S_0; [1 or 3][16][LD]: sums over other threads' tokens
   const int tid = threadIdx.x, head = blockIdx.y, request = blockIdx.z, first_column = blockIdx.x * kCarry;
   const int first = p.query_start[request], q_len = p.query_start[request + 1] - first, count = (q_len + kC - 1) / kC;
   if (count <= 0) return;
@@ -634,86 +675,138 @@ carry_kernel(const Problem p, const Solved in) {
     }
     cp_async_commit();
   };
-  const int n = (tid % QUADS) * 4, column = (tid / QUADS) * MINE;      // this thread's part of S
+  // this thread's part of S: four value columns and four key entries, summed over every TOKENS-th token of a chunk; the threads of the
+  // first tokens keep S
+  const int warp = tid >> 5, lane = tid & 31, turn = warp / NWARPS;
+  const int n = 32 * (warp % NWARPS) + 4 * (lane & 7), column = 4 * (lane >> 3);
+  const bool keeps = turn == 0;
   float* kept = p.states + (long long)p.state_slots[request] * p.state_stride + p.state_offset + ((size_t)head * p.vdim + first_column) * p.dim;
-  float s[MINE][4];
+  float s[4][4];
 #pragma unroll
-  for (int m = 0; m < MINE; ++m)
+  for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[m][e] = column + m < columns_here && n + e < p.dim ? kept[(size_t)(column + m) * p.dim + n + e] : 0.f;
-  auto store = [&](float* to) {
+    for (int e = 0; e < 4; ++e)
+      s[m][e] = keeps && column + m < columns_here && n + e < p.dim ? kept[(size_t)(column + m) * p.dim + n + e] : 0.f;
+  auto store = [&](float* to, bool wide) {
 #pragma unroll
-    for (int m = 0; m < MINE; ++m) {
+    for (int m = 0; m < 4; ++m) {
       if (column + m >= columns_here) continue;
+      float* at = to + (size_t)(column + m) * p.dim + n;
+      if (wide) {
+        if (n < p.dim) *reinterpret_cast<float4*>(at) = make_float4(s[m][0], s[m][1], s[m][2], s[m][3]);
+      } else {
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (n + e < p.dim) to[(size_t)(column + m) * p.dim + n + e] = s[m][e];
+        for (int e = 0; e < 4; ++e)
+          if (n + e < p.dim) at[e] = s[m][e];
+      }
     }
   };
   fetch(0, 0);
   for (int c = 0; c < count; ++c) {
     const int stage = c & 1, len = min(kC, q_len - c * kC);
     const float decay = p.chunk_decays[(place + c) * p.heads + head];
+    if (keeps) {
 #pragma unroll
-    for (int m = 0; m < MINE; ++m) *reinterpret_cast<float4*>(s_at + (column + m) * LD + n) = make_float4(s[m][0], s[m][1], s[m][2], s[m][3]);
+      for (int m = 0; m < 4; ++m) *reinterpret_cast<float4*>(s_at + (column + m) * LD + n) = make_float4(s[m][0], s[m][1], s[m][2], s[m][3]);
+    }
     cp_async_wait<0>();
     __syncthreads();                          // this chunk is there, S is there, the chunk before has been read
     if (c + 1 < count) fetch(c + 1, stage ^ 1);
-    store(p.chunk_states + ((place + c) * p.heads + head) * (size_t)p.vdim * p.dim + (size_t)first_column * p.dim);
+    if (keeps) store(p.chunk_states + ((place + c) * p.heads + head) * (size_t)p.vdim * p.dim + (size_t)first_column * p.dim, four_wide);
     {
-      // u = U - W S_0: tokens tt, tt + 32 and columns tp, tp + 8
-      const int tp = tid & 7, tt = tid >> 3;
-      const float* w0 = ws + stage * kC * LD + tt * LD;
-      unsigned long long acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
-#pragma unroll 8
-      for (int i = 0; i < NP; i += 4) {
-        const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(w0 + i), wb = *reinterpret_cast<const ulonglong2*>(w0 + 32 * LD + i);
-        const ulonglong2 sa = *reinterpret_cast<const ulonglong2*>(s_at + tp * LD + i);
-        const ulonglong2 sb = *reinterpret_cast<const ulonglong2*>(s_at + (tp + 8) * LD + i);
-        acc[0][0] = fma2(wa.y, sa.y, fma2(wa.x, sa.x, acc[0][0]));
-        acc[0][1] = fma2(wa.y, sb.y, fma2(wa.x, sb.x, acc[0][1]));
-        acc[1][0] = fma2(wb.y, sa.y, fma2(wb.x, sa.x, acc[1][0]));
-        acc[1][1] = fma2(wb.y, sb.y, fma2(wb.x, sb.x, acc[1][1]));
+      // W S_0 over a quarter of the key entries: tokens t0 + 8 i, columns c0 + 4 j
+      const int quarter = warp >> 1, t0 = 32 * (warp & 1) + (lane >> 2), c0 = lane & 3;
+      const float* w_at = ws + stage * kC * LD + t0 * LD + quarter * (NP / 4);
+      const float* s_row = s_at + c0 * LD + quarter * (NP / 4);
+      unsigned long long acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll
+      for (int k = 0; k < NP / 4; k += 4) {
+        ulonglong2 four[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) four[i] = *reinterpret_cast<const ulonglong2*>(w_at + 8 * i * LD + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const ulonglong2 state = *reinterpret_cast<const ulonglong2*>(s_row + 4 * j * LD + k);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[i][j] = fma2(four[i].y, state.y, fma2(four[i].x, state.x, acc[i][j]));
+        }
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int t = tt + 32 * i, c16 = tp + 8 * j;
-          const float u = us[stage * kC * kCarry + t * kCarry + c16] - both(acc[i][j]);
-          u_now[t * kCarry + c16] = u;
-          if (t < len && c16 < columns_here) in.u[((size_t)(first + c * kC + t) * p.heads + head) * p.vdim + first_column + c16] = u;
-        }
+        for (int j = 0; j < 4; ++j) parts[(quarter * kC + t0 + 8 * i) * kPartLd + c0 + 4 * j] = both(acc[i][j]);
     }
     __syncthreads();
-    unsigned long long sum[MINE][2];
+    {
+      const int t = tid >> 2, c4 = 4 * (tid & 3);
+      float4 u = *reinterpret_cast<const float4*>(us + stage * kC * kCarry + t * kCarry + c4);
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int m = 0; m < MINE; ++m) sum[m][0] = pack2(decay * s[m][0], decay * s[m][1]), sum[m][1] = pack2(decay * s[m][2], decay * s[m][3]);
-    const float* e_row = es + stage * kC * LD + n;
-#pragma unroll 8
-    for (int t = 0; t < len; ++t) {
-      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(e_row + t * LD);
-#pragma unroll
-      for (int m = 0; m < MINE; ++m) {
-        const float u = u_now[t * kCarry + column + m];
-        sum[m][0] = fma2(pack2(u, u), key.x, sum[m][0]);
-        sum[m][1] = fma2(pack2(u, u), key.y, sum[m][1]);
+      for (int q = 0; q < 4; ++q) {
+        const float4 part = *reinterpret_cast<const float4*>(parts + (q * kC + t) * kPartLd + c4);
+        sum = make_float4(sum.x + part.x, sum.y + part.y, sum.z + part.z, sum.w + part.w);
+      }
+      u = make_float4(u.x - sum.x, u.y - sum.y, u.z - sum.z, u.w - sum.w);
+      *reinterpret_cast<float4*>(u_now + t * kCarry + c4) = u;
+      if (t < len) {
+        float* at = in.u + ((size_t)(first + c * kC + t) * p.heads + head) * p.vdim + first_column + c4;
+        if (four_values) {
+          if (c4 < columns_here) *reinterpret_cast<float4*>(at) = u;
+        } else {
+          if (c4 < columns_here) at[0] = u.x;
+          if (c4 + 1 < columns_here) at[1] = u.y;
+          if (c4 + 2 < columns_here) at[2] = u.z;
+          if (c4 + 3 < columns_here) at[3] = u.w;
+        }
       }
     }
+    __syncthreads();
+    unsigned long long sum[4][2];
 #pragma unroll
-    for (int m = 0; m < MINE; ++m) {
-      unpack2(sum[m][0], s[m][0], s[m][1]);
-      unpack2(sum[m][1], s[m][2], s[m][3]);
+    for (int m = 0; m < 4; ++m) sum[m][0] = pack2(decay * s[m][0], decay * s[m][1]), sum[m][1] = pack2(decay * s[m][2], decay * s[m][3]);
+    const float* e_at = es + stage * kC * LD + n;
+#pragma unroll 8
+    for (int t = turn; t < len; t += TOKENS) {
+      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(e_at + t * LD);
+      const float4 u = *reinterpret_cast<const float4*>(u_now + t * kCarry + column);
+      const unsigned long long value[4] = {pack2(u.x, u.x), pack2(u.y, u.y), pack2(u.z, u.z), pack2(u.w, u.w)};
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        sum[m][0] = fma2(value[m], key.x, sum[m][0]);
+        sum[m][1] = fma2(value[m], key.y, sum[m][1]);
+      }
+    }
+    if (!keeps) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        *reinterpret_cast<ulonglong2*>(parts + ((turn - 1) * kCarry + column + m) * LD + n) = make_ulonglong2(sum[m][0], sum[m][1]);
+    }
+    __syncthreads();
+    if (keeps) {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        unpack2(sum[m][0], s[m][0], s[m][1]);
+        unpack2(sum[m][1], s[m][2], s[m][3]);
+#pragma unroll
+        for (int t = 1; t < TOKENS; ++t) {
+          const float4 part = *reinterpret_cast<const float4*>(parts + ((t - 1) * kCarry + column + m) * LD + n);
+          s[m][0] += part.x, s[m][1] += part.y, s[m][2] += part.z, s[m][3] += part.w;
+        }
+      }
     }
   }
-  store(kept);
+  if (keeps) store(kept, false);
 }
 
 // ------------------------------------------------------------------------------------------------------------ launches
 constexpr size_t local_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 3 * kC); }
 constexpr size_t read_bytes(int np) { return sizeof(float) * (size_t)(2 * kC * (np + 4) + 2 * kC * kLd + 4 * kC + np); }
 constexpr size_t solve_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 48 * kThreads + 5 * kC); }
-constexpr size_t carry_bytes(int np) { return sizeof(float) * (size_t)(4 * kC * (np + 4) + 3 * kC * kCarry + kCarry * (np + 4)); }
+constexpr size_t carry_bytes(int np) { return sizeof(float) * (size_t)(4 * kC * (np + 4) + 3 * kC * kCarry + kCarry * (np + 4) + 4 * kC * kPartLd); }
 
 template <typename Kernel>
 static bool allow(Kernel kernel, size_t bytes) {
