@@ -23,24 +23,44 @@
 // the bfloat16 form runs on the tensor cores.  In both a row's result depends on the row and its expert alone, not on
 // what else is in the batch or on where the row was sorted to.
 #include "common.cuh"
+#include "elementwise_vec.cuh"
 #include "mma_common.cuh"
 
 namespace ms {
 
 // Router logits, float32: logits[n][e] = sum_c x_n[c] W[e, c] + b[e].  A block of eight warps holds the rows of RT
 // tokens in shared memory (in their stored type: the conversion is exact) and takes `per_block` experts, warp w the
-// experts w, w + 8, ... of them: it reads an expert's weight row once, sixteen bytes per lane and two such loads
-// ahead of the sums, and forms the RT tokens' logits beside one another.  A logit is the fixed tree over the lanes'
-// sums of their own pieces in ascending order, so it does not depend on the token's neighbours or on the grid.
-template <typename T, int RT>
+// experts EW w .. EW w + EW - 1 and every 8 EW-th behind them: it reads an expert's weight row once, sixteen bytes per lane and eight
+// such loads ahead of the sums (the trip to the second-level cache, not the sums, is what a row costs: 2,048 tokens of
+// 16 rows take 14 us, 8 tokens of 60 rows 7, with two loads ahead 20 and 13; the first loads are made before the tokens are there), and forms the RT
+// tokens' logits beside one another; with EW = 2 a token's numbers are fetched and converted once for two experts.
+// A logit is the fixed tree over the lanes' sums of their own pieces in ascending order, so it does not depend on the token's neighbours
+// or on the grid.
+template <typename T> struct alignas(4 * sizeof(T)) Row4 { T v[4]; };
+
+template <typename T, int RT, int EW>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const T* __restrict__ x, const float* __restrict__ weight, const float* __restrict__ bias,
                      int width, int experts, int per_block, float* __restrict__ logits, int n_tokens) {
-  grid_dependency_wait();
-  grid_dependency_launch();
   extern __shared__ __align__(16) unsigned char router_smem[];
   T* xs = reinterpret_cast<T*>(router_smem);          // [RT][width]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int AHEAD = 8 / EW;
+  const bool wide = (width & 3) == 0;
+  const int e_first = blockIdx.y * per_block + EW * warp, e_end = min(experts, (int)(blockIdx.y + 1) * per_block);
+  float4 next[EW][AHEAD];
+  auto fetch = [&](int e, int c0) {
+#pragma unroll
+    for (int i = 0; i < EW; ++i)
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j) {
+        const int c = c0 + 128 * j + 4 * lane;
+        next[i][j] = c < width ? *reinterpret_cast<const float4*>(weight + (size_t)min(e + i, e_end - 1) * width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+  };
+  if (wide && e_first < e_end) fetch(e_first, 0);     // (weights: no kernel writes them)
+  grid_dependency_wait();
+  grid_dependency_launch();
   const int n0 = blockIdx.x * RT;
   constexpr int VEC = 16 / sizeof(T);                 // elements per 16-byte load
   if (width % VEC == 0) {
@@ -58,47 +78,58 @@ router_logits_kernel(const T* __restrict__ x, const float* __restrict__ weight, 
     }
   }
   __syncthreads();
-  const int e_end = min(experts, (blockIdx.y + 1) * per_block);
-  for (int e = blockIdx.y * per_block + warp; e < e_end; e += 8) {
-    const float* w = weight + (size_t)e * width;
-    float sum[RT];
+  for (int e = e_first; e < e_end; e += 8 * EW) {
+    float sum[EW][RT];
 #pragma unroll
-    for (int t = 0; t < RT; ++t) sum[t] = 0.f;
-    if ((width & 3) == 0) {
-      for (int c = lane * 4; c < width; c += 256) {
-        const float4 w0 = *reinterpret_cast<const float4*>(w + c);
-        const bool more = c + 128 < width;
-        const float4 w1 = more ? *reinterpret_cast<const float4*>(w + c + 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < EW; ++i)
 #pragma unroll
-        for (int t = 0; t < RT; ++t) {
-          const T* row = xs + t * width + c;
-          sum[t] += to_float(row[0]) * w0.x;
-          sum[t] += to_float(row[1]) * w0.y;
-          sum[t] += to_float(row[2]) * w0.z;
-          sum[t] += to_float(row[3]) * w0.w;
-        }
-        if (more) {
+      for (int t = 0; t < RT; ++t) sum[i][t] = 0.f;
+    if (wide) {
+      for (int c0 = 0; c0 < width; c0 += 128 * AHEAD) {
+        float4 now[EW][AHEAD];
+#pragma unroll
+        for (int i = 0; i < EW; ++i)
+#pragma unroll
+          for (int j = 0; j < AHEAD; ++j) now[i][j] = next[i][j];
+        if (c0 + 128 * AHEAD < width) fetch(e, c0 + 128 * AHEAD);
+        else if (e + 8 * EW < e_end) fetch(e + 8 * EW, 0);
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+          const int c = c0 + 128 * j + 4 * lane;
+          if (c >= width) continue;
 #pragma unroll
           for (int t = 0; t < RT; ++t) {
-            const T* row = xs + t * width + c + 128;
-            sum[t] += to_float(row[0]) * w1.x;
-            sum[t] += to_float(row[1]) * w1.y;
-            sum[t] += to_float(row[2]) * w1.z;
-            sum[t] += to_float(row[3]) * w1.w;
+            const Row4<T> row = *reinterpret_cast<const Row4<T>*>(xs + t * width + c);
+            const float4 four = make_float4(to_float(row.v[0]), to_float(row.v[1]), to_float(row.v[2]), to_float(row.v[3]));
+#pragma unroll
+            for (int i = 0; i < EW; ++i) {
+              sum[i][t] += four.x * now[i][j].x;
+              sum[i][t] += four.y * now[i][j].y;
+              sum[i][t] += four.z * now[i][j].z;
+              sum[i][t] += four.w * now[i][j].w;
+            }
           }
         }
       }
     } else {
-      for (int c = lane; c < width; c += 32) {
-        const float wc = w[c];
 #pragma unroll
-        for (int t = 0; t < RT; ++t) sum[t] += to_float(xs[t * width + c]) * wc;
+      for (int i = 0; i < EW; ++i) {
+        const float* w = weight + (size_t)min(e + i, e_end - 1) * width;
+        for (int c = lane; c < width; c += 32) {
+          const float wc = w[c];
+#pragma unroll
+          for (int t = 0; t < RT; ++t) sum[i][t] += to_float(xs[t * width + c]) * wc;
+        }
       }
     }
 #pragma unroll
-    for (int t = 0; t < RT; ++t) {
-      const float total = warp_sum(sum[t]);
-      if (lane == 0 && n0 + t < n_tokens) logits[(size_t)(n0 + t) * experts + e] = total + (bias ? bias[e] : 0.f);
+    for (int i = 0; i < EW; ++i) {
+      if (e + i >= e_end) break;
+#pragma unroll
+      for (int t = 0; t < RT; ++t) {
+        const float total = warp_sum(sum[i][t]);
+        if (lane == 0 && n0 + t < n_tokens) logits[(size_t)(n0 + t) * experts + e + i] = total + (bias ? bias[e + i] : 0.f);
+      }
     }
   }
 }
@@ -514,6 +545,48 @@ __global__ void expert_combine_kernel(const T* __restrict__ Y, int ldy, const in
   }
 }
 
+// The same, eight numbers a thread (sixteen-byte pieces in bfloat16), the rows of four choices on their way at a time; grid (tokens,
+// pieces of a row).  2,048 tokens, four choices of 2,048 numbers: 10 us, 20 number by number; and a decode step is
+// spread over more than a block a token (8 tokens, six choices: 4.8 us, 15).  The sums are the same sums.
+template <typename T>
+__global__ void __launch_bounds__(128)
+expert_combine_wide_kernel(const T* __restrict__ Y, int ldy, const int* __restrict__ place, const float* __restrict__ weights, int top,
+                           const T* __restrict__ shared, T* __restrict__ out, int width, const int* __restrict__ ids,
+                           int first_identity, const T* __restrict__ x, const float* __restrict__ shared_gate, int shared_gate_ld) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const size_t n = blockIdx.x;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= width) return;
+  Vec8 sum, row[4];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) sum.v[e] = 0.f;
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float factor[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k0 + u >= top) continue;
+      const size_t pair = n * top + k0 + u;
+      const bool identity = ids && ids[pair] >= first_identity;
+      row[u] = load8(identity ? x + n * width + c : Y + (size_t)place[pair] * ldy + c);
+      factor[u] = weights ? weights[pair] : 1.f;              // (no weights: the experts' inputs carried them)
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k0 + u >= top) continue;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sum.v[e] = weights ? sum.v[e] + factor[u] * row[u].v[e] : sum.v[e] + row[u].v[e];
+    }
+  }
+  if (shared) {
+    const float share = shared_gate ? 1.f / (1.f + expf(-shared_gate[n * shared_gate_ld])) : 1.f;
+    const Vec8 own = load8(shared + n * width + c);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sum.v[e] += share * own.v[e];
+  }
+  store8(out + n * width + c, sum);
+}
+
 // out[n, j] = clamped_glu(both[n, 2 j], both[n, 2 j + 1])
 template <typename T>
 __global__ void clamped_glu_kernel(const T* __restrict__ both, T* __restrict__ out, size_t total, float limit) {
@@ -559,7 +632,7 @@ static int launch_router_logits(const void* x, int dtype, const float* weight, c
   dim3 grid(token_tiles, (experts + per_block - 1) / per_block);
   const size_t smem = (size_t)rt * width * element;
 #define MS_ROUTER_LOGITS(RT)                                                                                                \
-  MS_EXP_DISPATCH(dtype, (ms::launch(router_logits_kernel<T, RT>, grid, 256, smem, stream, (const T*)x, weight, bias, width, \
+  MS_EXP_DISPATCH(dtype, (ms::launch(per_block > 8 ? router_logits_kernel<T, RT, 2> : router_logits_kernel<T, RT, 1>, grid, 256, smem, stream, (const T*)x, weight, bias, width, \
                                      experts, per_block, logits, n_tokens)))
   if (rt == 8) { MS_ROUTER_LOGITS(8); } else if (rt == 4) { MS_ROUTER_LOGITS(4); } else if (rt == 2) { MS_ROUTER_LOGITS(2); }
   else { MS_ROUTER_LOGITS(1); }
@@ -675,6 +748,14 @@ MS_EXPORT int ms_expert_combine(const void* Y, int dtype, int ldy, const int* pl
                                 const void* x, const float* shared_gate, int shared_gate_ld, cudaStream_t stream) {
   if (n_tokens == 0 || width == 0) return 0;
   MS_REQUIRE(ids == nullptr || x != nullptr, "expert_combine: identity experts need the tokens' rows");
+  auto aligned = [](const void* at) { return reinterpret_cast<size_t>(at) % 16 == 0; };
+  if (width % 8 == 0 && ldy % 8 == 0 && width <= 1024 * 65535 && aligned(Y) && aligned(out) && (!shared || aligned(shared)) && (!ids || aligned(x))) {
+    MS_EXP_DISPATCH(dtype, (ms::launch(expert_combine_wide_kernel<T>, dim3(n_tokens, (width + 1023) / 1024), 128, 0, stream, (const T*)Y, ldy,
+                                       place, weights, top, (const T*)shared, (T*)out, width, ids, first_identity, (const T*)x,
+                                       shared_gate, shared_gate_ld)));
+    MS_CHECK_LAUNCH("expert_combine");
+    return 0;
+  }
   MS_EXP_DISPATCH(dtype, (ms::launch(expert_combine_kernel<T>, n_tokens, 256, 0, stream, (const T*)Y, ldy, place, weights, top,
                                      (const T*)shared, (T*)out, width, ids, first_identity, (const T*)x, shared_gate,
                                      shared_gate_ld)));
