@@ -47,6 +47,31 @@ __global__ void unit_norm_heads_kernel(float* __restrict__ x, int ld, int col, i
   for (int c = lane; c < dim; c += 32) v[c] *= factor;
 }
 
+// The same for heads of up to 128 numbers whose rows lie on 16-byte boundaries: four numbers a lane, four (token, head) pairs a warp, so
+// that 2 KB a warp are on their way at a time.
+__global__ void unit_norm_heads_wide_kernel(float* __restrict__ x, int ld, int col, unsigned heads, int dim, float eps, float scale,
+                                            unsigned items) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  const int lane = threadIdx.x & 31;
+  const unsigned first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4;
+  float4* at[4];
+  float4 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned item = first + i;
+    const bool real = item < items && 4 * lane < dim;
+    at[i] = real ? reinterpret_cast<float4*>(x + (size_t)(item / heads) * ld + col + (size_t)(item % heads) * dim) + lane : nullptr;
+    v[i] = real ? *at[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float sum_sq = (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+    const float factor = scale / sqrtf(warp_sum(sum_sq) + eps);
+    if (at[i]) *at[i] = make_float4(v[i].x * factor, v[i].y * factor, v[i].z * factor, v[i].w * factor);
+  }
+}
+
 // One warp per (request, head).  logits [tokens, 2 heads] = [input | forget].  Lane l squashes the logits of token l of a
 // chunk of 32; the running maximum then walks the chunk's tokens in order (values handed round by shuffles), and each lane
 // writes its token's three factors.  The request's maximum is read from and left in states[slot, offset + head].
@@ -86,6 +111,76 @@ __global__ void exponential_gates_kernel(const float* __restrict__ logits, float
     }
   }
   if (lane == 0) *kept = peak;
+}
+
+// The same for portions of many tokens: one block per (head, request).  A token maps the maximum before it to max(f + m, i), and so
+// does a run of tokens, with F the sum of its f and I the maximum it leaves on its own: a thread composes its kGateRun tokens, a scan
+// over the threads gives every thread the maximum before its first, and it walks its tokens from there.  (Sums of f span only the tokens
+// of their run, so nothing cancels.)  2,011 tokens of 8 heads: 12 us, 74 as a chain of one warp a head
+// whose every token is two shuffles.
+constexpr int kGateRun = 8, kGateThreads = 256;
+
+__global__ void __launch_bounds__(kGateThreads)
+exponential_gates_scan_kernel(const float* __restrict__ logits, float cap, float* __restrict__ states, long long state_stride,
+                              int state_offset, const int* __restrict__ state_slots, const int* __restrict__ query_start, int heads,
+                              float* __restrict__ gates) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  __shared__ float2 warp_runs[2][kGateThreads / 32];
+  const int head = blockIdx.x, request = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q0 = query_start[request], q_len = query_start[request + 1] - q0;
+  if (q_len <= 0) return;
+  float* kept = states + (long long)state_slots[request] * state_stride + state_offset + head;
+  float carried = *kept;
+  int turn = 0;
+  for (int t0 = 0; t0 < q_len; t0 += kGateThreads * kGateRun, turn ^= 1) {
+    const int first = t0 + threadIdx.x * kGateRun;
+    float f[kGateRun], in[kGateRun];
+#pragma unroll
+    for (int j = 0; j < kGateRun; ++j) {
+      const float* row = logits + (size_t)(q0 + min(first + j, q_len - 1)) * 2 * heads + head;
+      in[j] = row[0], f[j] = row[heads];
+    }
+    float sum = 0.f, top = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kGateRun; ++j) {
+      in[j] = cap * tanhf(in[j] / cap);
+      f[j] = log_sigmoid_f(cap * tanhf(f[j] / cap));
+      if (first + j < q_len) {
+        top = fmaxf(top + f[j], in[j]);
+        sum += f[j];
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float sum_before = __shfl_up_sync(0xffffffffu, sum, o), top_before = __shfl_up_sync(0xffffffffu, top, o);
+      if (lane >= o) {
+        top = fmaxf(top_before + sum, top);
+        sum += sum_before;
+      }
+    }
+    if (lane == 31) warp_runs[turn][warp] = make_float2(sum, top);
+    __syncthreads();
+    float peak = carried;                                      // the maximum before this warp's first token, and after the last warp's
+    for (int w = 0; w < kGateThreads / 32; ++w) {
+      const float2 run = warp_runs[turn][w];
+      if (w < warp) peak = fmaxf(peak + run.x, run.y);
+      carried = fmaxf(carried + run.x, run.y);
+    }
+    const float sum_before = __shfl_up_sync(0xffffffffu, sum, 1), top_before = __shfl_up_sync(0xffffffffu, top, 1);
+    if (lane > 0) peak = fmaxf(peak + sum_before, top_before);
+#pragma unroll
+    for (int j = 0; j < kGateRun; ++j) {
+      if (first + j >= q_len) break;
+      const float next = fmaxf(f[j] + peak, in[j]);
+      float* out = gates + ((size_t)(q0 + first + j) * heads + head) * 3;
+      out[0] = expf(f[j] + peak - next);
+      out[1] = expf(in[j] - next);
+      out[2] = expf(-next);
+      peak = next;
+    }
+  }
+  if (threadIdx.x == 0) *kept = carried;
 }
 
 // logits [tokens, 2 heads] = [b | a]; gates [tokens, heads, 2] = (decay, beta).
@@ -406,21 +501,79 @@ low_rank_expand_tiled_kernel(const float* __restrict__ mid, int ld, int col, int
   }
 }
 
-// One warp per (token, head): v = y / bottom, v / sqrt(mean(v^2) + eps) * weight * act(gate).  Where a head's row is
-// at most 512 numbers, a multiple of four, and lies on 16-byte boundaries in all four arrays (`wide`), a lane keeps its
-// four-number pieces in registers between the sum and the output and every access is one piece; otherwise number by number.
+// v = y / bottom, v / sqrt(mean(v^2) + eps) * weight * act(gate), a row of y per (token, head), a warp for ROWS of them at a time.  Where
+// rows are a multiple of four numbers and lie on 16-byte boundaries in all four arrays, a lane keeps PIECES pieces of four numbers of
+// each row in registers between the sum and the output.  Bound by memory once enough of it is asked for at a time, hence four
+// pieces a lane whatever the row's length (2,048 x 16 rows of 128, 34 MB: 13 us, 37 one row at a time).
 template <typename T> struct alignas(sizeof(T) * 4) Four { T v[4]; };
 constexpr int kHeadPieces = 4;                               // pieces of four numbers a lane
 
+template <typename T, int PIECES, bool DIVIDE>
+__global__ void __launch_bounds__(256)
+head_norm_gate_kernel(const float* __restrict__ y, const float* __restrict__ bottom, const float* __restrict__ weight,
+                      int weight_per_head, const T* __restrict__ gate, int gate_ld, int gate_col, int activation, float eps,
+                      T* __restrict__ out, unsigned items, unsigned heads, int vdim) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  constexpr int ROWS = kHeadPieces / PIECES;
+  const int lane = threadIdx.x & 31, pieces = vdim >> 2;
+  const unsigned first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * ROWS;
+  float4 value[ROWS][PIECES];
+  Four<T> g[ROWS][PIECES];
+  float divisor[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const unsigned item = first + i;
+    const T* z = gate + (size_t)(item / heads) * gate_ld + gate_col + (size_t)(item % heads) * vdim;
+    const float4* row = reinterpret_cast<const float4*>(y + (size_t)item * vdim);
+    divisor[i] = DIVIDE && item < items ? bottom[item] : 1.f;
+#pragma unroll
+    for (int j = 0; j < PIECES; ++j) {
+      const int at = lane + 32 * j;
+      const bool real = item < items && at < pieces;
+      value[i][j] = real ? row[at] : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (real) g[i][j] = reinterpret_cast<const Four<T>*>(z)[at];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const unsigned item = first + i;
+    if (item >= items) return;
+    float sum_sq = 0.f;
+#pragma unroll
+    for (int j = 0; j < PIECES; ++j) {
+      float4& v = value[i][j];
+      if (DIVIDE) v.x /= divisor[i], v.y /= divisor[i], v.z /= divisor[i], v.w /= divisor[i];
+      sum_sq += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(sum_sq) / (float)vdim + eps);
+    const float4* w = reinterpret_cast<const float4*>(weight + (weight_per_head ? (size_t)(item % heads) * vdim : 0));
+    Four<T>* dst = reinterpret_cast<Four<T>*>(out + (size_t)item * vdim);
+#pragma unroll
+    for (int j = 0; j < PIECES; ++j) {
+      const int at = lane + 32 * j;
+      if (at >= pieces) continue;
+      const float4 scale = w[at], v = value[i][j];
+      const float v4[4] = {v.x * inv * scale.x, v.y * inv * scale.y, v.z * inv * scale.z, v.w * inv * scale.w};
+      Four<T> o;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float gv = to_float(g[i][j].v[e]);
+        o.v[e] = from_float<T>(v4[e] * (activation ? gv * sigmoid_f(gv) : sigmoid_f(gv)));
+      }
+      dst[at] = o;
+    }
+  }
+}
+
+// The same number by number, one warp per (token, head).
 template <typename T>
-__global__ void head_norm_gate_kernel(const float* __restrict__ y, const float* __restrict__ bottom,
-                                      const float* __restrict__ weight, int weight_per_head, const T* __restrict__ gate,
-                                      int gate_ld, int gate_col, int activation, float eps, T* __restrict__ out, int n_tokens,
-                                      int heads, int vdim, int wide) {
+__global__ void head_norm_gate_any_kernel(const float* __restrict__ y, const float* __restrict__ bottom, const float* __restrict__ weight,
+                                          int weight_per_head, const T* __restrict__ gate, int gate_ld, int gate_col, int activation,
+                                          float eps, T* __restrict__ out, long long items, int heads, int vdim) {
   grid_dependency_wait();
   grid_dependency_launch();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long items = (long long)n_tokens * heads;
   for (long long item = (long long)blockIdx.x * warps + warp; item < items; item += (long long)gridDim.x * warps) {
     const size_t token = (size_t)(item / heads);
     const int head = (int)(item % heads);
@@ -428,41 +581,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ y, const float* 
     const float divisor = bottom ? bottom[item] : 1.f;
     const float* w = weight + (weight_per_head ? (size_t)head * vdim : 0);
     const T* z = gate + token * gate_ld + gate_col + (size_t)head * vdim;
-    T* dst = out + (token * heads + head) * vdim;
-    if (wide) {
-      const int pieces = vdim >> 2;
-      float4 value[kHeadPieces];
-      Four<T> g[kHeadPieces];
-      float sum_sq = 0.f;
-#pragma unroll
-      for (int j = 0; j < kHeadPieces; ++j) {
-        const int at = lane + 32 * j;
-        value[j] = at < pieces ? reinterpret_cast<const float4*>(row)[at] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (at < pieces) g[j] = reinterpret_cast<const Four<T>*>(z)[at];
-      }
-#pragma unroll
-      for (int j = 0; j < kHeadPieces; ++j) {
-        value[j].x /= divisor, value[j].y /= divisor, value[j].z /= divisor, value[j].w /= divisor;
-        sum_sq += (value[j].x * value[j].x + value[j].y * value[j].y) + (value[j].z * value[j].z + value[j].w * value[j].w);
-      }
-      const float inv = 1.0f / sqrtf(warp_sum(sum_sq) / (float)vdim + eps);
-#pragma unroll
-      for (int j = 0; j < kHeadPieces; ++j) {
-        const int at = lane + 32 * j;
-        if (at < pieces) {
-          const float4 scale = reinterpret_cast<const float4*>(w)[at];
-          const float v4[4] = {value[j].x * inv * scale.x, value[j].y * inv * scale.y, value[j].z * inv * scale.z, value[j].w * inv * scale.w};
-          Four<T> o;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float gv = to_float(g[j].v[e]);
-            o.v[e] = from_float<T>(v4[e] * (activation ? gv * sigmoid_f(gv) : sigmoid_f(gv)));
-          }
-          reinterpret_cast<Four<T>*>(dst)[at] = o;
-        }
-      }
-      continue;
-    }
+    T* dst = out + (size_t)item * vdim;
     float sum_sq = 0.f;
     for (int c = lane; c < vdim; c += 32) {
       const float value = row[c] / divisor;
@@ -601,6 +720,14 @@ MS_EXPORT int ms_unit_norm_heads(float* x, int ld, int col, int heads, int dim, 
   if (n_tokens == 0 || heads == 0) return 0;
   MS_REQUIRE(dim > 0 && col >= 0 && col + heads * dim <= ld, "unit_norm_heads: %d heads of %d from column %d of rows of %d", heads, dim, col, ld);
   const int warps = 4;
+  if (dim % 4 == 0 && dim <= 128 && ld % 4 == 0 && col % 4 == 0 && reinterpret_cast<size_t>(x) % 16 == 0 &&
+      (long long)n_tokens * heads < (1LL << 31)) {
+    const unsigned items = (unsigned)n_tokens * (unsigned)heads;
+    ms::launch(unit_norm_heads_wide_kernel, (items + 4 * warps - 1) / (4 * warps), warps * 32, 0, stream, x, ld, col, (unsigned)heads, dim, eps,
+               scale, items);
+    MS_CHECK_LAUNCH("unit_norm_heads");
+    return 0;
+  }
   const long long blocks = ((long long)n_tokens * heads + warps - 1) / warps;
   MS_REQUIRE(blocks < 2147483647LL, "unit_norm_heads: %lld heads in one launch is too many", (long long)n_tokens * heads);
   ms::launch(unit_norm_heads_kernel, (unsigned)blocks, warps * 32, 0, stream, x, ld, col, heads, dim, eps, scale, n_tokens);
@@ -609,12 +736,19 @@ MS_EXPORT int ms_unit_norm_heads(float* x, int ld, int col, int heads, int dim, 
 }
 
 // logits float32 [tokens, 2 heads]; states float32 rows of state_stride numbers, the heads' maxima at state_offset;
-// gates float32 [tokens, heads, 3].
+// gates float32 [tokens, heads, 3].  max_query_len: an upper bound of the tokens a request brings; from 96 on (where the scans
+// behind these gates go in chunks too) the portions' maxima come from a parallel scan.
 MS_EXPORT int ms_exponential_gates(const float* logits, float cap, float* states, long long state_stride, int state_offset,
-                                   const int* state_slots, const int* query_start, int n_requests, int heads, float* gates,
-                                   cudaStream_t stream) {
+                                   const int* state_slots, const int* query_start, int n_requests, int max_query_len, int heads,
+                                   float* gates, cudaStream_t stream) {
   if (n_requests == 0 || heads == 0) return 0;
   MS_REQUIRE(cap > 0.f && n_requests <= 65535, "exponential_gates: cap %f, %d requests", cap, n_requests);
+  if (max_query_len >= 96) {
+    ms::launch(exponential_gates_scan_kernel, dim3(heads, n_requests), kGateThreads, 0, stream, logits, cap, states, state_stride,
+               state_offset, state_slots, query_start, heads, gates);
+    MS_CHECK_LAUNCH("exponential_gates");
+    return 0;
+  }
   const int warps = heads >= 4 ? 4 : heads;
   dim3 grid((heads + warps - 1) / warps, n_requests);
   ms::launch(exponential_gates_kernel, grid, warps * 32, 0, stream, logits, cap, states, state_stride, state_offset, state_slots,
@@ -769,17 +903,28 @@ MS_EXPORT int ms_head_norm_gate(const float* y, const float* bottom, const float
     MS_CHECK_LAUNCH("head_norm_gate");
     return 0;
   }
-  // blocks of eight warps that walk the (token, head) pairs with the grid's stride: at most sixteen blocks a multiprocessor
   const int warps = 8;
-  long long blocks = ((long long)n_tokens * heads + warps - 1) / warps;
-  if (blocks > 16LL * scan_sm_count()) blocks = 16LL * scan_sm_count();
+  const long long items = (long long)n_tokens * heads;
   const size_t element = dtype == MS_F32 ? 4 : 2;
-  const int wide = vdim % 4 == 0 && vdim <= 128 * kHeadPieces && gate_ld % 4 == 0 && gate_col % 4 == 0 &&
-                   reinterpret_cast<size_t>(y) % 16 == 0 && reinterpret_cast<size_t>(weight) % 16 == 0 &&
-                   reinterpret_cast<size_t>(gate) % (4 * element) == 0 && reinterpret_cast<size_t>(out) % (4 * element) == 0;
-  MS_REC_DISPATCH(dtype, (ms::launch(head_norm_gate_kernel<T>, (unsigned)blocks, warps * 32, 0, stream, y, bottom, weight,
-                                     weight_per_head, (const T*)gate, gate_ld, gate_col, activation, eps, (T*)out, n_tokens,
-                                     heads, vdim, wide)));
+  const bool wide = vdim % 4 == 0 && gate_ld % 4 == 0 && gate_col % 4 == 0 &&
+                    reinterpret_cast<size_t>(y) % 16 == 0 && reinterpret_cast<size_t>(weight) % 16 == 0 &&
+                    reinterpret_cast<size_t>(gate) % (4 * element) == 0 && reinterpret_cast<size_t>(out) % (4 * element) == 0;
+#define MS_HEAD_NORM(PIECES, DIVIDE)                                                                                          \
+  MS_REC_DISPATCH(dtype, (ms::launch(head_norm_gate_kernel<T, PIECES, DIVIDE>, (unsigned)((items + warps * kHeadPieces / PIECES - 1) / (warps * kHeadPieces / PIECES)), \
+                                     warps * 32, 0, stream, y, bottom, weight, weight_per_head, (const T*)gate, gate_ld, gate_col, activation, eps, \
+                                     (T*)out, (unsigned)items, (unsigned)heads, vdim)))
+#define MS_HEAD_NORM_PIECES(DIVIDE) \
+  if (vdim <= 128) { MS_HEAD_NORM(1, DIVIDE); } else if (vdim <= 256) { MS_HEAD_NORM(2, DIVIDE); } else { MS_HEAD_NORM(4, DIVIDE); }
+  if (wide && items < (1LL << 31)) {
+    if (bottom) { MS_HEAD_NORM_PIECES(true); } else { MS_HEAD_NORM_PIECES(false); }
+  } else {
+    long long blocks = (items + warps - 1) / warps;
+    if (blocks > 16LL * scan_sm_count()) blocks = 16LL * scan_sm_count();
+    MS_REC_DISPATCH(dtype, (ms::launch(head_norm_gate_any_kernel<T>, (unsigned)blocks, warps * 32, 0, stream, y, bottom, weight, weight_per_head,
+                                       (const T*)gate, gate_ld, gate_col, activation, eps, (T*)out, items, heads, vdim)));
+  }
+#undef MS_HEAD_NORM_PIECES
+#undef MS_HEAD_NORM
   MS_CHECK_LAUNCH("head_norm_gate");
   return 0;
 }

@@ -1065,7 +1065,7 @@ def exponential_gates(logits: torch.Tensor, cap: float, states: torch.Tensor, st
     _want(query_start, "query_start", torch.int32, (n_requests + 1,))
     stride = _state_rows(states, state_offset, heads)
     _check(library().ms_exponential_gates(_ptr(logits), _f(cap), _ptr(states), stride, _i(state_offset), _ptr(state_slots),
-                                          _ptr(query_start), _i(n_requests), _i(heads), _ptr(gates), _stream()))
+                                          _ptr(query_start), _i(n_requests), _i(max_query_len), _i(heads), _ptr(gates), _stream()))
 
 
 def decay_gates(logits: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, gates: torch.Tensor) -> None:
