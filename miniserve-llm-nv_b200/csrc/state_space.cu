@@ -93,6 +93,99 @@ causal_conv_silu_kernel(const T* __restrict__ proj, int ld, int col, int channel
   }
 }
 
+// The same for a fixed number of taps and rows on 8- or 16-byte boundaries: a thread owns four neighbouring channels, and eight tokens'
+// inputs are on their way at a time.  Bound by memory (2,048 tokens of 6,144 channels, 75 MB: 26 us, 46 channel by channel, two
+// bytes a lane and load).  Every sum is the same sum.
+template <typename T> struct alignas(4 * sizeof(T)) Channels { T v[4]; };
+
+template <typename T, typename U, int TAPS>
+__global__ void __launch_bounds__(128)
+causal_conv_wide_kernel(const T* __restrict__ proj, int ld, int col, int channels, const float* __restrict__ weight,
+                        const float* __restrict__ bias, const float* __restrict__ in_bias, int activation,
+                        float* __restrict__ states, long long state_stride, int state_offset, const int* __restrict__ state_slots,
+                        const int* __restrict__ query_start, U* __restrict__ out) {
+  grid_dependency_wait();
+  grid_dependency_launch();
+  constexpr int KEEP = TAPS - 1, TOGETHER = 8;
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  const int request = blockIdx.z;
+  const int q0 = query_start[request], q_len = query_start[request + 1] - q0;
+  const int t0 = blockIdx.y * kConvTokens;
+  if (c >= channels || t0 >= q_len) return;
+  float* state = states + (long long)state_slots[request] * state_stride + state_offset + c;     // [KEEP][channels]
+  const T* in = proj + (size_t)q0 * ld + col + c;
+  float w[4][TAPS], window[TAPS][4], b[4], ib[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (TAPS == 4) {                         // (the launch saw to the weight's alignment)
+      const float4 four = *reinterpret_cast<const float4*>(weight + (size_t)(c + e) * 4);
+      w[e][0] = four.x, w[e][TAPS - 3] = four.y, w[e][TAPS - 2] = four.z, w[e][TAPS - 1] = four.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) w[e][k] = weight[(size_t)(c + e) * TAPS + k];
+    }
+    b[e] = bias ? bias[c + e] : 0.f;
+    ib[e] = in_bias ? in_bias[c + e] : 0.f;
+  }
+  auto input = [&](int t, float (&to)[4]) {
+    const Channels<T> four = *reinterpret_cast<const Channels<T>*>(in + (size_t)t * ld);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) to[e] = to_float(four.v[e]) + ib[e];
+  };
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {           // window[k + 1]: input t0 - KEEP + k (window[0] is shifted out first)
+    const int i = t0 - KEEP + k;
+    if (i >= 0) {
+      input(i, window[k + 1]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) window[k + 1][e] = state[(size_t)(KEEP + i) * channels + e];
+    }
+  }
+  if (t0 == 0) {
+    // new state: the last KEEP inputs of (old state, this portion)
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) {
+      const int i = q_len - KEEP + j;
+      float v[4];
+      if (i >= 0) {
+        input(i, v);
+      } else {
+#pragma unroll
+        for (int k = 1; k < TAPS; ++k)
+          if (k == 1 + KEEP + i) {           // = old state[KEEP + i], read above, before this write
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = window[k][e];
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) state[(size_t)j * channels + e] = v[e];
+    }
+  }
+  const int t_end = min(q_len, t0 + kConvTokens);
+  for (int t = t0; t < t_end; t += TOGETHER) {
+    Channels<T> raw[TOGETHER];
+#pragma unroll
+    for (int u = 0; u < TOGETHER; ++u) raw[u] = *reinterpret_cast<const Channels<T>*>(in + (size_t)min(t + u, t_end - 1) * ld);
+#pragma unroll
+    for (int u = 0; u < TOGETHER; ++u) {
+      if (t + u >= t_end) break;
+      Channels<U> result;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) window[k][e] = window[k + 1][e];
+        window[KEEP][e] = to_float(raw[u].v[e]) + ib[e];
+        float sum = b[e];
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) sum += w[e][k] * window[k][e];
+        result.v[e] = from_float<U>(activation ? silu_f(sum) : sum);
+      }
+      *reinterpret_cast<Channels<U>*>(out + (size_t)(q0 + t + u) * channels + c) = result;
+    }
+  }
+}
+
 // The recurrence.  grid (column blocks of a head, heads, requests); a block of four warps owns 4 * CP channels (columns p)
 // of one head of one request, a warp CP of them, with the 32 lanes along the state: lane j holds the entries n = j,
 // j + 32, ... (R of them) of each of its columns in registers.  The tokens' B, C and x pass through shared memory in chunks
@@ -419,6 +512,22 @@ MS_EXPORT int ms_causal_conv(const void* proj, int dtype, int ld, int col, int c
   MS_REQUIRE(activation == 0 || activation == 1, "causal_conv: activation code %d", activation);
   const int chunks = (max_query_len + kConvTokens - 1) / kConvTokens;
   MS_REQUIRE(chunks <= 65535 && n_requests <= 65535, "causal_conv: grid %d x %d exceeds the launch limits", chunks, n_requests);
+  const size_t element = dtype == MS_F32 ? 4 : 2, out_element = out_like_proj ? element : 4;
+  if (taps >= 2 && taps <= 4 && (dtype == MS_F32 || dtype == MS_BF16) && channels % 4 == 0 && ld % 4 == 0 && col % 4 == 0 &&
+      reinterpret_cast<size_t>(proj) % (4 * element) == 0 && reinterpret_cast<size_t>(out) % (4 * out_element) == 0 &&
+      (taps != 4 || reinterpret_cast<size_t>(weight) % 16 == 0)) {
+    dim3 wide_grid((channels + 511) / 512, chunks, n_requests);
+#define MS_CONV_WIDE(U, TAPS)                                                                                                  \
+  MS_SS_DISPATCH(dtype, (ms::launch(causal_conv_wide_kernel<T, U, TAPS>, wide_grid, 128, 0, stream, (const T*)proj, ld, col, channels, weight, \
+                                    bias, in_bias, activation, states, state_stride, state_offset, state_slots, query_start, (U*)out)))
+#define MS_CONV_WIDE_TAPS(U) \
+  if (taps == 2) { MS_CONV_WIDE(U, 2); } else if (taps == 3) { MS_CONV_WIDE(U, 3); } else { MS_CONV_WIDE(U, 4); }
+    if (out_like_proj) { MS_CONV_WIDE_TAPS(T); } else { MS_CONV_WIDE_TAPS(float); }
+#undef MS_CONV_WIDE_TAPS
+#undef MS_CONV_WIDE
+    MS_CHECK_LAUNCH("causal_conv");
+    return 0;
+  }
   dim3 grid((channels + 127) / 128, chunks, n_requests);
   if (out_like_proj) {
     MS_SS_DISPATCH(dtype, (ms::launch(causal_conv_silu_kernel<T, T>, grid, 128, 0, stream, (const T*)proj, ld, col, channels, taps,
