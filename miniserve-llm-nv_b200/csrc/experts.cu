@@ -24,7 +24,7 @@
 // what else is in the batch or on where the row was sorted to.
 #include "common.cuh"
 #include "elementwise_vec.cuh"
-#include "mma_common.cuh"
+#include "expert_activation.cuh"
 
 namespace ms {
 
@@ -298,19 +298,6 @@ __global__ void expert_route_kernel(const int* __restrict__ ids, int pairs, int 
 constexpr int EBM = 64, EBN = 64, EBK = 16, ETM = 4, ETN = 4;
 
 // epilogues of the experts' products
-enum : int { kActNone = 0, kActReluSquare = 1, kActClampedGlu = 2, kActSiluGlu = 3 };
-
-// silu(s gate) (s up): the gated expert computed on s times its input (its first products are linear)
-__device__ __forceinline__ float silu_glu(float gate, float up, float s) {
-  const float g = s * gate;
-  return g / (1.f + expf(-g)) * (s * up);
-}
-
-// g = min(gate, limit), u = clamp(up, -limit, limit); g sigmoid(1.702 g) (u + 1)
-__device__ __forceinline__ float clamped_glu(float gate, float up, float limit) {
-  const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-  return g / (1.f + expf(-1.702f * g)) * (u + 1.f);
-}
 
 // C[i, :] = act(A[src(i), :] W_e^T) for every place i of expert e's segment; W [experts, N, K].  blockIdx.y walks the
 // row tiles of all segments one after the other (a segment's last tile may be partial); tiles beyond the last do nothing.
@@ -393,132 +380,6 @@ expert_linear_kernel(const T* __restrict__ A, int lda, const int* __restrict__ o
       C[(size_t)m * ldc + n] = from_float<T>(v);
     }
   }
-}
-
-// The same product on the tensor cores (bfloat16, mma.sync.m16n8k16, float32 sums): tiles of 64 rows x 128 columns, k in
-// steps of GBK through GSTAGES cp.async stages; eight warps, each 32 x 32 of the tile.  Rows of A are gathered through
-// `order` as above (a row's address is looked up once).  Inner size and column count multiples of 8.  (Measured against k
-// steps of 32 in three stages, which fit three blocks on a multiprocessor instead of two: steps of few rows, which only
-// stream the experts' weights, 25 -> 19 us per launch, half the barriers and twice the bytes on their way; prompt steps
-// 155 -> 147 us.)
-// Where the segments are long (prompt steps) the tiles have 128 rows, so that every weight fragment a warp fetches from shared
-// memory feeds four products instead of two (three stages then, two blocks a multiprocessor as before).
-constexpr int GBN = 128, GBK = 64;
-
-template <int GBM, int GSTAGES>
-__global__ void __launch_bounds__(256)
-expert_linear_mma_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __restrict__ order, int top,
-                         const __nv_bfloat16* __restrict__ W, __nv_bfloat16* __restrict__ C, int ldc,
-                         const int* __restrict__ offsets, int experts, int N, int K, int activation, float limit,
-                         const float* __restrict__ pair_scale) {
-  grid_dependency_wait();
-  grid_dependency_launch();
-  constexpr int GLD = GBK + 8;          // elements between the rows of a stage
-  constexpr int CPR = GBK / 8;          // 16-byte pieces per row of a stage
-  extern __shared__ __align__(16) unsigned char expert_smem[];
-  typedef __nv_bfloat16 (*StageA)[GBM][GLD];
-  typedef __nv_bfloat16 (*StageB)[GBN][GLD];
-  StageA As = reinterpret_cast<StageA>(expert_smem);
-  StageB Bs = reinterpret_cast<StageB>(expert_smem + sizeof(__nv_bfloat16) * GSTAGES * GBM * GLD);
-  __shared__ int src_row[GBM];
-  int tile = blockIdx.y, expert = 0, first = 0, end = 0;
-  for (; expert < experts; ++expert) {
-    first = offsets[expert];
-    end = offsets[expert + 1];
-    const int tiles = (end - first + GBM - 1) / GBM;
-    if (tile < tiles) break;
-    tile -= tiles;
-  }
-  if (expert == experts) return;
-  const int m0 = first + tile * GBM, n0 = blockIdx.x * GBN;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < GBM) {
-    const int i = m0 + tid;
-    src_row[tid] = i < end ? (order ? order[i] / top : i) : -1;
-  }
-  __syncthreads();
-  const __nv_bfloat16* We = W + (size_t)expert * N * K;
-  auto load_stage = [&](int stage, int k0) {
-#pragma unroll
-    for (int i = 0; i < GBM * CPR / 256; ++i) {                    // the A tile: its rows' addresses were looked up above
-      const int piece = tid + i * 256, r = piece / CPR, c = (piece % CPR) * 8;
-      const int src = src_row[r];
-      cp_async_16(&As[stage][r][c], A + (size_t)(src < 0 ? 0 : src) * lda + k0 + c, src >= 0 && k0 + c < K);
-    }
-#pragma unroll
-    for (int i = 0; i < GBN * CPR / 256; ++i) {
-      const int piece = tid + i * 256, r = piece / CPR, c = (piece % CPR) * 8;
-      const bool valid = n0 + r < N && k0 + c < K;
-      cp_async_16(&Bs[stage][r][c], We + (size_t)(valid ? n0 + r : 0) * K + (valid ? k0 + c : 0), valid);
-    }
-  };
-  const int k_tiles = (K + GBK - 1) / GBK;
-#pragma unroll
-  for (int s = 0; s < GSTAGES - 1; ++s) {
-    if (s < k_tiles) load_stage(s, s * GBK);
-    cp_async_commit();
-  }
-  const int warp_m = warp >> 2, warp_n = warp & 3;
-  constexpr int MI = GBM / 32;          // 16-row pieces of a warp's rows
-  float acc[MI][4][4];
-#pragma unroll
-  for (int i = 0; i < MI; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
-  for (int kt = 0; kt < k_tiles; ++kt) {
-    cp_async_wait<GSTAGES - 2>();
-    __syncthreads();
-    const int next = kt + GSTAGES - 1;
-    if (next < k_tiles) load_stage(next % GSTAGES, next * GBK);
-    cp_async_commit();
-    const int stage = kt % GSTAGES;
-#pragma unroll
-    for (int kk = 0; kk < GBK / 16; ++kk) {
-      unsigned a[MI][4], b[2][4];
-#pragma unroll
-      for (int mi = 0; mi < MI; ++mi)
-        ldmatrix_x4(a[mi], &As[stage][warp_m * (GBM / 2) + mi * 16 + (lane & 15)][kk * 16 + (lane >> 4) * 8]);
-#pragma unroll
-      for (int np = 0; np < 2; ++np)
-        ldmatrix_x4(b[np], &Bs[stage][warp_n * 32 + np * 16 + (lane & 7) + (lane >> 4) * 8][kk * 16 + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-      for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-        for (int np = 0; np < 2; ++np) {
-          mma_bf16(acc[mi][2 * np], a[mi], b[np][0], b[np][1]);
-          mma_bf16(acc[mi][2 * np + 1], a[mi], b[np][2], b[np][3]);
-        }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int mi = 0; mi < MI; ++mi)
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni) {
-      const int n = n0 + warp_n * 32 + ni * 8 + (lane & 3) * 2;
-      if (n >= N) continue;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int m = m0 + warp_m * (GBM / 2) + mi * 16 + (lane >> 2) + half * 8;
-        if (m >= end) continue;
-        float v0 = acc[mi][ni][2 * half], v1 = acc[mi][ni][2 * half + 1];
-        if (activation == kActClampedGlu) {         // (v0, v1) are a feature's gate and up sums
-          C[(size_t)m * ldc + n / 2] = __float2bfloat16_rn(clamped_glu(v0, v1, limit));
-          continue;
-        }
-        if (activation == kActSiluGlu) {
-          C[(size_t)m * ldc + n / 2] = __float2bfloat16_rn(silu_glu(v0, v1, pair_scale ? pair_scale[order[m]] : 1.f));
-          continue;
-        }
-        if (activation == kActReluSquare) {
-          v0 = fmaxf(v0, 0.f);
-          v1 = fmaxf(v1, 0.f);
-          v0 *= v0;
-          v1 *= v1;
-        }
-        *reinterpret_cast<__nv_bfloat162*>(C + (size_t)m * ldc + n) = __floats2bfloat162_rn(v0, v1);
-      }
-    }
 }
 
 // One block per token: out[n, c] = sum_k weights[n, k] * Y[place[n * top + k], c] (+ shared[n, c]), k ascending, float32.
@@ -715,24 +576,6 @@ MS_EXPORT int ms_expert_linear(const void* A, int dtype, int lda, const int* ord
              "expert_linear: a scale per pair goes with the silu-gated activation and gathered rows");
   const int row_tiles = (pairs + EBM - 1) / EBM + experts;      // every segment may end in a partial tile
   MS_REQUIRE(row_tiles <= 65535, "expert_linear: %d rows in one launch is too many", pairs);
-  if (dtype == MS_BF16 && K % 8 == 0 && N % 8 == 0 && lda % 8 == 0 && (ldc % 2 == 0 || activation >= kActClampedGlu)) {
-    // long segments (256 rows an expert on average, or more): tiles of 128 rows; else tiles of 64
-    const bool tall = pairs >= 256 * experts;
-    const int rows = tall ? 128 : 64, stages = tall ? 3 : 4;
-    dim3 mma_grid((N + GBN - 1) / GBN, (pairs + rows - 1) / rows + experts);
-    const size_t smem = sizeof(__nv_bfloat16) * stages * (rows + GBN) * (GBK + 8);
-    auto kernel = tall ? expert_linear_mma_kernel<128, 3> : expert_linear_mma_kernel<64, 4>;
-    static bool allowed[2] = {false, false};
-    if (!allowed[tall]) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) MS_FAIL("expert_linear: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
-      allowed[tall] = true;
-    }
-    ms::launch(kernel, mma_grid, 256, smem, stream, (const __nv_bfloat16*)A, lda, order, top,
-               (const __nv_bfloat16*)W, (__nv_bfloat16*)C, ldc, offsets, experts, N, K, activation, limit, pair_scale);
-    MS_CHECK_LAUNCH("expert_linear (tensor cores)");
-    return 0;
-  }
   dim3 grid((N + EBN - 1) / EBN, row_tiles);
   MS_EXP_DISPATCH(dtype, (ms::launch(expert_linear_kernel<T>, grid, 256, 0, stream, (const T*)A, lda, order, top, (const T*)W,
                                      (T*)C, ldc, offsets, experts, N, K, activation, limit, pair_scale)));

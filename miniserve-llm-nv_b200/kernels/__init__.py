@@ -1361,6 +1361,12 @@ def expert_linear(x: torch.Tensor, order: Optional[torch.Tensor], top: int, weig
         raise KernelError(f"expert_linear: x {tuple(x.shape)}, weight {tuple(weight.shape)}, out {tuple(out.shape)}")
     if order is not None:
         _want(order, "order", torch.int32, (pairs,))
+    if (x.dtype == torch.bfloat16 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and library().ms_expert_tcgen05_supports(_i(experts), _i(n), _i(k))):
+        _check(library().ms_expert_linear_tcgen05(_ptr(x), _i(k), _ptr(order), _i(top), _ptr(weight), _ptr(out), _i(out.shape[1]),
+                                                  _ptr(offsets), _i(experts), _i(pairs), _i(n), _i(k), _i(code), _f(limit),
+                                                  _ptr(pair_scale), _ptr(device_error_flag(x.device)), _stream()))
+        return
     _check(library().ms_expert_linear(_ptr(x), _i(_code(x.dtype)), _i(k), _ptr(order), _i(top), _ptr(weight), _ptr(out),
                                       _i(out.shape[1]), _ptr(offsets), _i(experts), _i(pairs), _i(n), _i(k), _i(code), _f(limit),
                                       _ptr(pair_scale), _stream()))
