@@ -819,9 +819,10 @@ def latent_prepare(proj: torch.Tensor, q_col: int, dkv_col: int, heads: int, dim
 
 def latent_attention_kernels(dtype: torch.dtype, rank: int, rot: int, heads: int, page_size: int) -> dict:
     """Which kernel :func:`latent_attention` runs for these sizes, as :func:`attention_kernels` says it for keys and
-    values: ``{"decode": name, "prompt": name}`` with ``mma.sync`` or ``general``."""
+    values: ``{"decode": name, "prompt": name}`` with ``tcgen05``, ``mma.sync`` or ``general``."""
     if dtype == torch.bfloat16 and USE_LATENT_MMA and library().ms_latent_attention_mma_supports(_i(rank), _i(rot), _i(heads)):
-        return {"decode": "mma.sync", "prompt": "mma.sync"}
+        prompt = library().ms_latent_attention_tcgen05_supports(_i(rank), _i(rot), _i(heads), _i(page_size))
+        return {"decode": "mma.sync", "prompt": "tcgen05" if prompt else "mma.sync"}
     return {"decode": "general", "prompt": "general"}
 
 
@@ -852,6 +853,13 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
     lib = library()
     page_size = cache.shape[1]
     if q_full.dtype == torch.bfloat16 and USE_LATENT_MMA and lib.ms_latent_attention_mma_supports(_i(rank), _i(dk - rank), _i(heads)):
+        if (max_query_len > 1 and lib.ms_latent_attention_tcgen05_supports(_i(rank), _i(dk - rank), _i(heads), _i(page_size))
+                and (q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0):
+            _check(lib.ms_latent_attention_tcgen05(
+                _ptr(q_full), _ptr(cache), _i(cache.shape[0]), _ptr(block_tables), _i(block_tables.shape[1]), _ptr(query_start),
+                _ptr(context_lens), _i(page_size), _i(heads), _i(rank), _i(dk - rank), _f(scale), _i(window if window else 0), _ptr(out),
+                _i(n_requests), _i(max_query_len), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
+            return
         reach = min(max_context_len, window) if window else max_context_len      # the most keys a token sees
         splits = lib.ms_latent_attention_mma_splits(_i(rank), _i(dk - rank), _i(heads), _i(n_requests), _i(max_query_len), _i(reach))
         part_o = part_lse = None

@@ -1,0 +1,59 @@
+"""Latent attention of prompt portions on the fifth-generation tensor cores, against float64: lengths around tiles of 128 rows and 64
+keys, portions that continue sequences, windows, pages smaller and larger than a tile, and stale numbers behind the context."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+STEPS = [([1, 2], [0, 0]), ([8, 1, 9], [0, 63, 64]), ([64, 65], [1, 191]), ([130], [0]), ([3, 40], [500, 0]), ([300, 1, 1], [0, 128, 700])]
+
+
+@pytest.mark.parametrize("rank,rot,heads,page", [(256, 32, 16, 64), (256, 32, 8, 16), (256, 64, 16, 128), (256, 0, 4, 8), (128, 16, 16, 32),
+                                                 (64, 48, 1, 64), (64, 64, 128, 64), (128, 32, 32, 192)])
+@pytest.mark.parametrize("new,before", STEPS)
+@pytest.mark.parametrize("window", [None, 70])
+def test_against_float64(rank, rot, heads, page, new, before, window):
+    from miniserve_b200 import kernels
+
+    g = torch.Generator(device="cuda").manual_seed(rank + heads + sum(new))
+    dk, scale, n = rank + rot, (rank + rot) ** -0.5, sum(new)
+    assert kernels.library().ms_latent_attention_tcgen05_supports(rank, rot, heads, page)
+    lens = [a + b for a, b in zip(new, before)]
+    counts = [(length + page - 1) // page for length in lens]
+    pages = torch.randperm(sum(counts), generator=g, device="cuda").to(torch.int32)
+    cache = torch.full((sum(counts), page, dk), float("nan"), device="cuda").bfloat16()      # (stale rows: nothing of them may be seen)
+    tables = torch.zeros((len(new), max(counts) + 1), dtype=torch.int32, device="cuda")
+    rows, at = [], 0
+    for r, (length, count) in enumerate(zip(lens, counts)):
+        tables[r, :count] = pages[at:at + count]
+        keys = (torch.randn((length, dk), generator=g, device="cuda") * 1.5).bfloat16()
+        keys[length // 2] *= 4                                             # (maxima that grow by more than 2^8 on the way)
+        filled = cache[pages[at:at + count].long()].reshape(count * page, dk)
+        filled[:length] = keys
+        cache[pages[at:at + count].long()] = filled.view(count, page, dk)
+        rows.append(keys.double())
+        at += count
+    q = (torch.randn((n, heads, dk), generator=g, device="cuda") * 2).bfloat16()
+    starts = [sum(new[:i]) for i in range(len(new) + 1)]
+
+    def ints(values):
+        return torch.tensor(values, dtype=torch.int32, device="cuda")
+
+    positions = ints([p for a, b in zip(new, before) for p in range(b, b + a)])
+    requests = ints([r for r, a in enumerate(new) for _ in range(a)])
+    out = torch.full((n, heads, rank), float("nan"), device="cuda").bfloat16()
+    kernels.latent_attention(q, cache, tables, requests, positions, ints(starts), ints(lens), max(new), max(lens), rank, scale, window, out)
+    kernels.check_device_errors(q.device)
+    for r, (a, b) in enumerate(zip(new, before)):
+        here, keys = q[starts[r]:starts[r + 1]].double(), rows[r]
+        scores = torch.einsum("thd,kd->htk", here, keys) * scale
+        key, token = torch.arange(a + b, device="cuda")[None, :], (b + torch.arange(a, device="cuda"))[:, None]
+        seen = (key <= token) & (key > token - (window or 1 << 30))
+        p = torch.softmax(scores.masked_fill(~seen, -torch.inf), dim=-1)
+        want = torch.einsum("htk,kd->thd", p, keys[:, :rank])
+        # probabilities rounded to bfloat16 (2^-9 of each) and the result once more: 2^-8 of the sums of magnitudes, and scores in
+        # float32, whose errors (dk 2^-23 of their magnitudes) enter the exponent
+        size = torch.einsum("htk,kd->thd", p, keys[:, :rank].abs())
+        slack = dk * 2.0 ** -23 * float((here.abs().amax() * keys.abs().amax() * dk * scale))
+        assert torch.all((out[starts[r]:starts[r + 1]].double() - want).abs() <= (2.0 ** -7 + slack) * size + 1e-6)
