@@ -861,6 +861,18 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
                 _i(n_requests), _i(max_query_len), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
             return
         reach = min(max_context_len, window) if window else max_context_len      # the most keys a token sees
+        if max_query_len == 1 and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
+                q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
+            splits = lib.ms_latent_decode_splits(_i(heads), _i(n_requests), _i(reach))
+            part_o = part_lse = None
+            if splits > 1:
+                part_o = torch.empty((n * heads * splits, rank), dtype=torch.float32, device=q_full.device)
+                part_lse = torch.empty((n * heads * splits,), dtype=torch.float32, device=q_full.device)
+            _check(lib.ms_latent_decode(
+                _ptr(q_full), _ptr(cache), _ptr(block_tables), _i(block_tables.shape[1]), _ptr(query_start), _ptr(context_lens),
+                _i(page_size), _i(heads), _i(rank), _i(dk - rank), _f(scale), _i(window if window else 0), _ptr(out), _ptr(part_o),
+                _ptr(part_lse), _i(splits), _i(n_requests), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
+            return
         splits = lib.ms_latent_attention_mma_splits(_i(rank), _i(dk - rank), _i(heads), _i(n_requests), _i(max_query_len), _i(reach))
         part_o = part_lse = None
         if splits > 1:

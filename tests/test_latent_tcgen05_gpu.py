@@ -1,5 +1,5 @@
-"""Latent attention of prompt portions on the fifth-generation tensor cores, against float64: lengths around tiles of 128 rows and 64
-keys, portions that continue sequences, windows, pages smaller and larger than a tile, and stale numbers behind the context."""
+"""Latent attention of prompt portions on the fifth-generation tensor cores, and of decode steps, against float64: lengths around tiles of
+128 rows and 64 keys, around pieces of 16 keys, portions that continue sequences, windows, pages smaller and larger than a tile, and stale numbers behind the context."""
 
 import pytest
 import torch
@@ -7,11 +7,12 @@ import torch
 pytestmark = pytest.mark.gpu
 
 STEPS = [([1, 2], [0, 0]), ([8, 1, 9], [0, 63, 64]), ([64, 65], [1, 191]), ([130], [0]), ([3, 40], [500, 0]), ([300, 1, 1], [0, 128, 700])]
+DECODE = [([1] * 6, [0, 15, 16, 63, 64, 65]), ([1], [5000]), ([1, 1, 1], [700, 2047, 191])]
 
 
 @pytest.mark.parametrize("rank,rot,heads,page", [(256, 32, 16, 64), (256, 32, 8, 16), (256, 64, 16, 128), (256, 0, 4, 8), (128, 16, 16, 32),
                                                  (64, 48, 1, 64), (64, 64, 128, 64), (128, 32, 32, 192)])
-@pytest.mark.parametrize("new,before", STEPS)
+@pytest.mark.parametrize("new,before", STEPS + DECODE)
 @pytest.mark.parametrize("window", [None, 70])
 def test_against_float64(rank, rot, heads, page, new, before, window):
     from miniserve_b200 import kernels
