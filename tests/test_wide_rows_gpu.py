@@ -143,3 +143,24 @@ def test_expert_combine(dtype, identity, n, top, width, weighted, shared):
     if shared:
         want = want + torch.sigmoid(gate[:, 1:2].double()) * own.double()
     assert close(out, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,rot,rank", [(1, 8, 16, 8), (16, 64, 32, 256), (3, 16, 64, 264), (8, 8, 48, 1024)])
+def test_latent_prepare_and_head_gate(dtype, heads, dim, rot, rank):
+    from miniserve_b200 import kernels
+
+    n = 7
+    proj = rand((n, heads * (dim + rot) + rank + rot + 8), dtype, 21)
+    slots, weight = ints([3, 0, -1, 9, 5, 6, 1]), rand((rank,), dtype, 22)
+    table = rand((n, rot // 2, 2), torch.float32, 23)
+    cache, q = rand((10, rank + rot), dtype, 24), rand((n, heads, rank + rot), dtype, 25)
+    want_cache, want_q = cache.cpu(), q.cpu()
+    args = (0, heads * (dim + rot), heads, dim, rot, rank)
+    plain_ops.latent_prepare(proj.cpu(), *args, slots.cpu(), weight.cpu(), 1e-5, table.cpu(), rot, want_cache, want_q)
+    kernels.latent_prepare(proj, *args, slots, weight, 1e-5, table, rot, cache.view(1, 10, rank + rot), q)
+    assert close(cache, want_cache, dtype) and close(q, want_q, dtype)
+    x, gate = rand((n, heads, dim), dtype, 26), rand((n, heads + 3), dtype, 27, 2.0)
+    want = x.double() * torch.sigmoid(gate[:, 2:2 + heads].double())[:, :, None]
+    kernels.head_gate(x, gate, 2)
+    assert close(x, want, dtype)
