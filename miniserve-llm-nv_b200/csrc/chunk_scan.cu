@@ -18,8 +18,8 @@
 //     carry_kernel   the chunks in order, sixteen columns of S a block: u, S_end; S_0 of every chunk
 //     read_kernel    y, with u for v
 //
-// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 120 us; selective,
-// 64 heads of 128 x 64, 2,048 tokens 496 -> 231 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 243 us.
+// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 110 us; selective,
+// 64 heads of 128 x 64, 2,048 tokens 496 -> 202 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 237 us.
 //
 // All arithmetic is float32 on float32 copies of the projections.  A token's result uses nothing of the tokens behind it (what is
 // masked is not multiplied: a zero would turn an infinity behind it into a NaN before it).
@@ -48,7 +48,7 @@ struct Problem {
   long long state_stride;
   int state_offset;
   const int *state_slots, *query_start;
-  int most;                                              // chunks of the longest portion: blockIdx.z = request * most + chunk
+  int requests, most;                                    // most: chunks of the longest portion: blockIdx.z = request * most + chunk
   float *chunk_states, *chunk_decays;                    // [places][heads][columns][dim], [places][heads]
   float *y, *bottom;
 };
@@ -64,6 +64,35 @@ __device__ __forceinline__ Where where_of(const Problem& p) {
   // (places of different requests do not meet: a portion of n tokens has at most one chunk more than it holds borders of 64
   // tokens counted from the step's first token)
   w.place = (size_t)(first / kC + w.request + c);
+  return w;
+}
+
+// The same for the c-th chunk of all portions, looked up by a whole warp; `count` is how many chunks there are (c beyond them: only that).
+__device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
+  const int lane = threadIdx.x & 31;
+  Where w = {};
+  count = 0;
+  for (int r0 = 0; r0 < p.requests; r0 += 32) {
+    int first = 0, tokens = 0;
+    if (r0 + lane < p.requests) first = p.query_start[r0 + lane], tokens = p.query_start[r0 + lane + 1] - first;
+    const int chunks = tokens > 0 ? (tokens + kC - 1) / kC : 0;
+    int upto = chunks;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const int before = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += before;
+    }
+    const unsigned found = __ballot_sync(0xffffffffu, count + upto > c);
+    if (found) {
+      const int at = __ffs(found) - 1;
+      first = __shfl_sync(0xffffffffu, first, at), tokens = __shfl_sync(0xffffffffu, tokens, at);
+      const int mine = c - count - __shfl_sync(0xffffffffu, upto - chunks, at);
+      w.request = r0 + at, w.left = tokens - mine * kC, w.len = min(w.left, kC), w.first = first + mine * kC;
+      w.place = (size_t)(first / kC + w.request + mine);
+      return w;
+    }
+    count += __shfl_sync(0xffffffffu, upto, 31);
+  }
   return w;
 }
 
@@ -157,15 +186,17 @@ __device__ __forceinline__ float both(unsigned long long two) {
   return a + b;
 }
 
-// G_t, the product of a chunk's decays up to token t, into every g[t] (64 threads).  Products of decays are formed in double precision and
-// rounded once: their errors would be the same for a whole row of scores, where the walk's fall on each number of S alone (float32
-// products left the delta form's state 1.6 times as far from the definition as the walk's).
-__device__ __forceinline__ void prefix_products(const double* keep, float* g, int t) {
-  double p = 1.0;
-#pragma unroll 8
-  for (int r = 0; r < kC; ++r)
-    if (r <= t) p *= keep[r];
-  g[t] = (float)p;
+// The product of a chunk's decays of tokens first <= r < end, as four chains of sixteen.  Products of decays are formed in double
+// precision and rounded once: their errors would be the same for a whole row of scores, where the walk's fall on each number of S
+// alone (float32 products left the delta form's state 1.6 times as far from the definition as the walk's).
+__device__ __forceinline__ double decay_between(const double* keep, int first, int end) {
+  double p[4] = {1.0, 1.0, 1.0, 1.0};
+#pragma unroll
+  for (int r = 0; r < 16; ++r)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (16 * b + r >= first && 16 * b + r < end) p[b] *= keep[16 * b + r];
+  return (p[0] * p[1]) * (p[2] * p[3]);
 }
 
 // ------------------------------------------------------------------------------------------------- a chunk's own matrix
@@ -193,10 +224,7 @@ local_kernel(const Problem p) {
   if (tid < kC) keep[tid] = gate.x;
   __syncthreads();
   if (tid < kC) {
-    double after = 1.0;                        // the decays behind the token
-#pragma unroll 8
-    for (int r = kC - 1; r > 0; --r)
-      if (r > tid) after *= keep[r];
+    const double after = decay_between(keep, tid + 1, kC);         // the decays behind the token
     weight[tid] = tid < w.len ? gate.y * (float)after : 0.f;
     if (tid == 0 && blockIdx.x == 0) p.chunk_decays[w.place * p.heads + head] = (float)(after * keep[0]);
   }
@@ -300,8 +328,11 @@ join_kernel(const Problem p) {
 }
 
 // ------------------------------------------------------------------------------------------------------- the rows of y
-// grid (value tiles, heads, chunks).  Bound by its multiply-adds: q k^T below the diagonal, scores times values, q S_0, which arrives
-// in the keys' place while the values are summed.
+// Two blocks a multiprocessor, each with a run of the work's units: 64 value columns of a head and a chunk.  Units that share their
+// queries and keys (a head's value tiles, the heads of a group) are neighbours, so that a block loads those and forms q k^T, which it
+// keeps in registers, once for several units, and the next unit's values and gates are on their way during the last product.  Bound by
+// its multiply-adds: q k^T below the diagonal, scores times values, q S_0, which arrives in the keys' place while the values are summed.
+// (A block per unit took 151, 79 and 80 us for the selective, memory and delta workloads at the top of this file, this 122, 72 and 77.)
 // (neighbouring threads have every fourth column of S_0: those lie in neighbouring rows)
 __device__ __forceinline__ int place_of_column(int c) { return (c & 32) + (c & 3) * 8 + ((c >> 2) & 7); }
 
@@ -310,8 +341,6 @@ __global__ void __launch_bounds__(kThreads, 2)
 read_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
-  const Where w = where_of(p);
-  if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* qs = chunk_smem;                     // [64][NP + 4]
   float* ks = qs + kC * (NP + 4);             // [64][NP + 4], then S_0, value column c in row place_of_column(c)
@@ -321,144 +350,229 @@ read_kernel(const Problem p) {
   float* weight = reinterpret_cast<float*>(keep + kC);
   float* decayed = weight + kC;               // G_t
   float* n0 = decayed + kC;                   // [NP] (memory form)
-  const int tid = threadIdx.x, head = blockIdx.y, kv_head = head / (p.heads / p.kv_heads), first_column = blockIdx.x * kTile;
-  const T* q = reinterpret_cast<const T*>(p.q.at) + (size_t)w.first * p.q.ld + p.q.col + kv_head * p.dim;
-  const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
-  const V* v = reinterpret_cast<const V*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim + first_column;
-  const float* start = p.chunk_states + (w.place * p.heads + head) * (size_t)p.columns * p.dim;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = lane & 7, ty = lane >> 3;
+  const int tiles = (p.vdim + kTile - 1) / kTile, per_group = p.heads / p.kv_heads;
   const bool four_wide = p.dim % 4 == 0;
-  float2 gate = make_float2(1.f, 0.f);
-  if (tid < w.len) gate = gate_of<FORM>(p, w.first + tid, head);
-  load_rows<T, NP>(qs, NP + 4, q, p.q.ld, w.len, p.dim, p.wide, p.input_act);
-  load_rows<T, NP>(ks, NP + 4, k, p.k.ld, w.len, p.dim, p.wide, p.input_act);
-  load_rows<V, kTile>(vs, kLd, v, p.v.ld, w.len, p.vdim - first_column, p.wide, p.input_act);
-  if (tid < kC) {
-    keep[tid] = gate.x;
-    weight[tid] = FORM == kDelta ? 1.f : gate.y;
-  }
-  if (FORM == kMemory && tid < NP) n0[tid] = tid < p.dim ? start[(size_t)p.vdim * p.dim + tid] : 0.f;
-  __syncthreads();
+  int count;
+  chunk_of(p, 0x7fffffff, count);
+  const long long units = (long long)count * p.heads * tiles;
+  const long long last = units * (blockIdx.x + 1) / gridDim.x;
+  long long unit = units * blockIdx.x / gridDim.x;
+  if (unit >= last) return;
+  // the unit's place: value tile, head, chunk
+  int tile, head, chunk;
   {
-    // scores[t][s] = D(t, s) w_s: a thread has column s and sixteen rows
-    const int s = tid & (kC - 1), t0 = (tid >> 6) * 16;
-    double product = 1.0;
-#pragma unroll 8
-    for (int r = 0; r < t0; ++r)
-      if (r > s) product *= keep[r];
-    const float mine = weight[s];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      if (t0 + r > s) product *= keep[t0 + r];
-      scores[(t0 + r) * kLd + s] = (float)product * mine;
-    }
-    if (tid < kC) prefix_products(keep, decayed, tid);
+    const long long rest = unit / tiles;
+    tile = (int)(unit % tiles), head = (int)(rest % p.heads), chunk = (int)(rest / p.heads);
   }
-  __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31, tx = lane & 7, ty = lane >> 3;
-  const Tile tile = score_tile(warp);
-  if (tile.row0 < w.len) {
-    unsigned long long acc[4][4];
-    dot_tile<NP>(qs, ks, tile.row0, tile.column0, tile.blocks, tx, ty, acc);
+  Where w = chunk_of(p, chunk, count);
+  // values: float32 ones that nothing is done to by asynchronous copies, 16-bit ones through registers, others when their unit begins
+  constexpr bool kCopied = sizeof(V) == 4;
+  constexpr int kPieces = kC * kTile * (int)sizeof(V) / 16 / kThreads, kEach = 16 / (int)sizeof(V), kPerRow = kTile / kEach;
+  uint4 ahead[kCopied ? 1 : kPieces];
+  auto request_values = [&]() {
+    const int first_column = tile * kTile;
+    const V* v = reinterpret_cast<const V*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim + first_column;
+    if (p.wide && !(kCopied && p.input_act)) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j >= tile.blocks) continue;
-        float* at = scores + (tile.row0 + ty + 4 * i) * kLd + tile.column0 + tx + 8 * j;
-        *at *= p.q_scale * both(acc[i][j]);                            // (s > t is never read)
+      for (int i = 0; i < kPieces; ++i) {
+        const int t = (tid + i * kThreads) / kPerRow, c = (tid + i * kThreads) % kPerRow * kEach;
+        const bool real = t < w.len && first_column + c < p.vdim;
+        if constexpr (kCopied) cp_async_16(vs + t * kLd + c, v + (real ? (size_t)t * p.v.ld + c : 0), real);
+        else ahead[i] = real ? *reinterpret_cast<const uint4*>(v + (size_t)t * p.v.ld + c) : make_uint4(0u, 0u, 0u, 0u);
       }
-  }
-  __syncthreads();                            // the scores are there, the keys have been read
-  if (four_wide) {
-    for (int i = tid; i < kTile * (NP / 4); i += kThreads) {
-      const int c = i / (NP / 4), n = i % (NP / 4) * 4;
-      const bool real = first_column + c < p.vdim && n < p.dim;
-      cp_async_16(ks + place_of_column(c) * (NP + 4) + n, start + (real ? (size_t)(first_column + c) * p.dim + n : 0), real);
     }
-  } else {
-    for (int i = tid; i < kTile * NP; i += kThreads) {
-      const int c = i / NP, n = i % NP;
-      ks[place_of_column(c) * (NP + 4) + n] = first_column + c < p.vdim && n < p.dim ? start[(size_t)(first_column + c) * p.dim + n] : 0.f;
+    cp_async_commit();
+  };
+  auto place_values = [&]() {
+    if (!p.wide || (kCopied && p.input_act)) {
+      const int first_column = tile * kTile;
+      const V* v = reinterpret_cast<const V*>(p.v.at) + (size_t)w.first * p.v.ld + p.v.col + (size_t)head * p.vdim + first_column;
+      load_rows<V, kTile>(vs, kLd, v, p.v.ld, w.len, p.vdim - first_column, p.wide, p.input_act);
+    } else if constexpr (!kCopied) {
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        const int t = (tid + i * kThreads) / kPerRow, c = (tid + i * kThreads) % kPerRow * kEach;
+        const V* from = reinterpret_cast<const V*>(&ahead[i]);
+#pragma unroll
+        for (int e = 0; e < kEach; e += 4) {
+          float4 four = make_float4(to_float(from[e]), to_float(from[e + 1]), to_float(from[e + 2]), to_float(from[e + 3]));
+          if (p.input_act) four = make_float4(silu_of(four.x), silu_of(four.y), silu_of(four.z), silu_of(four.w));
+          *reinterpret_cast<float4*>(vs + t * kLd + c + e) = four;
+        }
+      }
     }
-  }
-  cp_async_commit();
-  // results: 16 tokens and 32 value columns a warp, four neighbouring columns a thread; the two warps of a scheduler have 80 tokens' scores
+  };
+  auto gates_of = [&]() { return tid < w.len ? gate_of<FORM>(p, w.first + tid, head) : make_float2(1.f, 0.f); };
+  request_values();
+  float2 gate = gates_of();
+  float raw[4][4];                            // q k^T of the warp's tile
+  const Tile own = score_tile(warp);
   const int half = warp >> 2, row0 = 16 * (half ? 3 - (warp & 3) : warp & 3);
-  const bool busy = row0 < w.len;
-  unsigned long long out[4][2];
+  bool new_keys = true, new_head = true;
+  for (;; ++unit) {
+    __syncthreads();                          // the unit before has been read
+    if (new_keys) {
+      const int kv_head = head / per_group;
+      const T* q = reinterpret_cast<const T*>(p.q.at) + (size_t)w.first * p.q.ld + p.q.col + kv_head * p.dim;
+      const T* k = reinterpret_cast<const T*>(p.k.at) + (size_t)w.first * p.k.ld + p.k.col + kv_head * p.dim;
+      load_rows<T, NP>(qs, NP + 4, q, p.q.ld, w.len, p.dim, p.wide, p.input_act);
+      load_rows<T, NP>(ks, NP + 4, k, p.k.ld, w.len, p.dim, p.wide, p.input_act);
+      __syncthreads();
+      if (own.row0 < w.len) {
+        unsigned long long acc[4][4];
+        dot_tile<NP>(qs, ks, own.row0, own.column0, own.blocks, tx, ty, acc);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) out[i][0] = out[i][1] = 0ull;
-  const float* my_scores = scores + (row0 + ty) * kLd;
-  const float* my_values = vs + 32 * half + 4 * tx;
-  if (busy) {
-    for (int s = 0; s < row0; s += 4) {
-      float4 row[4];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) row[i] = *reinterpret_cast<const float4*>(my_scores + 4 * i * kLd + s);
+          for (int j = 0; j < 4; ++j) raw[i][j] = p.q_scale * both(acc[i][j]);
+      }
+      __syncthreads();                        // the keys have been read
+    }
+    const int first_column = tile * kTile;
+    const float* start = p.chunk_states + (w.place * p.heads + head) * (size_t)p.columns * p.dim;
+    place_values();
+    if (four_wide) {
+      for (int i = tid; i < kTile * (NP / 4); i += kThreads) {
+        const int c = i / (NP / 4), n = i % (NP / 4) * 4;
+        const bool real = first_column + c < p.vdim && n < p.dim;
+        cp_async_16(ks + place_of_column(c) * (NP + 4) + n, start + (real ? (size_t)(first_column + c) * p.dim + n : 0), real);
+      }
+    } else {
+      for (int i = tid; i < kTile * NP; i += kThreads) {
+        const int c = i / NP, n = i % NP;
+        ks[place_of_column(c) * (NP + 4) + n] = first_column + c < p.vdim && n < p.dim ? start[(size_t)(first_column + c) * p.dim + n] : 0.f;
+      }
+    }
+    cp_async_commit();
+    if (FORM == kMemory && tile == 0 && tid < NP) n0[tid] = tid < p.dim ? start[(size_t)p.vdim * p.dim + tid] : 0.f;
+    if (new_head) {
+      if (tid < kC) {
+        keep[tid] = gate.x;
+        weight[tid] = FORM == kDelta ? 1.f : gate.y;
+      }
+      __syncthreads();
+      // scores[t][s] = D(t, s) w_s: a thread has column s and sixteen rows
+      const int s = tid & (kC - 1), t0 = (tid >> 6) * 16;
+      double product = decay_between(keep, s + 1, t0);
+      const float mine = weight[s];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (s + u) * kLd);
+      for (int r = 0; r < 16; ++r) {
+        if (t0 + r > s) product *= keep[t0 + r];
+        scores[(t0 + r) * kLd + s] = (float)product * mine;
+      }
+      if (tid < kC) decayed[tid] = (float)decay_between(keep, 0, tid + 1);
+      __syncthreads();
+      if (own.row0 < w.len) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < own.blocks) scores[(own.row0 + ty + 4 * i) * kLd + own.column0 + tx + 8 * j] *= raw[i][j];        // (s > t is never read)
+      }
+    }
+    cp_async_wait<1>();
+    __syncthreads();                          // values and scores are there
+    // results: 16 tokens and 32 value columns a warp, four neighbouring columns a thread; the two warps of a scheduler have 80 tokens' scores
+    const bool busy = row0 < w.len;
+    unsigned long long out[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i][0] = out[i][1] = 0ull;
+    const float* my_scores = scores + (row0 + ty) * kLd;
+    const float* my_values = vs + 32 * half + 4 * tx;
+    if (busy) {
+      for (int s = 0; s < row0; s += 4) {
+        float4 row[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) row[i] = *reinterpret_cast<const float4*>(my_scores + 4 * i * kLd + s);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (s + u) * kLd);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float f = u == 0 ? row[i].x : u == 1 ? row[i].y : u == 2 ? row[i].z : row[i].w;
+            out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
+            out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {            // the tile's own tokens: each row up to itself
+        const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (row0 + u) * kLd);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (u <= ty + 4 * i) {
+            const float f = my_scores[4 * i * kLd + row0 + u];
+            out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
+            out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+          }
+      }
+      if (FORM == kSelective) {
+        const float skip = p.skip[head];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float f = u == 0 ? row[i].x : u == 1 ? row[i].y : u == 2 ? row[i].z : row[i].w;
-          out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
-          out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+          const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (row0 + ty + 4 * i) * kLd);
+          out[i][0] = fma2(pack2(skip, skip), value.x, out[i][0]);
+          out[i][1] = fma2(pack2(skip, skip), value.y, out[i][1]);
         }
       }
     }
+    if (FORM == kMemory && tile == 0) {
+      for (int t = 8 * warp; t < min(8 * warp + 8, w.len); ++t) {
+        float sum = 0.f, read = 0.f;
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {              // the tile's own tokens: each row up to itself
-      const ulonglong2 value = *reinterpret_cast<const ulonglong2*>(my_values + (row0 + u) * kLd);
+        for (int s = lane; s < kC; s += 32)
+          if (s <= t) sum += scores[t * kLd + s];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (u <= ty + 4 * i) {
-          const float f = my_scores[4 * i * kLd + row0 + u];
-          out[i][0] = fma2(pack2(f, f), value.x, out[i][0]);
-          out[i][1] = fma2(pack2(f, f), value.y, out[i][1]);
+        for (int n = lane; n < NP; n += 32) read += qs[t * (NP + 4) + n] * n0[n];
+        const float total = warp_sum(sum + decayed[t] * p.q_scale * read);
+        const size_t at = (size_t)(w.first + t) * p.heads + head;
+        if (lane == 0) p.bottom[at] = fmaxf(fabsf(total), p.gates[at * 3 + 2]) + 1e-6f;
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();                          // S_0 is there, values and scores have been read
+    const int my_head = head, my_len = w.len, column = first_column + 32 * half + 4 * tx;
+    float* at = p.y + ((size_t)(w.first + row0 + ty) * p.heads + my_head) * p.vdim + column;
+    const bool more = unit + 1 < last;
+    if (more) {                               // the next unit
+      new_keys = new_head = false;
+      if (++tile == tiles) {
+        tile = 0;
+        new_head = true;
+        if (++head == p.heads) {
+          head = 0;
+          w = chunk_of(p, ++chunk, count);
         }
+        new_keys = head % per_group == 0;
+      }
+      request_values();
+      if (new_head) gate = gates_of();
     }
-  }
-  if (FORM == kMemory && blockIdx.x == 0) {
-    for (int t = 8 * warp; t < min(8 * warp + 8, w.len); ++t) {
-      float sum = 0.f, read = 0.f;
+    if (busy) {
+      unsigned long long acc[4][4];
+      dot_tile<NP>(qs, ks, row0, 32 * half, 4, tx, ty, acc);
 #pragma unroll
-      for (int s = lane; s < kC; s += 32)
-        if (s <= t) sum += scores[t * kLd + s];
+      for (int i = 0; i < 4; ++i) {
+        const int t = row0 + ty + 4 * i;
+        if (t >= my_len) continue;
+        const float factor = p.q_scale * decayed[t];
+        float e[4];
+        unpack2(out[i][0], e[0], e[1]);
+        unpack2(out[i][1], e[2], e[3]);
 #pragma unroll
-      for (int n = lane; n < NP; n += 32) read += qs[t * (NP + 4) + n] * n0[n];
-      const float total = warp_sum(sum + decayed[t] * p.q_scale * read);
-      const size_t at = (size_t)(w.first + t) * p.heads + head;
-      if (lane == 0) p.bottom[at] = fmaxf(fabsf(total), p.gates[at * 3 + 2]) + 1e-6f;
+        for (int j = 0; j < 4; ++j) e[j] += factor * both(acc[i][j]);
+        float* row = at + (size_t)(4 * i) * p.heads * p.vdim;
+        if (p.vdim % 4 == 0) {
+          if (column < p.vdim) *reinterpret_cast<float4*>(row) = make_float4(e[0], e[1], e[2], e[3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (column + j < p.vdim) row[j] = e[j];
+        }
+      }
     }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-  if (!busy) return;
-  unsigned long long acc[4][4];
-  dot_tile<NP>(qs, ks, row0, 32 * half, 4, tx, ty, acc);
-  const float skip = FORM == kSelective ? p.skip[head] : 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = row0 + ty + 4 * i;
-    if (t >= w.len) continue;
-    const float factor = p.q_scale * decayed[t];
-    float e[4];
-    unpack2(out[i][0], e[0], e[1]);
-    unpack2(out[i][1], e[2], e[3]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      e[j] += factor * both(acc[i][j]);
-      if (FORM == kSelective) e[j] += skip * my_values[t * kLd + j];
-    }
-    const int column = first_column + 32 * half + 4 * tx;
-    float* at = p.y + ((size_t)(w.first + t) * p.heads + head) * p.vdim + column;
-    if (p.vdim % 4 == 0) {
-      if (column < p.vdim) *reinterpret_cast<float4*>(at) = make_float4(e[0], e[1], e[2], e[3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (column + j < p.vdim) at[j] = e[j];
-    }
+    if (!more) return;
   }
 }
 
@@ -496,10 +610,7 @@ solve_kernel(const Problem p, const Solved out) {
   {
     // a[s][t] = beta_t D(t, s): a thread has row t and sixteen s, the latest first
     const int t = tid & (kC - 1), s0 = (tid >> 6) * 16;
-    double product = 1.0;
-#pragma unroll 8
-    for (int r = kC - 1; r > s0 + 15; --r)
-      if (r <= t) product *= keep[r];
+    double product = decay_between(keep, s0 + 16, t + 1);
     const float mine = beta[t];
 #pragma unroll
     for (int r = 15; r >= 0; --r) {
@@ -507,14 +618,8 @@ solve_kernel(const Problem p, const Solved out) {
       if (s0 + r <= t) product *= keep[s0 + r];
     }
     if (tid < kC) {
-      double upto = 1.0, behind = 1.0;
-#pragma unroll 8
-      for (int r = 0; r < kC; ++r)
-        if (r <= tid) upto *= keep[r];
-      factor[tid] = beta[tid] * (float)upto;
-#pragma unroll 8
-      for (int r = kC - 1; r > 0; --r)
-        if (r > tid) behind *= keep[r];
+      factor[tid] = beta[tid] * (float)decay_between(keep, 0, tid + 1);
+      const double behind = decay_between(keep, tid + 1, kC);
       after[tid] = (float)behind;
       if (tid == 0 && blockIdx.x == 0) p.chunk_decays[w.place * p.heads + head] = (float)(behind * keep[0]);
     }
@@ -817,6 +922,10 @@ template <typename T, int FORM, int NP>
 static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
   const int tiles = (p.vdim + kTile - 1) / kTile;
   const dim3 grid(tiles, p.heads, n_requests * p.most);
+  const long long units = (long long)tiles * p.heads * n_requests * p.most;            // at most
+  int device = 0, sms = 148;
+  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  const dim3 readers((unsigned)min(units, 2ll * sms));
   if constexpr (FORM == kDelta) {
     auto solve = solve_kernel<T, NP>;
     auto carry = carry_kernel<NP>;
@@ -831,7 +940,7 @@ static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStre
     Problem reading = p;
     reading.v = Rows{solved.u, p.heads * p.vdim, 0};
     if (p.vdim % 4) reading.wide = 0;
-    ms::launch(read, grid, kThreads, read_bytes(NP), stream, reading);
+    ms::launch(read, readers, kThreads, read_bytes(NP), stream, reading);
   } else {
     auto local = local_kernel<T, FORM, NP>;
     auto read = read_kernel<T, T, FORM, NP>;
@@ -842,7 +951,7 @@ static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStre
     const size_t threads = (size_t)p.heads * p.columns * p.dim / (four ? 4 : 1);
     ms::launch(four ? join_kernel<4> : join_kernel<1>, dim3((unsigned)((threads + 255) / 256), n_requests), 256, 0, stream, p);
     MS_CHECK_LAUNCH("chunk_scan: chunks joined");
-    ms::launch(read, grid, kThreads, read_bytes(NP), stream, p);
+    ms::launch(read, readers, kThreads, read_bytes(NP), stream, p);
   }
   MS_CHECK_LAUNCH("chunk_scan: rows");
   return 0;
@@ -902,7 +1011,7 @@ MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const 
   p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim, p.columns = form == kMemory ? vdim + 1 : vdim;
   p.input_act = input_act, p.wide = wide, p.q_scale = q_scale, p.gates = gates;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
-  p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
+  p.requests = n_requests, p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
   const Solved solved{w, u, ke};
   if (dtype == MS_F32) return scan_form<float>(form, p, n_requests, solved, stream);
   if (dtype == MS_BF16) return scan_form<__nv_bfloat16>(form, p, n_requests, solved, stream);
@@ -931,6 +1040,6 @@ MS_EXPORT int ms_selective_chunk_scan(const float* conv, int conv_ld, const void
   p.q_scale = 1.f;
   p.step = proj, p.step_dtype = dtype, p.step_ld = ld, p.step_col = dt_col, p.step_bias = dt_bias, p.a_log = a_log, p.skip = d;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
-  p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
+  p.requests = n_requests, p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
   return scan_keys<float, kSelective>(p, n_requests, Solved{}, stream);
 }

@@ -106,6 +106,23 @@ def test_matrix_scan_in_chunks(form, dtype, heads, kv_heads, dim, vdim, lengths)
     assert torch.equal(states[untouched], start[untouched]) and torch.equal(states[:, :5], start[:, :5]) and torch.equal(states[:, -2:], start[:, -2:])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["memory", "delta", "decay"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(20, 5, 128, 136), (21, 7, 40, 130), (16, 16, 64, 64)])
+def test_a_block_reads_several_tiles_heads_chunks_and_requests(form, dtype, heads, kv_heads, dim, vdim):
+    """More than two blocks a multiprocessor have work for, of more requests than a warp has lanes, some without tokens: the walk's rows.
+    (Either way is within 2e-5 of the definition, see above: 4e-5 apart.)"""
+    lengths = [1, 0, 65, 3, 130] * 7 + [0, 0, 200, 64]
+    rows, cols, gates, slots, states, kv_heads, columns = problem(form, dtype, lengths, heads, kv_heads, dim, vdim, 11 + dim)
+    options = dict(input_activation="silu") if form == "decay" else {}
+    walked = states.clone()
+    y, bottom = run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, vdim, **options)
+    y_walk, bottom_walk = run(form, rows, cols, gates, slots, walked, lengths, heads, kv_heads, dim, vdim, chunk=0, **options)
+    pairs = [(y, y_walk), (states, walked)] + ([(bottom, bottom_walk)] if form == "memory" else [])
+    scale = max(1.0, float(y_walk.abs().max()))
+    assert all(float((a.double() - b.double()).abs().max()) <= 4e-5 * scale for a, b in pairs)
+
+
 @pytest.mark.parametrize("heads,P,N,G", [(4, 64, 128, 2), (3, 64, 64, 1), (2, 40, 24, 2), (2, 130, 100, 1), (1, 3, 7, 1)])
 @pytest.mark.parametrize("lengths", LENGTHS)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
