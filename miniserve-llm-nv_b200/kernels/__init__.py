@@ -781,7 +781,7 @@ def decode_attention_fused(qkv: torch.Tensor, slots: torch.Tensor, q_weight: Opt
         _ptr(qkv), _ptr(slots), _ptr(q_weight), _ptr(k_weight), _i(weight_code), _f(eps), _ptr(cos_sin), _ptr(k_pool),
         _ptr(v_pool), _ptr(block_tables), _i(block_tables.shape[1]), _ptr(query_start), _ptr(context_lens),
         _i(k_pool.shape[2]), _i(n_q), _i(n_kv), _i(head_dim), _f(scale), _i(window if window else 0), _ptr(out),
-        _ptr(part_o), _ptr(part_lse), _i(splits), _i(n), _stream()))
+        _ptr(part_o), _ptr(part_lse), _i(splits), _i(n), _i(k_pool.shape[0]), _ptr(device_error_flag(qkv.device)), _stream()))
 
 
 
