@@ -17,6 +17,9 @@
 // blockIdx.z whose partial results (float32, with the base-2 logarithm of their sums) the shared merge kernel adds.
 // In both, shared-memory rows are D_K + 8 elements apart, which puts the eight rows of an ldmatrix into eight different
 // bank groups for every D_K that is a multiple of 16, and a key row's page is looked up once per tile at most.
+//
+// They serve the sizes that attention_latent_tcgen05.cu (prompts) and attention_latent_decode.cu (single tokens) do not take: latents
+// of 96 and 512, numbers of heads or page sizes that a tile of 128 rows or 64 keys does not fit, other rotated parts.
 #include "common.cuh"
 #include "mma_common.cuh"
 
