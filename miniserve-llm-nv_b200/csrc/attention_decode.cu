@@ -16,7 +16,8 @@
 //   - where a tile of keys lies within a page (page sizes that are multiples of it), one TMA copy brings its keys and one its
 //     values.  A block is one warp, and what it has to issue, not the memory, sets its pace: sixteen bytes a copy are 64
 //     instructions a lane for a tile of 32 keys, each with an address (that path stays for other page sizes).  8 requests of
-//     1,777 to 4,096 tokens with 8 key/value heads of 128 (109 MB): 26.7 us that way, 24.0 here (a bulk copy a row: 36).
+//     1,777 to 4,096 tokens with 8 key/value heads of 128 (109 MB): 26.7 us that way, 24.0 so (a bulk copy a row: 36),
+//     22.7 since the heads are normed four at a time, their loads one trip to memory.
 // Arithmetic as in the separate kernels: float32 norm and rotation rounded once to bfloat16, float32 scores
 // and softmax, P rounded to bfloat16 for PV.
 #include "mma_common.cuh"
@@ -33,12 +34,25 @@ constexpr int ROWS = 16;           // query rows of a block's MMA tile: the grou
 template <int D> __host__ __device__ constexpr int per_lane() { return D / 64; }
 
 // Norm (optional) and half-split rotation (optional) of one head of D numbers spread over the warp: lane l
-// holds elements l * E .. l * E + E - 1 in lo[] and the same of the second half in hi[].
+// holds elements l * E .. l * E + E - 1 in lo[] and the same of the second half in hi[], and the like pieces of the weight and
+// of the token's (cos, sin).
 template <int D>
-__device__ __forceinline__ void norm_and_rotate(float (&lo)[per_lane<D>()], float (&hi)[per_lane<D>()], const void* weight,
-                                                int weight_dtype, float eps, const float* cos_sin_row, int lane) {
+struct HeadWeights {
+  float lo[per_lane<D>()], hi[per_lane<D>()];
+  __device__ __forceinline__ void load(const void* weight, int dtype, int lane) {
+    constexpr int E = per_lane<D>();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      lo[e] = weight != nullptr ? load_as_float(weight, dtype, lane * E + e) : 1.f;
+      hi[e] = weight != nullptr ? load_as_float(weight, dtype, D / 2 + lane * E + e) : 1.f;
+    }
+  }
+};
+template <int D>
+__device__ __forceinline__ void norm_and_rotate(float (&lo)[per_lane<D>()], float (&hi)[per_lane<D>()], bool norm, const HeadWeights<D>& weight,
+                                                float eps, bool rotate, const float2 (&cs)[per_lane<D>()]) {
   constexpr int E = per_lane<D>();
-  if (weight != nullptr) {
+  if (norm) {
     float squares = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e) squares += lo[e] * lo[e] + hi[e] * hi[e];
@@ -46,17 +60,16 @@ __device__ __forceinline__ void norm_and_rotate(float (&lo)[per_lane<D>()], floa
     const float inv = 1.0f / sqrtf(squares / (float)D + eps);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      lo[e] = lo[e] * inv * load_as_float(weight, weight_dtype, lane * E + e);
-      hi[e] = hi[e] * inv * load_as_float(weight, weight_dtype, D / 2 + lane * E + e);
+      lo[e] = lo[e] * inv * weight.lo[e];
+      hi[e] = hi[e] * inv * weight.hi[e];
     }
   }
-  if (cos_sin_row != nullptr) {
+  if (rotate) {
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      const float2 cs = *reinterpret_cast<const float2*>(cos_sin_row + 2 * (lane * E + e));
       const float a = lo[e], b = hi[e];
-      lo[e] = a * cs.x - b * cs.y;
-      hi[e] = b * cs.x + a * cs.y;
+      lo[e] = a * cs[e].x - b * cs[e].y;
+      hi[e] = b * cs[e].x + a * cs[e].y;
     }
   }
 }
@@ -201,6 +214,9 @@ attention_decode_fused_kernel(const __grid_constant__ CUtensorMap map_k, const _
   }
   // zeros for the rows of the query tile that hold no head
   for (int i = lane; i < ROWS * CHUNKS; i += 32) *reinterpret_cast<uint4*>(q_s + i * 8) = make_uint4(0u, 0u, 0u, 0u);
+  HeadWeights<D> q_norm, k_norm;                             // (no kernel of the step writes them)
+  q_norm.load(q_weight, weight_dtype, lane);
+  if (owns_new_key) k_norm.load(k_weight, weight_dtype, lane);
   grid_dependency_wait();
 
 #pragma unroll
@@ -216,23 +232,35 @@ attention_decode_fused_kernel(const __grid_constant__ CUtensorMap map_k, const _
   if constexpr (!TMA) cp_async_commit();
   __syncwarp();
 
-  // ---- the group's query heads: norm, rotation, into the tile
+  // ---- the new token's key and value: to the cache, and kept for this block's own last tile; the group's query heads: norm, rotation,
+  // into the tile, four at a time (their loads, and the key's and value's, are one trip to memory: a head after the other was one each)
   const __nv_bfloat16* token_row = qkv + (size_t)token * heads * D;
-  const float* cos_sin_row = cos_sin != nullptr ? cos_sin + (size_t)token * D : nullptr;
-  if (has_keys) {
-    for (int h = 0; h < group; ++h) {
-      float lo[E], hi[E];
-      load_head<D>(token_row + (size_t)(kv_head * group + h) * D, lo, hi, lane);
-      norm_and_rotate<D>(lo, hi, q_weight, weight_dtype, eps, cos_sin_row, lane);
-      store_head<D, 0>(q_s, h, lo, hi, lane);
-    }
-  }
-  // ---- the new token's key and value: to the cache, and kept for this block's own last tile
+  const bool rotate = cos_sin != nullptr;
+  float2 cs[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    cs[e] = rotate ? *reinterpret_cast<const float2*>(cos_sin + (size_t)token * D + 2 * (lane * E + e)) : make_float2(1.f, 0.f);
   float k_lo[E], k_hi[E], v_lo[E], v_hi[E];
   if (owns_new_key && inject) {
     load_head<D>(token_row + (size_t)(n_q + kv_head) * D, k_lo, k_hi, lane);
-    norm_and_rotate<D>(k_lo, k_hi, k_weight, weight_dtype, eps, cos_sin_row, lane);
     load_head<D>(token_row + (size_t)(n_q + n_kv + kv_head) * D, v_lo, v_hi, lane);
+  }
+  if (has_keys) {
+    for (int h0 = 0; h0 < group; h0 += 4) {
+      float lo[4][E], hi[4][E];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (h0 + j < group) load_head<D>(token_row + (size_t)(kv_head * group + h0 + j) * D, lo[j], hi[j], lane);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (h0 + j < group) {
+          norm_and_rotate<D>(lo[j], hi[j], q_weight != nullptr, q_norm, eps, rotate, cs);
+          store_head<D, 0>(q_s, h0 + j, lo[j], hi[j], lane);
+        }
+    }
+  }
+  if (owns_new_key && inject) {
+    norm_and_rotate<D>(k_lo, k_hi, k_weight != nullptr, k_norm, eps, rotate, cs);
     const size_t at = (((size_t)(slot / page_size) * n_kv + kv_head) * page_size + slot % page_size) * D;
     store_head<D, -1>(k_pool + at, 0, k_lo, k_hi, lane);
     store_head<D, -1>(v_pool + at, 0, v_lo, v_hi, lane);
