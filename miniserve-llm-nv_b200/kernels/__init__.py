@@ -721,11 +721,15 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
 FUSED_DECODE_ATTENTION = __import__("os").environ.get("MINISERVE_B200_FUSED_DECODE_ATTENTION", "1") == "1"
 
 
-# Steps of this many requests run :func:`decode_attention_fused` where it takes the sizes.  Measured at Qwen3-1.7B
-# sizes, context 4,096 (ms per step with / without): 1 request 1.341 / 1.330, 2: 1.370 / 1.366, 4: 1.490 / 1.549,
-# 8: 1.731 / 1.801, 16: 2.807 / 2.789, 64: 6.441 / 6.371.  With one or two requests there are few blocks and each
-# repeats the queries' norm and rotation; with many the kernel's larger register count costs residency.
+# Steps of this many requests run :func:`decode_attention_fused` where it takes the sizes: any page size, and pages that hold whole tiles
+# of keys with up to eight query heads to a key head.  Measured with four layers of 2,048, contexts of a third to all of
+# 4,096 (us per step, apart / inside).  Pages of 64, 16 heads over 8 of 128: 1 request 204 / 193, 2: 209 / 197, 8: 256 / 244, 16: 400 / 378,
+# 24: 445 / 426, 64: 747 / 708; 32 over 4: 1: 215 / 207, 16: 358 / 345, 24: 402 / 390, 64: 651 / 650; 32 over 8 of 64: 1: 200 / 184, 16:
+# 353 / 322, 24: 382 / 358, 64: 652 / 648; contexts up to 1,024: level to 6 % ahead, 24 requests up to 1.5 % behind.  128
+# requests: level.  16 heads over ONE of 128: 1: 200 / 203, 12: 285 / 289 (every block norms them all).  Pages of 16: 8: 257 / 259, 24:
+# 440 / 467, 64: 749 / 807 (the copies of sixteen bytes).
 FUSED_DECODE_ROWS = (3, 8)
+FUSED_DECODE_ROWS_WHOLE_TILES = (1, 64)
 
 
 def decode_attention_fused_supported(dtype: torch.dtype, head_dim: int, n_q: int, n_kv: int) -> bool:
@@ -735,9 +739,13 @@ def decode_attention_fused_supported(dtype: torch.dtype, head_dim: int, n_q: int
                 and library().ms_attention_decode_fused_supports(_i(head_dim), _i(n_q), _i(n_kv)))
 
 
-def decode_attention_fused_preferred(rows: int) -> bool:
-    """Whether a step of ``rows`` single tokens is faster with :func:`decode_attention_fused` (see FUSED_DECODE_ROWS)."""
-    return FUSED_DECODE_ROWS[0] <= rows <= FUSED_DECODE_ROWS[1]
+def decode_attention_fused_preferred(rows: int, head_dim: int = 0, group: int = 0, page_size: int = 0) -> bool:
+    """Whether a step of ``rows`` single tokens is faster with :func:`decode_attention_fused` (see FUSED_DECODE_ROWS);
+    ``head_dim``, ``group`` (query heads of a key head) and ``page_size``, where given, say whether pages hold whole tiles."""
+    first, last = FUSED_DECODE_ROWS
+    if page_size > 0 and page_size % (32 if head_dim == 128 else 64) == 0 and 0 < group <= 8:
+        first, last = min(first, FUSED_DECODE_ROWS_WHOLE_TILES[0]), max(last, FUSED_DECODE_ROWS_WHOLE_TILES[1])
+    return first <= rows <= last
 
 
 def decode_attention_fused(qkv: torch.Tensor, slots: torch.Tensor, q_weight: Optional[torch.Tensor],

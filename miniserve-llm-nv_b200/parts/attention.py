@@ -268,7 +268,7 @@ class Attention(Part):
             kernels.linear_pair_qkv(x, self.qkv_weight, slots, self.q_norm_weight, self.k_norm_weight, self.eps, fused[0],
                                     cache.key_pool, cache.value_pool, n_q, n_kv, q, row_stats=stats)
             self._attend(q, ctx, cache, attended)
-        elif self._decode_in_the_attention_kernel(ctx, fused, x.dtype):
+        elif self._decode_in_the_attention_kernel(ctx, cache, fused, x.dtype):
             # a step of single tokens: norm, rotation and append happen inside the split-key attention kernel
             kernels.decode_attention_fused(qkv, slots, self.q_norm_weight, self.k_norm_weight, self.eps, fused[0],
                                            cache.key_pool, cache.value_pool, cache.block_tables, ctx.query_start,
@@ -347,13 +347,14 @@ class Attention(Part):
                                 ctx.max_context_len, self.scale, self.window, attended,
                                 ctx.host_query_start or None, self.score_softcap, self._slopes_on_device)
 
-    def _decode_in_the_attention_kernel(self, ctx: StepContext, fused, dtype: torch.dtype) -> bool:
+    def _decode_in_the_attention_kernel(self, ctx: StepContext, cache: PagedKVView, fused, dtype: torch.dtype) -> bool:
         """Whether this step's norm, rotation and append run inside the attention kernel
         (``kernels.decode_attention_fused``): one token per request, a position encoding in that kernel's form (none,
         or half-split rotation over the whole head), no score modifiers, sizes that the kernel takes."""
         if ctx.max_query_len != 1 or ctx.n_tokens != ctx.n_requests or fused is None:
             return False
-        if not kernels.decode_attention_fused_preferred(ctx.n_requests):
+        if not kernels.decode_attention_fused_preferred(ctx.n_requests, self.head_dim, self.num_heads // self.num_kv_heads,
+                                                        cache.key_pool.shape[2]):
             return False
         cos_sin, rotary_dim, interleaved = fused
         if cos_sin is not None and (interleaved or rotary_dim != self.head_dim):

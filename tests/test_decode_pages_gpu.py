@@ -49,3 +49,12 @@ def test_the_page_size_changes_no_bit(lengths, d, n_q, n_kv, window):
         found.append(out)
     assert torch.isfinite(found[0].float()).all()
     assert all(torch.equal(found[0], other) for other in found[1:])
+
+
+@pytest.mark.parametrize("rows,head_dim,group,page_size,want", [
+    (2, 128, 2, 16, False), (3, 128, 2, 16, True), (9, 128, 2, 16, False), (1, 128, 2, 32, True), (64, 128, 8, 64, True), (65, 128, 2, 64, False),
+    (1, 64, 2, 32, False), (1, 64, 2, 128, True), (2, 128, 9, 64, False), (5, 128, 16, 64, True), (2, 0, 0, 0, False), (8, 0, 0, 0, True)])
+def test_which_decode_steps_take_it(rows, head_dim, group, page_size, want):
+    from miniserve_b200 import kernels
+
+    assert kernels.decode_attention_fused_preferred(rows, head_dim, group, page_size) is want
