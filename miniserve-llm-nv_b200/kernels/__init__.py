@@ -834,6 +834,10 @@ def latent_attention_kernels(dtype: torch.dtype, rank: int, rot: int, heads: int
     return {"decode": "general", "prompt": "general"}
 
 
+# Keys that a step of single tokens reads, for each sixteen of its heads, from which on ms_latent_decode takes it: its warps share nothing, and
+# meet once for longer.  A layer's step, us with ms_latent_attention_mma / with it: 2 requests of 2,400 keys 28.8 / 30.8, 8 of 2,400
+# 30.9 / 33.0, 16 of 2,400 33.8 / 35.0, 8 of 8,000 39.0 / 39.0, 16 of 8,000 57.5 / 52.8, 32 of 7,200 78 / 63.
+LATENT_DECODE_KEYS = 98304
 USE_LATENT_MMA = __import__("os").environ.get("MINISERVE_B200_LATENT_MMA", "1") == "1"
 
 
@@ -869,7 +873,7 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
                 _i(n_requests), _i(max_query_len), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
             return
         reach = min(max_context_len, window) if window else max_context_len      # the most keys a token sees
-        if max_query_len == 1 and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
+        if max_query_len == 1 and n * ((heads + 15) // 16) * reach >= LATENT_DECODE_KEYS and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
                 q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
             splits = lib.ms_latent_decode_splits(_i(heads), _i(n_requests), _i(reach))
             part_o = part_lse = None
@@ -940,10 +944,21 @@ def _state_rows(states: torch.Tensor, offset: int, length: int) -> int:
 
 CONV_ACTIVATIONS = {"none": 0, "silu": 1}
 MAX_CHUNK_SCRATCH = 1 << 30   # bytes of chunk states beyond which a scan walks its tokens
+# From which sizes on the scans in chunks are ahead of the walk: a longest portion of 256 tokens, or of 128 in a step of 512; the delta form,
+# whose chunks follow one another and whose walk gains from several requests, a longest portion of 128 x (1 + the number of such portions
+# that the step's tokens would fill).  Whole layers, walk / chunks in us: selective, 64 heads: 1 portion of 128: 74 / 87, 192: 95 / 87, 256: 113 /
+# 89, 4 of 128: 160 / 136; 32 heads: 192: 76 / 86, 256: 89 / 90, 320: 123 / 90; memory: 1 of 128: 93 / 104, 192: 102 / 105, 256: 123 / 107, 4 of 128:
+# 160 / 108; delta: 1 of 192: 134 / 136, 256: 163 / 139, 4 of 320: 251 / 270, 4 of 448: 339 / 335.
+CHUNK_SCAN_LONGEST, CHUNK_SCAN_OF_MANY, CHUNK_SCAN_DELTA = 256, (128, 512), 128
 
 
-def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device) -> Optional[tuple]:
+def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False) -> Optional[tuple]:
     """(chunk states, chunk decays) for the scans in chunks, or None where the step's tokens are walked one after the other."""
+    if delta:
+        if longest <= 0 or longest < CHUNK_SCAN_DELTA * (1 + (n + longest - 1) // longest):
+            return None
+    elif longest < CHUNK_SCAN_LONGEST and (longest < CHUNK_SCAN_OF_MANY[0] or n < CHUNK_SCAN_OF_MANY[1]):
+        return None
     chunk = library().ms_chunk_scan_chunk(_i(n_requests), _i(longest), _i(heads), _i(dim))
     if not chunk:
         return None
@@ -1177,7 +1192,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
         return
     scratch = None
     if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
-        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device)
+        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1)
     if scratch is not None:
         solved = [None] * 3
         if code == 1:

@@ -10,6 +10,15 @@ LENGTHS = [[64], [128, 1, 0, 65], [129, 63], [1, 200, 7], [96, 97, 98, 2, 511]]
 SIZES = [(4, 2, 128, 128), (2, 2, 64, 64), (3, 3, 40, 56), (2, 1, 100, 130), (1, 1, 33, 3), (2, 2, 128, 259), (2, 1, 6, 17)]
 
 
+@pytest.fixture(autouse=True)
+def in_chunks_from_96_tokens_on(monkeypatch):
+    """(in use only from the sizes on where it is faster)"""
+    from miniserve_b200 import kernels
+
+    for name, value in (("CHUNK_SCAN_LONGEST", 0), ("CHUNK_SCAN_DELTA", 0)):
+        monkeypatch.setattr(kernels, name, value)
+
+
 def ints(values):
     return torch.tensor(values, dtype=torch.int32, device="cuda")
 

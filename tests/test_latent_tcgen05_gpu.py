@@ -10,6 +10,14 @@ STEPS = [([1, 2], [0, 0]), ([8, 1, 9], [0, 63, 64]), ([64, 65], [1, 191]), ([130
 DECODE = [([1] * 6, [0, 15, 16, 63, 64, 65]), ([1], [5000]), ([1, 1, 1], [700, 2047, 191])]
 
 
+@pytest.fixture(autouse=True)
+def decode_steps_of_any_size(monkeypatch):
+    """(the kernel of decode steps is in use only from the sizes on where it is faster)"""
+    from miniserve_b200 import kernels
+
+    monkeypatch.setattr(kernels, "LATENT_DECODE_KEYS", 0)
+
+
 @pytest.mark.parametrize("rank,rot,heads,page", [(256, 32, 16, 64), (256, 32, 8, 16), (256, 64, 16, 128), (256, 0, 4, 8), (128, 16, 16, 32),
                                                  (64, 48, 1, 64), (64, 64, 128, 64), (128, 32, 32, 192)])
 @pytest.mark.parametrize("new,before", STEPS + DECODE)
