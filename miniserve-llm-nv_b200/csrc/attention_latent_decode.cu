@@ -71,8 +71,10 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                    ::"r"(t5::smem_u32(stage + lane * ROW)), "l"(row), "r"(DK * 2), "r"(t5::smem_u32(bar)) : "memory");
     }
-    for (int j = count * (ROW / 16) + lane; j < KEYS * (ROW / 16); j += 32)      // (behind the context: zeros)
-      *reinterpret_cast<uint4*>(stage + j * 16) = make_uint4(0u, 0u, 0u, 0u);
+    if (count < KEYS) {                                                          // behind the context: zeros
+      for (int j = count * (ROW / 16) + lane; j < KEYS * (ROW / 16); j += 32) *reinterpret_cast<uint4*>(stage + j * 16) = make_uint4(0u, 0u, 0u, 0u);
+      __syncwarp();                                                              // (other lanes read them; the copies' barrier does not order them)
+    }
   };
 #pragma unroll
   for (int i = 0; i < STAGES - 1; ++i)

@@ -66,3 +66,25 @@ def test_against_float64(rank, rot, heads, page, new, before, window):
         size = torch.einsum("htk,kd->thd", p, keys[:, :rank].abs())
         slack = dk * 2.0 ** -23 * float((here.abs().amax() * keys.abs().amax() * dk * scale))
         assert torch.all((out[starts[r]:starts[r + 1]].double() - want).abs() <= (2.0 ** -7 + slack) * size + 1e-6)
+
+
+def test_contexts_of_one_piece_after_a_step_of_stale_numbers():
+    """A warp whose range is one piece of sixteen keys, not all of them real, reads zeros behind the context, whatever the step before (of
+    NaN alone) has left in shared memory: a row of ones is then the answer exactly, since all keys have the same score."""
+    from miniserve_b200 import kernels
+
+    heads, rank, dk, page, n = 16, 256, 288, 64, 63
+    lens = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+    starts, tables = torch.arange(n + 1, dtype=torch.int32, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")[:, None].contiguous()
+    zeros = torch.zeros(n, dtype=torch.int32, device="cuda")
+    q = torch.ones((n, heads, dk), device="cuda").bfloat16()
+    stale = torch.full((n, page, dk), float("nan"), device="cuda").bfloat16()
+    cache = stale.clone()
+    for r in range(n):
+        cache[r, :r + 1] = 1.0
+    out = torch.empty((n, heads, rank), device="cuda").bfloat16()
+    for _ in range(20):
+        for pool in (stale, cache):
+            kernels.latent_attention(q, pool, tables, zeros, lens - 1, starts, lens, 1, n, rank, dk ** -0.5, None, out)
+        kernels.check_device_errors(q.device)
+        assert torch.all(out == 1.0)
