@@ -286,10 +286,14 @@ attention_decode_fused_kernel(const __grid_constant__ CUtensorMap map_k, const _
       __nv_bfloat16* vs = v_s + stage * BN * D;
       const int key0 = tile_begin + tile * BN;
       if constexpr (TMA) {
+        __syncwarp();                                         // every lane has read the stage that is fetched into next
         if (tile + STAGES - 1 < tile_hi) bring((stage + STAGES - 1) % STAGES, rows[STAGES - 1]);
         rows[STAGES - 1] = first_row(tile + STAGES);
         const bool ok = t5::mbar_wait(&full[stage], ((tile - tile_lo) / STAGES) & 1, error_flag, 52);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        if (!__all_sync(0xffffffffu, ok)) {
+          t5::let_copies_land(full, STAGES, min(tile_hi, tile + STAGES) - tile_lo, error_flag);
+          break;
+        }
         if (key0 + BN > key_end) {                            // what is masked in the scores must still be a number here
           for (int i = lane; i < (key0 + BN - key_end) * CHUNKS; i += 32)
             *reinterpret_cast<uint4*>(key_ptr<BN>(vs, key_end - key0 + i / CHUNKS, i % CHUNKS)) = make_uint4(0u, 0u, 0u, 0u);

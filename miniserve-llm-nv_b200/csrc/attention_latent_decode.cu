@@ -103,7 +103,10 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
 
   for (int i = 0; i < pieces; ++i) {
     const bool ok = t5::mbar_wait(&full[warp][i % STAGES], (i / STAGES) & 1, error_flag, 51);
-    if (!__all_sync(0xffffffffu, ok)) break;
+    if (!__all_sync(0xffffffffu, ok)) {
+      t5::let_copies_land(full[warp], STAGES, min(pieces, i + STAGES - 1), error_flag);
+      break;
+    }
     if (i + STAGES - 1 < pieces) request(i + STAGES - 1);                // (its stage's last reads lie before this wait)
     const unsigned char* kt = ring + (i % STAGES) * STAGE;
     float s[2][4], s_odd[2][4];                                          // two chains of products, added at the end

@@ -124,7 +124,8 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
       const int box = min(page_size, BN), boxes = BN / box;         // keys of a box, boxes of a tile and column block
       bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
+      int j = 0;
+      for (; j < n_tiles; ++j) {
         const int stage = j % STAGES;
         if (lane == 0) {
           ok = mbar_wait(&k_empty[stage], ((j / STAGES) & 1) ^ 1, error_flag, 31);
@@ -139,6 +140,10 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           const int row = key < key_end ? table[key / page_size] * page_size + key % page_size : table[0] * page_size;
           tma_load_2d(key_stage(stage) + (size_t)db * (BN * 128) + (size_t)(p * box) * 128, &map_k, &k_full[stage], db * 64, row);
         }
+      }
+      if (lane == 0 && (!ok || *reinterpret_cast<volatile int*>(error_flag) != 0)) {
+        let_copies_land(&q_full, 1, 1, error_flag);
+        let_copies_land(k_full, STAGES, j, error_flag);
       }
     }
   } else if (warp == 1) {

@@ -165,6 +165,7 @@ expert_tcgen05_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* _
           tma_load_2d(smem + (size_t)stage * L::STAGE_BYTES + L::A_BYTES, &map_w, &full_bar[stage], kb * BK, w_row);
         }
       }
+      if (!ok || *reinterpret_cast<volatile int*>(error_flag) != 0) let_copies_land(full_bar, STAGES, it, error_flag);
     }
   } else if (warp == 1) {
     if (lane == 0) {

@@ -34,6 +34,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int* e
   return false;
 }
 
+// After a wait that gave up: the copies still in flight, the last of `sent` through a ring of `stages` barriers, land before the block may
+// exit (its shared memory is then another's).  Each of these waits is bounded too.
+__device__ __forceinline__ void let_copies_land(uint64_t* full, int stages, int sent, int* error_flag) {
+  for (int j = sent - 1; j >= 0 && j >= sent - stages; --j) mbar_wait(&full[j % stages], (unsigned)(j / stages) & 1u, error_flag, 4);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
