@@ -13,16 +13,19 @@
 // (Four warps that share each piece of 32 keys meet three times for it, and fetch the queries' fragments again each time: a piece's
 // chain of some 2,900 clocks, not the memory, set the pace.)
 // 32 requests of 16 heads and some 7,200 keys (147 MB): 49 us that way, 35.5 here.
-#include "common.cuh"
-#include "mma_common.cuh"
+#include "attention_latent_tiles.cuh"
 #include "tcgen05.cuh"
 
 namespace ms {
 namespace latent_decode {
 
 constexpr int DV = 256, WARPS = 4, KEYS = 16, UNIT = WARPS * KEYS, STAGES = 3, OLD = DV + 4;
+constexpr int TILE_BUFFERS = 4;        // of attention_latent_tiles.cuh
 
-constexpr size_t smem_bytes(int nkc) { return (size_t)WARPS * STAGES * KEYS * (nkc * 32 + 16); }
+constexpr size_t smem_bytes(int nkc) {
+  const size_t rings = (size_t)WARPS * STAGES * KEYS * (nkc * 32 + 16), tiles = latent_tiles_smem(WARPS, TILE_BUFFERS, nkc * 16);
+  return rings > tiles ? rings : tiles;
+}
 
 // NKC: steps of 16 along a row of (256 + rot) numbers.
 template <int NKC>
@@ -31,7 +34,7 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
                      const int* __restrict__ block_tables, int table_stride, const int* __restrict__ query_start,
                      const int* __restrict__ context_lens, int page_size, int heads, float scale_log2, int window,
                      __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_lse, int splits,
-                     int* __restrict__ error_flag) {
+                     int ranges, int least, int tile_ranges, int* __restrict__ error_flag) {
   constexpr int DK = NKC * 16, ROW = NKC * 32 + 16, STAGE = KEYS * ROW;
   extern __shared__ __align__(128) unsigned char decode_smem[];
   __shared__ uint64_t full[WARPS][STAGES];
@@ -43,12 +46,21 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
   const int rows = q_len * heads, m0 = blockIdx.x * 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (m0 >= rows) return;
+  if ((window > 0 ? min(ctx, window) : ctx) < least) {
+    latent_decode_tiles<DV, WARPS, TILE_BUFFERS>(q_full, cache, block_tables, table_stride, query_start, context_lens, page_size, heads, DK,
+                                                 scale_log2, window, out, part_o, part_lse, splits, tile_ranges, decode_smem);
+    return;
+  }
   const int* table = block_tables + (size_t)req * table_stride;
   const int pos_last = ctx - q_len + (min(m0 + 16, rows) - 1) / heads, pos_first = ctx - q_len + m0 / heads;
   const int key_begin = window > 0 ? max(0, pos_first - window + 1) : 0;
   const int unit_begin = key_begin / UNIT, unit_end = pos_last / UNIT + 1;
-  const int per_split = (unit_end - unit_begin + splits - 1) / splits;
+  const int per_split = (unit_end - unit_begin + ranges - 1) / ranges;
   const int first_unit = unit_begin + split * per_split, units = min(unit_end, first_unit + per_split) - first_unit;
+  if (units <= 0 && splits > 1) {                // a range behind the request's keys: the merge reads no more of it than this
+    if (threadIdx.x < 16 && m0 + threadIdx.x < rows) part_lse[((size_t)q0 * heads + m0 + threadIdx.x) * splits + split] = -INFINITY;
+    return;
+  }
   const int first_key = first_unit * UNIT + warp * KEYS;
   // this warp's pieces: first_key, first_key + 64, ...
   const int pieces = units <= 0 ? 0 : units - (first_key + (units - 1) * UNIT > pos_last ? 1 : 0);
@@ -220,13 +232,13 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
 template <int NKC>
 static int launch(const void* q_full, const void* cache, const int* block_tables, int table_stride, const int* query_start,
                   const int* context_lens, int page_size, int heads, float scale, int window, void* out, float* part_o, float* part_lse,
-                  int splits, int n_requests, int* error_flag, cudaStream_t stream) {
+                  int splits, int ranges, int least, int tile_ranges, int n_requests, int* error_flag, cudaStream_t stream) {
   auto kernel = latent_decode_kernel<NKC>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(NKC));
   if (e != cudaSuccess) MS_FAIL("latent_decode: %zu bytes of shared memory refused: %s", smem_bytes(NKC), cudaGetErrorString(e));
   ms::launch(kernel, dim3((heads + 15) / 16, n_requests, splits), 32 * WARPS, smem_bytes(NKC), stream, (const __nv_bfloat16*)q_full,
              (const __nv_bfloat16*)cache, block_tables, table_stride, query_start, context_lens, page_size, heads,
-             scale * 1.4426950408889634f, window, (__nv_bfloat16*)out, part_o, part_lse, splits, error_flag);
+             scale * 1.4426950408889634f, window, (__nv_bfloat16*)out, part_o, part_lse, splits, ranges, least, tile_ranges, error_flag);
   MS_CHECK_LAUNCH("latent_decode");
   return 0;
 }
@@ -259,21 +271,24 @@ MS_EXPORT int ms_latent_decode_splits(int heads, int n_requests, int max_context
   return best;
 }
 
-// Arguments as ms_latent_attention_mma for steps of single tokens; error_flag: one int on the device that a kernel which gave up
-// waiting sets.  Cache rows on 16-byte boundaries.
+// Arguments as ms_latent_attention_mma for steps of single tokens.  A request's keys are cut into `ranges`; one that sees fewer than `least`
+// keys is attended to in tiles that its blocks' warps share (attention_latent_tiles.cuh), cut into tile_ranges.  Partial results are for
+// max(ranges, tile_ranges).  error_flag: one int on the device that a kernel which gave up waiting sets.  Cache rows on 16-byte boundaries.
 MS_EXPORT int ms_latent_decode(const void* q_full, const void* cache, const int* block_tables, int table_stride, const int* query_start,
                                const int* context_lens, int page_size, int heads, int rank, int rot, float scale, int window, void* out,
-                               float* part_o, float* part_lse, int splits, int n_requests, int n_tokens, int* error_flag,
+                               float* part_o, float* part_lse, int ranges, int least, int tile_ranges, int n_requests, int n_tokens, int* error_flag,
                                cudaStream_t stream) {
   if (n_tokens == 0 || n_requests == 0) return 0;
   MS_REQUIRE(ms_latent_decode_supports(rank, rot, heads) && page_size > 0, "latent_decode: %d + %d, %d heads, pages of %d", rank, rot, heads, page_size);
-  MS_REQUIRE(splits >= 1 && splits <= 32 && (splits == 1 || (part_o && part_lse)), "latent_decode: %d splits", splits);
+  const int splits = ranges > tile_ranges ? ranges : tile_ranges;
+  MS_REQUIRE(ranges >= 1 && tile_ranges >= 1 && splits <= 32 && (splits == 1 || (part_o && part_lse)), "latent_decode: %d ranges, or %d",
+             ranges, tile_ranges);
   MS_REQUIRE(n_requests <= 65535 && error_flag != nullptr, "latent_decode: %d requests, an error flag on the device is required", n_requests);
   MS_REQUIRE(((reinterpret_cast<size_t>(q_full) | reinterpret_cast<size_t>(cache) | reinterpret_cast<size_t>(out)) & 15) == 0,
              "latent_decode: operands must be 16-byte aligned");
   auto launch = rot == 0 ? latent_decode::launch<16> : rot == 32 ? latent_decode::launch<18> : latent_decode::launch<20>;
   if (launch(q_full, cache, block_tables, table_stride, query_start, context_lens, page_size, heads, scale, window, out, part_o, part_lse,
-             splits, n_requests, error_flag, stream))
+             splits, ranges, least, tile_ranges, n_requests, error_flag, stream))
     return 1;
   if (splits > 1) {
     launch_attention_combine<256>(part_o, part_lse, (__nv_bfloat16*)out, splits, n_tokens * heads, stream);

@@ -834,9 +834,12 @@ def latent_attention_kernels(dtype: torch.dtype, rank: int, rot: int, heads: int
     return {"decode": "general", "prompt": "general"}
 
 
-# Keys that a step of single tokens reads, for each sixteen of its heads, from which on ms_latent_decode takes it: its warps share nothing, and
-# meet once for longer.  A layer's step, us with ms_latent_attention_mma / with it: 2 requests of 2,400 keys 28.8 / 30.8, 8 of 2,400
-# 30.9 / 33.0, 16 of 2,400 33.8 / 35.0, 8 of 8,000 39.0 / 39.0, 16 of 8,000 57.5 / 52.8, 32 of 7,200 78 / 63.
+# From how many keys a request sees, times the step's requests and their tiles of sixteen heads, on ms_latent_decode's warps each take keys of
+# their own: they share nothing, and meet once for longer.  The kernel decides by each request's own length, because a captured step passes
+# the longest context allowed; only a step none of whose requests can be that long goes to ms_latent_attention_mma.  A
+# layer's captured step, us with shared tiles / own keys / this rule, bound 40,960: 4 requests of 100 keys 24.6 / 28.7 / 24.6, 8 of 600 26.7 /
+# 30.6 / 28.7, 8 of 8,000 39 / 41 / 41, 16 of 2,400 37 / 41 / 39, 16 of 8,000 57 / 53 / 54, 32 of 600 31 / 33 / 31, 32 of 8,000 75 / 63
+# / 63, 64 of 600 39 / 43 / 37, 64 of 2,400 65 / 62 / 62, 64 of 8,000 121 / 96 / 96 (the clock of such a measurement ticks in steps of 2).
 LATENT_DECODE_KEYS = 98304
 USE_LATENT_MMA = __import__("os").environ.get("MINISERVE_B200_LATENT_MMA", "1") == "1"
 
@@ -873,9 +876,12 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
                 _i(n_requests), _i(max_query_len), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
             return
         reach = min(max_context_len, window) if window else max_context_len      # the most keys a token sees
-        if max_query_len == 1 and n * ((heads + 15) // 16) * reach >= LATENT_DECODE_KEYS and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
+        tile_ranges = lib.ms_latent_attention_mma_splits(_i(rank), _i(dk - rank), _i(heads), _i(n_requests), _i(max_query_len), _i(reach))
+        least = LATENT_DECODE_KEYS // max(1, n * ((heads + 15) // 16))
+        if max_query_len == 1 and reach >= least and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
                 q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
-            splits = lib.ms_latent_decode_splits(_i(heads), _i(n_requests), _i(reach))
+            ranges = lib.ms_latent_decode_splits(_i(heads), _i(n_requests), _i(reach))
+            splits = max(ranges, tile_ranges)
             part_o = part_lse = None
             if splits > 1:
                 part_o = torch.empty((n * heads * splits, rank), dtype=torch.float32, device=q_full.device)
@@ -883,9 +889,10 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
             _check(lib.ms_latent_decode(
                 _ptr(q_full), _ptr(cache), _ptr(block_tables), _i(block_tables.shape[1]), _ptr(query_start), _ptr(context_lens),
                 _i(page_size), _i(heads), _i(rank), _i(dk - rank), _f(scale), _i(window if window else 0), _ptr(out), _ptr(part_o),
-                _ptr(part_lse), _i(splits), _i(n_requests), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
+                _ptr(part_lse), _i(ranges), _i(least), _i(tile_ranges), _i(n_requests), _i(n), _ptr(device_error_flag(q_full.device)),
+                _stream()))
             return
-        splits = lib.ms_latent_attention_mma_splits(_i(rank), _i(dk - rank), _i(heads), _i(n_requests), _i(max_query_len), _i(reach))
+        splits = tile_ranges
         part_o = part_lse = None
         if splits > 1:
             part_o = torch.empty((n * heads * splits, rank), dtype=torch.float32, device=q_full.device)

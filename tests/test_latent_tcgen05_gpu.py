@@ -88,3 +88,58 @@ def test_contexts_of_one_piece_after_a_step_of_stale_numbers():
             kernels.latent_attention(q, pool, tables, zeros, lens - 1, starts, lens, 1, n, rank, dk ** -0.5, None, out)
         kernels.check_device_errors(q.device)
         assert torch.all(out == 1.0)
+
+
+@pytest.mark.parametrize("rot,heads,window", [(32, 16, None), (64, 8, None), (32, 20, 2500)])
+def test_a_request_is_attended_to_by_what_its_own_keys_ask_for(monkeypatch, rot, heads, window):
+    """A captured step knows the longest context allowed, not the step's: which of the two ways a request takes is its own length's choice,
+    on the device.  One graph, replayed with short, long and mixed contexts, gives a short request the bits that the way for short
+    ones gives alone, and a long one those of the way for long ones."""
+    from miniserve_b200 import kernels
+
+    rank, page, limit, n = 256, 64, 40960, 48 if heads == 16 else 64
+    dk, border = rank + rot, 98304 // (n * ((heads + 15) // 16))
+    assert border <= (window or border)
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    cache = torch.randn((1 + (2 * border) // page, page, dk), generator=g, device="cuda").bfloat16()       # (all requests see the same pages)
+    tables = torch.arange(cache.shape[0], dtype=torch.int32, device="cuda").repeat(n, 1)
+    q = torch.randn((n, heads, dk), generator=g, device="cuda").bfloat16()
+    starts, zeros = torch.arange(n + 1, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    lens, out = torch.full((n,), 3, dtype=torch.int32, device="cuda"), torch.empty((n, heads, rank), device="cuda").bfloat16()
+
+    def step():
+        kernels.latent_attention(q, cache, tables, zeros, lens - 1, starts, lens, 1, limit, rank, dk ** -0.5, window, out)
+
+    found = {}
+    for name, keys in (("shared tiles", 1 << 60), ("own pieces", 0), ("rule", 98304)):
+        monkeypatch.setattr(kernels, "LATENT_DECODE_KEYS", keys)
+        step()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            step()
+        for mixture in ([1, border - 1, border, 2 * border], [17, 300], [border + 1, 2 * border - 5]):
+            lens.copy_(torch.tensor(mixture * n, dtype=torch.int32)[:n])
+            graph.replay()
+            found.setdefault(name, []).append((lens.clone(), out.clone()))
+    kernels.check_device_errors(q.device)
+    for (now, out_tiles), (_, out_pieces), (_, out_rule) in zip(*(found[name] for name in ("shared tiles", "own pieces", "rule"))):
+        short = now < border
+        assert torch.equal(out_rule[short], out_tiles[short]) and torch.equal(out_rule[~short], out_pieces[~short])
+        assert not short.any() or not torch.equal(out_tiles[short], out_pieces[short])
+
+
+@pytest.mark.parametrize("n,heads,bound,taken", [(2, 16, 49151, False), (2, 16, 49152, True), (3, 16, 40960, True), (3, 16, 32767, False),
+                                                 (64, 16, 1536, True), (64, 16, 1535, False), (64, 17, 768, True), (64, 17, 767, False)])
+def test_which_decode_steps_may_take_it(monkeypatch, n, heads, bound, taken):
+    from miniserve_b200 import kernels
+
+    monkeypatch.setattr(kernels, "LATENT_DECODE_KEYS", 98304)
+    lib, calls = kernels.library(), []
+    real = lib.ms_latent_decode
+    monkeypatch.setattr(lib, "ms_latent_decode", lambda *a: calls.append(1) or real(*a))
+    q, cache = torch.ones((n, heads, 288), device="cuda").bfloat16(), torch.ones((1, 64, 288), device="cuda").bfloat16()
+    ints = [torch.zeros((n, 1), dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")]
+    lens, out = torch.full((n,), 5, dtype=torch.int32, device="cuda"), torch.empty((n, heads, 256), device="cuda").bfloat16()
+    kernels.latent_attention(q, cache, ints[0], ints[1], lens - 1, torch.arange(n + 1, dtype=torch.int32, device="cuda"), lens, 1, bound, 256,
+                             0.1, None, out)
+    assert bool(calls) is taken and torch.all(out == 1.0)
