@@ -5,7 +5,7 @@
 //
 // A block has four warps that share nothing on the way: each takes every fourth piece of sixteen keys of the block's range, with the
 // queries' fragments (72 registers for 256 + 32) and its own output of 16 x 256 (128 registers) in registers, and a ring of three
-// pieces of its own, two on their way while one is multiplied.  A piece comes by one bulk copy a row (cp.async.bulk, sixteen
+// pieces of its own (two for 256 + 64), the others on their way while one is multiplied.  A piece comes by one bulk copy a row (cp.async.bulk, sixteen
 // instructions; rows lie sixteen bytes apart from one another's banks), counted by a barrier.  The probabilities go from the
 // scores' registers to the second product's operand without leaving the warp; the output is rescaled only when a row's maximum has
 // grown by more than 2^8.  At the end the four outputs meet in shared memory.  Rows that no kernel of this step writes are asked for
@@ -19,11 +19,13 @@
 namespace ms {
 namespace latent_decode {
 
-constexpr int DV = 256, WARPS = 4, KEYS = 16, UNIT = WARPS * KEYS, STAGES = 3, OLD = DV + 4;
+constexpr int DV = 256, WARPS = 4, KEYS = 16, UNIT = WARPS * KEYS, OLD = DV + 4;
 constexpr int TILE_BUFFERS = 4;        // of attention_latent_tiles.cuh
 
+// Pieces of a warp's ring: as many as let two blocks share a multiprocessor (three with a rotated part of 64 would not).
+__host__ __device__ constexpr int stages_of(int nkc) { return nkc <= 18 ? 3 : 2; }
 constexpr size_t smem_bytes(int nkc) {
-  const size_t rings = (size_t)WARPS * STAGES * KEYS * (nkc * 32 + 16), tiles = latent_tiles_smem(WARPS, TILE_BUFFERS, nkc * 16);
+  const size_t rings = (size_t)WARPS * stages_of(nkc) * KEYS * (nkc * 32 + 16), tiles = latent_tiles_smem(WARPS, TILE_BUFFERS, nkc * 16);
   return rings > tiles ? rings : tiles;
 }
 
@@ -35,7 +37,7 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
                      const int* __restrict__ context_lens, int page_size, int heads, float scale_log2, int window,
                      __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_lse, int splits,
                      int ranges, int least, int tile_ranges, int* __restrict__ error_flag) {
-  constexpr int DK = NKC * 16, ROW = NKC * 32 + 16, STAGE = KEYS * ROW;
+  constexpr int DK = NKC * 16, ROW = NKC * 32 + 16, STAGE = KEYS * ROW, STAGES = stages_of(NKC);
   extern __shared__ __align__(128) unsigned char decode_smem[];
   __shared__ uint64_t full[WARPS][STAGES];
   __shared__ float peaks[WARPS][16], sums[WARPS][16];
@@ -233,6 +235,7 @@ template <int NKC>
 static int launch(const void* q_full, const void* cache, const int* block_tables, int table_stride, const int* query_start,
                   const int* context_lens, int page_size, int heads, float scale, int window, void* out, float* part_o, float* part_lse,
                   int splits, int ranges, int least, int tile_ranges, int n_requests, int* error_flag, cudaStream_t stream) {
+  static_assert(2 * (smem_bytes(NKC) + 2048) <= 228 * 1024, "the ranges are chosen for two blocks a multiprocessor");
   auto kernel = latent_decode_kernel<NKC>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(NKC));
   if (e != cudaSuccess) MS_FAIL("latent_decode: %zu bytes of shared memory refused: %s", smem_bytes(NKC), cudaGetErrorString(e));
