@@ -48,52 +48,67 @@ struct Problem {
   long long state_stride;
   int state_offset;
   const int *state_slots, *query_start;
-  int requests, most;                                    // most: chunks of the longest portion: blockIdx.z = request * most + chunk
+  int requests, least;                                   // least: tokens from which on a portion is scanned here
   float *chunk_states, *chunk_decays;                    // [places][heads][columns][dim], [places][heads]
   float *y, *bottom;
 };
 
-struct Where { int request, first, len, left; size_t place; };      // a block's chunk: its first token, its tokens, those from it on
-__device__ __forceinline__ Where where_of(const Problem& p) {
-  Where w;
-  w.request = blockIdx.z / p.most;
-  const int c = blockIdx.z % p.most, first = p.query_start[w.request];
-  w.left = p.query_start[w.request + 1] - first - c * kC;
-  w.len = min(w.left, kC);
-  w.first = first + c * kC;
-  // (places of different requests do not meet: a portion of n tokens has at most one chunk more than it holds borders of 64
-  // tokens counted from the step's first token)
-  w.place = (size_t)(first / kC + w.request + c);
-  return w;
+// A block's chunk (its first token, its tokens, those of its portion from it on), or its portion and that one's first chunk.  Chunks are
+// numbered through the step's portions of at least `least` tokens, which is where their matrices lie in the scratch.
+struct Where { int request, first, len, left; size_t place; };
+struct Portion { int request, first, tokens; size_t place; };
+
+// The portions of 32 requests from r0 on, one a lane: its first token, its tokens (0: none, or too few for a chunk), and the chunks up to and
+// with it.
+struct Lane { int first, tokens, chunks, upto; };
+__device__ __forceinline__ Lane portions_from(const Problem& p, int r0) {
+  const int lane = threadIdx.x & 31;
+  Lane l = {};
+  if (r0 + lane < p.requests) l.first = p.query_start[r0 + lane], l.tokens = p.query_start[r0 + lane + 1] - l.first;
+  if (l.tokens < p.least) l.tokens = 0;
+  l.chunks = (l.tokens + kC - 1) / kC, l.upto = l.chunks;
+#pragma unroll
+  for (int d = 1; d < 32; d *= 2) {
+    const int before = __shfl_up_sync(0xffffffffu, l.upto, d);
+    if (lane >= d) l.upto += before;
+  }
+  return l;
 }
 
-// The same for the c-th chunk of all portions, looked up by a whole warp; `count` is how many chunks there are (c beyond them: only that).
+// The c-th chunk, looked up by a whole warp; `count` is how many there are (c beyond them: only that, and no tokens).
 __device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
-  const int lane = threadIdx.x & 31;
   Where w = {};
   count = 0;
   for (int r0 = 0; r0 < p.requests; r0 += 32) {
-    int first = 0, tokens = 0;
-    if (r0 + lane < p.requests) first = p.query_start[r0 + lane], tokens = p.query_start[r0 + lane + 1] - first;
-    const int chunks = tokens > 0 ? (tokens + kC - 1) / kC : 0;
-    int upto = chunks;
-#pragma unroll
-    for (int d = 1; d < 32; d *= 2) {
-      const int before = __shfl_up_sync(0xffffffffu, upto, d);
-      if (lane >= d) upto += before;
-    }
-    const unsigned found = __ballot_sync(0xffffffffu, count + upto > c);
+    const Lane l = portions_from(p, r0);
+    const unsigned found = __ballot_sync(0xffffffffu, count + l.upto > c);
     if (found) {
-      const int at = __ffs(found) - 1;
-      first = __shfl_sync(0xffffffffu, first, at), tokens = __shfl_sync(0xffffffffu, tokens, at);
-      const int mine = c - count - __shfl_sync(0xffffffffu, upto - chunks, at);
+      const int at = __ffs(found) - 1, first = __shfl_sync(0xffffffffu, l.first, at), tokens = __shfl_sync(0xffffffffu, l.tokens, at);
+      const int mine = c - count - __shfl_sync(0xffffffffu, l.upto - l.chunks, at);
       w.request = r0 + at, w.left = tokens - mine * kC, w.len = min(w.left, kC), w.first = first + mine * kC;
-      w.place = (size_t)(first / kC + w.request + mine);
+      w.place = (size_t)c;
       return w;
     }
-    count += __shfl_sync(0xffffffffu, upto, 31);
+    count += __shfl_sync(0xffffffffu, l.upto, 31);
   }
   return w;
+}
+
+// The k-th portion, looked up by a whole warp (no tokens: there are not as many).
+__device__ __forceinline__ Portion portion_of(const Problem& p, int k) {
+  int count = 0;
+  for (int r0 = 0; r0 < p.requests; r0 += 32) {
+    const Lane l = portions_from(p, r0);
+    const unsigned scanned = __ballot_sync(0xffffffffu, l.tokens > 0);
+    const unsigned found = __ballot_sync(0xffffffffu, l.tokens > 0 && __popc(scanned & ((1u << (threadIdx.x & 31)) - 1u)) == k);
+    if (found) {
+      const int at = __ffs(found) - 1;
+      return Portion{r0 + at, __shfl_sync(0xffffffffu, l.first, at), __shfl_sync(0xffffffffu, l.tokens, at),
+                     (size_t)(count + __shfl_sync(0xffffffffu, l.upto - l.chunks, at))};
+    }
+    k -= __popc(scanned), count += __shfl_sync(0xffffffffu, l.upto, 31);
+  }
+  return Portion{};
 }
 
 __device__ __forceinline__ float silu_of(float v) { return v * (1.f / (1.f + expf(-v))); }
@@ -207,7 +222,8 @@ __global__ void __launch_bounds__(kThreads)
 local_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
-  const Where w = where_of(p);
+  int count;
+  const Where w = chunk_of(p, blockIdx.z, count);
   if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* ks = chunk_smem;                     // [64][NP + 4]
@@ -296,13 +312,13 @@ __global__ void __launch_bounds__(256)
 join_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
-  const int request = blockIdx.y, first = p.query_start[request];
-  const int count = (p.query_start[request + 1] - first + kC - 1) / kC;
+  const Portion portion = portion_of(p, blockIdx.y);
+  const int count = (portion.tokens + kC - 1) / kC;
   const size_t all = (size_t)p.heads * p.columns * p.dim, at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * PER;
   if (count <= 0 || at >= all) return;
   const int head = (int)(at / ((size_t)p.columns * p.dim));
-  const size_t place = (size_t)(first / kC + request);
-  float* kept = p.states + (long long)p.state_slots[request] * p.state_stride + p.state_offset + at;
+  const size_t place = portion.place;
+  float* kept = p.states + (long long)p.state_slots[portion.request] * p.state_stride + p.state_offset + at;
   Piece<PER> s;
 #pragma unroll
   for (int e = 0; e < PER; ++e) s.v[e] = kept[e];
@@ -586,7 +602,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 solve_kernel(const Problem p, const Solved out) {
   grid_dependency_wait();
   grid_dependency_launch();
-  const Where w = where_of(p);
+  int count;
+  const Where w = chunk_of(p, blockIdx.z, count);
   if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* ks = chunk_smem;                     // [64][NP + 4]
@@ -739,10 +756,11 @@ carry_kernel(const Problem p, const Solved in) {
   float* s_at = us + 2 * kC * kCarry;         // [16][LD]
   float* u_now = s_at + kCarry * LD;          // [64][16]
   float* parts = u_now + kC * kCarry;         // [4][64][kPartLd]: quarters of W S_0; [1 or 3][16][LD]: sums over other threads' tokens
-  const int tid = threadIdx.x, head = blockIdx.y, request = blockIdx.z, first_column = blockIdx.x * kCarry;
-  const int first = p.query_start[request], q_len = p.query_start[request + 1] - first, count = (q_len + kC - 1) / kC;
+  const int tid = threadIdx.x, head = blockIdx.y, first_column = blockIdx.x * kCarry;
+  const Portion portion = portion_of(p, blockIdx.z);
+  const int request = portion.request, first = portion.first, q_len = portion.tokens, count = (q_len + kC - 1) / kC;
   if (count <= 0) return;
-  const size_t place = (size_t)(first / kC + request);
+  const size_t place = portion.place;
   const int columns_here = min(kCarry, p.vdim - first_column);
   const bool four_wide = p.dim % 4 == 0, four_values = p.vdim % 4 == 0;
   auto fetch = [&](int c, int stage) {
@@ -913,16 +931,23 @@ constexpr size_t read_bytes(int np) { return sizeof(float) * (size_t)(2 * kC * (
 constexpr size_t solve_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 48 * kThreads + 5 * kC); }
 constexpr size_t carry_bytes(int np) { return sizeof(float) * (size_t)(4 * kC * (np + 4) + 3 * kC * kCarry + kCarry * (np + 4) + 4 * kC * kPartLd); }
 
+// The portions and chunks that a step of n tokens brings at most.
+struct Bounds { int portions, chunks; };
+static Bounds bounds_of(int n_tokens, int n_requests, int least) {
+  const int portions = n_tokens / least < n_requests ? n_tokens / least : n_requests;
+  return Bounds{portions, n_tokens / kC + portions};
+}
+
 template <typename Kernel>
 static bool allow(Kernel kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
 
 template <typename T, int FORM, int NP>
-static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
+static int scan(const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
   const int tiles = (p.vdim + kTile - 1) / kTile;
-  const dim3 grid(tiles, p.heads, n_requests * p.most);
-  const long long units = (long long)tiles * p.heads * n_requests * p.most;            // at most
+  const dim3 grid(tiles, p.heads, most.chunks);
+  const long long units = (long long)tiles * p.heads * most.chunks;                    // at most
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const dim3 readers((unsigned)min(units, 2ll * sms));
@@ -932,10 +957,10 @@ static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStre
     auto read = read_kernel<T, float, kDelta, NP>;
     if (!allow(solve, solve_bytes(NP)) || !allow(carry, carry_bytes(NP)) || !allow(read, read_bytes(NP)))
       MS_FAIL("chunk_scan: shared memory refused");
-    ms::launch(solve, dim3((p.dim + p.vdim + kThreads - 1) / kThreads, p.heads, n_requests * p.most), kThreads, solve_bytes(NP), stream, p,
+    ms::launch(solve, dim3((p.dim + p.vdim + kThreads - 1) / kThreads, p.heads, most.chunks), kThreads, solve_bytes(NP), stream, p,
                solved);
     MS_CHECK_LAUNCH("chunk_scan: within the chunks");
-    ms::launch(carry, dim3((p.vdim + kCarry - 1) / kCarry, p.heads, n_requests), kThreads, carry_bytes(NP), stream, p, solved);
+    ms::launch(carry, dim3((p.vdim + kCarry - 1) / kCarry, p.heads, most.portions), kThreads, carry_bytes(NP), stream, p, solved);
     MS_CHECK_LAUNCH("chunk_scan: from chunk to chunk");
     Problem reading = p;
     reading.v = Rows{solved.u, p.heads * p.vdim, 0};
@@ -949,7 +974,7 @@ static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStre
     MS_CHECK_LAUNCH("chunk_scan: chunks alone");
     const bool four = p.dim % 4 == 0;
     const size_t threads = (size_t)p.heads * p.columns * p.dim / (four ? 4 : 1);
-    ms::launch(four ? join_kernel<4> : join_kernel<1>, dim3((unsigned)((threads + 255) / 256), n_requests), 256, 0, stream, p);
+    ms::launch(four ? join_kernel<4> : join_kernel<1>, dim3((unsigned)((threads + 255) / 256), most.portions), 256, 0, stream, p);
     MS_CHECK_LAUNCH("chunk_scan: chunks joined");
     ms::launch(read, readers, kThreads, read_bytes(NP), stream, p);
   }
@@ -958,15 +983,15 @@ static int scan(const Problem& p, int n_requests, const Solved& solved, cudaStre
 }
 
 template <typename T, int FORM>
-static int scan_keys(const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
-  return p.dim <= 64 ? scan<T, FORM, 64>(p, n_requests, solved, stream) : scan<T, FORM, 128>(p, n_requests, solved, stream);
+static int scan_keys(const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
+  return p.dim <= 64 ? scan<T, FORM, 64>(p, most, solved, stream) : scan<T, FORM, 128>(p, most, solved, stream);
 }
 
 template <typename T>
-static int scan_form(int form, const Problem& p, int n_requests, const Solved& solved, cudaStream_t stream) {
-  if (form == kMemory) return scan_keys<T, kMemory>(p, n_requests, solved, stream);
-  if (form == kDelta) return scan_keys<T, kDelta>(p, n_requests, solved, stream);
-  return scan_keys<T, kDecay>(p, n_requests, solved, stream);
+static int scan_form(int form, const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
+  if (form == kMemory) return scan_keys<T, kMemory>(p, most, solved, stream);
+  if (form == kDelta) return scan_keys<T, kDelta>(p, most, solved, stream);
+  return scan_keys<T, kDecay>(p, most, solved, stream);
 }
 
 }  // namespace chunk_scan
@@ -975,33 +1000,32 @@ static int scan_form(int form, const Problem& p, int n_requests, const Solved& s
 using namespace ms;
 using namespace ms::chunk_scan;
 
-// The tokens of a chunk (64) if the step's portions should be scanned in chunks, 0 if the walk, token after token, is the better
-// one or the only one: few tokens (a walk takes about 0.3 us a token, the launches of a scan 20 to 40 us before they have much to
-// do), keys of more than 128 entries, or more chunks than a launch's grid holds.
+// The tokens of a chunk (64) if portions of max_query_len tokens can be scanned in chunks, 0 if the walk, token after token, is the only
+// way: keys of more than 128 entries, or nothing to scan.  (From which sizes on the scans are ahead is the caller's rule.)
 MS_EXPORT int ms_chunk_scan_chunk(int n_requests, int max_query_len, int heads, int dim) {
-  if (n_requests <= 0 || heads <= 0 || heads > 65535 || dim <= 0 || dim > 128 || max_query_len < 96) return 0;
-  if ((long long)n_requests * ((max_query_len + kC - 1) / kC) > 65535) return 0;
-  return kC;
+  return n_requests > 0 && max_query_len > 0 && heads > 0 && heads <= 65535 && dim > 0 && dim <= 128 ? kC : 0;
 }
 
-// Arguments as ms_matrix_scan's forms 0 (memory), 1 (delta) and 2 (constant decay).  chunk_states float32 [places, heads, columns, dim] and
-// chunk_decays float32 [places, heads], places = n_tokens / 64 + n_requests; delta: w, ke float32 [n_tokens, heads, dim], u float32
-// [n_tokens, heads, vdim].  chunk_states and u on 16-byte boundaries.
+// Arguments as ms_matrix_scan's forms 0 (memory), 1 (delta) and 2 (constant decay); portions of fewer than `least` tokens are left
+// alone.  chunk_states float32 [places, heads, columns, dim] and chunk_decays float32 [places, heads], places = n_tokens / 64 +
+// min(n_requests, n_tokens / least), at most 65,535; delta: w, ke float32 [n_tokens, heads, dim], u float32 [n_tokens, heads, vdim].
+// chunk_states and u on 16-byte boundaries.
 MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const void* k, int k_ld, int k_col, const void* v, int v_ld,
                             int v_col, int dtype, float q_scale, const float* gates, float* states, long long state_stride,
-                            int state_offset, const int* state_slots, const int* query_start, int n_requests, int max_query_len,
+                            int state_offset, const int* state_slots, const int* query_start, int n_requests, int n_tokens, int least,
                             int heads, int kv_heads, int dim, int vdim, float* y, float* bottom, int input_act, float* chunk_states,
                             float* chunk_decays, float* w, float* u, float* ke, cudaStream_t stream) {
-  if (n_requests == 0 || max_query_len <= 0 || heads == 0) return 0;
+  if (n_requests == 0 || n_tokens == 0 || heads == 0) return 0;
   MS_REQUIRE(form >= kMemory && form <= kDecay, "chunk_scan: form %d", form);
   MS_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && dim >= 1 && dim <= 128 && vdim >= 1, "chunk_scan: %d/%d heads of %d/%d", heads,
              kv_heads, dim, vdim);
   MS_REQUIRE(form != kDelta || !input_act, "chunk_scan: the delta form takes its inputs as they are");
   MS_REQUIRE(form != kMemory || bottom != nullptr, "chunk_scan: the memory form writes the tokens' divisors");
   MS_REQUIRE(chunk_states && chunk_decays && (form != kDelta || (w && u && ke)), "chunk_scan: scratch is missing");
-  const int most = (max_query_len + kC - 1) / kC;
-  MS_REQUIRE(heads <= 65535 && (long long)n_requests * most <= 65535, "chunk_scan: %d heads, %d requests of %d chunks exceed the launch limits",
-             heads, n_requests, most);
+  MS_REQUIRE(least >= 1, "chunk_scan: portions of %d tokens and more", least);
+  const Bounds most = bounds_of(n_tokens, n_requests, least);
+  if (most.portions == 0) return 0;
+  MS_REQUIRE(heads <= 65535 && most.chunks <= 65535, "chunk_scan: %d heads, %d chunks exceed the launch limits", heads, most.chunks);
   const int per = dtype == MS_F32 ? 4 : 8;
   auto aligned = [](const void* at) { return reinterpret_cast<size_t>(at) % 16 == 0; };
   const int wide = aligned(q) && aligned(k) && aligned(v) && q_ld % per == 0 && k_ld % per == 0 && v_ld % per == 0 && q_col % per == 0 &&
@@ -1011,27 +1035,28 @@ MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const 
   p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim, p.columns = form == kMemory ? vdim + 1 : vdim;
   p.input_act = input_act, p.wide = wide, p.q_scale = q_scale, p.gates = gates;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
-  p.requests = n_requests, p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
+  p.requests = n_requests, p.least = least, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
   const Solved solved{w, u, ke};
-  if (dtype == MS_F32) return scan_form<float>(form, p, n_requests, solved, stream);
-  if (dtype == MS_BF16) return scan_form<__nv_bfloat16>(form, p, n_requests, solved, stream);
+  if (dtype == MS_F32) return scan_form<float>(form, p, most, solved, stream);
+  if (dtype == MS_BF16) return scan_form<__nv_bfloat16>(form, p, most, solved, stream);
   MS_FAIL("unknown element type code %d", dtype);
 }
 
-// Arguments as ms_selective_scan; scratch as above with columns = p (a head's channels) and dim = n_state.
+// Arguments as ms_selective_scan; `least` and scratch as above with columns = p (a head's channels) and dim = n_state.
 MS_EXPORT int ms_selective_chunk_scan(const float* conv, int conv_ld, const void* proj, int dtype, int ld, int dt_col, const float* dt_bias,
                                       const float* a_log, const float* d, float* states, long long state_stride, int state_offset,
-                                      const int* state_slots, const int* query_start, int n_requests, int max_query_len, int heads,
+                                      const int* state_slots, const int* query_start, int n_requests, int n_tokens, int least, int heads,
                                       int channels, int n_state, int groups, float* y, float* chunk_states, float* chunk_decays,
                                       cudaStream_t stream) {
-  if (n_requests == 0 || max_query_len <= 0) return 0;
+  if (n_requests == 0 || n_tokens == 0) return 0;
   MS_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "selective_chunk_scan: %d heads in %d groups", heads, groups);
   MS_REQUIRE(n_state >= 1 && n_state <= 128 && channels >= 1, "selective_chunk_scan: a state of %d numbers for %d channels", n_state, channels);
   MS_REQUIRE(dtype == MS_F32 || dtype == MS_BF16, "unknown element type code %d", dtype);
   MS_REQUIRE(chunk_states && chunk_decays, "selective_chunk_scan: scratch is missing");
-  const int most = (max_query_len + kC - 1) / kC;
-  MS_REQUIRE(heads <= 65535 && (long long)n_requests * most <= 65535,
-             "selective_chunk_scan: %d heads, %d requests of %d chunks exceed the launch limits", heads, n_requests, most);
+  MS_REQUIRE(least >= 1, "selective_chunk_scan: portions of %d tokens and more", least);
+  const Bounds most = bounds_of(n_tokens, n_requests, least);
+  if (most.portions == 0) return 0;
+  MS_REQUIRE(heads <= 65535 && most.chunks <= 65535, "selective_chunk_scan: %d heads, %d chunks exceed the launch limits", heads, most.chunks);
   const int inner = heads * channels;
   Problem p = {};
   p.v = Rows{conv, conv_ld, 0}, p.k = Rows{conv, conv_ld, inner}, p.q = Rows{conv, conv_ld, inner + groups * n_state};
@@ -1040,6 +1065,6 @@ MS_EXPORT int ms_selective_chunk_scan(const float* conv, int conv_ld, const void
   p.q_scale = 1.f;
   p.step = proj, p.step_dtype = dtype, p.step_ld = ld, p.step_col = dt_col, p.step_bias = dt_bias, p.a_log = a_log, p.skip = d;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
-  p.requests = n_requests, p.most = most, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
-  return scan_keys<float, kSelective>(p, n_requests, Solved{}, stream);
+  p.requests = n_requests, p.least = least, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
+  return scan_keys<float, kSelective>(p, most, Solved{}, stream);
 }

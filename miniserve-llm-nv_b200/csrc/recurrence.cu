@@ -229,7 +229,7 @@ matrix_scan_kernel(const T* __restrict__ q, int q_ld, int q_col, const T* __rest
                    float* __restrict__ states, long long state_stride, int state_offset,
                    const int* __restrict__ state_slots, const int* __restrict__ query_start, int heads, int kv_heads, int dim,
                    int vdim, int lpc_shift, int tok, float* __restrict__ y, float* __restrict__ bottom, int gate_ld,
-                   int gate_col, const float* __restrict__ channel_decay, int input_act) {
+                   int gate_col, const float* __restrict__ channel_decay, int input_act, int below) {
   grid_dependency_wait();
   grid_dependency_launch();
   extern __shared__ __align__(16) float matrix_smem[];
@@ -248,7 +248,7 @@ matrix_scan_kernel(const T* __restrict__ q, int q_ld, int q_col, const T* __rest
   const int head = blockIdx.y, request = blockIdx.z;
   const int kv_head = head / (heads / kv_heads);
   const int q0 = query_start[request], q_len = query_start[request + 1] - q0;
-  if (q_len <= 0) return;                                    // (the whole block)
+  if (q_len <= 0 || q_len >= below) return;                  // (the whole block)
   float* ks = matrix_smem;                                    // [tok][row]
   float* qs = ks + tok * row;                                 // [tok][row]
   float* vs = qs + tok * row;                                 // [tok][cols_per_block]
@@ -782,12 +782,13 @@ static int scan_sm_count() {
 // mode 2 (decay): gates [heads], the heads' constant decays; state [heads, vdim, dim].  mode 3 (channel delta): gates are rows
 // of gate_ld float32 numbers whose columns gate_col .. gate_col + heads hold the logits of beta; channel_decay float32
 // [tokens, heads, dim]; state [heads, vdim, dim].  mode 4 (channel decay): channel_decay as in mode 3, gates unused; the same state.  input_act != 0: q, k and v pass SiLU as they are read.
+// Portions of `below` tokens or more are left alone.
 MS_EXPORT int ms_matrix_scan(int mode, const void* q, int q_ld, int q_col, const void* k, int k_ld, int k_col, const void* v,
                              int v_ld, int v_col, int dtype, float q_scale, const float* gates, float* states,
                              long long state_stride, int state_offset, const int* state_slots, const int* query_start,
                              int n_requests, int max_query_len, int heads, int kv_heads, int dim, int vdim, float* y,
                              float* bottom, int gate_ld, int gate_col, const float* channel_decay, int input_act,
-                             cudaStream_t stream) {
+                             int below, cudaStream_t stream) {
   if (n_requests == 0 || max_query_len <= 0 || heads == 0) return 0;
   MS_REQUIRE(mode >= kModeMemory && mode <= kModeChannelDecay, "matrix_scan: mode %d", mode);
   MS_REQUIRE(mode != kModeChannelDecay || channel_decay != nullptr, "matrix_scan: the channel form needs the channels' decays");
@@ -833,7 +834,7 @@ MS_EXPORT int ms_matrix_scan(int mode, const void* q, int q_ld, int q_col, const
   MS_REC_DISPATCH(dtype, (ms::launch(matrix_scan_kernel<T, R, MODE>, grid, kScanThreads, smem, stream, (const T*)q, q_ld, q_col, \
                                      (const T*)k, k_ld, k_col, (const T*)v, v_ld, v_col, q_scale, gates, states, state_stride,  \
                                      state_offset, state_slots, query_start, heads, kv_heads, dim, vdim, lpc_shift, tok, y,     \
-                                     bottom, gate_ld, gate_col, channel_decay, input_act)))
+                                     bottom, gate_ld, gate_col, channel_decay, input_act, below)))
   if (mode == kModeMemory) {
     if (r == 4) { MS_MATRIX_SCAN(4, kModeMemory); } else if (r == 8) { MS_MATRIX_SCAN(8, kModeMemory); }
     else if (r == 16) { MS_MATRIX_SCAN(16, kModeMemory); } else { MS_MATRIX_SCAN(32, kModeMemory); }

@@ -215,7 +215,7 @@ selective_scan_kernel(const float* __restrict__ conv, int conv_ld, const T* __re
                       const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                       float* __restrict__ states, long long state_stride, int state_offset,
                       const int* __restrict__ state_slots, const int* __restrict__ query_start, int heads, int P, int N,
-                      int groups, float* __restrict__ y, int wide, int short_tok) {
+                      int groups, float* __restrict__ y, int wide, int short_tok, int below) {
   grid_dependency_wait();
   grid_dependency_launch();
   constexpr int COLS = kScanWarps * CP;
@@ -227,7 +227,7 @@ selective_scan_kernel(const float* __restrict__ conv, int conv_ld, const T* __re
   const int head = blockIdx.y, request = blockIdx.z;
   const int block_p0 = blockIdx.x * COLS, p0 = block_p0 + warp * CP;
   const int q0 = query_start[request], q_len = query_start[request + 1] - q0;
-  if (q_len <= 0) return;                                   // (the whole block)
+  if (q_len <= 0 || q_len >= below) return;                 // (the whole block)
   const int group = head / (heads / groups);
   const int inner = heads * P;
   const float* conv_x = conv + (size_t)q0 * conv_ld + head * P + block_p0;
@@ -548,12 +548,13 @@ MS_EXPORT int ms_scan_max_state() { return kScanMaxState; }
 
 // conv float32 [tokens, conv_ld] = [x: heads * P | B: groups * N | C: groups * N]; dt is column dt_col + head of proj;
 // dt_bias, a_log, d float32 [heads]; the heads' states [heads][P][N] at state_offset of a slot's row; y float32
-// [tokens, heads * P].  max_query_len: an upper bound of the tokens a request brings (it sizes the chunks).
+// [tokens, heads * P].  max_query_len: an upper bound of the tokens a request brings (it sizes the chunks).  Portions of
+// `below` tokens or more are left alone.
 MS_EXPORT int ms_selective_scan(const float* conv, int conv_ld, const void* proj, int dtype, int ld, int dt_col,
                                 const float* dt_bias, const float* a_log, const float* d, float* states,
                                 long long state_stride, int state_offset, const int* state_slots, const int* query_start,
                                 int n_requests, int max_query_len, int heads, int p, int n_state, int groups, float* y,
-                                cudaStream_t stream) {
+                                int below, cudaStream_t stream) {
   if (n_requests == 0 || max_query_len <= 0) return 0;
   MS_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "selective_scan: %d heads in %d groups", heads, groups);
   MS_REQUIRE(n_state >= 1 && n_state <= kScanMaxState, "selective_scan: a state of %d numbers per channel outside 1..%d",
@@ -581,7 +582,7 @@ MS_EXPORT int ms_selective_scan(const float* conv, int conv_ld, const void* proj
         configured[full + 2 * brief] = true;                                                                                   \
       }                                                                                                                        \
       ms::launch(kernel, grid, kScanWarps * 32, smem, stream, conv, conv_ld, (const T*)proj, ld, dt_col, dt_bias, a_log, d,    \
-                 states, state_stride, state_offset, state_slots, query_start, heads, p, n_state, groups, y, wide, tok);       \
+                 states, state_stride, state_offset, state_slots, query_start, heads, p, n_state, groups, y, wide, tok, below); \
     })                                                                                                                         \
   }
   if (per_lane <= 1) MS_SCAN(1, 4, 32) else if (per_lane <= 2) MS_SCAN(2, 4, 32) else if (per_lane <= 4) MS_SCAN(4, 4, 32) else MS_SCAN(8, 2, 16)

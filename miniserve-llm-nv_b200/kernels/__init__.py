@@ -16,7 +16,7 @@ import torch
 
 from . import build
 
-ABI_VERSION = 13
+ABI_VERSION = 14
 log = logging.getLogger("miniserve_b200")
 _library: Optional[ctypes.CDLL] = None
 
@@ -957,6 +957,11 @@ MAX_CHUNK_SCRATCH = 1 << 30   # bytes of chunk states beyond which a scan walks 
 # 89, 4 of 128: 160 / 136; 32 heads: 192: 76 / 86, 256: 89 / 90, 320: 123 / 90; memory: 1 of 128: 93 / 104, 192: 102 / 105, 256: 123 / 107, 4 of 128:
 # 160 / 108; delta: 1 of 192: 134 / 136, 256: 163 / 139, 4 of 320: 251 / 270, 4 of 448: 339 / 335.
 CHUNK_SCAN_LONGEST, CHUNK_SCAN_OF_MANY, CHUNK_SCAN_DELTA = 256, (128, 512), 128
+# In a step that is scanned in chunks, portions of fewer tokens than this, the decoded tokens beside a prompt above all, are walked: a chunk's
+# matrix passes through memory four more times than a state that is walked, and needs some forty tokens to be worth it (selective, 64
+# heads, where the state is largest).
+CHUNK_SCAN_LEAST = 32
+MAX_INT = 2 ** 31 - 1
 
 
 def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False) -> Optional[tuple]:
@@ -967,13 +972,18 @@ def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, 
     elif longest < CHUNK_SCAN_LONGEST and (longest < CHUNK_SCAN_OF_MANY[0] or n < CHUNK_SCAN_OF_MANY[1]):
         return None
     chunk = library().ms_chunk_scan_chunk(_i(n_requests), _i(longest), _i(heads), _i(dim))
-    if not chunk:
+    if not chunk or longest < CHUNK_SCAN_LEAST:
         return None
-    places = n // chunk + n_requests
-    if 4 * places * heads * columns * dim > MAX_CHUNK_SCRATCH:
+    places = n // chunk + min(n_requests, n // CHUNK_SCAN_LEAST)
+    if places > 65535 or 4 * places * heads * columns * dim > MAX_CHUNK_SCRATCH:
         return None
     return (torch.empty((places, heads, columns, dim), dtype=torch.float32, device=device),
             torch.empty((places, heads), dtype=torch.float32, device=device))
+
+
+def _none_short(n: int, n_requests: int, longest: int) -> bool:
+    """Whether ``n`` tokens of ``n_requests`` requests, of at most ``longest`` each, leave none with fewer than CHUNK_SCAN_LEAST."""
+    return n - (n_requests - 1) * longest >= CHUNK_SCAN_LEAST
 
 
 def causal_conv_silu(proj: torch.Tensor, col: int, weight: torch.Tensor, bias: torch.Tensor, states: torch.Tensor,
@@ -1044,13 +1054,17 @@ def selective_scan(conv: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias:
     if scratch is not None:
         _check(library().ms_selective_chunk_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
                                                  _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
-                                                 _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(longest), _i(heads),
-                                                 _i(head_dim), _i(state), _i(groups), _ptr(y), _ptr(scratch[0]), _ptr(scratch[1]), _stream()))
-        return
+                                                 _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n), _i(CHUNK_SCAN_LEAST),
+                                                 _i(heads), _i(head_dim), _i(state), _i(groups), _ptr(y), _ptr(scratch[0]),
+                                                 _ptr(scratch[1]), _stream()))
+        if _none_short(n, n_requests, longest):
+            return
+        longest = min(longest, CHUNK_SCAN_LEAST - 1)
     _check(library().ms_selective_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
                                        _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
                                        _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(longest),
-                                       _i(heads), _i(head_dim), _i(state), _i(groups), _ptr(y), _stream()))
+                                       _i(heads), _i(head_dim), _i(state), _i(groups), _ptr(y),
+                                       _i(MAX_INT if scratch is None else CHUNK_SCAN_LEAST), _stream()))
 
 
 def gated_group_norm(y: torch.Tensor, proj: torch.Tensor, z_col: int, weight: torch.Tensor, groups: int, eps: float,
@@ -1206,16 +1220,19 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
             solved = [torch.empty((n, heads, size), dtype=torch.float32, device=y.device) for size in (dim, vdim, dim)]
         _check(library().ms_chunk_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                        _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
-                                       _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(max_query_len),
-                                       _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _ptr(bottom),
+                                       _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n),
+                                       _i(CHUNK_SCAN_LEAST), _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _ptr(bottom),
                                        _i(CONV_ACTIVATIONS[input_activation]), _ptr(scratch[0]), _ptr(scratch[1]), _ptr(solved[0]),
                                        _ptr(solved[1]), _ptr(solved[2]), _stream()))
-        return
+        if _none_short(n, n_requests, max_query_len):
+            return
+        max_query_len = min(max_query_len, CHUNK_SCAN_LEAST - 1)
     _check(library().ms_matrix_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                     _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
                                     _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(max_query_len),
                                     _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _ptr(bottom), _i(gate_ld), _i(gate_col),
-                                    _ptr(channel_decay) if code >= 3 else None, _i(CONV_ACTIVATIONS[input_activation]), _stream()))
+                                    _ptr(channel_decay) if code >= 3 else None, _i(CONV_ACTIVATIONS[input_activation]),
+                                    _i(MAX_INT if scratch is None else CHUNK_SCAN_LEAST), _stream()))
 
 
 def channel_decays(logits: torch.Tensor, col: int, a_log: torch.Tensor, dt_bias: torch.Tensor, per_head: int, out: torch.Tensor) -> None:

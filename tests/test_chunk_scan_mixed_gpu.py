@@ -1,0 +1,98 @@
+"""Which steps are scanned in chunks, with the rules in force, and steps that mix portions with decoded tokens: those are walked beside the
+scan, as they are in a step of their own."""
+
+import pytest
+import torch
+
+from test_chunk_scan_gpu import ints, problem, run
+
+pytestmark = pytest.mark.gpu
+
+MIXED = [[300] + [1] * 40, [1, 31, 32, 33, 400, 0, 2], [1] * 33 + [260, 5, 700, 1]]
+
+
+def counted(monkeypatch, *names):
+    from miniserve_b200 import kernels
+
+    lib, calls = kernels.library(), dict.fromkeys(names, 0)
+    for name in names:
+        def wrapped(*args, _name=name, _real=getattr(lib, name)):
+            calls[_name] += 1
+            return _real(*args)
+        monkeypatch.setattr(lib, name, wrapped)
+    return calls
+
+
+@pytest.mark.parametrize("form", ["memory", "delta", "decay"])
+@pytest.mark.parametrize("lengths", MIXED)
+def test_matrix_scan(monkeypatch, form, lengths):
+    if form == "delta":
+        lengths = [3 * length if length >= 256 else length for length in lengths]      # (its rule asks for longer portions)
+    heads, kv_heads, dim, vdim = 4, 2, 64, 80
+    rows, cols, gates, slots, states, kv_heads, columns = problem(form, torch.bfloat16, lengths, heads, kv_heads, dim, vdim, 7)
+    walked = states.clone()
+    calls = counted(monkeypatch, "ms_chunk_scan", "ms_matrix_scan")
+    y, bottom = run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, vdim)
+    assert calls == {"ms_chunk_scan": 1, "ms_matrix_scan": 1}
+    y_walk, bottom_walk = run(form, rows, cols, gates, slots, walked, lengths, heads, kv_heads, dim, vdim, chunk=0)
+    assert calls == {"ms_chunk_scan": 1, "ms_matrix_scan": 2}
+    scale, at = max(1.0, float(y_walk.abs().max())), 0
+    for r, length in enumerate(lengths):
+        pairs = [(y[at:at + length], y_walk[at:at + length]), (states[slots[r]], walked[slots[r]])]
+        if form == "memory":
+            pairs.append((bottom[at:at + length], bottom_walk[at:at + length]))
+        for a, b in pairs:                                  # (either way is within 2e-5 of the definition)
+            assert torch.equal(a, b) if length < 32 else float((a - b).abs().max()) <= 4e-5 * scale
+        assert length < 32 or not torch.equal(states[slots[r]], walked[slots[r]])
+        at += length
+
+
+@pytest.mark.parametrize("lengths", MIXED)
+def test_selective_scan(monkeypatch, lengths):
+    from miniserve_b200 import kernels
+
+    heads, P, N, G = 4, 64, 100, 2
+    g = torch.Generator(device="cuda").manual_seed(len(lengths))
+    n, inner = sum(lengths), heads * P
+    conv = torch.randn((n, inner + 2 * G * N), generator=g, device="cuda") * 0.5
+    proj = (torch.randn((n, heads), generator=g, device="cuda") * 2).bfloat16()
+    dt_bias, a_log, skip = (torch.randn(heads, generator=g, device="cuda") for _ in range(3))
+    slots = torch.randperm(len(lengths), generator=g, device="cuda")
+    start = torch.randn((len(lengths), inner * N), generator=g, device="cuda") * 0.3
+    calls = counted(monkeypatch, "ms_selective_chunk_scan", "ms_selective_scan")
+
+    def scan(tokens, requests, **options):
+        """The rows of y and the states of a step of these requests (their tokens given)."""
+        states, y = start.clone(), torch.full((len(tokens), inner), float("nan"), device="cuda")
+        own = [lengths[r] for r in requests]
+        kernels.selective_scan(conv[tokens], proj[tokens], 0, dt_bias, a_log, skip, states, 0, slots[requests].to(torch.int32),
+                               ints([sum(own[:i]) for i in range(len(own) + 1)]), heads, P, N, G, y, max_query_len=max(own), **options)
+        return y, states
+
+    request_of = [r for r, length in enumerate(lengths) for _ in range(length)]
+    everything, short = list(range(len(lengths))), [r for r, length in enumerate(lengths) if length < 32]
+    short_tokens = [t for t in range(n) if lengths[request_of[t]] < 32]
+    long_tokens = [t for t in range(n) if lengths[request_of[t]] >= 32]
+    y, states = scan(list(range(n)), everything)
+    assert calls == {"ms_selective_chunk_scan": 1, "ms_selective_scan": 1}
+    y_alone, alone = scan(short_tokens, short)
+    assert torch.equal(y[short_tokens], y_alone) and torch.equal(states[slots[short]], alone[slots[short]])
+    y_walk, walked = scan(list(range(n)), everything, chunked=False)
+    assert calls == {"ms_selective_chunk_scan": 1, "ms_selective_scan": 3}
+    scale = max(1.0, float(y_walk.abs().max()))             # (either way is within 2e-5 of the definition)
+    assert float((y - y_walk)[long_tokens].abs().max()) <= 4e-5 * scale and float((states - walked).abs().max()) <= 4e-5 * scale
+
+
+@pytest.mark.parametrize("lengths,delta,taken,walk_beside", [
+    ([255], False, False, False), ([256], False, True, False), ([127, 385], False, True, False), ([127] * 5, False, False, False),
+    ([128] * 4, False, True, False), ([300, 200, 100], False, True, True), ([128] * 3 + [127], False, False, False), ([256, 32], False, True, False), ([256, 31], False, True, True),
+    ([255], True, False, False), ([256], True, True, False), ([383, 1], True, False, False), ([384, 1], True, True, True),
+    ([500] * 4, True, False, False), ([640] * 4, True, True, False)])
+def test_which_steps_are_scanned_in_chunks(monkeypatch, lengths, delta, taken, walk_beside):
+    """256 tokens, or 128 in a step of 512; the delta form 128 (1 + portions of that length that the step would fill).  Of more than two
+    unequal portions one may be too short for a chunk, as far as the host knows: the walk is launched beside the scan then."""
+    form = "delta" if delta else "memory"
+    rows, cols, gates, slots, states, kv_heads, columns = problem(form, torch.bfloat16, lengths, 1, 1, 8, 8, 3)
+    calls = counted(monkeypatch, "ms_chunk_scan", "ms_matrix_scan")
+    run(form, rows, cols, gates, slots, states, lengths, 1, kv_heads, 8, 8)
+    assert calls == {"ms_chunk_scan": int(taken), "ms_matrix_scan": int(walk_beside or not taken)}
