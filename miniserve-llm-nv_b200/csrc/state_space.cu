@@ -206,7 +206,7 @@ __device__ __forceinline__ void scan_copy(float* dst, const float* src, bool val
   }
 }
 
-// FULL: the state is a multiple of 32 numbers and the head's channels a multiple of the block's (no lane or column is idle,
+// FULL: the state is 32 R numbers and the head's channels a multiple of the block's (no lane or column is idle,
 // and no bound is tested per token).
 // SHORT: no request of the step brings TOK tokens, and the chunks are as long as the longest portion (a run-time number).
 template <typename T, int R, int CP, int TOK, bool FULL, bool SHORT>
@@ -564,7 +564,8 @@ MS_EXPORT int ms_selective_scan(const float* conv, int conv_ld, const void* proj
   // the copies into shared memory move four floats at a time where every row of B and C starts on a 16-byte boundary
   const int inner = heads * p;
   const int wide = (n_state % 4 == 0 && conv_ld % 4 == 0 && inner % 4 == 0 && (reinterpret_cast<uintptr_t>(conv) & 15) == 0) ? 1 : 0;
-  const int full = (n_state % 32 == 0 && p % (kScanWarps * (per_lane <= 4 ? 4 : 2)) == 0) ? 1 : 0;
+  const int lane_entries = per_lane <= 2 ? per_lane : per_lane <= 4 ? 4 : 8;             // (R below)
+  const int full = (n_state == 32 * lane_entries && p % (kScanWarps * (per_lane <= 4 ? 4 : 2)) == 0) ? 1 : 0;
   // columns per warp: four where a lane holds few entries (more products per load), two where it holds many
 #define MS_SCAN(R, CP, TOK)                                                                                                    \
   {                                                                                                                            \

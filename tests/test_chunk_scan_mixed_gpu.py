@@ -4,7 +4,7 @@ scan, as they are in a step of their own."""
 import pytest
 import torch
 
-from test_chunk_scan_gpu import ints, problem, run
+from test_chunk_scan_gpu import ints, problem, recurrence, run
 
 pytestmark = pytest.mark.gpu
 
@@ -51,7 +51,7 @@ def test_matrix_scan(monkeypatch, form, lengths):
 def test_selective_scan(monkeypatch, lengths):
     from miniserve_b200 import kernels
 
-    heads, P, N, G = 4, 64, 100, 2
+    heads, P, N, G = 4, 64, 96, 2
     g = torch.Generator(device="cuda").manual_seed(len(lengths))
     n, inner = sum(lengths), heads * P
     conv = torch.randn((n, inner + 2 * G * N), generator=g, device="cuda") * 0.5
@@ -96,3 +96,32 @@ def test_which_steps_are_scanned_in_chunks(monkeypatch, lengths, delta, taken, w
     calls = counted(monkeypatch, "ms_chunk_scan", "ms_matrix_scan")
     run(form, rows, cols, gates, slots, states, lengths, 1, kv_heads, 8, 8)
     assert calls == {"ms_chunk_scan": int(taken), "ms_matrix_scan": int(walk_beside or not taken)}
+
+
+@pytest.mark.parametrize("N", [32, 64, 96, 128, 160, 192, 224, 256])
+@pytest.mark.parametrize("lengths", [[1] * 5, [7, 1], [40]])
+def test_the_walk_with_states_of_any_multiple_of_32(N, lengths):
+    """A lane has 1, 2, 4 or 8 entries of a column: states of 96, 160, 192 and 224 numbers leave some of them empty."""
+    from miniserve_b200 import kernels
+
+    heads, P, G = 2, 32, 1
+    g = torch.Generator(device="cuda").manual_seed(N)
+    n, inner = sum(lengths), heads * P
+    conv = torch.randn((n, inner + 2 * G * N), generator=g, device="cuda") * 0.5
+    proj = torch.randn((n, heads), generator=g, device="cuda").bfloat16()
+    dt_bias, a_log, skip = (torch.randn(heads, generator=g, device="cuda") for _ in range(3))
+    start = torch.randn((len(lengths), inner * N), generator=g, device="cuda") * 0.3
+    states, y = start.clone(), torch.full((n, inner), float("nan"), device="cuda")
+    starts = [sum(lengths[:r]) for r in range(len(lengths) + 1)]
+    kernels.selective_scan(conv, proj, 0, dt_bias, a_log, skip, states, 0, ints(list(range(len(lengths)))), ints(starts), heads, P, N, G, y,
+                           max_query_len=max(lengths), chunked=False)
+    for r, length in enumerate(lengths):
+        here, rows = conv[starts[r]:starts[r + 1]].double(), slice(starts[r], starts[r + 1])
+        b, c = (here[:, at:at + N].view(length, 1, N).repeat_interleave(heads, 1) for at in (inner, inner + N))
+        x = here[:, :inner].view(length, heads, P)
+        dt = torch.nn.functional.softplus(proj[rows].double() + dt_bias.double())
+        want, after = recurrence("ssm", c, b, x, torch.exp(-torch.exp(a_log.double()) * dt), dt, start[r].double().view(heads, P, N))
+        want = (want + skip.double()[:, None] * x).reshape(length, inner)
+        scale = max(1.0, float(want.abs().max()))
+        assert float((y[rows].double() - want).abs().max()) <= 2e-5 * scale                 # (the walk's bound, as above)
+        assert float((states[r].double() - after.flatten()).abs().max()) <= 2e-5 * scale
