@@ -62,7 +62,7 @@ __device__ __forceinline__ void store_row(float (&v)[32], __nv_bfloat16* row, in
     count = 16, col >>= 1;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
-      v[i] = activation == kActSiluGlu ? silu_glu_bf16(v[2 * i], v[2 * i + 1], scale) : clamped_glu_bf16(v[2 * i], v[2 * i + 1], limit);
+      v[i] = activation == kActSiluGlu ? silu_glu(v[2 * i], v[2 * i + 1], scale) : clamped_glu(v[2 * i], v[2 * i + 1], limit);
   } else if (activation == kActReluSquare) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
