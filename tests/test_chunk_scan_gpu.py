@@ -17,6 +17,11 @@ def in_chunks_from_96_tokens_on(monkeypatch):
 
     for name, value in (("CHUNK_SCAN_LONGEST", 0), ("CHUNK_SCAN_DELTA", 0)):
         monkeypatch.setattr(kernels, name, value)
+    lib, scans = kernels.library(), []
+    for name in ("ms_chunk_scan", "ms_selective_chunk_scan"):
+        monkeypatch.setattr(lib, name, lambda *args, real=getattr(lib, name): scans.append(1) or real(*args))
+    yield
+    assert len(scans) >= 1                             # (not the walk compared with itself)
 
 
 def ints(values):

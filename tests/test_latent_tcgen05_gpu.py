@@ -61,10 +61,12 @@ def test_against_float64(rank, rot, heads, page, new, before, window):
         seen = (key <= token) & (key > token - (window or 1 << 30))
         p = torch.softmax(scores.masked_fill(~seen, -torch.inf), dim=-1)
         want = torch.einsum("htk,kd->thd", p, keys[:, :rank])
-        # probabilities rounded to bfloat16 (2^-9 of each) and the result once more: 2^-8 of the sums of magnitudes, and scores in
-        # float32, whose errors (dk 2^-23 of their magnitudes) enter the exponent
+        # probabilities rounded to bfloat16 (2^-9 of each, in the sum too) and the result once more: 3 2^-9 of the sums of magnitudes; and scores
+        # in float32, off by at most dk 2^-23 of the sums of their products' magnitudes, in a probability and in the sum of all
         size = torch.einsum("htk,kd->thd", p, keys[:, :rank].abs())
-        slack = dk * 2.0 ** -23 * float((here.abs().amax() * keys.abs().amax() * dk * scale))
+        products = torch.einsum("thd,kd->htk", here.abs(), keys.abs()) * scale
+        slack = 2 * dk * 2.0 ** -23 * (products * seen).amax(dim=-1).T[:, :, None]
+        assert float(slack.max()) < 2.0 ** -6
         assert torch.all((out[starts[r]:starts[r + 1]].double() - want).abs() <= (2.0 ** -7 + slack) * size + 1e-6)
 
 
@@ -143,3 +145,45 @@ def test_which_decode_steps_may_take_it(monkeypatch, n, heads, bound, taken):
     kernels.latent_attention(q, cache, ints[0], ints[1], lens - 1, torch.arange(n + 1, dtype=torch.int32, device="cuda"), lens, 1, bound, 256,
                              0.1, None, out)
     assert bool(calls) is taken and torch.all(out == 1.0)
+
+
+@pytest.mark.parametrize("rank,rot,heads,page", [(256, 32, 16, 64), (256, 64, 8, 16), (128, 32, 16, 32), (64, 16, 4, 128)])
+@pytest.mark.parametrize("new", [1, 3])
+@pytest.mark.parametrize("window", [None, 70])
+def test_the_key_at_a_border_decides(rank, rot, heads, page, new, window):
+    """One key's score is far above all others': the first or the last of a piece, a tile, a range, a page or the window, the newest, or one just
+    out of sight.  A key too many or too few changes the whole output."""
+    from miniserve_b200 import kernels
+
+    dk, g = rank + rot, torch.Generator(device="cuda").manual_seed(rank + heads)
+    cases = []
+    for length in (16, 17, 64, 65, 129, 400, 1300):
+        borders = {0, 15, 16, 31, 32, 63, 64, 127, 128, 191, 192, 255, 256, 639, 640, length - 2, length - 1}
+        if window:
+            borders |= {length - window - d for d in range(-1, new + 2)} | {(length - window) // 64 * 64}
+        cases += [(length, b) for b in sorted(borders) if 0 <= b < length]
+    width = (1300 + page - 1) // page
+    lens = torch.tensor([length for length, _ in cases], dtype=torch.int32, device="cuda")
+    n = len(cases)
+    cache = torch.full((n, width * page, dk), float("nan"), device="cuda").bfloat16()
+    for r, (length, border) in enumerate(cases):
+        cache[r, :length, :rank] = torch.randn((length, rank), generator=g, device="cuda").bfloat16()
+        cache[r, :length, rank:] = 0
+        cache[r, border, rank] = 16.0
+    tables = torch.arange(n * width, dtype=torch.int32, device="cuda").view(n, width)
+    q = torch.zeros((n * new, heads, dk), device="cuda").bfloat16()
+    q[:, :, rank] = 1.0
+    starts = torch.arange(n + 1, dtype=torch.int32, device="cuda") * new
+    positions = (lens[:, None] - new + torch.arange(new, device="cuda")).flatten().to(torch.int32)
+    requests = torch.arange(n, device="cuda").repeat_interleave(new).to(torch.int32)
+    out = torch.empty((n * new, heads, rank), device="cuda").bfloat16()
+    kernels.latent_attention(q, cache.view(n * width, page, dk), tables, requests, positions, starts, lens, new, 1300, rank, 1.0, window, out)
+    kernels.check_device_errors(q.device)
+    for r, (length, border) in enumerate(cases):
+        for t in range(new):
+            last = length - new + t
+            first = max(0, last - window + 1) if window else 0
+            rows = cache[r, first:last + 1].double()
+            p = torch.softmax(rows[:, rank], dim=0)
+            want, size = p @ rows[:, :rank], p @ rows[:, :rank].abs()
+            assert torch.all((out[r * new + t].double() - want).abs() <= 2.0 ** -7 * size + 1e-6), (length, border, t)
