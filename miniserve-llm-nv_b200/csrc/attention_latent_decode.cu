@@ -237,7 +237,7 @@ static int launch(const void* q_full, const void* cache, const int* block_tables
                   int splits, int ranges, int least, int tile_ranges, int n_requests, int* error_flag, cudaStream_t stream) {
   static_assert(2 * (smem_bytes(NKC) + 2048) <= 228 * 1024, "the ranges are chosen for two blocks a multiprocessor");
   auto kernel = latent_decode_kernel<NKC>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(NKC));
+  const cudaError_t e = allow_shared(kernel, smem_bytes(NKC));
   if (e != cudaSuccess) MS_FAIL("latent_decode: %zu bytes of shared memory refused: %s", smem_bytes(NKC), cudaGetErrorString(e));
   ms::launch(kernel, dim3((heads + 15) / 16, n_requests, splits), 32 * WARPS, smem_bytes(NKC), stream, (const __nv_bfloat16*)q_full,
              (const __nv_bfloat16*)cache, block_tables, table_stride, query_start, context_lens, page_size, heads,

@@ -414,7 +414,7 @@ int launch(const void* q, const void* cache, int n_pages, const int* block_table
     MS_REQUIRE(encode(&map_k, 2, cache, dims, strides, box), "latent_attention: tensor map of the cache failed");
   }
   auto kernel = latent_tcgen05_kernel<RANK>;
-  const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<RANK>::TOTAL);
+  const cudaError_t allowed = allow_shared(kernel, Layout<RANK>::TOTAL);
   if (allowed != cudaSuccess) MS_FAIL("latent_attention: %zu bytes of shared memory refused: %s", Layout<RANK>::TOTAL, cudaGetErrorString(allowed));
   const long long tiles = ((long long)max_query_len * heads + ROWS - 1) / ROWS;
   MS_REQUIRE(tiles <= 2147483647LL && n_requests <= 65535, "latent_attention: grid exceeds the launch limits");

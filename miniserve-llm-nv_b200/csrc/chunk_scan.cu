@@ -938,11 +938,6 @@ static Bounds bounds_of(int n_tokens, int n_requests, int least) {
   return Bounds{portions, n_tokens / kC + portions};
 }
 
-template <typename Kernel>
-static bool allow(Kernel kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-}
-
 template <typename T, int FORM, int NP>
 static int scan(const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
   const int tiles = (p.vdim + kTile - 1) / kTile;
@@ -955,7 +950,8 @@ static int scan(const Problem& p, const Bounds& most, const Solved& solved, cuda
     auto solve = solve_kernel<T, NP>;
     auto carry = carry_kernel<NP>;
     auto read = read_kernel<T, float, kDelta, NP>;
-    if (!allow(solve, solve_bytes(NP)) || !allow(carry, carry_bytes(NP)) || !allow(read, read_bytes(NP)))
+    if (allow_shared(solve, solve_bytes(NP)) != cudaSuccess || allow_shared(carry, carry_bytes(NP)) != cudaSuccess ||
+        allow_shared(read, read_bytes(NP)) != cudaSuccess)
       MS_FAIL("chunk_scan: shared memory refused");
     ms::launch(solve, dim3((p.dim + p.vdim + kThreads - 1) / kThreads, p.heads, most.chunks), kThreads, solve_bytes(NP), stream, p,
                solved);
@@ -969,7 +965,8 @@ static int scan(const Problem& p, const Bounds& most, const Solved& solved, cuda
   } else {
     auto local = local_kernel<T, FORM, NP>;
     auto read = read_kernel<T, T, FORM, NP>;
-    if (!allow(local, local_bytes(NP)) || !allow(read, read_bytes(NP))) MS_FAIL("chunk_scan: shared memory refused");
+    if (allow_shared(local, local_bytes(NP)) != cudaSuccess || allow_shared(read, read_bytes(NP)) != cudaSuccess)
+      MS_FAIL("chunk_scan: shared memory refused");
     ms::launch(local, grid, kThreads, local_bytes(NP), stream, p);
     MS_CHECK_LAUNCH("chunk_scan: chunks alone");
     const bool four = p.dim % 4 == 0;

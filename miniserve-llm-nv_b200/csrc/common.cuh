@@ -47,6 +47,12 @@ __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddep
 
 bool dependent_launch_enabled();  // defined in runtime.cu
 
+// Lets a kernel have `bytes` of dynamic shared memory on the current device: asked of the driver once per kernel and device (and again for
+// more), from any thread; a launch costs the host a lookup afterwards.
+cudaError_t allow_shared_bytes(const void* kernel, size_t bytes);  // defined in runtime.cu
+template <typename... Params>
+cudaError_t allow_shared(void (*kernel)(Params...), size_t bytes) { return allow_shared_bytes(reinterpret_cast<const void*>(kernel), bytes); }
+
 template <typename... Params, typename... Args>
 cudaError_t launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t config = {};

@@ -278,7 +278,7 @@ static int launch(const void* A, int lda, const int* order, int top, const void*
              "expert_linear: cuTensorMapEncodeTiled failed (%d experts of %d x %d)", experts, N, K);
   auto kernel = expert_tcgen05_kernel<BM, BN, STAGES>;
   const size_t smem = Layout<BM, BN, STAGES>::RING + sizeof(int) * 2 * ((size_t)experts + 1);
-  const cudaError_t allowed = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t allowed = allow_shared(kernel, smem);
   if (allowed != cudaSuccess) MS_FAIL("expert_linear: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(allowed));
   static int sms = 0;
   if (sms == 0) {

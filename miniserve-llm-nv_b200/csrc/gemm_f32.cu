@@ -230,7 +230,7 @@ static int launch_gemm_f32(Kernel kernel, int bm, int bn, int threads, int smem,
   const int grid_m = (M + bm - 1) / bm, grid_n = (N + bn - 1) / bn;
   MS_REQUIRE(grid_m <= 65535 && batch <= 65535, "gemm_f32: %d rows or %d products in one launch is too many", M, batch);
   if (smem > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_shared(kernel, (size_t)smem);
     if (e != cudaSuccess) MS_FAIL("gemm_f32: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
   }
   ms::launch(kernel, dim3(grid_n, grid_m, batch), threads, smem, stream, A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);

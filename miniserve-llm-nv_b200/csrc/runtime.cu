@@ -1,6 +1,7 @@
 // Library-wide state: the last error message and a version word for the bindings.
 #include "common.cuh"
 
+#include <pthread.h>
 #include <stdlib.h>
 
 namespace ms {
@@ -14,6 +15,31 @@ bool dependent_launch_enabled() {
     g_dependent_launch = (value != nullptr && value[0] == '0') ? 0 : 1;
   }
   return g_dependent_launch == 1;
+}
+
+// (kernel, device) and the bytes it may have, by open addressing; nothing in it throws.  Beyond its size the driver is asked each time.
+struct Allowed { const void* kernel; int device; size_t bytes; };
+constexpr int kAllowed = 512;
+static Allowed g_allowed[kAllowed];
+static pthread_mutex_t g_allowed_lock = PTHREAD_MUTEX_INITIALIZER;
+
+cudaError_t allow_shared_bytes(const void* kernel, size_t bytes) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  pthread_mutex_lock(&g_allowed_lock);
+  Allowed* entry = nullptr;
+  const size_t at = reinterpret_cast<size_t>(kernel) / 16 + (size_t)device;
+  for (int i = 0; i < kAllowed && entry == nullptr; ++i) {
+    Allowed* here = &g_allowed[(at + i) % kAllowed];
+    if (here->kernel == nullptr || (here->kernel == kernel && here->device == device)) entry = here;
+  }
+  if (entry == nullptr || entry->kernel == nullptr || entry->bytes < bytes) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && entry != nullptr) *entry = Allowed{kernel, device, bytes};
+  }
+  pthread_mutex_unlock(&g_allowed_lock);
+  return e;
 }
 }  // namespace ms
 
