@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import logging
+import math
 from typing import Optional, Union
 
 import torch
@@ -950,7 +951,7 @@ def _state_rows(states: torch.Tensor, offset: int, length: int) -> int:
 
 
 CONV_ACTIVATIONS = {"none": 0, "silu": 1}
-MAX_CHUNK_SCRATCH = 1 << 30   # bytes of chunk states beyond which a scan walks its tokens
+MAX_CHUNK_SCRATCH = 1 << 30   # bytes of scratch beyond which a scan walks its tokens
 # From which sizes on the scans in chunks are ahead of the walk: a longest portion of 256 tokens, or of 128 in a step of 512; the delta form,
 # whose chunks follow one another and whose walk gains from several requests, a longest portion of 128 x (1 + the number of such portions
 # that the step's tokens would fill).  Whole layers, walk / chunks in us: selective, 64 heads: 1 portion of 128: 74 / 87, 192: 95 / 87, 256: 113 /
@@ -965,7 +966,8 @@ MAX_INT = 2 ** 31 - 1
 
 
 def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False) -> Optional[tuple]:
-    """(chunk states, chunk decays) for the scans in chunks, or None where the step's tokens are walked one after the other."""
+    """(chunk states, chunk decays; delta: and W, U and the keys as a chunk's end sees them) for the scans in chunks, or None where the
+    step's tokens are walked one after the other."""
     if delta:
         if longest <= 0 or longest < CHUNK_SCAN_DELTA * (1 + (n + longest - 1) // longest):
             return None
@@ -975,10 +977,12 @@ def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, 
     if not chunk or longest < CHUNK_SCAN_LEAST:
         return None
     places = n // chunk + min(n_requests, n // CHUNK_SCAN_LEAST)
-    if places > 65535 or 4 * places * heads * columns * dim > MAX_CHUNK_SCRATCH:
+    shapes = [(places, heads, columns, dim), (places, heads)]
+    if delta:
+        shapes += [(n, heads, dim), (n, heads, columns), (n, heads, dim)]
+    if places > 65535 or 4 * sum(math.prod(shape) for shape in shapes) > MAX_CHUNK_SCRATCH:
         return None
-    return (torch.empty((places, heads, columns, dim), dtype=torch.float32, device=device),
-            torch.empty((places, heads), dtype=torch.float32, device=device))
+    return tuple(torch.empty(shape, dtype=torch.float32, device=device) for shape in shapes)
 
 
 def _none_short(n: int, n_requests: int, longest: int) -> bool:
@@ -1215,9 +1219,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
     if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
         scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1)
     if scratch is not None:
-        solved = [None] * 3
-        if code == 1:
-            solved = [torch.empty((n, heads, size), dtype=torch.float32, device=y.device) for size in (dim, vdim, dim)]
+        solved = scratch[2:] or [None] * 3
         _check(library().ms_chunk_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                        _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
                                        _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n),

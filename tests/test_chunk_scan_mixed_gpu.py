@@ -125,3 +125,14 @@ def test_the_walk_with_states_of_any_multiple_of_32(N, lengths):
         scale = max(1.0, float(want.abs().max()))
         assert float((y[rows].double() - want).abs().max()) <= 2e-5 * scale                 # (the walk's bound, as above)
         assert float((states[r].double() - after.flatten()).abs().max()) <= 2e-5 * scale
+
+
+@pytest.mark.parametrize("form,heads,dim,columns,most", [("memory", 8, 128, 257, 65215), ("delta", 16, 128, 128, 26196), ("decay", 16, 128, 128, 65471)])
+def test_beyond_a_gibibyte_of_scratch_a_scan_walks(form, heads, dim, columns, most):
+    """All of a form's scratch counts: the delta form's W, U and keys are more than its chunks' matrices."""
+    from miniserve_b200 import kernels
+
+    for n in (most, most + 200):
+        scratch = kernels._chunk_scratch(n, 1, n, heads, dim, columns, "meta", form == "delta")
+        assert (scratch is None) is (n > most)
+        assert scratch is None or sum(4 * t.numel() for t in scratch) <= 1 << 30
