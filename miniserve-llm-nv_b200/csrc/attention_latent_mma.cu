@@ -18,8 +18,9 @@
 // In both, shared-memory rows are D_K + 8 elements apart, which puts the eight rows of an ldmatrix into eight different
 // bank groups for every D_K that is a multiple of 16, and a key row's page is looked up once per tile at most.
 //
-// They serve the sizes that attention_latent_tcgen05.cu (prompts) and attention_latent_decode.cu (single tokens) do not take: latents
-// of 96 and 512, numbers of heads or page sizes that a tile of 128 rows or 64 keys does not fit, other rotated parts.
+// They serve what attention_latent_tcgen05.cu (prompts) and attention_latent_decode.cu (single tokens) do not take: latents of 96 and 512,
+// single tokens of any latent but 256, numbers of heads or page sizes that a tile of 128 rows or 64 keys does not fit, other rotated parts,
+// and decode steps none of whose requests can see enough keys (kernels.LATENT_DECODE_KEYS).
 #include "attention_latent_tiles.cuh"
 
 namespace ms {

@@ -9,8 +9,9 @@
 // Everything here is float32 arithmetic on float32 state; only the projection that the kernels read (z, the
 // convolution's inputs, dt) and the last kernel's output are in the model's compute type.  A request's tokens are
 // walked in order and every sum has a fixed order, so a position's result depends on the tokens before it alone, not
-// on how they were cut into steps, on what else is in the batch or on which state slot the request holds.  (Steps with
-// portions of 96 tokens and more are scanned in chunks, chunk_scan.cu: there the cutting changes a result's last bits.)
+// on how they were cut into steps, on what else is in the batch or on which state slot the request holds.  (Except where portions of 32
+// tokens and more are scanned in chunks, chunk_scan.cu, which is chosen for a step as a whole by rules in kernels/__init__.py: there the
+// cutting and the rest of the step change a result's last bits.)
 //
 // A request's state vector: [taps - 1][channels] convolution inputs, oldest first, then [heads][P][N] head states
 // (zero at admission: the zeros before a sequence's start and the empty state are the same thing).

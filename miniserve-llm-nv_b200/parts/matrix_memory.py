@@ -41,7 +41,8 @@ admission): for ``matrix_memory`` the heads' matrices with ``n`` as one more col
 norms, the recurrence and the output norm are float32 whatever the compute type (the gates' logits come from a float32
 product of their own); the wide projections are in the compute type.  Prompt portions, single tokens and mixed batches
 run the same kernels, which walk each request's tokens in order from the state its slot holds
-(``kernels.matrix_scan``); steps with portions of 96 tokens and more are scanned in chunks, to the same results up to rounding.
+(``kernels.matrix_scan``); the portions of steps that bring long ones (``kernels.CHUNK_SCAN_LONGEST`` and the lines beside it) are scanned
+in chunks, to the same results up to rounding, the decoded tokens beside them walked.
 """
 
 from __future__ import annotations
