@@ -8,8 +8,8 @@
 // pieces of its own (two for 256 + 64), the others on their way while one is multiplied.  A piece comes by one bulk copy a row (cp.async.bulk, sixteen
 // instructions; rows lie sixteen bytes apart from one another's banks), counted by a barrier.  The probabilities go from the
 // scores' registers to the second product's operand without leaving the warp; the output is rescaled only when a row's maximum has
-// grown by more than 2^8.  At the end the four outputs meet in shared memory.  Rows that no kernel of this step writes are asked for
-// before the wait for the kernel before.
+// grown by more than 2^8.  At the end the four outputs meet in shared memory.  (No row is asked for before the wait for the kernel before: a
+// caller may have written all of them just now.)
 // (Four warps that share each piece of 32 keys meet three times for it, and fetch the queries' fragments again each time: a piece's
 // chain of some 2,900 clocks, not the memory, set the pace.)
 // 32 requests of 16 heads and some 7,200 keys (147 MB): 49 us that way, 35.5 here.
@@ -163,10 +163,12 @@ latent_decode_kernel(const __nv_bfloat16* __restrict__ q_full, const __nv_bfloat
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const float p0 = exp2f(s[n][0] - use_a), p1 = exp2f(s[n][1] - use_a), p2 = exp2f(s[n][2] - use_b), p3 = exp2f(s[n][3] - use_b);
-      l_a += p0 + p1;
-      l_b += p2 + p3;
       p[2 * n] = pack_bf16(p0, p1);
       p[2 * n + 1] = pack_bf16(p2, p3);
+      // (the sum is that of the rounded ones: relative to a maximum that may lag behind, the largest is not 1, and its rounding would
+      // scale the whole output)
+      l_a += __uint_as_float(p[2 * n] << 16) + __uint_as_float(p[2 * n] & 0xffff0000u);
+      l_b += __uint_as_float(p[2 * n + 1] << 16) + __uint_as_float(p[2 * n + 1] & 0xffff0000u);
     }
 #pragma unroll
     for (int np = 0; np < DV / 16; ++np) {

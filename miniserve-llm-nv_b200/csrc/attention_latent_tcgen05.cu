@@ -10,12 +10,16 @@
 //   warps 1, 3   one thread each issues tcgen05.mma: warp 1 the scores, as far ahead as three score buffers in tensor memory allow, warp 3
 //                the outputs, with P read from tensor memory;
 //   warps 4..7   softmax of the even tiles, warps 8..11 of the odd ones, a thread a row: mask, running maximum (passed from group to
-//                group through shared memory), P as bfloat16 over the scores it came from; the output is rescaled only when a row's
-//                maximum has grown by more than 2^8.
+//                group through shared memory), P over the scores it came from, as two bfloat16 numbers (its rounding and what that
+//                leaves); the output is rescaled only when a row's maximum has grown by more than 2^8.
 // Bound by the tensor cores: a tile is (RANK + rot) / 16 products of 128 x 64 x 16 (48 clocks each) and four of 128 x RANK x 16 (128
-// clocks for 256), 1,376 clocks for a latent of 256 + 32, where the softmax takes two groups about 1,000.  Tiles of 64 keys
+// clocks for 256) for either part of P, 1,888 clocks for a latent of 256 + 32, where the softmax takes two groups about 1,200.  The second part
+// costs a third of the time, and is there because the largest probability of a row, relative to a maximum that lags behind, is not
+// 1: rounded, it put the layer further from float64 than tiles with the exact maximum do (0.00490 against 0.00488 for the prompt below; with both parts
+// 0.00476).  Tiles of 64 keys
 // because three of them fit beside the queries: of 128 keys two would, and a tile would be waited for.
-// 2,048 tokens of 16 heads, 256 + 32: 225 us on mma.sync (attention_latent_mma.cu), 58 here (36.5 GFLOP).
+// 2,048 tokens of 16 heads, 256 + 32: 225 us on mma.sync (attention_latent_mma.cu), 58 here with one part of P (36.5 GFLOP); the layer, whose
+// eager pass waits for the host, takes 140 us either way.
 // All mbarrier waits are bounded; a wait that runs out sets the error flag and every role drains and returns.
 #include "tcgen05.cuh"
 
@@ -203,6 +207,9 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)      // sixteen keys further: 16 rows of 128 bytes, 8 columns of packed P
           umma_bf16_a_tmem(tmem_base + o_column, p + kk * 8, values + kk * (16 * 128 / 16), idesc_pv, (j | kk) != 0 ? 1u : 0u);
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk)      // and what rounding has left of P
+          umma_bf16_a_tmem(tmem_base + o_column, p + BN / 2 + kk * 8, values + kk * (16 * 128 / 16), idesc_pv, 1u);
         umma_commit(&pv_done[j & 1]);
         umma_commit(&s_free[b]);
         umma_commit(&k_empty[stage]);
@@ -301,16 +308,20 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         for (int e = 0; e < 8; ++e) part_sum[e] = 0.f;
 #pragma unroll
         for (int c = 0; c < BN; c += 32) {
-          unsigned packed[16];
+          unsigned packed[16], rest[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float p0 = fast_exp2(v[c + i] * scale_log2 - base);
             const float p1 = fast_exp2(v[c + i + 1] * scale_log2 - base);
-            part_sum[(i >> 1) & 7] += p0 + p1;
             const __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
             packed[i / 2] = *reinterpret_cast<const unsigned*>(&two);
+            part_sum[(i >> 1) & 7] += p0 + p1;
+            const __nv_bfloat162 left = __floats2bfloat162_rn(p0 - __uint_as_float(packed[i / 2] << 16),
+                                                              p1 - __uint_as_float(packed[i / 2] & 0xffff0000u));
+            rest[i / 2] = *reinterpret_cast<const unsigned*>(&left);
           }
           tmem_store_16(s_addr + c / 2, packed);
+          tmem_store_16(s_addr + BN / 2 + c / 2, rest);
         }
         tmem_store_wait();
         tmem_fence_before();

@@ -187,3 +187,37 @@ def test_the_key_at_a_border_decides(rank, rot, heads, page, new, window):
             p = torch.softmax(rows[:, rank], dim=0)
             want, size = p @ rows[:, :rank], p @ rows[:, :rank].abs()
             assert torch.all((out[r * new + t].double() - want).abs() <= 2.0 ** -7 * size + 1e-6), (length, border, t)
+
+
+@pytest.mark.parametrize("new", [1, 80])
+def test_the_rounding_of_a_probability_does_not_scale_the_output(new):
+    """A key whose score lies 2^2 to 2^7.9 above the first ones' is what most of the output is.  Nothing is rescaled for that, so its probability
+    is no power of two, and is rounded: if the sum were that of the unrounded ones, every output would be off by that rounding too. (Measured
+    against the result's own rounding to bfloat16; both errors together would be 1.4 times that.)"""
+    from miniserve_b200 import kernels
+
+    heads, rank, rot, page, keys, n = 16, 256, 32, 64, 300, 40
+    dk, g = rank + rot, torch.Generator(device="cuda").manual_seed(new)
+    cache = torch.randn((5, page, dk), generator=g, device="cuda").bfloat16()
+    level = torch.full((5 * page,), -20.0, device="cuda")                          # of a key's score, in units of a token's
+    level[:160:16], level[210] = 1.0, 2.0                                          # (the first piece of every warp and range has one)
+    cache.view(-1, dk)[:, rank:] = 0
+    cache.view(-1, dk)[:, rank] = level.bfloat16()
+    q = torch.zeros((n * new, heads, dk), device="cuda").bfloat16()
+    unit = (2.0 + 5.9 * torch.rand((n * new, heads), generator=g, device="cuda")).bfloat16()     # base-2 distance of the two levels
+    q[:, :, rank] = unit
+    lens = torch.full((n,), keys, dtype=torch.int32, device="cuda")
+    starts = torch.arange(n + 1, dtype=torch.int32, device="cuda") * new
+    positions = (torch.arange(new, device="cuda") + keys - new).repeat(n).to(torch.int32)
+    requests = torch.arange(n, device="cuda").repeat_interleave(new).to(torch.int32)
+    tables = torch.arange(5, dtype=torch.int32, device="cuda").repeat(n, 1)
+    scale = 0.6931471805599453
+    out = torch.empty((n * new, heads, rank), device="cuda").bfloat16()
+    kernels.latent_attention(q, cache, tables, requests, positions, starts, lens, new, keys, rank, scale, None, out)
+    kernels.check_device_errors(q.device)
+    rows = cache.view(-1, dk)[:keys].double()
+    scores = torch.einsum("thd,kd->thk", q.double(), rows) * scale
+    scores = scores.masked_fill(torch.arange(keys, device="cuda") > positions[:, None, None], -torch.inf)
+    want = torch.einsum("thk,kd->thd", torch.softmax(scores, dim=-1), rows[:, :rank])
+    off, rounding = (out.double() - want).norm(), (want.bfloat16().double() - want).norm()
+    assert off <= 1.15 * rounding
