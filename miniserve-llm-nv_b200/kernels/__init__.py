@@ -9,6 +9,7 @@ built or loaded, raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import logging
 import math
 from typing import Optional, Union
@@ -47,6 +48,13 @@ def library() -> ctypes.CDLL:
             function.argtypes = [kinds[a] for a in arguments]
         _library = lib
     return _library
+
+
+@functools.lru_cache(maxsize=4096)
+def _asked(question: str, *sizes: int) -> int:
+    """The library's answer to a question about sizes alone (whether a kernel takes them, how it cuts them), asked once for each: an eager
+    pass asks a few for every layer, a microsecond each."""
+    return getattr(library(), question)(*sizes)
 
 
 launch_count = 0   # entry points of this library called so far (each launches one kernel, or a fixed few)
@@ -737,7 +745,7 @@ def decode_attention_fused_supported(dtype: torch.dtype, head_dim: int, n_q: int
     """Whether :func:`decode_attention_fused` takes these sizes (bfloat16, head size 64 or 128, at most 16
     query heads per key/value head); MINISERVE_B200_FUSED_DECODE_ATTENTION=0 turns it off."""
     return bool(FUSED_DECODE_ATTENTION and dtype == torch.bfloat16
-                and library().ms_attention_decode_fused_supports(_i(head_dim), _i(n_q), _i(n_kv)))
+                and _asked("ms_attention_decode_fused_supports", head_dim, n_q, n_kv))
 
 
 def decode_attention_fused_preferred(rows: int, head_dim: int = 0, group: int = 0, page_size: int = 0) -> bool:
@@ -781,7 +789,7 @@ def decode_attention_fused(qkv: torch.Tensor, slots: torch.Tensor, q_weight: Opt
     if cos_sin is not None:
         _want(cos_sin, "cos_sin", torch.float32, (n, head_dim // 2, 2))
     lib = library()
-    splits = lib.ms_attention_decode_fused_splits(_i(head_dim), _i(n), _i(n_kv), _i(max_context_len))
+    splits = _asked("ms_attention_decode_fused_splits", head_dim, n, n_kv, max_context_len)
     part_o = part_lse = None
     if splits > 1:
         part_o = torch.empty((n * n_q * splits, head_dim), dtype=torch.float32, device=qkv.device)
@@ -868,8 +876,8 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
     _want(context_lens, "context_lens", torch.int32, (n_requests,))
     lib = library()
     page_size = cache.shape[1]
-    if q_full.dtype == torch.bfloat16 and USE_LATENT_MMA and lib.ms_latent_attention_mma_supports(_i(rank), _i(dk - rank), _i(heads)):
-        if (max_query_len > 1 and lib.ms_latent_attention_tcgen05_supports(_i(rank), _i(dk - rank), _i(heads), _i(page_size))
+    if q_full.dtype == torch.bfloat16 and USE_LATENT_MMA and _asked("ms_latent_attention_mma_supports", rank, dk - rank, heads):
+        if (max_query_len > 1 and _asked("ms_latent_attention_tcgen05_supports", rank, dk - rank, heads, page_size)
                 and (q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0):
             _check(lib.ms_latent_attention_tcgen05(
                 _ptr(q_full), _ptr(cache), _i(cache.shape[0]), _ptr(block_tables), _i(block_tables.shape[1]), _ptr(query_start),
@@ -877,11 +885,11 @@ def latent_attention(q_full: torch.Tensor, cache: torch.Tensor, block_tables: to
                 _i(n_requests), _i(max_query_len), _i(n), _ptr(device_error_flag(q_full.device)), _stream()))
             return
         reach = min(max_context_len, window) if window else max_context_len      # the most keys a token sees
-        tile_ranges = lib.ms_latent_attention_mma_splits(_i(rank), _i(dk - rank), _i(heads), _i(n_requests), _i(max_query_len), _i(reach))
+        tile_ranges = _asked("ms_latent_attention_mma_splits", rank, dk - rank, heads, n_requests, max_query_len, reach)
         least = LATENT_DECODE_KEYS // max(1, n * ((heads + 15) // 16))
-        if max_query_len == 1 and reach >= least and lib.ms_latent_decode_supports(_i(rank), _i(dk - rank), _i(heads)) and (
+        if max_query_len == 1 and reach >= least and _asked("ms_latent_decode_supports", rank, dk - rank, heads) and (
                 q_full.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
-            ranges = lib.ms_latent_decode_splits(_i(heads), _i(n_requests), _i(reach))
+            ranges = _asked("ms_latent_decode_splits", heads, n_requests, reach)
             splits = max(ranges, tile_ranges)
             part_o = part_lse = None
             if splits > 1:
@@ -962,18 +970,28 @@ CHUNK_SCAN_LONGEST, CHUNK_SCAN_OF_MANY, CHUNK_SCAN_DELTA = 256, (128, 512), 128
 # matrix passes through memory four more times than a state that is walked, and needs some forty tokens to be worth it (selective, 64
 # heads, where the state is largest).
 CHUNK_SCAN_LEAST = 32
+# The walk takes such short ones and the portions at the same time, the scan one after the other: with memory and constant decays, from a
+# few on, each asks for two more tokens of the longest portion.  Memory, 8 heads of 128 x 256, us walked
+# / in chunks: 256 tokens and 24 single ones 155 / 128, 256 and 64 165 / 194, 400 and 64 230 / 198.
+CHUNK_SCAN_BESIDE = (28, 2)
+WALK_BESIDE_CHUNK = 31     # tokens of a chunk of that walk, at most
 MAX_INT = 2 ** 31 - 1
 
 
-def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False) -> Optional[tuple]:
+def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False,
+                   beside: int = 0) -> Optional[tuple]:
     """(chunk states, chunk decays; delta: and W, U and the keys as a chunk's end sees them) for the scans in chunks, or None where the
     step's tokens are walked one after the other."""
     if delta:
         if longest <= 0 or longest < CHUNK_SCAN_DELTA * (1 + (n + longest - 1) // longest):
             return None
-    elif longest < CHUNK_SCAN_LONGEST and (longest < CHUNK_SCAN_OF_MANY[0] or n < CHUNK_SCAN_OF_MANY[1]):
-        return None
-    chunk = library().ms_chunk_scan_chunk(_i(n_requests), _i(longest), _i(heads), _i(dim))
+    else:
+        # how many requests are too short, at least: what the longest one leaves is not enough for the others to be longer
+        short = n_requests - 1 - max(0, n - longest - (n_requests - 1)) // (CHUNK_SCAN_LEAST - 1)
+        more = beside * max(0, short - CHUNK_SCAN_BESIDE[0])
+        if longest < CHUNK_SCAN_LONGEST + more and (longest < CHUNK_SCAN_OF_MANY[0] + more or n < CHUNK_SCAN_OF_MANY[1]):
+            return None
+    chunk = _asked("ms_chunk_scan_chunk", n_requests, longest, heads, dim)
     if not chunk or longest < CHUNK_SCAN_LEAST:
         return None
     places = n // chunk + min(n_requests, n // CHUNK_SCAN_LEAST)
@@ -1063,7 +1081,7 @@ def selective_scan(conv: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias:
                                                  _ptr(scratch[1]), _stream()))
         if _none_short(n, n_requests, longest):
             return
-        longest = min(longest, CHUNK_SCAN_LEAST - 1)
+        longest = min(longest, WALK_BESIDE_CHUNK)
     _check(library().ms_selective_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
                                        _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
                                        _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(longest),
@@ -1170,7 +1188,8 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
     ``"channel_decay"`` of few long portions runs in chunks that need not wait for one another (a walk from zero per chunk, a join
     of the chunks' matrices, a walk from the joined ones): ``chunk`` None lets the library choose, 0 forbids it, a number is
     the chunk's tokens.  ``"memory"``, ``"delta"`` and ``"decay"`` of portions of many tokens run as matrix products over chunks of 64
-    tokens (``csrc/chunk_scan.cu``) unless ``chunk`` is 0."""
+    tokens (``csrc/chunk_scan.cu``; CHUNK_SCAN_LONGEST says from when on) unless ``chunk`` is 0, which walks them; other numbers are
+    refused there."""
     code = MATRIX_SCAN_MODES[mode]
     n = y.shape[0]
     for name, tensor in (("q", q), ("k", k), ("v", v)):
@@ -1217,7 +1236,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
         return
     scratch = None
     if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
-        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1)
+        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1, CHUNK_SCAN_BESIDE[1])
     if scratch is not None:
         solved = scratch[2:] or [None] * 3
         _check(library().ms_chunk_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
@@ -1228,7 +1247,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
                                        _ptr(solved[1]), _ptr(solved[2]), _stream()))
         if _none_short(n, n_requests, max_query_len):
             return
-        max_query_len = min(max_query_len, CHUNK_SCAN_LEAST - 1)
+        max_query_len = min(max_query_len, WALK_BESIDE_CHUNK)
     _check(library().ms_matrix_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                     _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
                                     _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(max_query_len),
@@ -1431,7 +1450,7 @@ def expert_linear(x: torch.Tensor, order: Optional[torch.Tensor], top: int, weig
     if order is not None:
         _want(order, "order", torch.int32, (pairs,))
     if (x.dtype == torch.bfloat16 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-            and library().ms_expert_tcgen05_supports(_i(experts), _i(n), _i(k))):
+            and _asked("ms_expert_tcgen05_supports", experts, n, k)):
         _check(library().ms_expert_linear_tcgen05(_ptr(x), _i(k), _ptr(order), _i(top), _ptr(weight), _ptr(out), _i(out.shape[1]),
                                                   _ptr(offsets), _i(experts), _i(pairs), _i(n), _i(k), _i(code), _f(limit),
                                                   _ptr(pair_scale), _ptr(device_error_flag(x.device)), _stream()))

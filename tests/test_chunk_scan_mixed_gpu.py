@@ -1,6 +1,9 @@
 """Which steps are scanned in chunks, with the rules in force, and steps that mix portions with decoded tokens: those are walked beside the
 scan, as they are in a step of their own."""
 
+import importlib
+
+import helpers
 import pytest
 import torch
 
@@ -8,7 +11,7 @@ from test_chunk_scan_gpu import ints, problem, recurrence, run
 
 pytestmark = pytest.mark.gpu
 
-MIXED = [[300] + [1] * 40, [1, 31, 32, 33, 400, 0, 2], [1] * 33 + [260, 5, 700, 1]]
+MIXED = [[310] + [1] * 40, [1, 31, 32, 33, 400, 0, 2], [1] * 33 + [260, 5, 700, 1]]
 
 
 def counted(monkeypatch, *names):
@@ -86,11 +89,13 @@ def test_selective_scan(monkeypatch, lengths):
 @pytest.mark.parametrize("lengths,delta,taken,walk_beside", [
     ([255], False, False, False), ([256], False, True, False), ([127, 385], False, True, False), ([127] * 5, False, False, False),
     ([128] * 4, False, True, False), ([300, 200, 100], False, True, True), ([128] * 3 + [127], False, False, False), ([256, 32], False, True, False), ([256, 31], False, True, True),
+    ([256] + [1] * 28, False, True, True), ([256] + [1] * 29, False, False, False), ([327] + [1] * 64, False, False, False), ([328] + [1] * 64, False, True, True),
     ([255], True, False, False), ([256], True, True, False), ([383, 1], True, False, False), ([384, 1], True, True, True),
     ([500] * 4, True, False, False), ([640] * 4, True, True, False)])
 def test_which_steps_are_scanned_in_chunks(monkeypatch, lengths, delta, taken, walk_beside):
     """256 tokens, or 128 in a step of 512; the delta form 128 (1 + portions of that length that the step would fill).  Of more than two
-    unequal portions one may be too short for a chunk, as far as the host knows: the walk is launched beside the scan then."""
+    unequal portions one may be too short for a chunk, as far as the host knows: the walk is launched beside the scan then.  More
+    than 28 requests that are too short ask for a longer portion, two tokens each."""
     form = "delta" if delta else "memory"
     rows, cols, gates, slots, states, kv_heads, columns = problem(form, torch.bfloat16, lengths, 1, 1, 8, 8, 3)
     calls = counted(monkeypatch, "ms_chunk_scan", "ms_matrix_scan")
@@ -136,3 +141,26 @@ def test_beyond_a_gibibyte_of_scratch_a_scan_walks(form, heads, dim, columns, mo
         scratch = kernels._chunk_scratch(n, 1, n, heads, dim, columns, "meta", form == "delta")
         assert (scratch is None) is (n > most)
         assert scratch is None or sum(4 * t.numel() for t in scratch) <= 1 << 30
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("design,name,scan,walk", [("kivurax", "c", "ms_chunk_scan", "ms_matrix_scan"), ("kivurax", "d", "ms_chunk_scan", "ms_matrix_scan"),
+                                                   ("zozezen", "c", "ms_selective_chunk_scan", "ms_selective_scan")])
+def test_a_long_prompt_beside_decoded_tokens_of_a_model(tmp_path, monkeypatch, dtype, design, name, scan, walk):
+    """A step of the whole engine: 430 tokens of one prompt and the next token of each of nine requests, every logit against the plain
+    whole-sequence computation, before and after it too."""
+    tests, parts = importlib.import_module(f"test_{design}_gpu"), importlib.import_module(f"{design}_helpers")
+    folder = parts.make_folder(tmp_path, name, seed=21)
+    vocab = parts.CONFIGS[name]["vocab"]
+    short = {f"s{i}": helpers.random_tokens(vocab, n, seed=30 + i) for i, n in enumerate((3, 5, 9, 17, 18, 33, 40, 65, 7))}
+    requests = dict(short, long=helpers.random_tokens(vocab, 432, seed=50))
+    steps = [dict(step=0, entries=[dict(id=rid, tokens=t[:-2], want=list(range(len(t) - 2))) for rid, t in short.items()], end=[]),
+             dict(step=1, entries=[dict(id="s0", tokens=short["s0"][-2:-1], want=[0]), dict(id="long", tokens=requests["long"][:430], want=list(range(430)))]
+                  + [dict(id=rid, tokens=t[-2:-1], want=[0]) for rid, t in list(short.items())[1:]], end=[]),
+             dict(step=2, entries=[dict(id="long", tokens=requests["long"][430:], want=[0, 1])]
+                  + [dict(id=rid, tokens=t[-1:], want=[0]) for rid, t in short.items()], end=list(requests))]
+    runtime = tests.build(folder, dtype, 120, 8, max_seqs=10)
+    calls = counted(monkeypatch, scan, walk)
+    got = helpers.collect(steps, tests.replay(runtime, steps))
+    tests.check(folder, dtype, requests, got)
+    assert calls[scan] >= 1 and calls[walk] >= 3 * calls[scan]         # (a layer walks in all three steps, beside the scan in the second)
