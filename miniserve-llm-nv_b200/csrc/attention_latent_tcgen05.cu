@@ -18,8 +18,8 @@
 // 1: rounded, it put the layer further from float64 than tiles with the exact maximum do (0.00490 against 0.00488 for the prompt below; with both parts
 // 0.00476).  Tiles of 64 keys
 // because three of them fit beside the queries: of 128 keys two would, and a tile would be waited for.
-// 2,048 tokens of 16 heads, 256 + 32: 225 us on mma.sync (attention_latent_mma.cu), 58 here with one part of P (36.5 GFLOP); the layer, whose
-// eager pass waits for the host, takes 140 us either way.
+// 2,048 tokens of 16 heads, 256 + 32: 225 us on mma.sync (attention_latent_mma.cu), 63 here, 58 with one part of P (36.5 GFLOP of scores and
+// one part); the layer, whose eager pass waits for the host, takes 135 to 140 us either way.
 // All mbarrier waits are bounded; a wait that runs out sets the error flag and every role drains and returns.
 #include "tcgen05.cuh"
 

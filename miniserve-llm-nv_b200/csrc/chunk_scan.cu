@@ -21,7 +21,7 @@
 // Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 110 us; selective,
 // 64 heads of 128 x 64, 2,048 tokens 496 -> 202 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 237 us.
 //
-// All arithmetic is float32 on float32 copies of the projections.  A token's result uses nothing of the tokens behind it (what is
+// All arithmetic is float32 on float32 copies of the projections, products of decays in double.  A token's result uses nothing of the tokens behind it (what is
 // masked is not multiplied: a zero would turn an infinity behind it into a NaN before it).
 #include "common.cuh"
 #include "mma_common.cuh"
@@ -61,11 +61,11 @@ struct Portion { int request, first, tokens; size_t place; };
 // The portions of 32 requests from r0 on, one a lane: its first token, its tokens (0: none, or too few for a chunk), and the chunks up to and
 // with it.
 struct Lane { int first, tokens, chunks, upto; };
-__device__ __forceinline__ Lane portions_from(const Problem& p, int r0) {
+__device__ __forceinline__ Lane portions_from(const int* query_start, int requests, int least, int r0) {
   const int lane = threadIdx.x & 31;
   Lane l = {};
-  if (r0 + lane < p.requests) l.first = p.query_start[r0 + lane], l.tokens = p.query_start[r0 + lane + 1] - l.first;
-  if (l.tokens < p.least) l.tokens = 0;
+  if (r0 + lane < requests) l.first = query_start[r0 + lane], l.tokens = query_start[r0 + lane + 1] - l.first;
+  if (l.tokens < least) l.tokens = 0;
   l.chunks = (l.tokens + kC - 1) / kC, l.upto = l.chunks;
 #pragma unroll
   for (int d = 1; d < 32; d *= 2) {
@@ -75,12 +75,13 @@ __device__ __forceinline__ Lane portions_from(const Problem& p, int r0) {
   return l;
 }
 
-// The c-th chunk, looked up by a whole warp; `count` is how many there are (c beyond them: only that, and no tokens).
-__device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
+// The c-th chunk, looked up by a whole warp; `count` is how many there are (c beyond them: only that, and no tokens).  Several requests are
+// searched out of line: a single one's kernels then need no more registers than without a search.
+__device__ __noinline__ Where search_chunk(const int* query_start, int requests, int least, int c, int* all) {
   Where w = {};
-  count = 0;
-  for (int r0 = 0; r0 < p.requests; r0 += 32) {
-    const Lane l = portions_from(p, r0);
+  int count = 0;
+  for (int r0 = 0; r0 < requests; r0 += 32) {
+    const Lane l = portions_from(query_start, requests, least, r0);
     const unsigned found = __ballot_sync(0xffffffffu, count + l.upto > c);
     if (found) {
       const int at = __ffs(found) - 1, first = __shfl_sync(0xffffffffu, l.first, at), tokens = __shfl_sync(0xffffffffu, l.tokens, at);
@@ -91,14 +92,23 @@ __device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
     }
     count += __shfl_sync(0xffffffffu, l.upto, 31);
   }
+  *all = count;
+  return w;
+}
+__device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
+  if (p.requests > 1) return search_chunk(p.query_start, p.requests, p.least, c, &count);
+  Where w = {};
+  const int first = p.query_start[0], tokens = p.query_start[1] - first;
+  count = (tokens + kC - 1) / kC;
+  if (c < count) w.left = tokens - c * kC, w.len = min(w.left, kC), w.first = first + c * kC, w.place = (size_t)c;
   return w;
 }
 
 // The k-th portion, looked up by a whole warp (no tokens: there are not as many).
-__device__ __forceinline__ Portion portion_of(const Problem& p, int k) {
+__device__ __noinline__ Portion search_portion(const int* query_start, int requests, int least, int k) {
   int count = 0;
-  for (int r0 = 0; r0 < p.requests; r0 += 32) {
-    const Lane l = portions_from(p, r0);
+  for (int r0 = 0; r0 < requests; r0 += 32) {
+    const Lane l = portions_from(query_start, requests, least, r0);
     const unsigned scanned = __ballot_sync(0xffffffffu, l.tokens > 0);
     const unsigned found = __ballot_sync(0xffffffffu, l.tokens > 0 && __popc(scanned & ((1u << (threadIdx.x & 31)) - 1u)) == k);
     if (found) {
@@ -109,6 +119,10 @@ __device__ __forceinline__ Portion portion_of(const Problem& p, int k) {
     k -= __popc(scanned), count += __shfl_sync(0xffffffffu, l.upto, 31);
   }
   return Portion{};
+}
+__device__ __forceinline__ Portion portion_of(const Problem& p, int k) {
+  if (p.requests > 1) return search_portion(p.query_start, p.requests, p.least, k);
+  return Portion{0, p.query_start[0], p.query_start[1] - p.query_start[0], 0};
 }
 
 __device__ __forceinline__ float silu_of(float v) { return v * (1.f / (1.f + expf(-v))); }
@@ -218,7 +232,7 @@ __device__ __forceinline__ double decay_between(const double* keep, int first, i
 // grid (value tiles, heads, chunks).  Bound by its multiply-adds, 64 x 64 x dim a block: a thread has four or eight value columns and
 // four key entries, a token costs it a read of keys and one or two of values for eight or sixteen packed multiply-adds.
 template <typename T, int FORM, int NP>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, NP == 128 ? 4 : 1)              // (as many as the shared memory has room for)
 local_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
