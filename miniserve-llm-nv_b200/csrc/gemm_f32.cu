@@ -1,7 +1,8 @@
 // True float32 matrix product for the 32-bit path: C[M, N] = A[M, K] * W[N, K]^T with
 // both operands stored K-major, as activations and `[out, in]` weights are.  Plain FFMA
 // on the CUDA cores: no tensor cores and no reduced-precision mode, so a fault that
-// bfloat16 rounding would hide shows up.  Each output element is one thread's sum over
+// bfloat16 rounding would hide shows up.  (Sums of 1,536 products and more are formed on the tensor
+// cores from exact parts of the operands, see gemm_f32_tcgen05.cu.)  Each output element is one thread's sum over
 // k in ascending order, whatever M is, so a row's result does not depend on the batch.
 #include "common.cuh"
 

@@ -1515,8 +1515,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, row_stats: 
     """``out[M, N] = x[M, K] @ weight[N, K]^T``.  (``row_stats``: see :func:`linear_wide`; the caller has asked
     :func:`fold_supported` first.)
 
-    float32 operands run through the library's own FFMA kernel (true 32-bit, no tensor-core
-    mode).  bfloat16 operands go to cuBLAS through ``torch.mm`` with float32 accumulation;
+    float32 operands run through the library's own kernels: FFMA, or for long sums tensor cores
+    on three bfloat16 parts of each operand that add up to it exactly (nearer to 64 bits than the FFMA
+    sums; which of the two is a question of N and K alone).  bfloat16 operands go to cuBLAS through ``torch.mm`` with float32 accumulation;
     ``out`` may then be bfloat16 or float32.
     """
     m, k = x.shape
@@ -1533,6 +1534,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, row_stats: 
         _want(x, "x", torch.float32)
         _want(weight, "weight", torch.float32)
         _want(out, "out", torch.float32)
+        if _asked("ms_gemm_f32_tcgen05_takes", n, k) and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
+            scratch = torch.empty(_asked("ms_gemm_f32_tcgen05_scratch", m, k), dtype=torch.uint8, device=x.device)
+            _check(library().ms_gemm_f32_tcgen05(_ptr(x), _ptr(weight), _ptr(out), _i(m), _i(n), _i(k), _i(k), _i(k), _i(n), _ptr(scratch),
+                                                 _ptr(device_error_flag(x.device)), _stream()))
+            return
         _check(library().ms_gemm_f32(_ptr(x), _ptr(weight), _ptr(out), _i(m), _i(n), _i(k), _i(k), _i(k), _i(n),
                                      _stream()))
         return

@@ -1,0 +1,59 @@
+"""The float32 product on the tensor cores (three bfloat16 parts of each operand) against float64, at sizes around its tiles of rows,
+its stages of 64 k and its clusters."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(m, n, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(m, k, generator=g, device="cuda"), torch.randn(n, k, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1536), (1, 2048, 6144), (16, 128, 1540), (17, 129, 2052), (145, 300, 1604), (144, 4096, 2048), (289, 5000, 1536),
+                                   (33, 12288, 1600), (130, 8192, 1024), (700, 2816, 1568), (5, 20000, 1600)])
+def test_long_sums(m, n, k):
+    """An addition to a stage's sum drops what lies behind 24 bits (up to 2^-23 of what is summed so far, in a stage's last four steps and
+    the small products before them), stages are added with one rounding each: (K / 64 + 8) 2^-23 of the sum of the magnitudes is well
+    above both.  And a row's bits do not depend on the rows beside it."""
+    from miniserve_b200 import kernels
+
+    assert kernels._asked("ms_gemm_f32_tcgen05_takes", n, k)
+    x, w = operands(m, n, k, m + n + k)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    kernels.linear(x, w, out)
+    want = x.double() @ w.double().T
+    bound = (k / 64 + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    assert torch.all((out.double() - want).abs() <= bound)
+    # the distance that float32 sums in ascending order have grows with sqrt(K / 2) roundings of 2^-25 each; this one must not exceed it
+    assert float((out.double() - want).norm() / want.norm()) <= (k / 2) ** 0.5 * 2.0 ** -25
+    for row in {0, m // 2, m - 1}:
+        alone = torch.empty((1, n), device="cuda")
+        kernels.linear(x[row:row + 1].contiguous(), w, alone)
+        assert torch.equal(alone[0], out[row])
+    kernels.check_device_errors(x.device)
+
+
+@pytest.mark.parametrize("n", [300, 20000])
+def test_numbers_at_the_ends_of_the_range(n):
+    """Infinities, NaNs, overflowing sums and operands near the largest number give what the plain product gives (one block a tile, and
+    clusters)."""
+    from miniserve_b200 import kernels
+
+    x, w = operands(37, n, 1600, 3)
+    x[3, 5], x[4, 7], w[7, 9], w[n - 1, 1599] = float("inf"), float("nan"), float("-inf"), float("inf")
+    x[8], w[11], x[9, 3], w[:, 3] = 3.0e38, 3.0e38, 3.4028e38, 0.25
+    out = torch.empty((37, n), device="cuda")
+    kernels.linear(x, w, out)
+    # the same rows one number past a 16-byte boundary: the plain kernel
+    room = torch.empty(37 * 1600 + 1, device="cuda")[1:]
+    plain = torch.empty((37, n), device="cuda")
+    kernels.linear(room.copy_(x.reshape(-1)).view(37, 1600), w, plain)
+    finite = torch.isfinite(plain)
+    assert torch.equal(torch.isfinite(out), finite) and not finite[3].any() and torch.isfinite(out[9, :7]).all()
+    assert torch.equal(torch.nan_to_num(out, nan=7.0)[~finite], torch.nan_to_num(plain, nan=7.0)[~finite])
+    scale = x.double().abs() @ w.double().abs().T
+    assert torch.all(((out.double() - plain.double()).abs() <= 1600 * 2.0 ** -23 * scale)[finite])
+    kernels.check_device_errors(x.device)
