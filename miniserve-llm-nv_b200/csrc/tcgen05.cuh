@@ -26,8 +26,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
       : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return done != 0;
 }
-// Waits for the phase of the given parity; false (and the error flag set) if it does not come.
+// Waits for the phase of the given parity; false (and the error flag set) if it does not come.  The loop stays a loop: unrolled, it took a
+// large part of a kernel's instruction cache for turns that are hardly ever taken (quantised attention of a decode step 36.6 us, now 35.7; quantised experts 140.7, 138.4).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int* error_flag, int code) {
+#pragma unroll 1
   for (unsigned spin = 0; spin < SPIN_LIMIT; ++spin)
     if (mbar_try_wait(bar, parity)) return true;
   atomicExch(error_flag, code);
