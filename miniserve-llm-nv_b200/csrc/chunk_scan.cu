@@ -1,6 +1,7 @@
 // Recurrences with one decay per token and head, S_t = g_t S_(t-1) + w_t v_t k_t^T, y_t = S_t q_t, for portions of many tokens: what
 // ms_matrix_scan (memory, delta and constant-decay forms) and ms_selective_scan do token after token, as matrix products over chunks
-// of 64 tokens.  Walked, a portion is a chain of as many steps as it has tokens, whose every step waits for shared memory and for a
+// of 64 tokens, on the float32 pipe.  Where there is more work the products run on the tensor cores, over chunks of 128 (chunk_scan_tcgen05.cu;
+// which of the two is the caller's rule): of the delta form, whose chunks follow one another, what is read then, and the rest here.  Walked, a portion is a chain of as many steps as it has tokens, whose every step waits for shared memory and for a
 // butterfly of shuffles; in chunks nearly all of it is products whose operands a thread uses several times.
 //
 // With D(t, s) = g_(s+1) .. g_t (products of the factors themselves, not differences of their logarithms: a difference of two large
@@ -18,126 +19,20 @@
 //     carry_kernel   the chunks in order, sixteen columns of S a block: u, S_end; S_0 of every chunk
 //     read_kernel    y, with u for v
 //
-// Measured (one request in bfloat16, the scan's launches together): memory form, 8 heads of 128 x 256, 2,011 tokens 658 -> 110 us; selective,
-// 64 heads of 128 x 64, 2,048 tokens 496 -> 202 us; delta, 16 heads of 128 x 128, portions of 1,500 and 548 tokens 566 -> 237 us.
+// Measured (one request in bfloat16, the scan's launches together; us walked, here, on the tensor cores): memory form, 8 heads of 128 x 256,
+// 2,048 tokens 658, 119, 65; selective, 64 heads of 128 x 64, 2,048 tokens 496, 210, 124; delta, 16 heads of 128 x 128, 2,048 tokens 566, 234, 212;
+// 512 tokens of the same (here, tensor cores): 43, 34; 69, 58; 71, 76.
 //
 // All arithmetic is float32 on float32 copies of the projections, products of decays in double.  A token's result uses nothing of the tokens behind it (what is
 // masked is not multiplied: a zero would turn an infinity behind it into a NaN before it).
-#include "common.cuh"
+#include "chunk_scan.cuh"
 #include "mma_common.cuh"
 
 namespace ms {
 namespace chunk_scan {
 
-constexpr int kC = 64, kThreads = 256, kTile = 64;       // tokens of a chunk; value columns of a block
+constexpr int kC = kSolved, kThreads = 256, kTile = 64;  // tokens of a chunk; value columns of a block
 constexpr int kLd = kTile + 4;
-enum Form : int { kMemory = 0, kDelta = 1, kDecay = 2, kSelective = 3 };
-
-struct Rows { const void* at; int ld, col; };            // a head's rows: column col + head * size
-
-struct Problem {
-  Rows q, k, v;
-  int heads, kv_heads, dim, vdim, columns;               // columns of a head's state: vdim, and one more in the memory form
-  int input_act, wide;                                   // SiLU on q, k, v; rows on 16-byte boundaries in whole 16-byte pieces
-  float q_scale;
-  const float* gates;                                    // memory [N, H, 3], delta [N, H, 2], decay [H]
-  const void* step;                                      // selective: step sizes' logits, type, rows, first column
-  int step_dtype, step_ld, step_col;
-  const float *step_bias, *a_log, *skip;
-  float* states;
-  long long state_stride;
-  int state_offset;
-  const int *state_slots, *query_start;
-  int requests, least;                                   // least: tokens from which on a portion is scanned here
-  float *chunk_states, *chunk_decays;                    // [places][heads][columns][dim], [places][heads]
-  float *y, *bottom;
-};
-
-// A block's chunk (its first token, its tokens, those of its portion from it on), or its portion and that one's first chunk.  Chunks are
-// numbered through the step's portions of at least `least` tokens, which is where their matrices lie in the scratch.
-struct Where { int request, first, len, left; size_t place; };
-struct Portion { int request, first, tokens; size_t place; };
-
-// The portions of 32 requests from r0 on, one a lane: its first token, its tokens (0: none, or too few for a chunk), and the chunks up to and
-// with it.
-struct Lane { int first, tokens, chunks, upto; };
-__device__ __forceinline__ Lane portions_from(const int* query_start, int requests, int least, int r0) {
-  const int lane = threadIdx.x & 31;
-  Lane l = {};
-  if (r0 + lane < requests) l.first = query_start[r0 + lane], l.tokens = query_start[r0 + lane + 1] - l.first;
-  if (l.tokens < least) l.tokens = 0;
-  l.chunks = (l.tokens + kC - 1) / kC, l.upto = l.chunks;
-#pragma unroll
-  for (int d = 1; d < 32; d *= 2) {
-    const int before = __shfl_up_sync(0xffffffffu, l.upto, d);
-    if (lane >= d) l.upto += before;
-  }
-  return l;
-}
-
-// The c-th chunk, looked up by a whole warp; `count` is how many there are (c beyond them: only that, and no tokens).  Several requests are
-// searched out of line: a single one's kernels then need no more registers than without a search.
-__device__ __noinline__ Where search_chunk(const int* query_start, int requests, int least, int c, int* all) {
-  Where w = {};
-  int count = 0;
-  for (int r0 = 0; r0 < requests; r0 += 32) {
-    const Lane l = portions_from(query_start, requests, least, r0);
-    const unsigned found = __ballot_sync(0xffffffffu, count + l.upto > c);
-    if (found) {
-      const int at = __ffs(found) - 1, first = __shfl_sync(0xffffffffu, l.first, at), tokens = __shfl_sync(0xffffffffu, l.tokens, at);
-      const int mine = c - count - __shfl_sync(0xffffffffu, l.upto - l.chunks, at);
-      w.request = r0 + at, w.left = tokens - mine * kC, w.len = min(w.left, kC), w.first = first + mine * kC;
-      w.place = (size_t)c;
-      return w;
-    }
-    count += __shfl_sync(0xffffffffu, l.upto, 31);
-  }
-  *all = count;
-  return w;
-}
-__device__ __forceinline__ Where chunk_of(const Problem& p, int c, int& count) {
-  if (p.requests > 1) return search_chunk(p.query_start, p.requests, p.least, c, &count);
-  Where w = {};
-  const int first = p.query_start[0], tokens = p.query_start[1] - first;
-  count = (tokens + kC - 1) / kC;
-  if (c < count) w.left = tokens - c * kC, w.len = min(w.left, kC), w.first = first + c * kC, w.place = (size_t)c;
-  return w;
-}
-
-// The k-th portion, looked up by a whole warp (no tokens: there are not as many).
-__device__ __noinline__ Portion search_portion(const int* query_start, int requests, int least, int k) {
-  int count = 0;
-  for (int r0 = 0; r0 < requests; r0 += 32) {
-    const Lane l = portions_from(query_start, requests, least, r0);
-    const unsigned scanned = __ballot_sync(0xffffffffu, l.tokens > 0);
-    const unsigned found = __ballot_sync(0xffffffffu, l.tokens > 0 && __popc(scanned & ((1u << (threadIdx.x & 31)) - 1u)) == k);
-    if (found) {
-      const int at = __ffs(found) - 1;
-      return Portion{r0 + at, __shfl_sync(0xffffffffu, l.first, at), __shfl_sync(0xffffffffu, l.tokens, at),
-                     (size_t)(count + __shfl_sync(0xffffffffu, l.upto - l.chunks, at))};
-    }
-    k -= __popc(scanned), count += __shfl_sync(0xffffffffu, l.upto, 31);
-  }
-  return Portion{};
-}
-__device__ __forceinline__ Portion portion_of(const Problem& p, int k) {
-  if (p.requests > 1) return search_portion(p.query_start, p.requests, p.least, k);
-  return Portion{0, p.query_start[0], p.query_start[1] - p.query_start[0], 0};
-}
-
-__device__ __forceinline__ float silu_of(float v) { return v * (1.f / (1.f + expf(-v))); }
-
-// (g_t, w_t) of a token (delta: w is beta).
-template <int FORM>
-__device__ __forceinline__ float2 gate_of(const Problem& p, int token, int head) {
-  const size_t at = (size_t)token * p.heads + head;
-  if (FORM == kMemory) return make_float2(p.gates[at * 3], p.gates[at * 3 + 1]);
-  if (FORM == kDelta) return make_float2(p.gates[at * 2], p.gates[at * 2 + 1]);
-  if (FORM == kDecay) return make_float2(p.gates[head], 1.f);
-  const float raw = load_as_float(p.step, p.step_dtype, (size_t)token * p.step_ld + p.step_col + head) + p.step_bias[head];
-  const float step = raw > 20.f ? raw : log1pf(expf(raw));           // softplus; above 20 the two agree in float32
-  return make_float2(expf(-expf(p.a_log[head]) * step), step);
-}
 
 // 64 rows of WIDTH numbers into shared memory as float32, zeros beyond `len` rows and `width` numbers.
 template <typename T, int WIDTH>
@@ -237,7 +132,7 @@ local_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
   int count;
-  const Where w = chunk_of(p, blockIdx.z, count);
+  const Where w = chunk_of<kC>(p, blockIdx.z, count);
   if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* ks = chunk_smem;                     // [64][NP + 4]
@@ -326,7 +221,7 @@ __global__ void __launch_bounds__(256)
 join_kernel(const Problem p) {
   grid_dependency_wait();
   grid_dependency_launch();
-  const Portion portion = portion_of(p, blockIdx.y);
+  const Portion portion = portion_of<kC>(p, blockIdx.y);
   const int count = (portion.tokens + kC - 1) / kC;
   const size_t all = (size_t)p.heads * p.columns * p.dim, at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * PER;
   if (count <= 0 || at >= all) return;
@@ -384,7 +279,7 @@ read_kernel(const Problem p) {
   const int tiles = (p.vdim + kTile - 1) / kTile, per_group = p.heads / p.kv_heads;
   const bool four_wide = p.dim % 4 == 0;
   int count;
-  chunk_of(p, 0x7fffffff, count);
+  chunk_of<kC>(p, 0x7fffffff, count);
   const long long units = (long long)count * p.heads * tiles;
   const long long last = units * (blockIdx.x + 1) / gridDim.x;
   long long unit = units * blockIdx.x / gridDim.x;
@@ -395,7 +290,7 @@ read_kernel(const Problem p) {
     const long long rest = unit / tiles;
     tile = (int)(unit % tiles), head = (int)(rest % p.heads), chunk = (int)(rest / p.heads);
   }
-  Where w = chunk_of(p, chunk, count);
+  Where w = chunk_of<kC>(p, chunk, count);
   // values: float32 ones that nothing is done to by asynchronous copies, 16-bit ones through registers, others when their unit begins
   constexpr bool kCopied = sizeof(V) == 4;
   constexpr int kPieces = kC * kTile * (int)sizeof(V) / 16 / kThreads, kEach = 16 / (int)sizeof(V), kPerRow = kTile / kEach;
@@ -572,7 +467,7 @@ read_kernel(const Problem p) {
         new_head = true;
         if (++head == p.heads) {
           head = 0;
-          w = chunk_of(p, ++chunk, count);
+          w = chunk_of<kC>(p, ++chunk, count);
         }
         new_keys = head % per_group == 0;
       }
@@ -617,7 +512,7 @@ solve_kernel(const Problem p, const Solved out) {
   grid_dependency_wait();
   grid_dependency_launch();
   int count;
-  const Where w = chunk_of(p, blockIdx.z, count);
+  const Where w = chunk_of<kC>(p, blockIdx.z, count);
   if (w.len <= 0) return;
   extern __shared__ __align__(16) float chunk_smem[];
   float* ks = chunk_smem;                     // [64][NP + 4]
@@ -771,7 +666,10 @@ carry_kernel(const Problem p, const Solved in) {
   float* u_now = s_at + kCarry * LD;          // [64][16]
   float* parts = u_now + kC * kCarry;         // [4][64][kPartLd]: quarters of W S_0; [1 or 3][16][LD]: sums over other threads' tokens
   const int tid = threadIdx.x, head = blockIdx.y, first_column = blockIdx.x * kCarry;
-  const Portion portion = portion_of(p, blockIdx.z);
+  const Portion portion = portion_of<kC>(p, blockIdx.z);
+  // (what is read on the tensor cores starts from every second chunk's S_0)
+  const int every = p.records != nullptr ? kChunk / kC : 1;
+  const size_t kept_place = p.records != nullptr ? portion_of<kChunk>(p, blockIdx.z).place : portion.place;
   const int request = portion.request, first = portion.first, q_len = portion.tokens, count = (q_len + kC - 1) / kC;
   if (count <= 0) return;
   const size_t place = portion.place;
@@ -849,7 +747,7 @@ carry_kernel(const Problem p, const Solved in) {
     cp_async_wait<0>();
     __syncthreads();                          // this chunk is there, S is there, the chunk before has been read
     if (c + 1 < count) fetch(c + 1, stage ^ 1);
-    if (keeps) store(p.chunk_states + ((place + c) * p.heads + head) * (size_t)p.vdim * p.dim + (size_t)first_column * p.dim, four_wide);
+    if (keeps && c % every == 0) store(p.chunk_states + ((kept_place + c / every) * p.heads + head) * (size_t)p.vdim * p.dim + (size_t)first_column * p.dim, four_wide);
     {
       // W S_0 over a quarter of the key entries: tokens t0 + 8 i, columns c0 + 4 j
       const int quarter = warp >> 1, t0 = 32 * (warp & 1) + (lane >> 2), c0 = lane & 3;
@@ -945,15 +843,8 @@ constexpr size_t read_bytes(int np) { return sizeof(float) * (size_t)(2 * kC * (
 constexpr size_t solve_bytes(int np) { return sizeof(float) * (size_t)(kC * (np + 4) + kC * kLd + 48 * kThreads + 5 * kC); }
 constexpr size_t carry_bytes(int np) { return sizeof(float) * (size_t)(4 * kC * (np + 4) + 3 * kC * kCarry + kCarry * (np + 4) + 4 * kC * kPartLd); }
 
-// The portions and chunks that a step of n tokens brings at most.
-struct Bounds { int portions, chunks; };
-static Bounds bounds_of(int n_tokens, int n_requests, int least) {
-  const int portions = n_tokens / least < n_requests ? n_tokens / least : n_requests;
-  return Bounds{portions, n_tokens / kC + portions};
-}
-
 template <typename T, int FORM, int NP>
-static int scan(const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
+static int scan(const Problem& p, const Bounds& most, const Bounds& kept, const Solved& solved, cudaStream_t stream) {
   const int tiles = (p.vdim + kTile - 1) / kTile;
   const dim3 grid(tiles, p.heads, most.chunks);
   const long long units = (long long)tiles * p.heads * most.chunks;                    // at most
@@ -974,6 +865,10 @@ static int scan(const Problem& p, const Bounds& most, const Solved& solved, cuda
     MS_CHECK_LAUNCH("chunk_scan: from chunk to chunk");
     Problem reading = p;
     reading.v = Rows{solved.u, p.heads * p.vdim, 0};
+    if (p.records != nullptr) {
+      reading.v_dtype = MS_F32, reading.v_wide = p.vdim % 4 == 0;
+      return launch_read(reading, kept, stream);
+    }
     if (p.vdim % 4) reading.wide = 0;
     ms::launch(read, readers, kThreads, read_bytes(NP), stream, reading);
   } else {
@@ -994,15 +889,26 @@ static int scan(const Problem& p, const Bounds& most, const Solved& solved, cuda
 }
 
 template <typename T, int FORM>
-static int scan_keys(const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
-  return p.dim <= 64 ? scan<T, FORM, 64>(p, most, solved, stream) : scan<T, FORM, 128>(p, most, solved, stream);
+static int scan_keys(const Problem& p, const Bounds& most, const Bounds& kept, const Solved& solved, cudaStream_t stream) {
+  return p.dim <= 64 ? scan<T, FORM, 64>(p, most, kept, solved, stream) : scan<T, FORM, 128>(p, most, kept, solved, stream);
 }
 
 template <typename T>
-static int scan_form(int form, const Problem& p, const Bounds& most, const Solved& solved, cudaStream_t stream) {
-  if (form == kMemory) return scan_keys<T, kMemory>(p, most, solved, stream);
-  if (form == kDelta) return scan_keys<T, kDelta>(p, most, solved, stream);
-  return scan_keys<T, kDecay>(p, most, solved, stream);
+static int scan_form(int form, const Problem& p, const Bounds& most, const Bounds& kept, const Solved& solved, cudaStream_t stream) {
+  if (form == kMemory) return scan_keys<T, kMemory>(p, most, kept, solved, stream);
+  if (form == kDelta) return scan_keys<T, kDelta>(p, most, kept, solved, stream);
+  return scan_keys<T, kDecay>(p, most, kept, solved, stream);
+}
+
+// All of a scan: on the tensor cores where there are records (the decays first, which nothing else waits for long).
+static int scan_any(int form, const Problem& p, int n_tokens, const Solved& solved, cudaStream_t stream) {
+  const Bounds most = bounds_of<kC>(n_tokens, p.requests, p.least), kept = bounds_of<kChunk>(n_tokens, p.requests, p.least);
+  if (p.records != nullptr) {
+    if (launch_gates(form, p, kept, stream)) return 1;
+    if (form != kDelta) return launch_local(p, kept, stream) || launch_read(p, kept, stream);
+  }
+  if (form == kSelective) return scan_keys<float, kSelective>(p, most, kept, solved, stream);
+  return p.qk_dtype == MS_F32 ? scan_form<float>(form, p, most, kept, solved, stream) : scan_form<__nv_bfloat16>(form, p, most, kept, solved, stream);
 }
 
 }  // namespace chunk_scan
@@ -1017,24 +923,33 @@ MS_EXPORT int ms_chunk_scan_chunk(int n_requests, int max_query_len, int heads, 
   return n_requests > 0 && max_query_len > 0 && heads > 0 && heads <= 65535 && dim > 0 && dim <= 128 ? kC : 0;
 }
 
+// Tokens of a chunk on the tensor cores, and the floats of such a chunk's record (per head).
+MS_EXPORT int ms_chunk_scan_tokens() { return kChunk; }
+MS_EXPORT int ms_chunk_scan_record() { return kRecord; }
+
 // Arguments as ms_matrix_scan's forms 0 (memory), 1 (delta) and 2 (constant decay); portions of fewer than `least` tokens are left
 // alone.  chunk_states float32 [places, heads, columns, dim] and chunk_decays float32 [places, heads], places = n_tokens / 64 +
 // min(n_requests, n_tokens / least), at most 65,535; delta: w, ke float32 [n_tokens, heads, dim], u float32 [n_tokens, heads, vdim].
-// chunk_states and u on 16-byte boundaries.
+// records not null: on the tensor cores.  chunk_states has places = n_tokens / 128 + min(n_requests, n_tokens / least) then, and records are
+// float32 [those places, heads, ms_chunk_scan_record()]; only the delta form needs chunk_decays; not with input_act.  All on 16-byte
+// boundaries.  error_flag: one int on the device that a kernel which gave up waiting sets.
 MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const void* k, int k_ld, int k_col, const void* v, int v_ld,
                             int v_col, int dtype, float q_scale, const float* gates, float* states, long long state_stride,
                             int state_offset, const int* state_slots, const int* query_start, int n_requests, int n_tokens, int least,
                             int heads, int kv_heads, int dim, int vdim, float* y, float* bottom, int input_act, float* chunk_states,
-                            float* chunk_decays, float* w, float* u, float* ke, cudaStream_t stream) {
+                            float* chunk_decays, float* w, float* u, float* ke, float* records, int* error_flag, cudaStream_t stream) {
   if (n_requests == 0 || n_tokens == 0 || heads == 0) return 0;
   MS_REQUIRE(form >= kMemory && form <= kDecay, "chunk_scan: form %d", form);
   MS_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && dim >= 1 && dim <= 128 && vdim >= 1, "chunk_scan: %d/%d heads of %d/%d", heads,
              kv_heads, dim, vdim);
   MS_REQUIRE(form != kDelta || !input_act, "chunk_scan: the delta form takes its inputs as they are");
   MS_REQUIRE(form != kMemory || bottom != nullptr, "chunk_scan: the memory form writes the tokens' divisors");
-  MS_REQUIRE(chunk_states && chunk_decays && (form != kDelta || (w && u && ke)), "chunk_scan: scratch is missing");
+  MS_REQUIRE(chunk_states && (chunk_decays || (records && form != kDelta)) && (form != kDelta || (w && u && ke)) && (!records || error_flag),
+             "chunk_scan: scratch is missing");
+  MS_REQUIRE(!records || !input_act, "chunk_scan: the tensor cores take inputs as they are");
+  MS_REQUIRE(dtype == MS_F32 || dtype == MS_BF16, "unknown element type code %d", dtype);
   MS_REQUIRE(least >= 1, "chunk_scan: portions of %d tokens and more", least);
-  const Bounds most = bounds_of(n_tokens, n_requests, least);
+  const Bounds most = bounds_of<kC>(n_tokens, n_requests, least);
   if (most.portions == 0) return 0;
   MS_REQUIRE(heads <= 65535 && most.chunks <= 65535, "chunk_scan: %d heads, %d chunks exceed the launch limits", heads, most.chunks);
   const int per = dtype == MS_F32 ? 4 : 8;
@@ -1044,13 +959,11 @@ MS_EXPORT int ms_chunk_scan(int form, const void* q, int q_ld, int q_col, const 
   Problem p = {};
   p.q = Rows{q, q_ld, q_col}, p.k = Rows{k, k_ld, k_col}, p.v = Rows{v, v_ld, v_col};
   p.heads = heads, p.kv_heads = kv_heads, p.dim = dim, p.vdim = vdim, p.columns = form == kMemory ? vdim + 1 : vdim;
-  p.input_act = input_act, p.wide = wide, p.q_scale = q_scale, p.gates = gates;
+  p.qk_dtype = p.v_dtype = dtype, p.input_act = input_act, p.wide = p.v_wide = wide, p.q_scale = q_scale, p.gates = gates;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
   p.requests = n_requests, p.least = least, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y, p.bottom = bottom;
-  const Solved solved{w, u, ke};
-  if (dtype == MS_F32) return scan_form<float>(form, p, most, solved, stream);
-  if (dtype == MS_BF16) return scan_form<__nv_bfloat16>(form, p, most, solved, stream);
-  MS_FAIL("unknown element type code %d", dtype);
+  p.records = records, p.error_flag = error_flag;
+  return scan_any(form, p, n_tokens, Solved{w, u, ke}, stream);
 }
 
 // Arguments as ms_selective_scan; `least` and scratch as above with columns = p (a head's channels) and dim = n_state.
@@ -1058,24 +971,26 @@ MS_EXPORT int ms_selective_chunk_scan(const float* conv, int conv_ld, const void
                                       const float* a_log, const float* d, float* states, long long state_stride, int state_offset,
                                       const int* state_slots, const int* query_start, int n_requests, int n_tokens, int least, int heads,
                                       int channels, int n_state, int groups, float* y, float* chunk_states, float* chunk_decays,
-                                      cudaStream_t stream) {
+                                      float* records, int* error_flag, cudaStream_t stream) {
   if (n_requests == 0 || n_tokens == 0) return 0;
   MS_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "selective_chunk_scan: %d heads in %d groups", heads, groups);
   MS_REQUIRE(n_state >= 1 && n_state <= 128 && channels >= 1, "selective_chunk_scan: a state of %d numbers for %d channels", n_state, channels);
   MS_REQUIRE(dtype == MS_F32 || dtype == MS_BF16, "unknown element type code %d", dtype);
-  MS_REQUIRE(chunk_states && chunk_decays, "selective_chunk_scan: scratch is missing");
+  MS_REQUIRE(chunk_states && (chunk_decays || (records && error_flag)), "selective_chunk_scan: scratch is missing");
   MS_REQUIRE(least >= 1, "selective_chunk_scan: portions of %d tokens and more", least);
-  const Bounds most = bounds_of(n_tokens, n_requests, least);
+  const Bounds most = bounds_of<kC>(n_tokens, n_requests, least);
   if (most.portions == 0) return 0;
   MS_REQUIRE(heads <= 65535 && most.chunks <= 65535, "selective_chunk_scan: %d heads, %d chunks exceed the launch limits", heads, most.chunks);
   const int inner = heads * channels;
   Problem p = {};
   p.v = Rows{conv, conv_ld, 0}, p.k = Rows{conv, conv_ld, inner}, p.q = Rows{conv, conv_ld, inner + groups * n_state};
   p.heads = heads, p.kv_heads = groups, p.dim = n_state, p.vdim = channels, p.columns = channels;
-  p.wide = conv_ld % 4 == 0 && inner % 4 == 0 && n_state % 4 == 0 && channels % 4 == 0 && reinterpret_cast<size_t>(conv) % 16 == 0;
+  p.qk_dtype = p.v_dtype = MS_F32;
+  p.wide = p.v_wide = conv_ld % 4 == 0 && inner % 4 == 0 && n_state % 4 == 0 && channels % 4 == 0 && reinterpret_cast<size_t>(conv) % 16 == 0;
   p.q_scale = 1.f;
   p.step = proj, p.step_dtype = dtype, p.step_ld = ld, p.step_col = dt_col, p.step_bias = dt_bias, p.a_log = a_log, p.skip = d;
   p.states = states, p.state_stride = state_stride, p.state_offset = state_offset, p.state_slots = state_slots, p.query_start = query_start;
   p.requests = n_requests, p.least = least, p.chunk_states = chunk_states, p.chunk_decays = chunk_decays, p.y = y;
-  return scan_keys<float, kSelective>(p, most, Solved{}, stream);
+  p.records = records, p.error_flag = error_flag;
+  return scan_any(kSelective, p, n_tokens, Solved{}, stream);
 }

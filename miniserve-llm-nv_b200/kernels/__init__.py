@@ -18,7 +18,7 @@ import torch
 
 from . import build
 
-ABI_VERSION = 14
+ABI_VERSION = 15
 log = logging.getLogger("miniserve_b200")
 _library: Optional[ctypes.CDLL] = None
 
@@ -978,12 +978,32 @@ CHUNK_SCAN_BESIDE = (28, 2)
 # tokens and 64 single ones: 242 us with 31, 200 with 4.
 WALK_BESIDE_CHUNK = 4
 MAX_INT = 2 ** 31 - 1
+# From which work on (tokens x heads x key entries x value columns) a scan in chunks runs on the tensor cores, where a block of 128 tokens and 64
+# columns takes the same time whatever there is in it: with operands of three parts each when two value tiles or two blocks of key entries
+# share what a block prepares, with bfloat16 ones always for more than 64 key entries.  The scans alone, float32 pipe / tensor cores
+# in us at 256, 512, 1,000 and 2,048 tokens: memory, 8 heads of 128 x 256: 37 / 27, 43 / 34, 75 / 47, 119 / 65; 16 of 64 x 128: 28 / 25, 31 / 33, 51 / 41,
+# 88 / 66; selective, 64 heads of 128 x 64: 42 / 37, 69 / 58, 114 / 81, 210 / 124; 32 of 128 x 64: 35 / 37, 41 / 37, 65 / 49, 111 / 72; 32 of 64 x 128: 29 / 32, 47 / 47,
+# 74 / 66, 126 / 99; delta, 16 heads of 128 x 128: 57 / 56, 71 / 76, 125 / 118, 234 / 212; 32 of 64 x 64: 41 / 51, 51 / 67, 96 / 120, 188 / 234.  Portions that
+# fill a chunk badly cost as much as whole ones: their mean is asked for, or one that is half of the step.
+TENSOR_SCAN_WORK, TENSOR_SCAN_EXACT, TENSOR_SCAN_MEAN = 240_000_000, 100_000_000, 96
+
+
+def _scanned_on_tensor_cores(n: int, n_requests: int, longest: int, heads: int, dim: int, vdim: int, as_they_are: bool) -> bool:
+    """Whether a step that is scanned in chunks is scanned on the tensor cores (``as_they_are``: q, k and v are bfloat16 and nothing is done to
+    them, so that each is one exact part)."""
+    work = n * heads * dim * vdim
+    if as_they_are:
+        large = dim > 64 or work >= TENSOR_SCAN_EXACT
+    else:
+        large = (dim > 64 or vdim > 64) and work >= TENSOR_SCAN_WORK
+    return large and (2 * longest >= n or n >= TENSOR_SCAN_MEAN * n_requests)
 
 
 def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, columns: int, device, delta: bool = False,
-                   beside: int = 0) -> Optional[tuple]:
+                   beside: int = 0, tensor_cores: bool = False) -> Optional[tuple]:
     """(chunk states, chunk decays; delta: and W, U and the keys as a chunk's end sees them) for the scans in chunks, or None where the
-    step's tokens are walked one after the other."""
+    step's tokens are walked one after the other.  ``tensor_cores``: the states are fewer, and the last
+    are the records of decays (or not, where those do not fit)."""
     if delta:
         if longest <= 0 or longest < CHUNK_SCAN_DELTA * (1 + (n + longest - 1) // longest):
             return None
@@ -1002,7 +1022,17 @@ def _chunk_scratch(n: int, n_requests: int, longest: int, heads: int, dim: int, 
         shapes += [(n, heads, dim), (n, heads, columns), (n, heads, dim)]
     if places > 65535 or 4 * sum(math.prod(shape) for shape in shapes) > MAX_CHUNK_SCRATCH:
         return None
+    if tensor_cores:
+        kept = n // _asked("ms_chunk_scan_tokens") + min(n_requests, n // CHUNK_SCAN_LEAST)
+        wanted = [(kept, heads, columns, dim)] + shapes[1:] + [(kept, heads, _asked("ms_chunk_scan_record"))]
+        if 4 * sum(math.prod(shape) for shape in wanted) <= MAX_CHUNK_SCRATCH:       # (small matrices: the records are larger)
+            shapes = wanted
     return tuple(torch.empty(shape, dtype=torch.float32, device=device) for shape in shapes)
+
+
+def _records(scratch: tuple, delta: bool = False) -> Optional[torch.Tensor]:
+    """The records of decays among a scan's scratch: there are some if it is for the tensor cores."""
+    return scratch[-1] if len(scratch) > (5 if delta else 2) else None
 
 
 def _none_short(n: int, n_requests: int, longest: int) -> bool:
@@ -1074,13 +1104,15 @@ def selective_scan(conv: torch.Tensor, proj: torch.Tensor, dt_col: int, dt_bias:
         raise KernelError(f"selective_scan: {heads} heads in {groups} groups, state {state}, dt from column {dt_col} of rows of {ld}")
     stride = _state_rows(states, state_offset, inner * state)
     longest = n if max_query_len is None else max_query_len
-    scratch = _chunk_scratch(n, n_requests, longest, heads, state, head_dim, y.device) if chunked else None
+    tensor_cores = _scanned_on_tensor_cores(n, n_requests, longest, heads, state, head_dim, False)
+    scratch = _chunk_scratch(n, n_requests, longest, heads, state, head_dim, y.device, tensor_cores=tensor_cores) if chunked else None
     if scratch is not None:
         _check(library().ms_selective_chunk_scan(_ptr(conv), _i(conv.shape[1]), _ptr(proj), _i(_code(proj.dtype)), _i(ld), _i(dt_col),
                                                  _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(states), stride, _i(state_offset),
                                                  _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n), _i(CHUNK_SCAN_LEAST),
                                                  _i(heads), _i(head_dim), _i(state), _i(groups), _ptr(y), _ptr(scratch[0]),
-                                                 _ptr(scratch[1]), _stream()))
+                                                 _ptr(scratch[1]), _ptr(_records(scratch)),
+                                                 _ptr(device_error_flag(y.device)) if tensor_cores else None, _stream()))
         if _none_short(n, n_requests, longest):
             return
         longest = min(longest, WALK_BESIDE_CHUNK)
@@ -1189,8 +1221,8 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
 
     ``"channel_decay"`` of few long portions runs in chunks that need not wait for one another (a walk from zero per chunk, a join
     of the chunks' matrices, a walk from the joined ones): ``chunk`` None lets the library choose, 0 forbids it, a number is
-    the chunk's tokens.  ``"memory"``, ``"delta"`` and ``"decay"`` of portions of many tokens run as matrix products over chunks of 64
-    tokens (``csrc/chunk_scan.cu``; CHUNK_SCAN_LONGEST says from when on) unless ``chunk`` is 0, which walks them; other numbers are
+    the chunk's tokens.  ``"memory"``, ``"delta"`` and ``"decay"`` of portions of many tokens run as matrix products over chunks of 64 or, on the
+    tensor cores, 128 tokens (``csrc/chunk_scan.cu``; CHUNK_SCAN_LONGEST and TENSOR_SCAN_WORK say from when on) unless ``chunk`` is 0, which walks them; other numbers are
     refused there."""
     code = MATRIX_SCAN_MODES[mode]
     n = y.shape[0]
@@ -1238,15 +1270,18 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
         return
     scratch = None
     if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
-        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1, CHUNK_SCAN_BESIDE[1])
+        tensor_cores = input_activation == "none" and _scanned_on_tensor_cores(
+            n, n_requests, max_query_len, heads, dim, vdim, code != 1 and q.dtype == torch.bfloat16)
+        scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1, CHUNK_SCAN_BESIDE[1], tensor_cores)
     if scratch is not None:
-        solved = scratch[2:] or [None] * 3
+        solved = scratch[2:5] if code == 1 else [None] * 3
         _check(library().ms_chunk_scan(_i(code), _ptr(q), _i(q.shape[1]), _i(q_col), _ptr(k), _i(k.shape[1]), _i(k_col), _ptr(v),
                                        _i(v.shape[1]), _i(v_col), _i(_code(q.dtype)), _f(q_scale), _ptr(gates), _ptr(states), stride,
                                        _i(state_offset), _ptr(state_slots), _ptr(query_start), _i(n_requests), _i(n),
                                        _i(CHUNK_SCAN_LEAST), _i(heads), _i(kv_heads), _i(dim), _i(vdim), _ptr(y), _ptr(bottom),
                                        _i(CONV_ACTIVATIONS[input_activation]), _ptr(scratch[0]), _ptr(scratch[1]), _ptr(solved[0]),
-                                       _ptr(solved[1]), _ptr(solved[2]), _stream()))
+                                       _ptr(solved[1]), _ptr(solved[2]), _ptr(_records(scratch, code == 1)),
+                                       _ptr(device_error_flag(y.device)) if tensor_cores else None, _stream()))
         if _none_short(n, n_requests, max_query_len):
             return
         max_query_len = min(max_query_len, WALK_BESIDE_CHUNK)

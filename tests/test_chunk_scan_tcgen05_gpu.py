@@ -1,0 +1,104 @@
+"""The scans in chunks on the tensor cores (chunks of 128 tokens, operands in exact bfloat16 parts): the tests of the scans in chunks at lengths and
+sizes around the borders of chunks, tiles of 64 value columns and blocks of 64 key entries, and what only these kernels have."""
+
+import pytest
+import torch
+
+import test_chunk_scan_gpu as scans
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [[128], [127, 1, 0, 129], [257, 63], [1, 200, 7], [96, 64, 65, 2, 511]]
+SIZES = [(4, 2, 128, 128), (2, 2, 64, 64), (3, 3, 40, 56), (2, 1, 100, 130), (1, 1, 33, 3), (2, 2, 128, 259), (2, 1, 6, 17), (2, 1, 72, 64)]
+
+
+@pytest.fixture
+def on_tensor_cores(monkeypatch):
+    from miniserve_b200 import kernels
+
+    for name in ("CHUNK_SCAN_LONGEST", "CHUNK_SCAN_DELTA"):
+        monkeypatch.setattr(kernels, name, 0)
+    monkeypatch.setattr(kernels, "_scanned_on_tensor_cores", lambda *args: True)
+    lib, records = kernels.library(), []
+    for name in ("ms_chunk_scan", "ms_selective_chunk_scan"):
+        monkeypatch.setattr(lib, name, lambda *args, real=getattr(lib, name): records.append(args[-3]) or real(*args))
+    yield
+    assert records and all(records)                    # (not the float32 pipe)
+    kernels.check_device_errors(torch.device("cuda:0"))
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["memory", "delta"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", SIZES)
+@pytest.mark.parametrize("lengths", LENGTHS)
+def test_against_the_definition(form, dtype, heads, kv_heads, dim, vdim, lengths):
+    scans.test_matrix_scan_in_chunks(form, dtype, heads, kv_heads, dim, vdim, lengths)
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("heads,P,N,G", [(4, 64, 128, 2), (3, 64, 64, 1), (2, 40, 24, 2), (2, 130, 100, 1), (1, 3, 7, 1)])
+@pytest.mark.parametrize("lengths", LENGTHS)
+def test_selective(heads, P, N, G, lengths):
+    scans.test_selective_scan_in_chunks(torch.bfloat16, heads, P, N, G, lengths)
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["memory", "delta", "decay"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(20, 5, 128, 136), (21, 7, 40, 130), (16, 16, 64, 64)])
+def test_runs_of_units(form, dtype, heads, kv_heads, dim, vdim):
+    """More units than multiprocessors, of more requests than a warp has lanes, some without tokens, some too short: the walk's rows.  (Either
+    way is within 2e-5 of the definition, see there: 4e-5 apart.)"""
+    lengths = [1, 0, 65, 3, 130] * 7 + [0, 0, 200, 64]
+    rows, cols, gates, slots, states, kv_heads, columns = scans.problem(form, dtype, lengths, heads, kv_heads, dim, vdim, 11 + dim)
+    walked = states.clone()
+    y, bottom = scans.run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, vdim)
+    y_walk, bottom_walk = scans.run(form, rows, cols, gates, slots, walked, lengths, heads, kv_heads, dim, vdim, chunk=0)
+    pairs = [(y, y_walk), (states, walked)] + ([(bottom, bottom_walk)] if form == "memory" else [])
+    scale = max(1.0, float(y_walk.abs().max()))
+    assert all(float((a.double() - b.double()).abs().max()) <= 4e-5 * scale for a, b in pairs)
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("form", ["memory", "delta", "decay"])
+def test_an_infinity_reaches_no_token_before_it(form):
+    scans.test_an_infinity_reaches_no_token_before_it(form)
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form,which", [("memory", 0), ("memory", 1), ("memory", 2), ("decay", 2), ("delta", 0)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.0e38])
+def test_what_is_not_finite_is_summed_plainly(form, which, dtype, value):
+    """One number of the queries, keys or values: the rows and matrices that it reaches are those of the walk, the others its to the bound."""
+    lengths, bad = [300], 77
+    rows, cols, gates, slots, states, kv_heads, columns = scans.problem(form, dtype, lengths, 2, 2, 72, 96, 21)
+    rows[bad, cols[which] + 5] = value
+    walked = states.clone()
+    y, bottom = scans.run(form, rows, cols, gates, slots, states, lengths, 2, kv_heads, 72, 96)
+    y_walk, bottom_walk = scans.run(form, rows, cols, gates, slots, walked, lengths, 2, kv_heads, 72, 96, chunk=0)
+    usual = 30.0                                       # (results of the other numbers are below it; 3e38 times an ordinary number is not)
+    # (An infinite query's own bottom is the floor in chunks, on either pipe: infinities of both signs meet in q n.)
+    for a, b in [(y, y_walk), (states, walked)] + ([(bottom, bottom_walk)] if form == "memory" and which else []):
+        small = b.abs() <= usual
+        assert torch.equal(a.abs() <= usual, small)
+        assert float((a - b).abs()[small].max()) <= 4e-5 * usual
+
+
+def test_which_scans_run_there(monkeypatch):
+    from miniserve_b200 import kernels
+
+    taken = kernels._scanned_on_tensor_cores
+    # memory and constant decay in bfloat16: always with more than 64 key entries, or enough work
+    assert taken(256, 1, 256, 8, 128, 256, True) and not taken(512, 1, 512, 16, 64, 128, True) and taken(1000, 1, 1000, 16, 64, 128, True)
+    # three parts: two tiles or two blocks, and more work
+    assert not taken(256, 1, 256, 64, 128, 64, False) and taken(512, 1, 512, 64, 128, 64, False) and not taken(2048, 1, 2048, 32, 64, 64, False)
+    # portions that leave chunks empty
+    assert not taken(2048, 30, 200, 8, 128, 256, True) and taken(2048, 20, 200, 8, 128, 256, True) and taken(1100, 65, 1036, 8, 128, 256, True)
+    # records that do not fit: the float32 pipe's scratch
+    n = 1_000_000
+    assert len(kernels._chunk_scratch(n, 1, n, 8, 65, 9, "meta", tensor_cores=True)) == 2
+    monkeypatch.setattr(kernels, "_scanned_on_tensor_cores", lambda *args: True)
+    rows, cols, gates, slots, states, kv_heads, columns = scans.problem("memory", torch.bfloat16, [300], 1, 1, 8, 8, 3)
+    scans.run("memory", rows, cols, gates, slots, states, [300], 1, kv_heads, 8, 8)
