@@ -128,9 +128,9 @@ __device__ __forceinline__ float2 gate_of(const Problem& p, int token, int head)
 //   F      [3][128] pairs   for the rows of block w + 1 (of 32): decays from s to the block's start, times w_s and the scale of the queries
 //   diag   [4][32][32]      within block w: the same from token j (row) to token t (column)
 //   G      [128]            decays from the chunk's start to t, times the scale
-//   end    [128]            decays from behind s to the chunk's end, times w_s
+//   end    [128] pairs      decays from behind s to the chunk's end, times w_s
 //   all    [1]              the product of all
-constexpr int kRecordA = 0, kRecordF = 256, kRecordDiag = 1024, kRecordG = 5120, kRecordEnd = 5248, kRecordAll = 5376, kRecord = 5380;
+constexpr int kRecordA = 0, kRecordF = 256, kRecordDiag = 1024, kRecordG = 5120, kRecordEnd = 5248, kRecordAll = 5504, kRecord = 5508;
 
 // The portions and chunks of C tokens that a step of n tokens brings at most.
 struct Bounds { int portions, chunks; };

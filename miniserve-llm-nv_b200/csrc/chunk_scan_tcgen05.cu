@@ -7,7 +7,9 @@
 // Float32 operands are cut into three bfloat16 parts that add up to them exactly, and the six products of parts that reach a float32's last
 // bit are summed, smallest first; what comes in bfloat16 already (queries, keys and values straight from a projection) is one part, and its
 // products with three parts are three.  An addition in tensor memory drops the bits behind its last instead of rounding, so a sum
-// lives there for 64 numbers only (16 or 32 where it is a score, whose error a row's values share) and sums of those are added in float32 registers.
+// lives there for 64 numbers only (16 or 32 where it is a score, whose error a row's values share, or a state's) and sums of those are added in
+// float32 registers; what such sums lose on average is in the decays (gates_kernel).  Relative errors against 64 bits, the float32 pipe's and these:
+// memory form, 128 x 256, bfloat16, y 1.04e-7 and 0.74e-7, states 0.74e-7 and 0.46e-7; all positive 0.67e-7 and 0.41e-7; selective, 64 x 128, 1.66e-7 and 0.95e-7, 0.79e-7 and 0.74e-7.
 //
 // In the read kernel the scores pass from tensor memory through registers, where they get their decays, back to tensor memory as the parts of the
 // next product's operand: they are never in memory.
@@ -42,6 +44,14 @@ __device__ __forceinline__ float2 pair_of(double v) {
   return make_float2(hi, is_finite(hi) ? (float)(v - (double)hi) : 0.f);
 }
 
+// What the sums in tensor memory lose on average, relative to the result, since their additions drop bits: of a row by way of its scores, of one by way of
+// S_0, of a chunk's own matrix.  The decays are made larger by as much, which leaves the losses' spread.  Measured on operands of either sign and
+// on positive ones, 8 heads' worth of each: rows of exact scores 6.3e-8 and 8.2e-8 (key entries in one block 5.1e-8, 6.1e-8), of scores of
+// three parts 8.3e-8 and 9.5e-8 (7.6e-8, 8.5e-8); S_0 of 64 entries and more 5.9e-8 and 7.8e-8, of 32 4.0e-8 and 4.5e-8; matrices 3.8e-8, 4.7e-8.
+__device__ __forceinline__ double rows_loss(const Problem& p) { return p.qk_dtype == MS_BF16 ? (p.dim > 64 ? 7.2e-8 : 5.6e-8) : p.dim > 64 ? 8.9e-8 : 8.0e-8; }
+__device__ __forceinline__ double start_loss(const Problem& p) { return 1.7e-8 + 1.25e-8 * min(4, (p.dim + 15) / 16); }
+constexpr double kMatrixLoss = 4.2e-8;
+
 template <int FORM>
 __global__ void __launch_bounds__(kChunk)
 gates_kernel(const __grid_constant__ Problem p) {
@@ -57,7 +67,7 @@ gates_kernel(const __grid_constant__ Problem p) {
     gate = gate_of<FORM>(p, w.first + t, head);
     if (FORM == kDelta) gate.y = 1.f;        // (what reads take for w v is u)
   }
-  const double g = gate.x, weight = gate.y, scaled = weight * (double)p.q_scale;
+  const double g = gate.x, weight = gate.y, scaled = weight * (double)p.q_scale * (1.0 + rows_loss(p));
   double upto = g, behind = g;               // products of the block's decays up to and with t, from t on
 #pragma unroll
   for (int d = 1; d < 32; d *= 2) {
@@ -79,10 +89,10 @@ gates_kernel(const __grid_constant__ Problem p) {
     reinterpret_cast<float2*>(record + kRecordF)[(b - 1) * kChunk + t] = block < b ? pair_of(product * scaled) : make_float2(0.f, 0.f);
     if (block < b) product *= blocks[b];
   }
-  record[kRecordEnd + t] = t < w.len ? (float)(product * weight) : 0.f;
+  reinterpret_cast<float2*>(record + kRecordEnd)[t] = t < w.len ? pair_of(product * weight * (1.0 + kMatrixLoss)) : make_float2(0.f, 0.f);
   double from_start = upto;
   for (int b = 0; b < block; ++b) from_start *= blocks[b];
-  record[kRecordG + t] = (float)(from_start * (double)p.q_scale);
+  record[kRecordG + t] = (float)(from_start * (double)p.q_scale * (1.0 + start_loss(p)));
   if (t == kChunk - 1) record[kRecordAll] = (float)from_start;
   double d = 1.0;
   for (int j = 31; j >= 0; --j) {            // D(t, block's token j), t's own block
@@ -133,19 +143,27 @@ __device__ __forceinline__ void floats_of(const Raw& r, int dtype, float (&v)[8]
   for (int e = 0; e < 8; ++e)
     v[e] = __uint_as_float(dtype == MS_F32 ? w[e] : e % 2 == 0 ? w[e / 2] << 16 : w[e / 2] & 0xffff0000u);
 }
-// Two numbers' parts, packed; exact: what is left behind two roundings to eight bits has eight bits.
-__device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
+// Two numbers' parts, packed; exact: what is left behind two roundings to eight bits has eight bits.  What rounding the numbers themselves
+// left (`more_a`, `more_b`: they are products) goes into the last part, and only that is rounded.
+__device__ __forceinline__ void cut(float a, float b, float more_a, float more_b, unsigned& hi, unsigned& mid, unsigned& lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
   a -= __uint_as_float(hi << 16), b -= __uint_as_float(hi & 0xffff0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
   a -= __uint_as_float(mid << 16), b -= __uint_as_float(mid & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b + more_b), "f"(a + more_a));
 }
+__device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) { cut(a, b, 0.f, 0.f, hi, mid, lo); }
 __device__ __forceinline__ void cut_eight(const float (&v)[8], uint4 (&part)[3]) {
   cut(v[0], v[1], part[0].x, part[1].x, part[2].x);
   cut(v[2], v[3], part[0].y, part[1].y, part[2].y);
   cut(v[4], v[5], part[0].z, part[1].z, part[2].z);
   cut(v[6], v[7], part[0].w, part[1].w, part[2].w);
+}
+__device__ __forceinline__ void cut_eight(const float (&v)[8], const float (&more)[8], uint4 (&part)[3]) {
+  cut(v[0], v[1], more[0], more[1], part[0].x, part[1].x, part[2].x);
+  cut(v[2], v[3], more[2], more[3], part[0].y, part[1].y, part[2].y);
+  cut(v[4], v[5], more[4], more[5], part[0].z, part[1].z, part[2].z);
+  cut(v[6], v[7], more[6], more[7], part[0].w, part[1].w, part[2].w);
 }
 // Whether any of eight leading parts is an infinity or a NaN: zero times it is not zero.
 __device__ __forceinline__ bool any_endless(const uint4& v) {
@@ -360,10 +378,10 @@ __device__ __noinline__ void plain_row(const Problem& p, size_t place, int first
   }
 }
 // The same for a number of a chunk's own matrix.
-__device__ __noinline__ float plain_entry(const Problem& p, const float* weights, int first, int len, int head, int column, int entry) {
+__device__ __noinline__ float plain_entry(const Problem& p, const float2* weights, int first, int len, int head, int column, int entry) {
   float sum = 0.f;
   for (int s = 0; s < len; ++s)
-    sum = fmaf(weights[s] * value_at(p, first + s, head, column), number_at(p, p.k, p.qk_dtype, first + s, head / (p.heads / p.kv_heads) * p.dim + entry), sum);
+    sum = fmaf(weights[s].x * value_at(p, first + s, head, column), number_at(p, p.k, p.qk_dtype, first + s, head / (p.heads / p.kv_heads) * p.dim + entry), sum);
   return sum;
 }
 
@@ -468,7 +486,7 @@ read_kernel(const __grid_constant__ Problem p) {
     };
     float sum[32];
     unsigned results[2] = {0, 0};
-    auto add_results = [&](int halves) {
+    auto add_results = [&](int halves, float scale) {          // (of what there is)
 #pragma unroll 1
       for (int h = 0; h < halves; ++h) {
         waits.wait(&result_full[h], (h == 0 ? results[0]++ : results[1]++) & 1, 77);
@@ -479,8 +497,9 @@ read_kernel(const __grid_constant__ Problem p) {
           tmem_load_16_nowait(row + 64 * h + i0, v);
           tmem_load_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) sum[i0 + i] += v[i];
+          for (int i = 0; i < 16; ++i) sum[i0 + i] = fmaf(sum[i0 + i], scale, v[i]);
         }
+        scale = 1.f;
       }
     };
     // a unit's results to memory: eight columns at a time by way of shared memory, so that a store takes whole sectors.  Rows from a value on
@@ -560,7 +579,7 @@ read_kernel(const __grid_constant__ Problem p) {
       const float decayed = record_at(p, u)[kRecordG + t];
 #pragma unroll
       for (int i = 0; i < 32; ++i) sum[i] = 0.f;
-      add_results(NB);
+      add_results(NB, 1.f);
       cp_async_wait<1>();
       if (tid == 0) endless[(n + 2) & 3] = kChunk;       // (every warp is done with the results of the unit before the last)
 #pragma unroll 1
@@ -600,9 +619,7 @@ read_kernel(const __grid_constant__ Problem p) {
       }
       if (more) request_values(next);
       else cp_async_commit();
-#pragma unroll
-      for (int i = 0; i < 32; ++i) sum[i] *= decayed;
-      add_results(2);
+      add_results(2, decayed);
       before = u, u = next;
     }
     cp_async_wait<0>();
@@ -789,7 +806,7 @@ read_kernel(const __grid_constant__ Problem p) {
 
 // ------------------------------------------------------------------------------------------------- a chunk's own matrix
 // The same roles; a unit is the product of the keys (their 64-entry blocks are the MMA's rows, read transposed) and the 64 weighted value
-// columns over the chunk's tokens, each half of them a sum.  Values and results have two buffers each.  Bound by the cutting of keys and
+// columns over the chunk's tokens, each quarter of them a sum.  Values and results have two buffers each.  Bound by the cutting of keys and
 // values and, in the memory form, by what it writes: the float32 pipe's kernel and this, 2,048 tokens: memory, 8 heads of 128 x 256, 28.9 and 15.8 us;
 // selective, 64 of 128 x 64, 57.9 and 28.2.  The join has half as many matrices: 14.2 and 10.1, 43.8 and 16.2 us.
 template <int KP, int NB>
@@ -819,7 +836,7 @@ local_kernel(const __grid_constant__ Problem p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kFirstIssuer) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(&tmem_base_s)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base_s)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tmem_fence_before();
@@ -835,13 +852,13 @@ local_kernel(const __grid_constant__ Problem p) {
     const int c = threadIdx.x & 7, row0 = threadIdx.x >> 3;
     const bool one_column = p.columns > p.vdim;
     uint4* raw_values = reinterpret_cast<uint4*>(v_s + 2 * L::VALUES) + threadIdx.x;
-    float weight[4];
+    float2 weight[4];
     auto request_values = [&](const Unit& u) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         stage_eight(raw_values + 2 * i * kFetchers, p.v.at, p.v_dtype, value_index(p, u, row0 + 32 * i), values_valid(p, u, row0 + 32 * i), p.v_wide);
       cp_async_commit();
-      const float* weights = record_at(p, u) + kRecordEnd + row0;
+      const float2* weights = reinterpret_cast<const float2*>(record_at(p, u) + kRecordEnd) + row0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) weight[i] = weights[32 * i];
     };
@@ -864,12 +881,16 @@ local_kernel(const __grid_constant__ Problem p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int token = row0 + 32 * i;
-        float v[8];
+        float v[8], more[8];
         uint4 part[3];
         floats_of(staged_eight(raw_values + 2 * i * kFetchers, p.v_dtype), p.v_dtype, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = weight[i] * (e == one ? 1.f : v[e]);
-        cut_eight(v, part);
+        for (int e = 0; e < 8; ++e) {
+          const float value = e == one ? 1.f : v[e];
+          v[e] = weight[i].x * value;
+          more[e] = fmaf(weight[i].y, value, fmaf(weight[i].x, value, -v[e]));
+        }
+        cut_eight(v, more, part);
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(v_s + buffer * L::VALUES + q * kRowsBlock + place_of(token, c)) = part[q];
       }
@@ -890,10 +911,11 @@ local_kernel(const __grid_constant__ Problem p) {
       waits.wait(&result_full[buffer], (n >> 1) & 1, 86);
       tmem_fence_after();
       float sum[32];
-      tmem_load_32(row + 128 * buffer + 32 * half, sum);
-      if (u.len > 64) {
+      tmem_load_32(row + 256 * buffer + 32 * half, sum);
+#pragma unroll 1
+      for (int part = 1; part * 32 < u.len; ++part) {
         float v[32];
-        tmem_load_32(row + 128 * buffer + 64 + 32 * half, v);
+        tmem_load_32(row + 256 * buffer + 64 * part + 32 * half, v);
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[i] += v[i];
       }
@@ -916,7 +938,7 @@ local_kernel(const __grid_constant__ Problem p) {
         }
         if (zero != 0.f || zero != zero) {
           for (int i = 0; i < here; ++i)
-            to[(size_t)i * p.dim] = plain_entry(p, record_at(p, u) + kRecordEnd, u.first, u.len, u.head, column + i, entry);
+            to[(size_t)i * p.dim] = plain_entry(p, reinterpret_cast<const float2*>(record_at(p, u) + kRecordEnd), u.first, u.len, u.head, column + i, entry);
         }
       }
       __syncwarp();
@@ -941,8 +963,8 @@ local_kernel(const __grid_constant__ Problem p) {
           products<KP, 3>([&](int i, int j, bool first) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_bf16(tmem + 128 * buffer + 64 * h, a + (uint64_t)(i * NB * (kRowsBlock / 16) + 128 * k), b + (uint64_t)(j * (kRowsBlock / 16) + 128 * k),
-                        umma_idesc(kChunk, width, true) | 1u << 15, !first || k != 0);        // (bit 15: A transposed as well)
+              umma_bf16(tmem + 256 * buffer + 128 * h + 64 * (k >> 1), a + (uint64_t)(i * NB * (kRowsBlock / 16) + 128 * k), b + (uint64_t)(j * (kRowsBlock / 16) + 128 * k),
+                        umma_idesc(kChunk, width, true) | 1u << 15, !first || k % 2 != 0);        // (bit 15: A transposed as well)
           });
         umma_commit(&values_free[buffer]);
         umma_commit(&result_full[buffer]);
@@ -954,7 +976,7 @@ local_kernel(const __grid_constant__ Problem p) {
   __syncthreads();
   if (warp == kFirstIssuer) {
     tmem_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
 }
 
