@@ -8,7 +8,9 @@ are compiled in parallel and a progress line is printed every few seconds, becau
 first build takes the better part of a minute.
 
 The sources include no framework headers: they export plain C functions over raw device
-pointers, so the build needs nvcc and a host compiler and nothing else.
+pointers, so the build needs nvcc and a host compiler and nothing else.  The calls of them
+(``csrc/calls.cpp``, a module for this interpreter) are built beside the library where the
+interpreter's headers are there; elsewhere ctypes makes them.
 """
 
 from __future__ import annotations
@@ -18,11 +20,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
+from typing import Optional
 
 PACKAGE_DIR = Path(__file__).resolve().parent.parent
 SOURCE_DIR = PACKAGE_DIR / "csrc"
@@ -33,6 +37,8 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
 ]
+CALLS_NAME = "miniserve_b200_calls"
+CALLS_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
 
 
 class KernelBuildError(RuntimeError):
@@ -179,3 +185,35 @@ def library_path(verbose: bool = True) -> Path:
     if verbose:
         _say(f"built {library} in {time.time() - started:.0f} s")
     return library
+
+
+def calls_path() -> Optional[Path]:
+    """Path of an up-to-date module of the calls (``csrc/calls.cpp``), building it first if needed; None where it cannot be built."""
+    source = SOURCE_DIR / "calls.cpp"
+    table = "".join(f'{{"{name}", call<{", ".join([result, *arguments])}>}},\n' for name, (result, arguments) in sorted(exported_signatures().items())
+                    if result in ("int", "longlong"))
+    digest = hashlib.sha256("\n".join((table, source.read_text(), sys.version, *CALLS_FLAGS)).encode()).hexdigest()
+    build_dir = _build_dir()
+    module = build_dir / f"{CALLS_NAME}_{digest[:16]}.so"
+    if module.is_file():
+        return module
+    include = sysconfig.get_paths()["include"]
+    compiler = shutil.which("g++") or shutil.which("c++")
+    if compiler is None or not (Path(include) / "Python.h").is_file():
+        return None
+    work = Path(tempfile.mkdtemp(prefix=f"calls_{os.getpid()}_", dir=build_dir))
+    try:
+        (work / "trampolines.inc").write_text(table)
+        built = work / "calls.so"
+        result = subprocess.run([compiler, *CALLS_FLAGS, "-I", include, f'-DTRAMPOLINES="{work / "trampolines.inc"}"', str(source), "-o", str(built)],
+                                capture_output=True, text=True)
+        if result.returncode != 0:
+            _say(f"the calls' module is not built (ctypes makes the calls): {result.stderr[-2000:]}")
+            return None
+        for old in build_dir.glob(f"{CALLS_NAME}_*.so"):
+            if old != module:
+                old.unlink(missing_ok=True)
+        os.replace(built, module)
+    finally:
+        shutil.rmtree(work, ignore_errors=True)
+    return module
