@@ -704,7 +704,9 @@ read_kernel(const __grid_constant__ Problem p) {
           multiply_start(width);
         }
       }
-      if (n > 0) waits.wait(&parts_free, (n - 1) & 1, 72);
+      // (Once a head, not once a unit: within a head the two warps that issue the MMAs need nothing of the other six, and could take the barrier
+      // two phases on while one of those has not looked at it yet.  From head to head they need every warp's parts.)
+      if (u.new_head && heads > 0) waits.wait(&parts_free, (heads - 1) & 1, 72);
       if (u.new_head) {
         const float skip = p.skip != nullptr ? p.skip[u.head] : 0.f;
         const float2* factor = factors + (heads & 1) * 192 + (quarter == 2 ? 32 : quarter == 3 ? 96 : 0);
@@ -789,7 +791,7 @@ read_kernel(const __grid_constant__ Problem p) {
                                !first || k != 0);
           });
           umma_commit(&result_full[h]);
-          umma_commit(&parts_free);
+          if (u.tile + 1 == run.tiles && at + 1 < run.last) umma_commit(&parts_free);        // (and somebody waits for it)
         }
         __syncwarp();
       }
