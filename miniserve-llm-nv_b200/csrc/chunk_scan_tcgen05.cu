@@ -8,7 +8,7 @@
 // bit are summed, smallest first; what comes in bfloat16 already (queries, keys and values straight from a projection) is one part, and its
 // products with three parts are three.  An addition in tensor memory drops the bits behind its last instead of rounding, so a sum
 // lives there for 64 numbers only (16 or 32 where it is a score, whose error a row's values share, or a state's) and sums of those are added in
-// float32 registers; what such sums lose on average is in the decays (gates_kernel).  Relative errors against 64 bits, the float32 pipe's and these:
+// float32 registers; what such sums drop on average is in the decays (gates_kernel).  Relative errors against 64 bits, the float32 pipe's and these:
 // memory form, 128 x 256, bfloat16, y 1.04e-7 and 0.74e-7, states 0.74e-7 and 0.46e-7; all positive 0.67e-7 and 0.41e-7; selective, 64 x 128, 1.66e-7 and 0.95e-7, 0.79e-7 and 0.74e-7.
 //
 // In the read kernel the scores pass from tensor memory through registers, where they get their decays, back to tensor memory as the parts of the
@@ -44,13 +44,25 @@ __device__ __forceinline__ float2 pair_of(double v) {
   return make_float2(hi, is_finite(hi) ? (float)(v - (double)hi) : 0.f);
 }
 
-// What the sums in tensor memory lose on average, relative to the result, since their additions drop bits: of a row by way of its scores, of one by way of
-// S_0, of a chunk's own matrix.  The decays are made larger by as much, which leaves the losses' spread.  Measured on operands of either sign and
-// on positive ones, 8 heads' worth of each: rows of exact scores 6.3e-8 and 8.2e-8 (key entries in one block 5.1e-8, 6.1e-8), of scores of
-// three parts 8.3e-8 and 9.5e-8 (7.6e-8, 8.5e-8); S_0 of 64 entries and more 5.9e-8 and 7.8e-8, of 32 4.0e-8 and 4.5e-8; matrices 3.8e-8, 4.7e-8.
-__device__ __forceinline__ double rows_loss(const Problem& p) { return p.qk_dtype == MS_BF16 ? (p.dim > 64 ? 7.2e-8 : 5.6e-8) : p.dim > 64 ? 8.9e-8 : 8.0e-8; }
-__device__ __forceinline__ double start_loss(const Problem& p) { return 1.7e-8 + 1.25e-8 * min(4, (p.dim + 15) / 16); }
-constexpr double kMatrixLoss = 4.2e-8;
+// An addition in tensor memory drops the bits behind its last, towards zero: half a unit of the last place on average, 4.3e-8 of a result.  Half a unit
+// added to what is summed makes of dropping bits the rounding of them, so a decay that a summed number is multiplied with is larger by a `share` of
+// itself.  How much: 4.3e-8 for the last step of a row's sums, as much again for a score's own sum of 16 key entries (half of that where products of
+// bfloat16 numbers meet, which have 16 bits: their sums drop less), a quarter to a half more where such a sum takes two steps; S_0's sums of up to four
+// steps find a part of the sum at each.  Measured, on operands of either sign and on positive ones: rows of exact scores 6.3e-8 and 8.2e-8 (key entries in
+// one block 5.1e-8, 6.1e-8), of scores of three parts 8.3e-8 and 9.5e-8 (7.6e-8, 8.5e-8); S_0 of 64 entries and more 5.9e-8 and 7.8e-8, of 32 4.0e-8
+// and 4.5e-8; matrices 3.8e-8, 4.7e-8.  The shares are the means of the two.
+//
+// A decay of at most eight bits (one, powers of two) gets none: products with it may be exact, and small whole numbers' sums are.  Other rows with
+// such decays keep what their sums drop.  A score that is exact (bfloat16 queries and keys of a few entries, whole numbers) under another decay gets
+// up to 4e-8 too much: its own sum has dropped nothing.  Those are the two ends: rows of positive numbers are off by 0.5e-7 with the shares, 1.1e-7 without.
+// What is summed outside of tensor memory (plain_row, plain_entry) takes the share off again.
+__device__ __forceinline__ double rows_share(const Problem& p) { return p.qk_dtype == MS_BF16 ? (p.dim > 64 ? 7.2e-8 : 5.6e-8) : p.dim > 64 ? 8.9e-8 : 8.0e-8; }
+__device__ __forceinline__ double start_share(const Problem& p) { return 1.7e-8 + 1.25e-8 * min(4, (p.dim + 15) / 16); }
+constexpr double kMatrixShare = 4.2e-8;
+__device__ __forceinline__ bool few_bits(float v) { return (__float_as_uint(v) & 0xffffu) == 0u; }
+__device__ __forceinline__ double with_share(double v, double share) { return few_bits((float)v) ? v : v * (1.0 + share); }
+// (of a factor out of a record, in float32: a factor with its share has few bits only by chance)
+__device__ __forceinline__ float without_share(float v, double share) { return few_bits(v) ? v : (float)((double)v * (1.0 - share)); }
 
 template <int FORM>
 __global__ void __launch_bounds__(kChunk)
@@ -67,7 +79,7 @@ gates_kernel(const __grid_constant__ Problem p) {
     gate = gate_of<FORM>(p, w.first + t, head);
     if (FORM == kDelta) gate.y = 1.f;        // (what reads take for w v is u)
   }
-  const double g = gate.x, weight = gate.y, scaled = weight * (double)p.q_scale * (1.0 + rows_loss(p));
+  const double g = gate.x, weight = gate.y, scaled = weight * (double)p.q_scale, share = rows_share(p);
   double upto = g, behind = g;               // products of the block's decays up to and with t, from t on
 #pragma unroll
   for (int d = 1; d < 32; d *= 2) {
@@ -86,19 +98,19 @@ gates_kernel(const __grid_constant__ Problem p) {
   double product = behind;                   // from behind t to the start of block b
 #pragma unroll
   for (int b = 1; b < 4; ++b) {
-    reinterpret_cast<float2*>(record + kRecordF)[(b - 1) * kChunk + t] = block < b ? pair_of(product * scaled) : make_float2(0.f, 0.f);
+    reinterpret_cast<float2*>(record + kRecordF)[(b - 1) * kChunk + t] = block < b ? pair_of(with_share(product * scaled, share)) : make_float2(0.f, 0.f);
     if (block < b) product *= blocks[b];
   }
-  reinterpret_cast<float2*>(record + kRecordEnd)[t] = t < w.len ? pair_of(product * weight * (1.0 + kMatrixLoss)) : make_float2(0.f, 0.f);
+  reinterpret_cast<float2*>(record + kRecordEnd)[t] = t < w.len ? pair_of(with_share(product * weight, kMatrixShare)) : make_float2(0.f, 0.f);
   double from_start = upto;
   for (int b = 0; b < block; ++b) from_start *= blocks[b];
-  record[kRecordG + t] = (float)(from_start * (double)p.q_scale * (1.0 + start_loss(p)));
+  record[kRecordG + t] = (float)with_share(from_start * (double)p.q_scale, start_share(p));
   if (t == kChunk - 1) record[kRecordAll] = (float)from_start;
   double d = 1.0;
   for (int j = 31; j >= 0; --j) {            // D(t, block's token j), t's own block
     const double next = __shfl_sync(0xffffffffu, g, (j + 1) & 31), w_j = __shfl_sync(0xffffffffu, scaled, j);
     if (j < lane) d *= next;
-    record[kRecordDiag + (block * 32 + j) * 32 + lane] = j <= lane ? (float)(d * w_j) : 0.f;
+    record[kRecordDiag + (block * 32 + j) * 32 + lane] = j <= lane ? (float)with_share(d * w_j, share) : 0.f;
   }
 }
 
@@ -362,15 +374,15 @@ __device__ __noinline__ void plain_row(const Problem& p, size_t place, int first
     float sum = 0.f;
     for (int n = 0; n < p.dim; ++n)
       sum = fmaf(number_at(p, p.q, p.qk_dtype, first + t, kv_head * p.dim + n), start[(size_t)(column + c) * p.dim + n], sum);
-    sum *= record[kRecordG + t];
+    sum *= without_share(record[kRecordG + t], start_share(p));
     for (int s = 0; s <= t; ++s) {
       float dot = 0.f;
       for (int n = 0; n < p.dim; ++n)
         dot = fmaf(number_at(p, p.q, p.qk_dtype, first + t, kv_head * p.dim + n),
                    number_at(p, p.k, p.qk_dtype, first + s, kv_head * p.dim + n), dot);
       float score;
-      if ((s >> 5) < (t >> 5)) score = dot * (a.x * record[kRecordF + 2 * (((t >> 5) - 1) * kChunk + s)]);
-      else score = dot * record[kRecordDiag + s * 32 + (t & 31)];
+      if ((s >> 5) < (t >> 5)) score = dot * (a.x * without_share(record[kRecordF + 2 * (((t >> 5) - 1) * kChunk + s)], rows_share(p)));
+      else score = dot * without_share(record[kRecordDiag + s * 32 + (t & 31)], rows_share(p));
       if (s == t && p.skip != nullptr) score += p.skip[head];
       sum = fmaf(score, value_at(p, first + s, head, column + c), sum);
     }
@@ -381,7 +393,7 @@ __device__ __noinline__ void plain_row(const Problem& p, size_t place, int first
 __device__ __noinline__ float plain_entry(const Problem& p, const float2* weights, int first, int len, int head, int column, int entry) {
   float sum = 0.f;
   for (int s = 0; s < len; ++s)
-    sum = fmaf(weights[s].x * value_at(p, first + s, head, column), number_at(p, p.k, p.qk_dtype, first + s, head / (p.heads / p.kv_heads) * p.dim + entry), sum);
+    sum = fmaf(without_share(weights[s].x, kMatrixShare) * value_at(p, first + s, head, column), number_at(p, p.k, p.qk_dtype, first + s, head / (p.heads / p.kv_heads) * p.dim + entry), sum);
   return sum;
 }
 

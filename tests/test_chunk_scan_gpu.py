@@ -64,7 +64,7 @@ def problem(form, dtype, lengths, heads, kv_heads, dim, vdim, seed):
     return rows, (q_col, k_col, v_col), gates, slots, states, kv_heads, columns
 
 
-def run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, vdim, **options):
+def run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, vdim, scale=0.7, **options):
     from miniserve_b200 import kernels
 
     n = rows.shape[0]
@@ -74,7 +74,7 @@ def run(form, rows, cols, gates, slots, states, lengths, heads, kv_heads, dim, v
     for length in lengths:
         starts.append(starts[-1] + length)
     kernels.matrix_scan(form, rows, cols[0], rows, cols[1], rows, cols[2], gates, states, 5, slots.to(torch.int32), ints(starts), max(lengths),
-                        heads, kv_heads, dim, vdim, y, q_scale=0.7, bottom=bottom, **options)
+                        heads, kv_heads, dim, vdim, y, q_scale=scale, bottom=bottom, **options)
     return y, bottom
 
 

@@ -60,6 +60,59 @@ def test_runs_of_units(form, dtype, heads, kv_heads, dim, vdim):
     assert all(float((a.double() - b.double()).abs().max()) <= 4e-5 * scale for a, b in pairs)
 
 
+def distances(form, dtype, dim, vdim, length, kind, heads=4):
+    """2-norm of the difference from float64 over that of the result: y (and the memory form's divisors), states.  Operands of either sign, positive
+    ones, or small whole numbers whose decays are one."""
+    rows, cols, gates, slots, states, kv_heads, columns = scans.problem(form, dtype, [length], heads, heads, dim, vdim, 31 + dim + length)
+    if kind == "positive":
+        rows, states = rows.abs(), states.abs()
+    scale = 0.7
+    if kind == "whole":
+        rows, states, gates, scale = (rows.float() * 4).round().clamp(-2, 2).to(dtype), (states * 6).round(), torch.ones_like(gates), 1.0
+    start = states[slots[0], 5:5 + heads * columns * dim].double().view(heads, columns, dim)
+    y, bottom = scans.run(form, rows, cols, gates, slots, states, [length], heads, heads, dim, vdim, scale=scale)
+    here = rows.double()
+    q, k, v = (here[:, at:at + heads * size].view(length, heads, size) for at, size in zip(cols, (dim, dim, vdim)))
+    keep = gates.double().expand(length, heads) if form == "decay" else gates.double()[:, :, 0]
+    write = torch.ones_like(keep) if form == "decay" else gates.double()[:, :, 1]
+    want, after = scans.recurrence(form, scale * q, k, v, keep, write, start)
+
+    def off(found, exact):
+        return float((found.double() - exact).norm() / exact.norm())
+
+    found = [off(y, want[:, :, :vdim]), off(states[slots[0], 5:5 + heads * columns * dim], after.flatten())]
+    if form == "memory":
+        found[0] = max(found[0], off(bottom, torch.maximum(want[:, :, vdim].abs(), gates.double()[:, :, 2]) + 1e-6))
+    return found
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("kind,y_bound,state_bound", [("either sign", 0.9e-7, 0.65e-7), ("positive", 0.7e-7, 0.55e-7)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["memory", "decay"])
+@pytest.mark.parametrize("dim,vdim", [(16, 64), (33, 40), (64, 128), (72, 96), (128, 256)])
+@pytest.mark.parametrize("length", [33, 128, 300])
+def test_distance_from_64_bits(form, dtype, dim, vdim, length, kind, y_bound, state_bound):
+    """What is rounded once is off by 0.29 units of the last place (root mean square), 2.5e-8 of the number: a state is the sum of four such sums, which
+    are smaller than it, and is rounded with each of them (a constant decay's powers are rounded alike in all of a head's numbers, which adds as
+    much once more: 0.59e-7 with 64 columns); a row's scores are off by as much again, and its numbers by more where they have either sign.  What the
+    sums in tensor memory drop, half a unit at each of several steps, would come on top of that (positive numbers without the decays' shares:
+    y 0.86e-7 to 1.3e-7, states 0.59e-7 to 0.72e-7)."""
+    y, state = distances(form, dtype, dim, vdim, length, kind)
+    assert y <= y_bound and state <= state_bound
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("form", ["memory", "decay"])
+@pytest.mark.parametrize("dim,vdim", [(6, 17), (64, 128), (128, 64)])
+@pytest.mark.parametrize("length", [33, 300])
+def test_small_whole_numbers_stay_exact(form, dtype, dim, vdim, length):
+    """Decays and weights of one, sums below 2^24.  (The divisors have 1e-6 added to them: a rounding, 2^-24 of the number at most.)"""
+    y, state = distances(form, dtype, dim, vdim, length, "whole")
+    assert y <= (2.0 ** -24 if form == "memory" else 0.0) and state == 0.0
+
+
 @pytest.mark.usefixtures("on_tensor_cores")
 @pytest.mark.parametrize("form", ["memory", "delta", "decay"])
 def test_an_infinity_reaches_no_token_before_it(form):
