@@ -364,37 +364,111 @@ __device__ __forceinline__ void store_result(const Problem& p, size_t token, int
   if (column < p.vdim) p.y[token * p.vdim + column] = v;
   else p.bottom[token] = keep && v != v ? v : fmaxf(fabsf(v), p.gates[token * 3 + 2]) + 1e-6f;
 }
-// Row t of a chunk, `count` value columns from `column` on, by plain multiply-adds and to memory: see the top of this file.
-__device__ __noinline__ void plain_row(const Problem& p, size_t place, int first, int head, int t, int column, int count) {
-  const float* record = p.records + (place * p.heads + head) * (size_t)kRecord;
-  const float* start = p.chunk_states + (place * p.heads + head) * (size_t)p.columns * p.dim;
-  const int kv_head = head / (p.heads / p.kv_heads);
-  const float2 a = reinterpret_cast<const float2*>(record + kRecordA)[t];
-  for (int c = 0; c < count; ++c) {
-    float sum = 0.f;
-    for (int n = 0; n < p.dim; ++n)
-      sum = fmaf(number_at(p, p.q, p.qk_dtype, first + t, kv_head * p.dim + n), start[(size_t)(column + c) * p.dim + n], sum);
-    sum *= without_share(record[kRecordG + t], start_share(p));
-    for (int s = 0; s <= t; ++s) {
-      float dot = 0.f;
-      for (int n = 0; n < p.dim; ++n)
-        dot = fmaf(number_at(p, p.q, p.qk_dtype, first + t, kv_head * p.dim + n),
-                   number_at(p, p.k, p.qk_dtype, first + s, kv_head * p.dim + n), dot);
-      float score;
-      if ((s >> 5) < (t >> 5)) score = dot * (a.x * without_share(record[kRecordF + 2 * (((t >> 5) - 1) * kChunk + s)], rows_share(p)));
-      else score = dot * without_share(record[kRecordDiag + s * 32 + (t & 31)], rows_share(p));
-      if (s == t && p.skip != nullptr) score += p.skip[head];
-      sum = fmaf(score, value_at(p, first + s, head, column + c), sum);
+// Whether anything holds for a thread of the operand warps (a barrier of theirs).
+__device__ __forceinline__ bool any_fetcher(bool what) {
+  unsigned any;
+  asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, 6, %2, p; selp.u32 %0, 1, 0, q; }"
+               : "=r"(any) : "r"((unsigned)what), "n"(kFetchers) : "memory");
+  return any != 0;
+}
+// Rows of a unit by plain multiply-adds and to memory: see the top of this file.  Of row t, columns 32 h to 32 h + 31 of the tile if bit t of
+// rows[h] is set.  All operand warps take part, with the keys, S_0 and 32 rows' queries and scores at a time in shared memory (`room`).  A prompt of 2,048 tokens with a NaN
+// among its first keys, 8 heads of 128 x 256, whose every later row is summed again: 1.3 ms (0.12 without it); a thread for each row and half a tile, 189 ms.
+template <int NB> struct PlainRoom {
+  static constexpr int LD = 64 * NB + 1, KEYS = 0, START = KEYS + kChunk * LD, QUERIES = START + kTile * LD, SCORES = QUERIES + 32 * LD;
+  static constexpr int FLOATS = SCORES + 32 * (kChunk + 1);
+};
+template <int NB>
+__device__ __noinline__ void plain_rows(const Problem& p, const Unit u, const unsigned (&rows)[2][4], float* room) {
+  using R = PlainRoom<NB>;
+  float *ks = room + R::KEYS, *start = room + R::START, *qs = room + R::QUERIES, *scores = room + R::SCORES;
+  const int tid = threadIdx.x, columns = columns_at(p, u), kv = u.head / (p.heads / p.kv_heads) * p.dim;
+  const float* record = record_at(p, u);
+  const double share = rows_share(p);
+#pragma unroll 8
+  for (int i = tid; i < u.len * p.dim; i += kFetchers) ks[i / p.dim * R::LD + i % p.dim] = number_at(p, p.k, p.qk_dtype, u.first + i / p.dim, kv + i % p.dim);
+#pragma unroll 8
+  for (int i = tid; i < columns * p.dim; i += kFetchers) start[i / p.dim * R::LD + i % p.dim] = start_at(p, u)[i];
+#pragma unroll 1
+  for (int block = 0; block < 4; ++block) {
+    const unsigned mine = rows[0][block] | rows[1][block];
+    const int t0 = 32 * block;
+    if (mine == 0u) continue;
+    any_fetcher(false);                      // (the block before has been read)
+#pragma unroll 8
+    for (int i = tid; i < min(32, u.len - t0) * p.dim; i += kFetchers)
+      qs[i / p.dim * R::LD + i % p.dim] = number_at(p, p.q, p.qk_dtype, u.first + t0 + i / p.dim, kv + i % p.dim);
+    any_fetcher(false);
+    {
+      const int r = tid >> 3, t = t0 + r;
+      if (mine >> r & 1u) {
+        const float2 a = reinterpret_cast<const float2*>(record + kRecordA)[t];
+        for (int s0 = tid & 7; s0 <= t; s0 += 32) {              // (four at a time)
+          float dot[4] = {0.f, 0.f, 0.f, 0.f};
+          for (int n = 0; n < p.dim; ++n) {
+            const float query = qs[r * R::LD + n];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dot[j] = fmaf(query, ks[min(s0 + 8 * j, t) * R::LD + n], dot[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int s = s0 + 8 * j;
+            if (s > t) continue;
+            float score = s < t0 ? dot[j] * (a.x * without_share(record[kRecordF + 2 * ((block - 1) * kChunk + s)], share))
+                                 : dot[j] * without_share(record[kRecordDiag + s * 32 + r], share);
+            if (s == t && p.skip != nullptr) score += p.skip[u.head];
+            scores[r * (kChunk + 1) + s] = score;
+          }
+        }
+      }
     }
-    store_result(p, (size_t)(first + t) * p.heads + head, column + c, sum, false);
+    any_fetcher(false);
+    const int c = tid & 63, r0 = 8 * (tid >> 6), column = u.tile * kTile + c;
+    if (c < columns) {
+      float sum[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) sum[r] = 0.f;
+      for (int n = 0; n < p.dim; ++n) {
+        const float from = start[c * R::LD + n];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) sum[r] = fmaf(qs[(r0 + r) * R::LD + n], from, sum[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) sum[r] *= without_share(record[kRecordG + t0 + r0 + r], start_share(p));
+      const int last = min(t0 + r0 + 8, u.len);
+      for (int s0 = 0; s0 < last; s0 += 8) {
+        float value[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) value[j] = value_at(p, u.first + min(s0 + j, last - 1), u.head, column);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+            if (s0 + j <= t0 + r0 + r) sum[r] = fmaf(scores[(r0 + r) * (kChunk + 1) + s0 + j], value[j], sum[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (rows[c >> 5][block] >> (r0 + r) & 1u) store_result(p, (size_t)(u.first + t0 + r0 + r) * p.heads + u.head, column, sum[r], false);
+    }
   }
 }
-// The same for a number of a chunk's own matrix.
-__device__ __noinline__ float plain_entry(const Problem& p, const float2* weights, int first, int len, int head, int column, int entry) {
-  float sum = 0.f;
-  for (int s = 0; s < len; ++s)
-    sum = fmaf(without_share(weights[s].x, kMatrixShare) * value_at(p, first + s, head, column), number_at(p, p.k, p.qk_dtype, first + s, head / (p.heads / p.kv_heads) * p.dim + entry), sum);
-  return sum;
+// A warp's numbers of a chunk's own matrix (an entry a lane, `here` columns from `column` on) by plain multiply-adds, where `to` has one that is not finite.
+__device__ __noinline__ void plain_entries(const Problem& p, const Unit u, int column, int here, int entry, float* to) {
+  const float2* weights = reinterpret_cast<const float2*>(record_at(p, u) + kRecordEnd);
+  const int lane = threadIdx.x & 31, kv = u.head / (p.heads / p.kv_heads) * p.dim;
+  float sum[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < u.len; ++s) {
+    const float key = entry < p.dim ? number_at(p, p.k, p.qk_dtype, u.first + s, kv + entry) : 0.f;
+    const float value = lane < here ? without_share(weights[s].x, kMatrixShare) * value_at(p, u.first + s, u.head, column + lane) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) sum[i] = fmaf(__shfl_sync(0xffffffffu, value, i), key, sum[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (entry < p.dim && i < here && !is_finite(to[(size_t)i * p.dim])) to[(size_t)i * p.dim] = sum[i];
 }
 
 // ------------------------------------------------------------------------------------------------------- the rows of y
@@ -421,6 +495,9 @@ struct ReadLayout {
   static constexpr size_t BYTES = 1024 + QUERIES + SECOND + FACTORS + ROOM;
 };
 constexpr unsigned kScores = 0, kParts = 128, kResult = 320;
+static_assert(PlainRoom<1>::FLOATS * 4 <= ReadLayout<1, 1, 1>::QUERIES + ReadLayout<1, 1, 1>::SECOND &&
+                  PlainRoom<2>::FLOATS * 4 <= ReadLayout<1, 1, 2>::QUERIES + ReadLayout<1, 1, 2>::SECOND,
+              "rows that are summed again have no room");
 
 template <int QP, int VP, int NB>
 __global__ void __launch_bounds__(kReadThreads, 1)
@@ -431,6 +508,7 @@ read_kernel(const __grid_constant__ Problem p) {
   unsigned char *k_s = q_s + L::QUERIES, *slots = k_s;
   float2* factors = reinterpret_cast<float2*>(q_s + L::QUERIES + L::SECOND);         // [2][192]: 32, 64 and 96 tokens' for the blocks 1, 2, 3
   __shared__ uint64_t keys_full, scores_full, scores_read, slot_full[2], result_full[2], parts_full, parts_free;
+  __shared__ unsigned again[2][4];           // rows that are summed again
   __shared__ int endless[4];                 // first token whose value is not finite, of the last units
   __shared__ unsigned tmem_base_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -635,18 +713,19 @@ read_kernel(const __grid_constant__ Problem p) {
       before = u, u = next;
     }
     cp_async_wait<0>();
-    if (__any_sync(0xffffffffu, !finite)) {  // the rows with a result that is not finite, again
-      __syncwarp();
-      u = first_unit(p, run);
-      for (int at = run.unit; at < run.last; ++at, next_unit(p, run, u)) {
-        const int column = u.tile * kTile + 32 * half, here = min(32, p.columns - column);
+    if (any_fetcher(!finite)) {              // the rows with a result that is not finite, again (shared memory is free by now)
+      Unit one = first_unit(p, run);
+      for (int at = run.unit; at < run.last; ++at, next_unit(p, run, one)) {
+        const int column = one.tile * kTile + 32 * half, here = min(32, p.columns - column);
         bool bad = false;
-        for (int i = 0; i < here && t < u.len; ++i) {
-          const size_t token = (size_t)(u.first + t) * p.heads + u.head;
+        for (int i = 0; i < here && t < one.len; ++i) {
+          const size_t token = (size_t)(one.first + t) * p.heads + one.head;
           bad = bad || !is_finite(column + i < p.vdim ? p.y[token * p.vdim + column + i] : p.bottom[token]);
         }
-        if (bad) plain_row(p, u.place, u.first, u.head, t, column, here);
-        __syncwarp();
+        const unsigned mask = __ballot_sync(0xffffffffu, bad);
+        if (lane == 0) again[half][quarter] = mask;
+        if (any_fetcher(mask != 0u)) plain_rows<NB>(p, one, again, reinterpret_cast<float*>(q_s));
+        any_fetcher(false);                  // (read, all of it)
       }
     }
   } else {
@@ -938,10 +1017,10 @@ local_kernel(const __grid_constant__ Problem p) {
       if (lane == 0) mbar_arrive(&result_empty[buffer]);
       const int column = u.tile * kTile + 32 * half;
       float* to = p.chunk_states + ((u.place * p.heads + u.head) * (size_t)p.columns + column) * p.dim + entry;
+      const int here = min(32, p.columns - column);
+      float zero = 0.f;                      // a sum of zeros unless one of them is not finite
       if (entry < p.dim) {
-        const int here = min(32, p.columns - column);
         float* at_column = to;
-        float zero = 0.f;                    // a sum of zeros unless one of them is not finite
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           if (i < here) {
@@ -950,11 +1029,8 @@ local_kernel(const __grid_constant__ Problem p) {
           }
           at_column += p.dim;
         }
-        if (zero != 0.f || zero != zero) {
-          for (int i = 0; i < here; ++i)
-            to[(size_t)i * p.dim] = plain_entry(p, reinterpret_cast<const float2*>(record_at(p, u) + kRecordEnd), u.first, u.len, u.head, column + i, entry);
-        }
       }
+      if (__any_sync(0xffffffffu, zero != zero)) plain_entries(p, u, column, here, entry, to);
       __syncwarp();
     }
   } else {

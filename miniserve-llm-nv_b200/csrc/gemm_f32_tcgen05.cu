@@ -70,12 +70,6 @@ __device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mi
 }
 
 __device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
-__device__ __noinline__ float plain_sum(const float* a, const float* w, int count) {
-  float sum = 0.f;
-  for (int k = 0; k < count; ++k) sum = fmaf(a[k], w[k], sum);
-  return sum;
-}
-
 __device__ __forceinline__ void tmem_load_8_nowait(unsigned taddr, float (&v)[8]) {
   unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -91,6 +85,51 @@ __device__ __forceinline__ float4 load_shared_of(unsigned cluster_address) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_address) : "memory");
   return v;
+}
+
+// What a block has stored in its rows of W and the columns c_first <= c < c_last of its tile and is not finite, by plain multiply-adds in ascending k.  All of
+// its threads take part, with slices of 32 k in shared memory: 389 rows of NaNs, 2,048 x 6,144, take 1.8 ms (0.10 without); a thread for each such sum 32 ms.
+constexpr int kAgain = 8, kAgainGroups = kThreads / kRows;       // columns a thread, threads a row of W
+__device__ __noinline__ void plain_sums(const Args& p, float* room, int n0, int m0, int c_first, int c_last) {
+  float *ws = room, *as = room + kRows * 36;                     // [128][36], [40][32]
+  const int n = threadIdx.x % kRows, group = threadIdx.x / kRows;
+#pragma unroll 1
+  for (int c0 = c_first; c0 < c_last; c0 += kAgain * kAgainGroups) {
+    const int mine = c0 + group * kAgain;
+    unsigned bad = 0;
+#pragma unroll
+    for (int e = 0; e < kAgain; ++e)
+      if (mine + e < c_last && m0 + mine + e < p.M && n0 + n < p.N && !is_finite(p.C[(size_t)(m0 + mine + e) * p.ldc + n0 + n])) bad |= 1u << e;
+    if (!__syncthreads_or(bad != 0u)) continue;
+    const bool any = __any_sync(0xffffffffu, bad != 0u);
+    float sum[kAgain];
+#pragma unroll
+    for (int e = 0; e < kAgain; ++e) sum[e] = 0.f;
+#pragma unroll 1
+    for (int k0 = 0; k0 < p.K; k0 += 32) {
+      for (int i = threadIdx.x; i < (kRows + kAgain * kAgainGroups) * 8; i += kThreads) {
+        const int row = i / 8, k = i % 8 * 4, c = c0 + row - kRows;
+        const bool of_w = row < kRows, there = k0 + k < p.K && (of_w ? n0 + row < p.N : c < c_last && m0 + c < p.M);
+        const float* from = of_w ? p.W + (size_t)(n0 + row) * p.ldw : p.A + (size_t)(m0 + c) * p.lda;
+        const float4 v = there ? *reinterpret_cast<const float4*>(from + k0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(of_w ? ws + row * 36 + k : as + (row - kRows) * 32 + k) = v;
+      }
+      __syncthreads();
+      const int here = any ? min(32, p.K - k0) : 0;
+      for (int k = 0; k < here; k += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + n * 36 + k);
+#pragma unroll
+        for (int e = 0; e < kAgain; ++e) {
+          const float4 a = *reinterpret_cast<const float4*>(as + (group * kAgain + e) * 32 + k);
+          sum[e] = fmaf(a.w, w.w, fmaf(a.z, w.z, fmaf(a.y, w.y, fmaf(a.x, w.x, sum[e]))));
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int e = 0; e < kAgain; ++e)
+      if (bad >> e & 1u) p.C[(size_t)(m0 + mine + e) * p.ldc + n0 + n] = sum[e];
+  }
 }
 
 // [3][rows][ld] bfloat16 parts of rows of A, four numbers a thread.  Bound by memory: ten bytes a number.
@@ -111,7 +150,7 @@ cut_rows_kernel(const float* __restrict__ A, int lda, int rows, int K, int ld, u
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const Args p) {
+gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Args p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ uint64_t full[kMaxPieces], empty[kMaxPieces], rows_full[kMaxPieces], rows_empty[kMaxPieces], cut_full[2], cut_empty[2], sum_full[2], sum_empty[2];
@@ -154,6 +193,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   grid_dependency_launch();
 
   float acc[kUnits][8];                      // of the summing warps
+  bool finite = true;                        // what this thread has stored
   if (warp < 8) {
     // ---------------- rows of W into tensor memory: half a stage a warp
     const int half = warp >> 2;
@@ -227,7 +267,6 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     const int n_in = (warp & 3) * 32 + lane;
     if (splits == 1) {
       if (ok && n0 + n_in < p.N) {
-        bool finite = true;
         float* out = p.C + (size_t)m0 * p.ldc + n0 + n_in;
 #pragma unroll
         for (int u = 0; u < kUnits; ++u) {
@@ -238,10 +277,6 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
               out[(size_t)(c0 + e) * p.ldc] = acc[u][e];
               finite = finite && is_finite(acc[u][e]);
             }
-        }
-        if (!finite) {                         // (its own stores, read back)
-          for (int c = half * 8; c < tn && m0 + c < p.M; c += c % 8 == 7 ? 9 : 1)
-            if (!is_finite(out[(size_t)c * p.ldc])) out[(size_t)c * p.ldc] = plain_sum(p.A + (size_t)(m0 + c) * p.lda, p.W + (size_t)(n0 + n_in) * p.ldw, p.K);
         }
       }
     } else {
@@ -324,12 +359,15 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   }
 
   tmem_fence_before();
-  __syncthreads();
+  const bool again = __syncthreads_or(!finite);
   if (warp == 17) {
     tmem_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(columns) : "memory");
   }
-  if (splits == 1) return;
+  if (splits == 1) {
+    if (again) plain_sums(p, reinterpret_cast<float*>(smem), n0, m0, 0, tn);
+    return;
+  }
   cluster_sync_all();                        // every rank's sums are there
   const int c_first = tn * rank / splits, c_last = tn * (rank + 1) / splits;
   const bool wide = (p.ldc & 3) == 0 && (reinterpret_cast<size_t>(p.C) & 15) == 0;
@@ -343,8 +381,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       v[0] += part.x, v[1] += part.y, v[2] += part.z, v[3] += part.w;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (n0 + n + e < p.N && !is_finite(v[e])) v[e] = plain_sum(p.A + (size_t)(m0 + c) * p.lda, p.W + (size_t)(n0 + n + e) * p.ldw, p.K);
+    for (int e = 0; e < 4; ++e) finite = finite && (n0 + n + e >= p.N || is_finite(v[e]));
     float* out = p.C + (size_t)(m0 + c) * p.ldc + n0 + n;
     if (wide && n0 + n + 4 <= p.N) {
       *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
@@ -355,6 +392,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     }
   }
   cluster_sync_all();                        // nobody reads this block's sums any more
+  if (__syncthreads_or(!finite)) plain_sums(p, reinterpret_cast<float*>(smem), n0, m0, c_first, c_last);
 }
 
 // Rows of 32 numbers a box: float32 ones 128 bytes wide, parts 64, either with the swizzle of that width.

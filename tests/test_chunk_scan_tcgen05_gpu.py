@@ -155,3 +155,25 @@ def test_which_scans_run_there(monkeypatch):
     monkeypatch.setattr(kernels, "_scanned_on_tensor_cores", lambda *args: True)
     rows, cols, gates, slots, states, kv_heads, columns = scans.problem("memory", torch.bfloat16, [300], 1, 1, 8, 8, 3)
     scans.run("memory", rows, cols, gates, slots, states, [300], 1, kv_heads, 8, 8)
+
+
+@pytest.mark.usefixtures("on_tensor_cores")
+@pytest.mark.parametrize("form,dtype", [("memory", torch.bfloat16), ("delta", torch.float32)])
+def test_a_token_that_is_not_finite_costs_no_orders_of_magnitude(form, dtype):
+    """A NaN in an early token's keys is in every later row and state: all of them are summed again, by whole blocks.  (Measured: 11 times the time without
+    it; by a thread for each row and half a tile, 1,600 times.)"""
+    lengths = [1000]
+    rows, cols, gates, slots, states, kv_heads, columns = scans.problem(form, dtype, lengths, 8, 8, 128, 256, 17)
+    times = []
+    for value in (0.0, float("nan")):
+        rows[3, cols[1]:cols[2]] = value
+        for _ in range(3):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            kept = states.clone()
+            start.record()
+            y, _ = scans.run(form, rows, cols, gates, slots, kept, lengths, 8, kv_heads, 128, 256)
+            end.record()
+            end.synchronize()
+        times.append(start.elapsed_time(end))
+    assert torch.isfinite(y[:3]).all() and not torch.isfinite(y[3:]).any()
+    assert times[1] <= 30 * times[0]
