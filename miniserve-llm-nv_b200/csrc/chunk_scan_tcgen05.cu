@@ -4,8 +4,8 @@
 //   join_long_kernel  what each chunk starts from, and the request's new state
 //   read_kernel    y
 //
-// Float32 operands are cut into three bfloat16 parts that add up to them exactly, and the six products of parts that reach a float32's last
-// bit are summed, smallest first; what comes in bfloat16 already (queries, keys and values straight from a projection) is one part, and its
+// Float32 operands are cut into three bfloat16 parts that add up to them exactly (from 2^-110 on; the parts of smaller ones end at 2^-133), and the six
+// products of parts that reach a float32's last bit are summed, smallest first; what comes in bfloat16 already (queries, keys and values straight from a projection) is one part, and its
 // products with three parts are three.  An addition in tensor memory drops the bits behind its last instead of rounding, so a sum
 // lives there for 64 numbers only (16 or 32 where it is a score, whose error a row's values share, or a state's) and sums of those are added in
 // float32 registers; what such sums drop on average is in the decays (gates_kernel).  Relative errors against 64 bits, the float32 pipe's and these:

@@ -1,6 +1,7 @@
 // The float32 product C[M, N] = A[M, K] * W[N, K]^T on the fifth-generation tensor cores, as exact as the one on the CUDA cores: every
 // operand is cut into three bfloat16 parts that add up to it exactly (x = hi + mid + lo: 24 bits in three times eight), and of the nine
-// products of parts the six that reach a float32's last bit are summed (the other three are at most 2^-26 of a product each).
+// products of parts the six that reach a float32's last bit are summed (the other three are at most 2^-26 of a product each).  Numbers below
+// 2^-110 are more than their parts, which end at 2^-133; see `as_it_is` for what comes of that.
 //
 // What the tensor cores do not do is round: an addition to an accumulator in tensor memory drops the bits behind its last, always
 // towards zero, and over a sum of 2,048 that leaves five times the error of float32 additions (2.1e-6 against 4e-7, measured).  So a
@@ -23,8 +24,8 @@
 //   warp 19        fetches the parts of A into a second ring.  A kernel before this one cuts A: every block would cut its rows again, which
 //                  took as long as the MMAs.
 //
-// A sum that is not finite (an operand was not, or one of the products above has left the range that float32 has) is formed again by
-// plain multiply-adds, so that infinities and NaNs are those of the plain product.
+// A sum that is not finite (an operand was not, or one of the products above has left the range that float32 has) or is very small is formed again by
+// plain multiply-adds, so that infinities and NaNs are those of the plain product, and small operands count whole.
 //
 // Bound by the MMAs' operands: a stage of 144 rows takes 2,245 clocks, its 24 MMAs 1,730 when nothing else reads shared memory (16 rows:
 // 1,800, an MMA of any width takes 65).  One row / 389 rows (us; the plain kernels in brackets): 12,288 x 2,048 44 / 110 (49 / 513), 2,048 x
@@ -69,7 +70,13 @@ __device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mi
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
 }
 
-__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// Whether a sum is taken as it is: finite, and zero or at least 2^-100.  What operands below 2^-110 lack in their parts is 2^-134 of the other operand at
+// most, 2^-25 of such a sum while a row's magnitudes add up to less than 2^9.  Smaller sums are formed again (rows of 1e-36 times
+// rows of ordinary numbers came out with 14 bits).
+__device__ __forceinline__ bool as_it_is(float v) {
+  const unsigned twice = __float_as_uint(v) << 1;          // (without the sign)
+  return twice == 0u || (twice >= 27u << 24 && twice < 255u << 24);
+}
 __device__ __forceinline__ void tmem_load_8_nowait(unsigned taddr, float (&v)[8]) {
   unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -87,7 +94,7 @@ __device__ __forceinline__ float4 load_shared_of(unsigned cluster_address) {
   return v;
 }
 
-// What a block has stored in its rows of W and the columns c_first <= c < c_last of its tile and is not finite, by plain multiply-adds in ascending k.  All of
+// What a block has stored in its rows of W and the columns c_first <= c < c_last of its tile and cannot stay as it is, by plain multiply-adds in ascending k.  All of
 // its threads take part, with slices of 32 k in shared memory: 389 rows of NaNs, 2,048 x 6,144, take 1.8 ms (0.10 without); a thread for each such sum 32 ms.
 constexpr int kAgain = 8, kAgainGroups = kThreads / kRows;       // columns a thread, threads a row of W
 __device__ __noinline__ void plain_sums(const Args& p, float* room, int n0, int m0, int c_first, int c_last) {
@@ -99,7 +106,7 @@ __device__ __noinline__ void plain_sums(const Args& p, float* room, int n0, int 
     unsigned bad = 0;
 #pragma unroll
     for (int e = 0; e < kAgain; ++e)
-      if (mine + e < c_last && m0 + mine + e < p.M && n0 + n < p.N && !is_finite(p.C[(size_t)(m0 + mine + e) * p.ldc + n0 + n])) bad |= 1u << e;
+      if (mine + e < c_last && m0 + mine + e < p.M && n0 + n < p.N && !as_it_is(p.C[(size_t)(m0 + mine + e) * p.ldc + n0 + n])) bad |= 1u << e;
     if (!__syncthreads_or(bad != 0u)) continue;
     const bool any = __any_sync(0xffffffffu, bad != 0u);
     float sum[kAgain];
@@ -193,7 +200,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   grid_dependency_launch();
 
   float acc[kUnits][8];                      // of the summing warps
-  bool finite = true;                        // what this thread has stored
+  bool fine = true;                          // what this thread has stored
   if (warp < 8) {
     // ---------------- rows of W into tensor memory: half a stage a warp
     const int half = warp >> 2;
@@ -275,7 +282,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
           for (int e = 0; e < 8; ++e)
             if (c0 + e < tn && m0 + c0 + e < p.M) {
               out[(size_t)(c0 + e) * p.ldc] = acc[u][e];
-              finite = finite && is_finite(acc[u][e]);
+              fine = fine && as_it_is(acc[u][e]);
             }
         }
       }
@@ -359,7 +366,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
   }
 
   tmem_fence_before();
-  const bool again = __syncthreads_or(!finite);
+  const bool again = __syncthreads_or(!fine);
   if (warp == 17) {
     tmem_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(columns) : "memory");
@@ -381,7 +388,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
       v[0] += part.x, v[1] += part.y, v[2] += part.z, v[3] += part.w;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) finite = finite && (n0 + n + e >= p.N || is_finite(v[e]));
+    for (int e = 0; e < 4; ++e) fine = fine && (n0 + n + e >= p.N || as_it_is(v[e]));
     float* out = p.C + (size_t)(m0 + c) * p.ldc + n0 + n;
     if (wide && n0 + n + 4 <= p.N) {
       *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
@@ -392,7 +399,7 @@ gemm_f32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     }
   }
   cluster_sync_all();                        // nobody reads this block's sums any more
-  if (__syncthreads_or(!finite)) plain_sums(p, reinterpret_cast<float*>(smem), n0, m0, c_first, c_last);
+  if (__syncthreads_or(!fine)) plain_sums(p, reinterpret_cast<float*>(smem), n0, m0, c_first, c_last);
 }
 
 // Rows of 32 numbers a box: float32 ones 128 bytes wide, parts 64, either with the swizzle of that width.

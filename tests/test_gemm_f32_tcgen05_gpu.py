@@ -59,6 +59,27 @@ def test_numbers_at_the_ends_of_the_range(n):
     kernels.check_device_errors(x.device)
 
 
+@pytest.mark.parametrize("n", [300, 20000])
+@pytest.mark.parametrize("of_x,of_w", [(1e-36, 1.0), (1.0, 1e-36), (1e-18, 1e-18), (3e-34, 0.02)])
+def test_small_numbers(n, of_x, of_w):
+    """Operands whose parts end before they do (below 2^-110) count whole: the distance that float32 sums have, see above.  Rows of ordinary numbers
+    beside them, and zeros, are what they are alone."""
+    from miniserve_b200 import kernels
+
+    x, w = operands(21, n, 1600, 9)
+    ordinary = torch.empty((21, n), device="cuda")
+    kernels.linear(x, w, ordinary)
+    x[5:] *= of_x
+    x[20] = 0.0
+    w[:n - 7] *= of_w
+    out = torch.empty((21, n), device="cuda")
+    kernels.linear(x, w, out)
+    small, want = out[5:20, :n - 7].double(), x[5:20].double() @ w[:n - 7].double().T
+    assert float((small - want).norm() / want.norm()) <= 800 ** 0.5 * 2.0 ** -25
+    assert torch.equal(out[:5, n - 7:], ordinary[:5, n - 7:]) and not out[20].any()
+    kernels.check_device_errors(x.device)
+
+
 def test_numbers_that_are_not_finite_cost_no_orders_of_magnitude():
     """Sums that are not finite are formed again by whole blocks.  (Measured: all of them 17 times the time of none;
     by a thread for each, 310 times.)"""
