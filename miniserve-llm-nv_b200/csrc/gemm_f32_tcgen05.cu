@@ -34,6 +34,8 @@
 //
 // Every wait on an mbarrier is bounded: a wait that does not finish sets the error flag that the host checks, all roles drain and
 // tensor memory is freed on every path.
+#include <algorithm>
+
 #include "tcgen05.cuh"
 
 namespace ms {
@@ -425,19 +427,15 @@ using namespace ms::t5f;
 // 23 against 19, 6,144 x 1,536 27 against 25; with 389 rows all of these are two to four times as fast here.
 MS_EXPORT int ms_gemm_f32_tcgen05_takes(int N, int K) { return K % 4 == 0 && (K >= 1536 || (K >= 1024 && N >= 8192)); }
 
-// Bytes of scratch (on a 16-byte boundary) for the parts of M rows of K.
-MS_EXPORT long long ms_gemm_f32_tcgen05_scratch(int M, int K) { return 6LL * M * ((K + 7) / 8 * 8); }
+// Rows of A that are cut and multiplied at a time.  More are a loop of launches, so that no number of rows is too large and the scratch stays that of
+// these (1.5 times their size).  They fill the processors well: 114 tiles of 144 rows, with 2,048 rows of W 12.3 rounds.
+static int rows_at_a_time(int K) { return (int)std::min(16384LL, ((1LL << 31) - 1) / (K / 4)); }
 
-// C[M, N] = A[M, K] * W[N, K]^T in float32; bases on 16-byte boundaries, rows of a multiple of four numbers apart.
-MS_EXPORT int ms_gemm_f32_tcgen05(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, void* scratch,
-                                  int* error_flag, cudaStream_t stream) {
-  if (M == 0 || N == 0) return 0;
-  MS_REQUIRE(K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && lda >= K && ldw >= K && ldc >= N, "gemm_f32_tcgen05: %d x %d x %d, rows of %d %d %d",
-             M, N, K, lda, ldw, ldc);
-  MS_REQUIRE(((reinterpret_cast<size_t>(A) | reinterpret_cast<size_t>(W) | reinterpret_cast<size_t>(scratch)) & 15) == 0,
-             "gemm_f32_tcgen05: operands must be 16-byte aligned");
-  MS_REQUIRE(error_flag != nullptr && scratch != nullptr, "gemm_f32_tcgen05: an error flag and scratch on the device are required");
-  MS_REQUIRE((long long)M * (K / 4) < (1LL << 31) && M <= (1 << 29), "gemm_f32_tcgen05: %d rows of %d in one launch is too much", M, K);
+// Bytes of scratch (on a 16-byte boundary) for the parts of M rows of K.
+MS_EXPORT long long ms_gemm_f32_tcgen05_scratch(int M, int K) { return 6LL * std::min(M, rows_at_a_time(K)) * (((long long)K + 7) / 8 * 8); }
+
+static int multiply(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, void* scratch, int* error_flag,
+                    cudaStream_t stream) {
   // Clusters of c blocks, a block a multiprocessor, that run at a time (cudaOccupancyMaxActiveClusters): the largest c that lets all tiles of
   // W run at once, with 256 k a block at least.
   constexpr int kActive[8] = {148, 74, 45, 33, 26, 22, 15, 15};
@@ -459,7 +457,6 @@ MS_EXPORT int ms_gemm_f32_tcgen05(const float* A, const float* W, float* C, int 
     if (rows == 16) break;
   }
   const int tiles_m = (M + tn - 1) / tn;
-  MS_REQUIRE(tiles_m <= 65535, "gemm_f32_tcgen05: %d rows in one launch is too many", M);
   // The rings: two and a half stages of A and four pieces of W in the largest tiles.
   constexpr int kShared = 226 * 1024 - 1024;
   const int row_pieces = tn > 128 ? 5 : 6;
@@ -486,5 +483,20 @@ MS_EXPORT int ms_gemm_f32_tcgen05(const float* A, const float* W, float* C, int 
   config.attrs = attributes, config.numAttrs = dependent_launch_enabled() ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&config, gemm_f32_tcgen05_kernel, map_w, map_a, args);
   if (e != cudaSuccess) MS_FAIL("gemm_f32_tcgen05: launch failed: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+// C[M, N] = A[M, K] * W[N, K]^T in float32; bases on 16-byte boundaries, rows of a multiple of four numbers apart.
+MS_EXPORT int ms_gemm_f32_tcgen05(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, void* scratch,
+                                  int* error_flag, cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  MS_REQUIRE(K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && lda >= K && ldw >= K && ldc >= N, "gemm_f32_tcgen05: %d x %d x %d, rows of %d %d %d",
+             M, N, K, lda, ldw, ldc);
+  MS_REQUIRE(((reinterpret_cast<size_t>(A) | reinterpret_cast<size_t>(W) | reinterpret_cast<size_t>(scratch)) & 15) == 0,
+             "gemm_f32_tcgen05: operands must be 16-byte aligned");
+  MS_REQUIRE(error_flag != nullptr && scratch != nullptr, "gemm_f32_tcgen05: an error flag and scratch on the device are required");
+  const int rows = rows_at_a_time(K);
+  for (long long m = 0; m < M; m += rows)
+    if (multiply(A + m * lda, W, C + m * ldc, (int)std::min((long long)rows, M - m), N, K, lda, ldw, ldc, scratch, error_flag, stream)) return 1;
   return 0;
 }

@@ -36,6 +36,27 @@ def test_long_sums(m, n, k):
     kernels.check_device_errors(x.device)
 
 
+@pytest.mark.parametrize("m,n,k", [(16384, 130, 1536), (16385, 130, 1536), (32768 + 37, 5, 1536), ((1 << 33) // 1536 + 1, 1, 1536)])
+def test_many_rows(m, n, k):
+    """More rows than are multiplied at a time, and more numbers than 2^33: a row's bits are those that it has alone."""
+    from miniserve_b200 import kernels
+
+    x, w = torch.zeros((m, k), device="cuda"), operands(1, n, k, 4)[1]
+    looked_at = sorted({0, 1, 16383, m // 2, m - 2, m - 1})
+    x[looked_at] = torch.randn((len(looked_at), k), device="cuda")
+    out, few = torch.full((m, n), float("nan"), device="cuda"), torch.empty((len(looked_at), n), device="cuda")
+    kernels.linear(x, w, out)
+    kernels.linear(x[looked_at].contiguous(), w, few)
+    assert torch.equal(out[looked_at], few) and torch.count_nonzero(out) == torch.count_nonzero(few) and few.any()
+    kernels.check_device_errors(x.device)
+
+
+def test_scratch_is_bounded():
+    from miniserve_b200 import kernels
+
+    assert kernels._asked("ms_gemm_f32_tcgen05_scratch", 1 << 24, 10944) == 6 * 16384 * 10944
+
+
 @pytest.mark.parametrize("n", [300, 20000])
 def test_numbers_at_the_ends_of_the_range(n):
     """Infinities, NaNs, overflowing sums and operands near the largest number give what the plain product gives (one block a tile, and
