@@ -1001,21 +1001,29 @@ MAX_INT = 2 ** 31 - 1
 # From which work on (tokens x heads x key entries x value columns) a scan in chunks runs on the tensor cores, where a block of 128 tokens and 64
 # columns takes the same time whatever there is in it: with operands of three parts each when two value tiles or two blocks of key entries
 # share what a block prepares, with bfloat16 ones always for more than 64 key entries.  The scans alone, float32 pipe / tensor cores
-# in us at 256, 512, 1,000 and 2,048 tokens: memory, 8 heads of 128 x 256: 37 / 27, 43 / 34, 75 / 47, 119 / 65; 16 of 64 x 128: 28 / 25, 31 / 33, 51 / 41,
-# 88 / 66; selective, 64 heads of 128 x 64: 42 / 37, 69 / 58, 114 / 81, 210 / 124; 32 of 128 x 64: 35 / 37, 41 / 37, 65 / 49, 111 / 72; 32 of 64 x 128: 29 / 32, 47 / 47,
-# 74 / 66, 126 / 99; delta, 16 heads of 128 x 128: 57 / 56, 71 / 76, 125 / 118, 234 / 212; 32 of 64 x 64: 41 / 51, 51 / 67, 96 / 120, 188 / 234.  Portions that
+# in us at 256, 512, 1,000 and 2,048 tokens.  bfloat16: memory, 8 heads of 128 x 256: 40 / 29, 47 / 42, 73 / 55, 115 / 73; 1 head 28 / 25 to 43 / 28 (from 1,000
+# tokens on); 64 of 128 x 16: 45 / 35, 72 / 46, 130 / 71, 237 / 121; 16 of 64 x 128: 29 / 28, 32 / 41, 50 / 50, 87 / 74; 32 of 64 x 64 (which wait for TENSOR_SCAN_WORK):
+# 29 / 33, 32 / 42, 55 / 59, 99 / 85.  float32: selective, 64 of 128 x 64: 45 / 46, 61 / 55, 103 / 78, 203 / 127; 32 of 64 x 128: 31 / 40, 43 / 49, 69 / 67, 123 / 106; delta, 16 of
+# 128 x 128: 58 / 56, 76 / 79, 126 / 125, 246 / 230.  More work is asked for where a pipe of float32 is ahead for longer: the delta form with one block of key
+# entries (32 of 64 x 128: 50 / 59, 79 / 89, 149 / 156, 271 / 275) and the memory form, each of whose heads has keys of its own, with one (64 of 64 x 128: 49 / 65, 84 / 98, 145 / 164,
+# 310 / 290) or with a last tile of few columns besides the ones (64 of 128 x 64: 47 / 64, 76 / 93, 149 / 144, 284 / 266).  Portions that
 # fill a chunk badly cost as much as whole ones: their mean is asked for, or one that is half of the step.
 TENSOR_SCAN_WORK, TENSOR_SCAN_EXACT, TENSOR_SCAN_MEAN = 240_000_000, 100_000_000, 96
 
 
-def _scanned_on_tensor_cores(n: int, n_requests: int, longest: int, heads: int, dim: int, vdim: int, as_they_are: bool) -> bool:
+def _scanned_on_tensor_cores(n: int, n_requests: int, longest: int, heads: int, dim: int, vdim: int, as_they_are: bool, form: str = "selective") -> bool:
     """Whether a step that is scanned in chunks is scanned on the tensor cores (``as_they_are``: q, k and v are bfloat16 and nothing is done to
     them, so that each is one exact part)."""
     work = n * heads * dim * vdim
     if as_they_are:
-        large = dim > 64 or work >= TENSOR_SCAN_EXACT
+        large = dim > 64 or work >= (TENSOR_SCAN_EXACT if vdim > 64 else TENSOR_SCAN_WORK)
     else:
-        large = (dim > 64 or vdim > 64) and work >= TENSOR_SCAN_WORK
+        wanted = TENSOR_SCAN_WORK
+        if form == "memory" and vdim >= 64 and (vdim + 1) % 64 < 32:
+            wanted *= 2
+        if form != "selective" and dim <= 64:
+            wanted *= 4
+        large = (dim > 64 or vdim > 64) and work >= wanted
     return large and (2 * longest >= n or n >= TENSOR_SCAN_MEAN * n_requests)
 
 
@@ -1291,7 +1299,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
     scratch = None
     if code <= 2 and chunk is None and not (code == 1 and input_activation != "none"):
         tensor_cores = input_activation == "none" and _scanned_on_tensor_cores(
-            n, n_requests, max_query_len, heads, dim, vdim, code != 1 and q.dtype == torch.bfloat16)
+            n, n_requests, max_query_len, heads, dim, vdim, code != 1 and q.dtype == torch.bfloat16, mode)
         scratch = _chunk_scratch(n, n_requests, max_query_len, heads, dim, columns, y.device, code == 1, CHUNK_SCAN_BESIDE[1], tensor_cores)
     if scratch is not None:
         solved = scratch[2:5] if code == 1 else [None] * 3

@@ -147,6 +147,11 @@ def test_which_scans_run_there(monkeypatch):
     assert taken(256, 1, 256, 8, 128, 256, True) and not taken(512, 1, 512, 16, 64, 128, True) and taken(1000, 1, 1000, 16, 64, 128, True)
     # three parts: two tiles or two blocks, and more work
     assert not taken(256, 1, 256, 64, 128, 64, False) and taken(512, 1, 512, 64, 128, 64, False) and not taken(2048, 1, 2048, 32, 64, 64, False)
+    # one value tile and one block; a memory form's tile of ones, and its own keys; the delta form's single block
+    assert not taken(2048, 1, 2048, 16, 64, 64, True) and taken(2048, 1, 2048, 32, 64, 64, True)
+    assert not taken(512, 1, 512, 64, 128, 64, False, "memory") and taken(2048, 1, 2048, 32, 128, 64, False, "memory")
+    assert taken(512, 1, 512, 64, 96, 96, False, "memory") and not taken(1000, 1, 1000, 64, 64, 128, False, "memory")
+    assert not taken(1000, 1, 1000, 32, 64, 128, False, "delta") and taken(2048, 1, 2048, 64, 64, 128, False, "delta")
     # portions that leave chunks empty
     assert not taken(2048, 30, 200, 8, 128, 256, True) and taken(2048, 20, 200, 8, 128, 256, True) and taken(1100, 65, 1036, 8, 128, 256, True)
     # records that do not fit: the float32 pipe's scratch
