@@ -54,15 +54,19 @@ def library() -> ctypes.CDLL:
 
 
 def _take_calls(lib: ctypes.CDLL) -> None:
-    """Puts the native calls (``csrc/calls.cpp``) in the place of ctypes' for the entry points that return a number.  A call's arguments
-    cost ctypes 0.12 us each; eager passes that the host bounds took 138 us (latent attention, 256 tokens) and 88.6 (gated linear attention,
-    three prompts of about 50) and take 127 and 79.6."""
+    """Puts the native calls (``csrc/calls.cpp``) in the place of ctypes' for the entry points that return a number; where their module is not
+    there or does not load, ctypes makes the calls.  A call's arguments cost ctypes 0.12 us each; eager passes that the host bounds took
+    132 us (latent attention, a prompt of 2,048 tokens) and 87 (gated linear attention, three prompts of about 50), and take 125 and 75."""
     path = build.calls_path()
     if path is None:
         return
     loader = importlib.machinery.ExtensionFileLoader(build.CALLS_NAME, str(path))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(build.CALLS_NAME, loader))
-    loader.exec_module(module)
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader(build.CALLS_NAME, loader))
+        loader.exec_module(module)
+    except (ImportError, OSError) as error:
+        log.warning("the calls' module does not load, ctypes makes the calls: %s", error)
+        return
     for name in build.exported_signatures():
         function = getattr(lib, name)
         entry = module.entry(name, ctypes.cast(function, ctypes.c_void_p).value, function)

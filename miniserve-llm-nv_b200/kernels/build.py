@@ -188,18 +188,23 @@ def library_path(verbose: bool = True) -> Path:
 
 
 def calls_path() -> Optional[Path]:
-    """Path of an up-to-date module of the calls (``csrc/calls.cpp``), building it first if needed; None where it cannot be built."""
+    """Path of an up-to-date module of the calls (``csrc/calls.cpp``), building it first if needed; None where it cannot be built (a
+    compiler that has refused these sources is not asked again)."""
     source = SOURCE_DIR / "calls.cpp"
     table = "".join(f'{{"{name}", call<{", ".join([result, *arguments])}>}},\n' for name, (result, arguments) in sorted(exported_signatures().items())
                     if result in ("int", "longlong"))
-    digest = hashlib.sha256("\n".join((table, source.read_text(), sys.version, *CALLS_FLAGS)).encode()).hexdigest()
+    digest = hashlib.sha256("\n".join((table, source.read_text(), *CALLS_FLAGS)).encode()).hexdigest()
+    abi = sysconfig.get_config_var("SOABI") or sys.implementation.cache_tag          # (every interpreter has a module of its own)
     build_dir = _build_dir()
-    module = build_dir / f"{CALLS_NAME}_{digest[:16]}.so"
+    module = build_dir / f"{CALLS_NAME}_{abi}_{digest[:16]}.so"
+    refused = module.with_suffix(".refused")
     if module.is_file():
         return module
     include = sysconfig.get_paths()["include"]
     compiler = shutil.which("g++") or shutil.which("c++")
     if compiler is None or not (Path(include) / "Python.h").is_file():
+        return None
+    if refused.is_file() and refused.read_text() == compiler:
         return None
     work = Path(tempfile.mkdtemp(prefix=f"calls_{os.getpid()}_", dir=build_dir))
     try:
@@ -209,8 +214,9 @@ def calls_path() -> Optional[Path]:
                                 capture_output=True, text=True)
         if result.returncode != 0:
             _say(f"the calls' module is not built (ctypes makes the calls): {result.stderr[-2000:]}")
+            refused.write_text(compiler)
             return None
-        for old in build_dir.glob(f"{CALLS_NAME}_*.so"):
+        for old in build_dir.glob(f"{CALLS_NAME}_{abi}_*"):
             if old != module:
                 old.unlink(missing_ok=True)
         os.replace(built, module)

@@ -55,3 +55,44 @@ def test_as_ctypes(module, name):
             assert direct(*wrong) == "general"
     entry.restype = ctypes.c_int
     assert entry.restype is ctypes.c_int
+
+
+@pytest.fixture
+def elsewhere(tmp_path, monkeypatch):
+    """A build folder of its own."""
+    monkeypatch.setattr(build, "_build_dir", lambda: tmp_path)
+    return tmp_path
+
+
+def test_a_module_that_does_not_load_leaves_the_calls_to_ctypes(module, elsewhere, monkeypatch):
+    from miniserve_b200 import kernels
+
+    broken = elsewhere / "broken.so"
+    broken.write_bytes(b"not a module")
+    monkeypatch.setattr(build, "calls_path", lambda: broken)
+
+    class Library:
+        def __getattr__(self, name):
+            raise AssertionError("nothing is replaced")
+
+    kernels._take_calls(Library())
+
+
+def test_another_interpreters_module_stays(module, elsewhere):
+    ours = elsewhere / f"{build.CALLS_NAME}_{build.sysconfig.get_config_var('SOABI')}_0123456789abcdef.so"
+    theirs = elsewhere / f"{build.CALLS_NAME}_cpython-399-x86_64-linux-gnu_0123456789abcdef.so"
+    for path in (ours, theirs):
+        path.write_bytes(b"")
+    built = build.calls_path()
+    assert built.is_file() and theirs.is_file() and not ours.is_file()
+
+
+def test_a_compiler_that_refuses_is_asked_once(module, elsewhere, monkeypatch):
+    asked = []
+
+    class Refusal:
+        returncode, stderr = 1, "no"
+
+    monkeypatch.setattr(build.subprocess, "run", lambda command, **_: asked.append(command) or Refusal())
+    assert build.calls_path() is None and build.calls_path() is None and len(asked) == 1
+    assert [path.suffix for path in elsewhere.iterdir()] == [".refused"]
