@@ -34,8 +34,6 @@ constexpr int kTile = 64;                    // value columns of a unit
 constexpr int kFetchers = 256, kThreads = 576, kFirstIssuer = 16, kReadThreads = 512;
 constexpr unsigned kRowsBlock = kChunk * 128, kTileBlock = kTile * 128;        // bytes of 64 bfloat16 columns of 128 rows, of 64
 
-__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
-
 // ------------------------------------------------------------------------------------------------------------- decays
 // grid (heads, chunks), a token a thread.  Products of decays are formed in double precision and rounded once (a pair of floats where they
 // are a factor of one more product): their errors would be the same for a whole row of scores, where the walk's fall on each number of S alone.
@@ -60,7 +58,9 @@ __device__ __forceinline__ double rows_share(const Problem& p) { return p.qk_dty
 __device__ __forceinline__ double start_share(const Problem& p) { return 1.7e-8 + 1.25e-8 * min(4, (p.dim + 15) / 16); }
 constexpr double kMatrixShare = 4.2e-8;
 __device__ __forceinline__ bool few_bits(float v) { return (__float_as_uint(v) & 0xffffu) == 0u; }
-__device__ __forceinline__ double with_share(double v, double share) { return few_bits((float)v) ? v : v * (1.0 + share); }
+__device__ __forceinline__ double with_share(double v, double share) {
+  return (__double2loint(v) | (__double2hiint(v) & 0x1fff)) == 0 ? v : fma(v, share, v);
+}
 // (of a factor out of a record, in float32: a factor with its share has few bits only by chance)
 __device__ __forceinline__ float without_share(float v, double share) { return few_bits(v) ? v : (float)((double)v * (1.0 - share)); }
 
@@ -155,16 +155,6 @@ __device__ __forceinline__ void floats_of(const Raw& r, int dtype, float (&v)[8]
   for (int e = 0; e < 8; ++e)
     v[e] = __uint_as_float(dtype == MS_F32 ? w[e] : e % 2 == 0 ? w[e / 2] << 16 : w[e / 2] & 0xffff0000u);
 }
-// Two numbers' parts, packed; exact: what is left behind two roundings to eight bits has eight bits.  What rounding the numbers themselves
-// left (`more_a`, `more_b`: they are products) goes into the last part, and only that is rounded.
-__device__ __forceinline__ void cut(float a, float b, float more_a, float more_b, unsigned& hi, unsigned& mid, unsigned& lo) {
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-  a -= __uint_as_float(hi << 16), b -= __uint_as_float(hi & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
-  a -= __uint_as_float(mid << 16), b -= __uint_as_float(mid & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b + more_b), "f"(a + more_a));
-}
-__device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) { cut(a, b, 0.f, 0.f, hi, mid, lo); }
 __device__ __forceinline__ void cut_eight(const float (&v)[8], uint4 (&part)[3]) {
   cut(v[0], v[1], part[0].x, part[1].x, part[2].x);
   cut(v[2], v[3], part[0].y, part[1].y, part[2].y);
@@ -328,16 +318,6 @@ __device__ __forceinline__ int values_valid(const Problem& p, const Unit& u, int
   return row < u.len ? p.vdim - u.tile * kTile - 8 * (int)(threadIdx.x & 7) : 0;
 }
 
-__device__ __forceinline__ void tmem_load_16_nowait(unsigned taddr, float (&v)[16]) {
-  unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_store_8(unsigned taddr, const unsigned (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
 template <int ID, int THREADS> __device__ __forceinline__ void named_barrier() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
 __device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 

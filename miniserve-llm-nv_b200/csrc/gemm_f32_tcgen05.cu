@@ -63,15 +63,6 @@ struct Args {
   int* error_flag;
 };
 
-// Two numbers' parts, packed; exact: what is left behind two roundings to eight bits has eight bits.
-__device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-  a -= __uint_as_float(hi << 16), b -= __uint_as_float(hi & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
-  a -= __uint_as_float(mid << 16), b -= __uint_as_float(mid & 0xffff0000u);
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
-}
-
 // Whether a sum is taken as it is: finite, and zero or at least 2^-100.  What operands below 2^-110 lack in their parts is 2^-134 of the other operand at
 // most, 2^-25 of such a sum while a row's magnitudes add up to less than 2^9.  Smaller sums are formed again (rows of 1e-36 times
 // rows of ordinary numbers came out with 14 bits).
@@ -79,12 +70,6 @@ __device__ __forceinline__ bool as_it_is(float v) {
   const unsigned twice = __float_as_uint(v) << 1;          // (without the sign)
   return twice == 0u || (twice >= 27u << 24 && twice < 255u << 24);
 }
-__device__ __forceinline__ void tmem_load_8_nowait(unsigned taddr, float (&v)[8]) {
-  unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
-}
-
 // Descriptor of a K-major tile of 32 k: rows of 64 bytes with the 64-byte swizzle, groups of eight rows 512 bytes apart.
 __device__ __forceinline__ uint64_t rows_desc(const void* smem_tile) {
   return (uint64_t)((smem_u32(smem_tile) & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;

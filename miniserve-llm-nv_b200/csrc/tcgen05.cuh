@@ -26,8 +26,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
       : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return done != 0;
 }
-// Waits for the phase of the given parity; false (and the error flag set) if it does not come.  The loop stays a loop: unrolled, it took a
-// large part of a kernel's instruction cache for turns that are hardly ever taken (quantised attention of a decode step 36.6 us, now 35.7; quantised experts 140.7, 138.4).
+// Waits for the phase of the given parity; false (and the error flag set) if it does not come.  The loop stays a loop: unrolled at a kernel's many
+// waits it takes a large part of the instruction cache (selective scan of 2,048 tokens, 64 heads of 128 x 64: 134 us, as a loop 127; float32 product of
+// 389 x 12,288 x 2,048 within 1 %, attention and experts of a decode step within what runs differ by).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int* error_flag, int code) {
 #pragma unroll 1
   for (unsigned spin = 0; spin < SPIN_LIMIT; ++spin)
@@ -88,6 +89,24 @@ __device__ __forceinline__ void umma_bf16(unsigned tmem_d, uint64_t a_desc, uint
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// Two numbers' parts, packed; exact from 2^-110 on: what is left behind two roundings to eight bits has eight bits.
+__device__ __forceinline__ void cut(float& a, float& b, unsigned& hi, unsigned& mid) {        // (and what is left)
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+  a -= __uint_as_float(hi << 16), b -= __uint_as_float(hi & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(b), "f"(a));
+  a -= __uint_as_float(mid << 16), b -= __uint_as_float(mid & 0xffff0000u);
+}
+__device__ __forceinline__ void cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
+  cut(a, b, hi, mid);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b), "f"(a));
+}
+// Of numbers that are products: what rounding them left (`more_a`, `more_b`) goes into the last part, and only that is rounded.
+__device__ __forceinline__ void cut(float a, float b, float more_a, float more_b, unsigned& hi, unsigned& mid, unsigned& lo) {
+  cut(a, b, hi, mid);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b + more_b), "f"(a + more_a));
+}
+
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -119,6 +138,17 @@ __device__ __forceinline__ void tmem_load_32_nowait(unsigned taddr, float (&v)[3
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_load_16_nowait(unsigned taddr, float (&v)[16]) {
+  unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_load_8_nowait(unsigned taddr, float (&v)[8]) {
+  unsigned* r = reinterpret_cast<unsigned*>(&v[0]);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_store_32(unsigned taddr, const unsigned (&r)[32]) {
@@ -137,6 +167,10 @@ __device__ __forceinline__ void tmem_store_16(unsigned taddr, const unsigned (&r
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_store_8(unsigned taddr, const unsigned (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
