@@ -157,9 +157,28 @@ def test_which_scans_run_there(monkeypatch):
     # records that do not fit: the float32 pipe's scratch
     n = 1_000_000
     assert len(kernels._chunk_scratch(n, 1, n, 8, 65, 9, "meta", tensor_cores=True)) == 2
-    monkeypatch.setattr(kernels, "_scanned_on_tensor_cores", lambda *args: True)
+
+
+def test_records_that_do_not_fit_leave_a_scan_to_the_float32_pipe(monkeypatch):
+    """The scratch of either way is allowed, or of the float32 pipe's alone: which kernels run, and that those give what they give by themselves."""
+    from miniserve_b200 import kernels
+
+    monkeypatch.setattr(kernels, "CHUNK_SCAN_LONGEST", 0)
     rows, cols, gates, slots, states, kv_heads, columns = scans.problem("memory", torch.bfloat16, [300], 1, 1, 8, 8, 3)
-    scans.run("memory", rows, cols, gates, slots, states, [300], 1, kv_heads, 8, 8)
+    library, records, found = kernels.library(), [], []
+    monkeypatch.setattr(library, "ms_chunk_scan", lambda *args, real=library.ms_chunk_scan: records.append(args[-3]) or real(*args))
+    # floats of the pipe: five chunks' matrices and decays; of the tensor cores: three matrices, decays, three records
+    limit = 4 * (5 * 9 * 8 + 5)
+    for wanted, scratch in ((True, kernels.MAX_CHUNK_SCRATCH), (True, limit), (False, limit)):
+        monkeypatch.setattr(kernels, "MAX_CHUNK_SCRATCH", scratch)
+        monkeypatch.setattr(kernels, "_scanned_on_tensor_cores", lambda *args: wanted)
+        kept = states.clone()
+        y, bottom = scans.run("memory", rows, cols, gates, slots, kept, [300], 1, kv_heads, 8, 8)
+        found.append((y, bottom, kept))
+    assert records[0] and not records[1] and not records[2]
+    assert all(torch.equal(a, b) for a, b in zip(found[1], found[2]))
+    assert all(torch.allclose(a, b, rtol=4e-5, atol=4e-5) for a, b in zip(found[0], found[1]))
+    kernels.check_device_errors(torch.device("cuda:0"))
 
 
 @pytest.mark.usefixtures("on_tensor_cores")
