@@ -8,8 +8,13 @@
 // products of parts that reach a float32's last bit are summed, smallest first; what comes in bfloat16 already (queries, keys and values straight from a projection) is one part, and its
 // products with three parts are three.  An addition in tensor memory drops the bits behind its last instead of rounding, so a sum
 // lives there for 64 numbers only (16 or 32 where it is a score, whose error a row's values share, or a state's) and sums of those are added in
-// float32 registers; what such sums drop on average is in the decays (gates_kernel).  Relative errors against 64 bits, the float32 pipe's and these:
-// memory form, 128 x 256, bfloat16, y 1.04e-7 and 0.74e-7, states 0.74e-7 and 0.46e-7; all positive 0.67e-7 and 0.41e-7; selective, 64 x 128, 1.66e-7 and 0.95e-7, 0.79e-7 and 0.74e-7.
+// float32 registers; what such sums drop on average is in the decays (gates_kernel).  Relative errors against 64 bits (2-norm), the float32 pipe's and these,
+// portions of 33 to 2,048 tokens: memory form, 8 heads of 128 x 256, bfloat16, y 1.05e-7 and 0.74e-7, states 0.72e-7 to 0.79e-7 and 0.41e-7 to 0.47e-7; positive operands y
+// 0.68e-7 and 0.49e-7; decays near one y 1.2e-7 to 2.0e-7 and 0.74e-7 to 0.92e-7; selective, 64 channels, states of 128, y 1.6e-7 and 0.9e-7, states 0.7e-7 to 0.8e-7 both.
+//
+// Who comes here: the memory form with bfloat16 or float32 inputs, the selective form and the delta form's read with float32 ones.  The constant decay
+// comes only from a caller that has nothing done to the inputs (the engine's layer asks for SiLU, which the float32 pipe's kernels apply), the
+// delta form's bfloat16 queries with float32 values only from one whose inputs are bfloat16 (the engine's are not).
 //
 // In the read kernel the scores pass from tensor memory through registers, where they get their decays, back to tensor memory as the parts of the
 // next product's operand: they are never in memory.
@@ -462,8 +467,9 @@ __device__ __noinline__ void plain_entries(const Problem& p, const Unit u, int c
 // A slot's next operand is announced only after its last results have been read, so that one barrier says both.  (Every unit takes the
 // same steps whatever its tokens: waits by parity must not be overtaken.)
 //
-// What binds it is the chain between the roles (keys cut, scores into registers and back, results out), not a unit: on 2,048 tokens the MMAs take a
-// fifth of the time and memory a quarter.  The float32 pipe's kernel, which its multiply-adds bound, and this: memory form, 8 heads of 128 x 256 in bfloat16,
+// What binds it is the chain between the roles (keys cut, scores into registers and back, results out), not a unit: on 2,048 tokens the tensor pipe is busy
+// for 11 % of the cycles (memory form) and 22 % (selective), the memory system for 23 to 28 %, and warps wait for loads and for barriers
+// (profiles/scan_tcgen05_ncu.md).  The float32 pipe's kernel, which its multiply-adds bound, and this: memory form, 8 heads of 128 x 256 in bfloat16,
 // 74.1 and 36.9 us; selective, 64 of 128 x 64, 121.5 and 73.3; delta, 16 of 128 x 128, 75.8 and 51.4.
 template <int QP, int VP, int NB>
 struct ReadLayout {

@@ -1254,7 +1254,7 @@ def matrix_scan(mode: str, q: torch.Tensor, q_col: int, k: torch.Tensor, k_col: 
     ``"channel_decay"`` of few long portions runs in chunks that need not wait for one another (a walk from zero per chunk, a join
     of the chunks' matrices, a walk from the joined ones): ``chunk`` None lets the library choose, 0 forbids it, a number is
     the chunk's tokens.  ``"memory"``, ``"delta"`` and ``"decay"`` of portions of many tokens run as matrix products over chunks of 64 or, on the
-    tensor cores, 128 tokens (``csrc/chunk_scan.cu``; CHUNK_SCAN_LONGEST and TENSOR_SCAN_WORK say from when on) unless ``chunk`` is 0, which walks them; other numbers are
+    tensor cores and without an activation on the way in, 128 tokens (``csrc/chunk_scan.cu``; CHUNK_SCAN_LONGEST and TENSOR_SCAN_WORK say from when on) unless ``chunk`` is 0, which walks them; other numbers are
     refused there."""
     code = MATRIX_SCAN_MODES[mode]
     n = y.shape[0]
@@ -1584,7 +1584,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, row_stats: 
 
     float32 operands run through the library's own kernels: FFMA, or for long sums tensor cores
     on three bfloat16 parts of each operand that add up to it exactly (nearer to 64 bits than the FFMA
-    sums; which of the two is a question of N and K alone).  bfloat16 operands go to cuBLAS through ``torch.mm`` with float32 accumulation;
+    sums; which of the two is a question of N, K and of bases on 16-byte boundaries, never of M).  bfloat16 operands go to cuBLAS through ``torch.mm`` with float32 accumulation;
     ``out`` may then be bfloat16 or float32.
     """
     m, k = x.shape
