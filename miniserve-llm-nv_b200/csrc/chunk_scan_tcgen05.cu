@@ -468,8 +468,8 @@ __device__ __noinline__ void plain_entries(const Problem& p, const Unit u, int c
 // same steps whatever its tokens: waits by parity must not be overtaken.)
 //
 // What binds it is the chain between the roles (keys cut, scores into registers and back, results out), not a unit: on 2,048 tokens the tensor pipe is busy
-// for 11 % of the cycles (memory form) and 22 % (selective), the memory system for 23 to 28 %, and warps wait for loads and for barriers
-// (profiles/scan_tcgen05_ncu.md).  The float32 pipe's kernel, which its multiply-adds bound, and this: memory form, 8 heads of 128 x 256 in bfloat16,
+// for 11 % of the cycles (memory form) and 22 % (selective), the memory system for 23 to 28 %, and warps wait for loads and for barriers.
+// The float32 pipe's kernel, which its multiply-adds bound, and this: memory form, 8 heads of 128 x 256 in bfloat16,
 // 74.1 and 36.9 us; selective, 64 of 128 x 64, 121.5 and 73.3; delta, 16 of 128 x 128, 75.8 and 51.4.
 template <int QP, int VP, int NB>
 struct ReadLayout {

@@ -28,7 +28,7 @@
 // plain multiply-adds, so that infinities and NaNs are those of the plain product, and small operands count whole.
 //
 // Bound by the MMAs' operands: a stage of 144 rows takes 2,245 clocks, its 24 MMAs 1,730 when nothing else reads shared memory (16 rows:
-// 1,800, an MMA of any width takes 65); the tensor pipe is busy for 62 % of the cycles at 389 x 12,288 x 2,048 (profiles/scan_tcgen05_ncu.md).  One row / 389 rows (us; the plain kernels in brackets): 12,288 x 2,048 44 / 110 (49 / 513), 2,048 x
+// 1,800, an MMA of any width takes 65); the tensor pipe is busy for 62 % of the cycles at 389 x 12,288 x 2,048.  One row / 389 rows (us; the plain kernels in brackets): 12,288 x 2,048 44 / 110 (49 / 513), 2,048 x
 // 6,144 30 / 93 (51 / 345), 2,048 x 2,048 19 / 54 (23 / 121), 21,888 x 2,560 97 / 257 (106 / 1,093).  Distance from 64 bits (2-norm,
 // normal operands): K = 2,048 1.0e-7 to 1.3e-7 (plain 8.1e-7), K = 6,144 1.2e-7 (1.4e-6), K = 256 0.9e-7 (3e-7).
 //
